@@ -1,71 +1,319 @@
 // True 32-bit matrix product for the verification path: C[M,N] = A[M,K] * W[N,K]^T (+ bias).
 // Plain FFMA on CUDA cores: no tensor-core instruction is issued, so no operand is
-// ever rounded to TF32 or bfloat16.  Every output element accumulates k = 0..K-1 in
-// ascending order in one thread, so a row's result does not depend on how many other
-// rows are in the batch (nn.Linear layout, mini_llm/nn/attention.py:102-111).
+// ever rounded to TF32 or bfloat16 (nn.Linear layout, mini_llm/nn/attention.py:102-111).
+//
+// The order of an output's sum is a function of K alone: k is cut into segments of kSegment and segments into at most
+// eight blocks (block_length).  A segment is accumulated in ascending k by fused multiply-adds from zero, a block is the
+// sum of its segments in ascending order, the output the sum of its blocks in ascending order.  Every kernel below keeps
+// that order, so a row's bits do not depend on how many other rows are in the batch or on which kernel took it.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace b200 {
 
-constexpr int BM = 64, BN = 64, BK = 16;
+namespace cg = cooperative_groups;
 
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K,
-                int lda, int ldc) {
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Ws[BK][BN + 4];
+constexpr int kSegment = 128;
+// Blocks of 1,024, longer ones where K is longer than eight of those: whole segments.
+inline int block_length(int K) {
+  const int eighth = ((K + 7) / 8 + kSegment - 1) / kSegment * kSegment;
+  return eighth > 8 * kSegment ? eighth : 8 * kSegment;
+}
+
+// ------------------------------------------------------------------------------------------ tiles
+// A cluster per BM x BN tile, one CTA for each block of K, (BM / TM) x (BN / TN) threads with TM x TN outputs each (rows
+// ty * 4 + g BM / (TM / 4), columns likewise: every fragment is one 16-byte read that neighbouring threads share or lay
+// side by side).  Two buffers of BK columns in shared memory and two more in registers: rows are asked for two steps ahead (with one, a step of
+// 0.8 us was the latency of its loads).  The
+// sums of finished segments wait in shared memory, one private 16-byte column per thread, so that registers hold one
+// accumulator an output and two or three CTAs fit an SM; at the end the CTAs of a cluster share out the outputs and add the
+// blocks' sums up through distributed shared memory.  Bound by the FMA pipe and the reads of shared memory beside it:
+// 509 x 6144 x 1024 161 us (40 TFLOP/s of the 74 that the pipe could do; 292 us with one 64 x 64 tile kernel and 4-byte
+// accesses), 509 x 1024 x 3072 89 us (189).
+// VEC: rows of A and W start on 16-byte boundaries and K is a multiple of 4; otherwise elements are loaded one by one.
+constexpr int kBK = 16;
+constexpr size_t tile_smem(int bm, int bn) { return sizeof(float) * (static_cast<size_t>(bm) * bn + 2 * kBK * (bm + 4 + bn + 4)); }
+
+template <int BM, int BN, int TM, int TN, bool VEC>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                     float* __restrict__ C, int M, int N, int K, int lda, int ldc, int block) {
+  constexpr int THREADS = (BM / TM) * (BN / TN), BK = kBK, PA = BM + 4, PW = BN + 4;
+  constexpr int RPP = THREADS / 4;                                  // rows a pass of 16-byte loads covers
+  constexpr int LA = BM / RPP, LW = BN / RPP;
+  constexpr int SM_ = BM / (TM / 4), SN_ = BN / (TN / 4);           // distance of a thread's groups of four rows, columns
+  static_assert(TM % 4 == 0 && TN % 4 == 0 && kSegment % BK == 0 && BM % RPP == 0 && BN % RPP == 0, "tile shape");
+  extern __shared__ __align__(16) float smem[];
+  float* As = smem;                                                 // [2][BK][PA]
+  float* Ws = As + 2 * BK * PA;                                     // [2][BK][PW]
+  float4* sums = reinterpret_cast<float4*>(Ws + 2 * BK * PW);       // [TM * TN / 4][THREADS]
+  pdl_trigger();
+  pdl_wait();
+  cg::cluster_group cluster = cg::this_cluster();
+  const int blocks = cluster.num_blocks(), rank = cluster.block_rank();
+  const int tid = threadIdx.x;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x / blocks * BN;
+  const int k_begin = rank * block, k_end = min(K, k_begin + block);
+  const int tx = tid % (BN / TN), ty = tid / (BN / TN);
+  const int lrow = tid >> 2, lk = (tid & 3) * 4;
+  struct Rows { float4 a[LA], w[LW]; };
+
+  auto load4 = [&](const float* base, int row, int rows, int ld, int k) -> float4 {
+    if (row >= rows || k >= k_end) return make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* p = base + static_cast<size_t>(row) * ld + k;
+    if (VEC) return *reinterpret_cast<const float4*>(p);
+    return make_float4(p[0], k + 1 < k_end ? p[1] : 0.f, k + 2 < k_end ? p[2] : 0.f, k + 3 < k_end ? p[3] : 0.f);
+  };
+  auto fetch = [&](Rows& r, int k0) {
+#pragma unroll
+    for (int i = 0; i < LA; ++i) r.a[i] = load4(A, m0 + lrow + RPP * i, M, lda, k0 + lk);
+#pragma unroll
+    for (int i = 0; i < LW; ++i) r.w[i] = load4(W, n0 + lrow + RPP * i, N, K, k0 + lk);
+  };
+  auto stash = [&](const Rows& r, int buf) {
+    float* as = As + (buf * BK + lk) * PA + lrow;
+    float* ws = Ws + (buf * BK + lk) * PW + lrow;
+#pragma unroll
+    for (int i = 0; i < LA; ++i) {
+      as[RPP * i] = r.a[i].x; as[PA + RPP * i] = r.a[i].y; as[2 * PA + RPP * i] = r.a[i].z; as[3 * PA + RPP * i] = r.a[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < LW; ++i) {
+      ws[RPP * i] = r.w[i].x; ws[PW + RPP * i] = r.w[i].y; ws[2 * PW + RPP * i] = r.w[i].z; ws[3 * PW + RPP * i] = r.w[i].w;
+    }
+  };
+
+  // two neighbouring columns share a register pair: one packed instruction does two fused multiply-adds, each
+  // rounded as by itself
+  float2 acc[TM][TN / 2];
+  auto clear = [&]() {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN / 2; ++j) acc[i][j] = make_float2(0.f, 0.f);
+  };
+  clear();
+  // `spent` goes on its way to hold the rows behind the next ones; `next` was asked for a step ago
+  auto step = [&](int k0, int buf, Rows& spent, const Rows& next) {
+    const bool more = k0 + BK < k_end;
+    fetch(spent, k0 + 2 * BK);
+    const float* as = As + buf * BK * PA + ty * 4;
+    const float* ws = Ws + buf * BK * PW + tx * 4;
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      float a[TM];
+      float2 w[TN / 2];
+#pragma unroll
+      for (int i = 0; i < TM; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(as + k * PA + i / 4 * SM_);
+        a[i] = v.x; a[i + 1] = v.y; a[i + 2] = v.z; a[i + 3] = v.w;
+      }
+#pragma unroll
+      for (int j = 0; j < TN; j += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(ws + k * PW + j / 4 * SN_);
+        w[j / 2] = make_float2(v.x, v.y);
+        w[j / 2 + 1] = make_float2(v.z, v.w);
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), w[j], acc[i][j]);
+    }
+    if ((k0 + BK - k_begin) % kSegment == 0 || !more) {             // the segment is complete
+      const bool first = k0 - k_begin < kSegment;
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN / 4; ++j) {
+          float4* s = sums + (i * (TN / 4) + j) * THREADS + tid;
+          const float4 t = first ? make_float4(0.f, 0.f, 0.f, 0.f) : *s;
+          *s = make_float4(t.x + acc[i][2 * j].x, t.y + acc[i][2 * j].y, t.z + acc[i][2 * j + 1].x, t.w + acc[i][2 * j + 1].y);
+        }
+      clear();
+    }
+    if (more) stash(next, buf ^ 1);
+    __syncthreads();
+  };
+  Rows even, odd;
+  fetch(even, k_begin);
+  fetch(odd, k_begin + BK);
+  stash(even, 0);
+  __syncthreads();
+  for (int k0 = k_begin; k0 < k_end; k0 += 2 * BK) {
+    step(k0, 0, even, odd);
+    if (k0 + BK < k_end) step(k0 + BK, 1, odd, even);
+  }
+  if (blocks > 1) cluster.sync();                                   // every block's sums are in its CTA's shared memory
+  const bool wide = VEC && ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
+  for (int q = rank; q < TM * TN / 4; q += blocks) {
+    const int i = q / (TN / 4), j = q % (TN / 4);
+    const int m = m0 + ty * 4 + i / 4 * SM_ + i % 4, n = n0 + tx * 4 + j * SN_;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int b = 0; b < blocks; ++b) {
+      const float4 t = (blocks > 1 ? cluster.map_shared_rank(sums, b) : sums)[q * THREADS + tid];
+      v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+    }
+    if (m >= M || n >= N) continue;
+    float* c = C + static_cast<size_t>(m) * ldc + n;
+    const float out[4] = {v.x, v.y, v.z, v.w};
+    if (bias == nullptr && wide && n + 4 <= N) {
+      *reinterpret_cast<float4*>(c) = v;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (n + e < N) c[e] = out[e] + (bias ? bias[n + e] : 0.f);
+    }
+  }
+  if (blocks > 1) cluster.sync();                                   // nobody leaves while its sums are being read
+}
+
+// ------------------------------------------------------------------------------------------ few rows
+// Up to eight rows of A per CTA beside kRowsW rows of W: the time is that of streaming W.  A thread forms the sums of one
+// segment of one weight row against every row of A (1 x 151,936 x 1024: 93 us = 6.7 TB/s, where tiles took 708); kSegments segments of all the CTA's weight rows are in shared memory
+// at a time, copied there 16 bytes at a time without passing through registers, two or three CTAs an SM so that one's copies
+// run under the other's arithmetic.  Rows are padded by 16 bytes: the eight threads of a 128-byte phase then read from
+// different banks.
+constexpr int kRowsW = 8, kSegments = 16, kPass = kSegments * kSegment;
+constexpr size_t few_smem(int pitch) { return sizeof(float) * kRowsW * pitch; }
+
+template <int MB>
+__global__ void __launch_bounds__(kRowsW * kSegments)
+gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                    float* __restrict__ C, int M, int N, int K, int lda, int ldc, int pitch, int block) {
+  extern __shared__ __align__(16) float ws[];                    // [kRowsW][pitch]
+  __shared__ float sums[kSegments][MB][kRowsW];
   pdl_trigger();
   pdl_wait();
   const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int tx = tid & 15, ty = tid >> 4;  // 16 x 16 threads, each 4 x 4 outputs
-  float acc[4][4] = {};
-  // each thread loads 4 consecutive k of one row for A and for W
-  const int lrow = tid >> 2, lk = (tid & 3) * 4;
-  for (int k0 = 0; k0 < K; k0 += BK) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int k = k0 + lk + i;
-      const int am = m0 + lrow, wn = n0 + lrow;
-      As[lk + i][lrow] = (am < M && k < K) ? A[static_cast<size_t>(am) * lda + k] : 0.f;
-      Ws[lk + i][lrow] = (wn < N && k < K) ? W[static_cast<size_t>(wn) * K + k] : 0.f;
+  const int n0 = blockIdx.x * kRowsW, m0 = blockIdx.y * MB;
+  const int n = tid % kRowsW, seg = tid / kRowsW;
+  const int rows = min(MB, M - m0);
+  const float* a0 = A + static_cast<size_t>(m0) * lda;
+  float total = 0.f, part = 0.f;                                 // of output (tid / kRowsW, tid % kRowsW), for tid < MB * kRowsW
+  for (int k0 = 0; k0 < K; k0 += kPass) {
+    const int span = min(kPass, K - k0), quads = span / 4;       // K is a multiple of 4 here
+    for (int r = tid / 32; r < kRowsW; r += kRowsW * kSegments / 32) {
+      if (n0 + r >= N) continue;                                 // never read: that row's outputs are not stored
+      const float* src = W + static_cast<size_t>(n0 + r) * K + k0;
+      const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(ws + r * pitch));
+      for (int q = tid % 32; q < quads; q += 32)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + q * 16), "l"(src + q * 4) : "memory");
     }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
+    float acc[MB];
 #pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      float a[4], w[4];
+    for (int m = 0; m < MB; ++m) acc[m] = 0.f;
+    const int first = seg * kSegment, last = min(first + kSegment, span);
+    if (n0 + n < N) {
+      const float* wrow = ws + n * pitch;
+#pragma unroll 4
+      for (int k = first; k < last; k += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(wrow + k);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = Ws[k][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+        for (int m = 0; m < MB; ++m) {
+          const float4 a = *reinterpret_cast<const float4*>(a0 + static_cast<size_t>(m < rows ? m : 0) * lda + k0 + k);
+          acc[m] = fmaf(a.x, w.x, acc[m]);
+          acc[m] = fmaf(a.y, w.y, acc[m]);
+          acc[m] = fmaf(a.z, w.z, acc[m]);
+          acc[m] = fmaf(a.w, w.w, acc[m]);
+        }
+      }
     }
+#pragma unroll
+    for (int m = 0; m < MB; ++m) sums[seg][m][n] = acc[m];
     __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n < N) C[static_cast<size_t>(m) * ldc + n] = acc[i][j] + (bias ? bias[n] : 0.f);
+    if (tid < MB * kRowsW) {
+      const int used = (span + kSegment - 1) / kSegment;
+      for (int s = 0; s < used; ++s) {
+        part += sums[s][tid / kRowsW][tid % kRowsW];
+        if ((k0 + (s + 1) * kSegment) % block == 0) {             // the block is complete
+          total += part;
+          part = 0.f;
+        }
+      }
     }
+    __syncthreads();                                             // the sums and the rows have been read
   }
+  if (tid < MB * kRowsW) {
+    const int m = m0 + tid / kRowsW, nn = n0 + tid % kRowsW;
+    if (m < M && nn < N) C[static_cast<size_t>(m) * ldc + nn] = (K % block ? total + part : total) + (bias ? bias[nn] : 0.f);
+  }
+}
+
+template <int BM, int BN, int TM, int TN, bool VEC>
+int launch_tiles(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, cudaStream_t stream) {
+  static DeviceOnce once;
+  const int status = configure_once(once, gemm_f32_tile_kernel<BM, BN, TM, TN, VEC>, tile_smem(BM, BN));
+  if (status) return status;
+  const int block = block_length(K), blocks = (K + block - 1) / block;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3((N + BN - 1) / BN * blocks, (M + BM - 1) / BM);
+  config.blockDim = dim3((BM / TM) * (BN / TN));
+  config.dynamicSmemBytes = tile_smem(BM, BN);
+  config.stream = stream;
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = blocks;
+  attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attributes;
+  config.numAttrs = pdl_enabled() ? 2 : 1;
+  cudaLaunchKernelEx(&config, gemm_f32_tile_kernel<BM, BN, TM, TN, VEC>, A, W, bias, C, M, N, K, lda, ldc, block);
+  return launch_status();
+}
+
+template <int MB>
+int launch_few(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, cudaStream_t stream) {
+  static DeviceOnce once;
+  const int status = configure_once(once, gemm_f32_few_kernel<MB>, few_smem(kPass + 4));
+  if (status) return status;
+  const dim3 grid((N + kRowsW - 1) / kRowsW, (M + MB - 1) / MB);
+  const int pitch = (K < kPass ? K : kPass) + 4;      // a short K takes less shared memory: more CTAs an SM
+  launch(gemm_f32_few_kernel<MB>, grid, dim3(kRowsW * kSegments), few_smem(pitch), stream, A, W, bias, C, M, N, K, lda, ldc, pitch,
+         block_length(K));
+  return launch_status();
 }
 
 }  // namespace b200
 
-extern "C" int b200_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M,
-                             int N, int K, int lda, int ldc, cudaStream_t stream) {
+// `kernel`: 0 chooses by size; 1: few rows, 2: tiles of 64 x 64, 3: tiles of 128 x 64 (for tests and measurements).
+extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,
+                                     int ldc, int kernel, cudaStream_t stream) {
+  using namespace b200;
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || lda < K || ldc < N) return B200_ERR_BAD_SIZE;
-  dim3 grid((N + b200::BN - 1) / b200::BN, (M + b200::BM - 1) / b200::BM);
-  if (grid.y > 65535) return B200_ERR_TOO_LARGE;
-  b200::launch(b200::gemm_f32_kernel, dim3(grid), dim3(256), 0, stream, A, W, bias, C, M, N, K, lda, ldc);
-  return b200::launch_status();
+  const bool vec = K % 4 == 0 && lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(W) % 16 == 0;
+  const int blocks = (K + block_length(K) - 1) / block_length(K);
+  const long long small = static_cast<long long>((M + 63) / 64) * ((N + 63) / 64) * blocks;
+  const long long large = static_cast<long long>((M + 127) / 128) * ((N + 63) / 64) * blocks;
+  if (kernel == 0) {
+    // Up to 8 rows the weights cross once and that is the time (1 x 1024 x 3072: 7.9 us against 37.6 with tiles; 8 x 151,936 x
+    // 1024: 285 against 495).  Every further eight rows read them again, from the L2 while the product is small: 24 x 6144
+    // x 1024 37.5 against 39.0, 24 x 1024 x 3072 25.6 against 37.8, 64 x 6144 x 1024 83 against 40.
+    // Tiles of 128 rows do a third more arithmetic per byte of shared memory read; where they would be fewer than about
+    // 1.7 an SM, tiles of 64 fill the SMs better (509 x 4096 x 1024: 109 us against 116; 509 x 1024 x 3072: 109 against 89).
+    if (vec && (M <= 8 || (M <= 24 && small < 148))) kernel = 1;
+    else kernel = large >= 250 && M > 64 ? 3 : 2;
+  }
+  if ((M + 63) / 64 > 65535) return B200_ERR_TOO_LARGE;
+  if (kernel == 1) {
+    if (!vec) return B200_ERR_BAD_SIZE;
+    if (M == 1) return launch_few<1>(A, W, bias, C, M, N, K, lda, ldc, stream);
+    if (M == 2) return launch_few<2>(A, W, bias, C, M, N, K, lda, ldc, stream);
+    if (M <= 4) return launch_few<4>(A, W, bias, C, M, N, K, lda, ldc, stream);
+    return launch_few<8>(A, W, bias, C, M, N, K, lda, ldc, stream);
+  }
+  if (kernel == 3)
+    return vec ? launch_tiles<128, 64, 8, 8, true>(A, W, bias, C, M, N, K, lda, ldc, stream)
+               : launch_tiles<128, 64, 8, 8, false>(A, W, bias, C, M, N, K, lda, ldc, stream);
+  return vec ? launch_tiles<64, 64, 8, 4, true>(A, W, bias, C, M, N, K, lda, ldc, stream)
+             : launch_tiles<64, 64, 8, 4, false>(A, W, bias, C, M, N, K, lda, ldc, stream);
+}
+
+extern "C" int b200_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M,
+                             int N, int K, int lda, int ldc, cudaStream_t stream) {
+  return b200_gemm_f32_variant(A, W, bias, C, M, N, K, lda, ldc, 0, stream);
 }

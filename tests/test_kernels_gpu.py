@@ -97,6 +97,30 @@ def test_gemm_f32_is_exact_and_batch_invariant(m, n, k):
     assert torch.equal(alone[0], out[m // 2])
 
 
+# edges of the tiles (64, 128 rows; 64 columns), of the weight rows a CTA takes (8), of a segment (128) and of a block (1,024;
+# longer ones from K = 8,192 on), widths that are no multiple of 4
+@pytest.mark.parametrize("m,n,k", [(1, 7, 4), (2, 9, 132), (3, 65, 1024), (8, 64, 1028), (9, 63, 2052), (24, 40, 4100), (25, 130, 128),
+                                   (65, 61, 1152), (129, 200, 96), (300, 129, 2048), (5, 66, 1027), (70, 20, 9000), (4, 24, 17000)])
+def test_gemm_f32_kernels_agree_bit_for_bit(m, n, k):
+    from llm_runtime_study_b200.ops import native
+
+    torch.manual_seed(4)
+    x, w, b = dev(torch.randn(m, k)), dev(torch.randn(n, k)), dev(torch.randn(n))
+    results = [F().linear_f32(x, w, b)]
+    for kernel in (1, 2, 3):
+        if kernel == 1 and k % 4:
+            continue                    # 16-byte rows only
+        out = torch.full((m, n), float("nan"), device=x.device)
+        native.call("b200_gemm_f32_variant", x.data_ptr(), w.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, k, n, kernel, native.stream_ptr())
+        results.append(out)
+    for out in results[1:]:
+        assert torch.equal(out, results[0])
+    want = x.double() @ w.double().T + b.double()
+    # a chain of at most 128 fused multiply-adds and one of at most 64 + 8 sums, each half a unit in the last place (6e-8) of partial
+    # sums whose size is that of the whole sum (sqrt(k)) or less
+    assert float((results[0].double() - want).abs().max()) < 6e-8 * 200 * math.sqrt(k)
+
+
 def _scatter_to_pages(k, v, page_size, nkv, d, dtype, seed=0, extra_pages=3):
     """Put contiguous k, v [T, nkv, d] into shuffled pages; return pools + table row."""
 
