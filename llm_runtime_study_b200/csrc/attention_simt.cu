@@ -16,11 +16,29 @@
 // Values may have a head size `dv` of their own.  Two further rules: a bias by the logarithm of the distance
 // (S <- S - r1_j * ln(1 + r2_j * (p - t)) with two numbers per query head) and a mask in blocks (`chunk` > 0: position p
 // sees t only if floor(p / chunk) = floor(t / chunk), blocks counted from position 0 of the sequence).
+//
+// Two kernels keep that order bit for bit: one warp per token and head (single decoded tokens, and every size), and tiles
+// of query rows that share the keys and values of a prompt portion (float32).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace b200 {
 
-// kMaxChunks x 32 columns of values at most; the key size is bounded by shared memory only
+// What the rules make of a product q . k: every rounding is spelled out, so that the kernels cannot differ in it.
+struct ScoreRules {
+  float scale, softcap, inv_cap, slope, r1, r2;
+  bool log_bias;
+  __device__ __forceinline__ float operator()(float dot, int distance) const {
+    float s = __fmul_rn(dot, scale);
+    if (softcap > 0.f) s = __fmul_rn(softcap, tanhf(__fmul_rn(s, inv_cap)));
+    s = __fmaf_rn(-slope, static_cast<float>(distance), s);
+    if (log_bias) s = __fmaf_rn(-r1, log1pf(__fmul_rn(r2, static_cast<float>(distance))), s);
+    return s;
+  }
+};
+
+// One warp per token and head.  kMaxChunks x 32 columns of values at most; the key size is bounded by shared memory only
 template <typename T, int kMaxChunks>
 __global__ void __launch_bounds__(128)
 paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_pool,
@@ -51,9 +69,8 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_poo
   // the sink is a key of score 0 (or sinks[head]) and value 0 that every row sees: it starts the running maximum and sum
   float m = sink ? 0.f : -INFINITY, l = sink || sinks != nullptr ? 1.f : 0.f;
   if (sinks != nullptr) m = sinks[head];
-  const float slope = slopes ? slopes[head] : 0.f;
-  const float inv_cap = softcap > 0.f ? 1.f / softcap : 0.f;
-  const float r1 = log_r1 ? log_r1[head] : 0.f, r2 = log_r2 ? log_r2[head] : 0.f;
+  const ScoreRules rules{scale, softcap, softcap > 0.f ? 1.f / softcap : 0.f, slopes ? slopes[head] : 0.f,
+                         log_r1 ? log_r1[head] : 0.f, log_r2 ? log_r2[head] : 0.f, log_r1 != nullptr};
   float acc[kMaxChunks];
 #pragma unroll
   for (int c = 0; c < kMaxChunks; ++c) acc[c] = 0.f;
@@ -69,6 +86,7 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_poo
       const T* krow = k_pool + ((static_cast<size_t>(page) * nkv + kvh) * page_size + t % page_size) * d;
       float dot = 0.f;
       if (d % VN == 0) {         // rows of keys then start on 16-byte boundaries
+#pragma unroll 8
         for (int i = 0; i < d; i += VN) {
           float f[VN];
           Vec<T>::unpack(*reinterpret_cast<const typename Vec<T>::type*>(krow + i), f);
@@ -78,30 +96,39 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_poo
       } else {
         for (int i = 0; i < d; ++i) dot = fmaf(qs[i], to_float(krow[i]), dot);
       }
-      s = dot * scale;
-      if (softcap > 0.f) s = softcap * tanhf(s * inv_cap);
-      s -= slope * static_cast<float>(p - t);
-      if (log_r1 != nullptr) s -= r1 * log1pf(r2 * static_cast<float>(p - t));
+      s = rules(dot, p - t);
     }
     const float m_tile = warp_max(s);
     if (m_tile == -INFINITY) continue;
     const float m_new = fmaxf(m, m_tile);
     const float corr = expf(m - m_new);  // m = -inf -> 0
     const float pl = valid ? expf(s - m_new) : 0.f;
-    l = l * corr + warp_sum(pl);
+    l = __fmaf_rn(l, corr, warp_sum(pl));
 #pragma unroll
     for (int c = 0; c < kMaxChunks; ++c) acc[c] *= corr;
     const int count = min(32, p - t0 + 1);
-    for (int j = 0; j < count; ++j) {
-      const float pj = __shfl_sync(0xffffffffu, pl, j);
-      if (pj == 0.f) continue;
-      const int tj = t0 + j;
-      const int page = table[tj / page_size];
-      const T* vrow = v_pool + ((static_cast<size_t>(page) * nkv + kvh) * page_size + tj % page_size) * v_row;
+    // the values of kAhead keys are asked for before the first is used (each lane holds its own key's page)
+    constexpr int kAhead = kMaxChunks <= 4 ? 8 : (kMaxChunks <= 8 ? 4 : 2);
+    for (int j0 = 0; j0 < count; j0 += kAhead) {
+      float pj[kAhead], vj[kAhead][kMaxChunks];
 #pragma unroll
-      for (int c = 0; c < kMaxChunks; ++c) {
-        const int i = lane + 32 * c;
-        if (i < dv) acc[c] = fmaf(pj, to_float(vrow[i]), acc[c]);
+      for (int e = 0; e < kAhead; ++e) {
+        pj[e] = __shfl_sync(0xffffffffu, pl, (j0 + e) & 31);
+        const int pg = __shfl_sync(0xffffffffu, page, (j0 + e) & 31);
+        if (j0 + e >= count) pj[e] = 0.f;
+        if (pj[e] == 0.f) continue;          // masked, or too small to count: its value is not read
+        const T* vrow = v_pool + ((static_cast<size_t>(pg) * nkv + kvh) * page_size + (t0 + j0 + e) % page_size) * v_row;
+#pragma unroll
+        for (int c = 0; c < kMaxChunks; ++c) {
+          const int i = lane + 32 * c;
+          vj[e][c] = i < dv ? to_float(vrow[i]) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < kAhead; ++e) {
+        if (pj[e] == 0.f) continue;
+#pragma unroll
+        for (int c = 0; c < kMaxChunks; ++c) acc[c] = fmaf(pj[e], vj[e][c], acc[c]);
       }
     }
     m = m_new;
@@ -113,6 +140,235 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_poo
     const int i = lane + 32 * c;
     if (i < dv) orow[i] = from_float<T>(acc[c] * inv);
   }
+}
+
+// Prompt portions in float32: a CTA holds 32 rows (32 / group consecutive tokens of one request times the query heads
+// that share a key head) and walks the keys in the tiles of 32 that the kernel above takes them in; keys and values pass
+// through shared memory once for all rows, the next tile's on their way while this one is worked on.  A thread owns four
+// rows and, of a tile, the keys c and c + 16: the sum of its two weights and four shuffles are then the sum that 32 lanes
+// form by xor shuffles, and every other sum is one chain, so the results are the same bits.  A weight of zero reads no
+// value here either (a later token's value may be anything): only a warp that has one takes the loop that asks.
+// One warp per token and head reads every key for every row from the L2: 509 tokens, 16 heads of 128 over 8: 574 us; so: 133
+// (64 rows a CTA 161: fewer CTAs, one an SM).  Bound by the reads of shared memory beside the FMA pipe.
+constexpr int kTileRows = 32, kTileKeys = 32, kTileThreads = kTileRows * 4, kPPitch = kTileKeys + 4;
+constexpr size_t attention_tile_smem(int dmax) {
+  return sizeof(float) * (static_cast<size_t>(kTileRows + 2 * kTileKeys) * (dmax + 4) + kTileRows * kPPitch);
+}
+
+struct TileParams {
+  const float* q; const float* k_pool; const float* v_pool; float* out;
+  const int* positions; const int* q_start; const int* block_table;
+  int entries, table_stride, page_size, nq, nkv, d, dv, per_tile, window, chunk, sink;
+  float scale, softcap;
+  const float* slopes; const float* log_r1; const float* log_r2; const float* sinks;
+};
+
+template <int DMAX>
+__global__ void __launch_bounds__(kTileThreads) paged_attention_tile_kernel(const TileParams p) {
+  constexpr int PITCH = DMAX + 4, CG = DMAX > 64 ? 2 : 1;   // CG: groups of four value columns a thread owns
+  extern __shared__ __align__(16) float smem[];
+  float* qs = smem;                                     // [32][PITCH]
+  float* ks = qs + kTileRows * PITCH;                   // [32][PITCH]
+  float* vs = ks + kTileKeys * PITCH;                   // [32][PITCH]
+  float* ps = vs + kTileKeys * PITCH;                   // [32][kPPitch]
+  pdl_trigger();
+  pdl_wait();
+  // the tile's request: every request has its own tiles, the last one (with most keys) first
+  int entry = 0, tile = blockIdx.x, first = 0, tokens = 0;
+  for (;; ++entry) {
+    if (entry == p.entries) return;
+    first = p.q_start[entry];
+    tokens = p.q_start[entry + 1] - first;
+    const int tiles = (tokens + p.per_tile - 1) / p.per_tile;
+    if (tile < tiles) {
+      tile = tiles - 1 - tile;
+      break;
+    }
+    tile -= tiles;
+  }
+  first += tile * p.per_tile;
+  tokens = min(p.per_tile, tokens - tile * p.per_tile);
+  const int tid = threadIdx.x, c = tid % 16, rg = tid / 16;
+  const int group = p.nq / p.nkv, kvh = blockIdx.y;
+  const int* table = p.block_table + static_cast<size_t>(entry) * p.table_stride;
+  const int d = p.d, dv = p.dv, quads = d / 4, vquads = dv / 4;
+
+  for (int idx = tid; idx < kTileRows * quads; idx += kTileThreads) {
+    const int row = idx / quads, i = idx % quads * 4, t = row / group;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < tokens) v = *reinterpret_cast<const float4*>(p.q + (static_cast<size_t>(first + t) * p.nq + kvh * group + row % group) * d + i);
+    *reinterpret_cast<float4*>(qs + row * PITCH + i) = v;
+  }
+  const float inv_cap = p.softcap > 0.f ? 1.f / p.softcap : 0.f;
+  float slope[4], r1[4], r2[4];
+  int pos[4], w0[4];
+  float m[4], l[4];
+  float2 acc[4][2 * CG];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int row = rg * 4 + r, t = row / group, head = kvh * group + row % group;
+    pos[r] = t < tokens ? p.positions[first + t] : -1;   // -1: no such row; it sees no key
+    w0[r] = p.window > 0 ? max(0, pos[r] - p.window + 1) : 0;
+    if (p.chunk > 0) w0[r] = max(w0[r], pos[r] / p.chunk * p.chunk);
+    slope[r] = p.slopes ? p.slopes[head] : 0.f;
+    r1[r] = p.log_r1 ? p.log_r1[head] : 0.f;
+    r2[r] = p.log_r2 ? p.log_r2[head] : 0.f;
+    m[r] = p.sinks ? p.sinks[head] : (p.sink ? 0.f : -INFINITY);
+    l[r] = p.sink || p.sinks ? 1.f : 0.f;
+#pragma unroll
+    for (int j = 0; j < 2 * CG; ++j) acc[r][j] = make_float2(0.f, 0.f);
+  }
+  const int p_first = p.positions[first], p_last = p.positions[first + tokens - 1];    // positions ascend within a request
+  int lowest = p.window > 0 ? max(0, p_first - p.window + 1) : 0;
+  if (p.chunk > 0) lowest = max(lowest, p_first / p.chunk * p.chunk);
+
+  // Four threads copy a row of a tile, 16 bytes at a time, zeros where there is no page; the row's page is looked up a
+  // tile ahead of its keys and serves its values too.
+  const int crow = tid / (kTileThreads / kTileKeys), cquad = tid % (kTileThreads / kTileKeys);
+  auto page_of = [&](int t) { return t <= p_last ? table[t / p.page_size] : -1; };
+  auto ask = [&](const float* pool, float* to, int page, int t, int width, int nquads) {
+    const float* src = pool + ((static_cast<size_t>(max(page, 0)) * p.nkv + kvh) * p.page_size + t % p.page_size) * width;
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(to + crow * PITCH));
+    const int bytes = page >= 0 ? 16 : 0;
+    for (int i = cquad; i < nquads; i += kTileThreads / kTileKeys)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst + i * 16), "l"(src + i * 4), "r"(bytes) : "memory");
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+
+  int t0 = lowest / kTileKeys * kTileKeys;
+  int page = page_of(t0 + crow), next_page = page_of(t0 + kTileKeys + crow);
+  ask(p.k_pool, ks, page, t0 + crow, d, quads);
+  ask(p.v_pool, vs, page, t0 + crow, dv, vquads);
+  for (; t0 <= p_last; t0 += kTileKeys) {
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");            // the keys; the values may still be on their way
+    __syncthreads();
+    const int ahead_page = page_of(t0 + 2 * kTileKeys + crow);
+    int key_page[2];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) key_page[n] = page_of(t0 + c + 16 * n);
+    float s[4][2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) s[r][0] = s[r][1] = 0.f;
+    const float* qrow = qs + rg * 4 * PITCH;
+    const float* krow = ks + c * PITCH;
+#pragma unroll 4
+    for (int i = 0; i < d; i += 4) {
+      float4 qv[4], kv[2];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) qv[r] = *reinterpret_cast<const float4*>(qrow + r * PITCH + i);
+#pragma unroll
+      for (int n = 0; n < 2; ++n) kv[n] = *reinterpret_cast<const float4*>(krow + n * 16 * PITCH + i);
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          s[r][n] = fmaf(qv[r].x, kv[n].x, s[r][n]);
+          s[r][n] = fmaf(qv[r].y, kv[n].y, s[r][n]);
+          s[r][n] = fmaf(qv[r].z, kv[n].z, s[r][n]);
+          s[r][n] = fmaf(qv[r].w, kv[n].w, s[r][n]);
+        }
+    }
+    bool full = true;                                                 // no weight of this thread's is zero
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const ScoreRules rules{p.scale, p.softcap, inv_cap, slope[r], r1[r], r2[r], p.log_r1 != nullptr};
+      bool valid[2];
+      float top = -INFINITY;
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const int t = t0 + c + 16 * n;
+        valid[n] = key_page[n] >= 0 && t <= pos[r] && t >= w0[r];
+        s[r][n] = valid[n] ? rules(s[r][n], pos[r] - t) : -INFINITY;
+        top = fmaxf(top, s[r][n]);
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      float w[2] = {0.f, 0.f}, corr = 1.f;
+      const bool any = top != -INFINITY;
+      const float m_new = any ? fmaxf(m[r], top) : m[r];
+      if (any) {
+        corr = expf(m[r] - m_new);
+#pragma unroll
+        for (int n = 0; n < 2; ++n) w[n] = valid[n] ? expf(s[r][n] - m_new) : 0.f;
+      }
+      float sum = __fadd_rn(w[0], w[1]);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (any) {
+        l[r] = __fmaf_rn(l[r], corr, sum);
+        m[r] = m_new;
+#pragma unroll
+        for (int j = 0; j < 2 * CG; ++j) { acc[r][j].x *= corr; acc[r][j].y *= corr; }
+      }
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        ps[(rg * 4 + r) * kPPitch + c + 16 * n] = w[n];
+        full = full && w[n] != 0.f;
+      }
+    }
+    full = __all_sync(0xffffffffu, full);                             // then all 32 keys exist, for all rows of the warp
+    __syncthreads();                                                  // the keys have been read, all weights are written
+    const bool more = t0 + kTileKeys <= p_last;
+    if (more) {
+      ask(p.k_pool, ks, next_page, t0 + kTileKeys + crow, d, quads);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");          // the values
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    auto add_values = [&](auto ask_first, int count) {
+      for (int j = 0; j < count; j += 4) {
+        float4 pw[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) pw[r] = *reinterpret_cast<const float4*>(ps + (rg * 4 + r) * kPPitch + j);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float4 vv[CG];
+#pragma unroll
+          for (int g = 0; g < CG; ++g) vv[g] = *reinterpret_cast<const float4*>(vs + (j + e) * PITCH + (g * 64 + c * 4) % DMAX);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const float w = e == 0 ? pw[r].x : e == 1 ? pw[r].y : e == 2 ? pw[r].z : pw[r].w;
+            if (decltype(ask_first)::value && w == 0.f) continue;
+#pragma unroll
+            for (int g = 0; g < CG; ++g) {
+              acc[r][2 * g] = __ffma2_rn(make_float2(w, w), make_float2(vv[g].x, vv[g].y), acc[r][2 * g]);
+              acc[r][2 * g + 1] = __ffma2_rn(make_float2(w, w), make_float2(vv[g].z, vv[g].w), acc[r][2 * g + 1]);
+            }
+          }
+        }
+      }
+    };
+    if (full) add_values(std::false_type(), kTileKeys);
+    else add_values(std::true_type(), min(kTileKeys, p_last - t0 + 1));
+    __syncthreads();                                                  // the values and the weights have been read
+    if (more) ask(p.v_pool, vs, next_page, t0 + kTileKeys + crow, dv, vquads);
+    next_page = ahead_page;
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int row = rg * 4 + r, t = row / group;
+    if (t >= tokens) continue;
+    const float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
+    float* orow = p.out + (static_cast<size_t>(first + t) * p.nq + kvh * group + row % group) * dv;
+#pragma unroll
+    for (int g = 0; g < CG; ++g) {
+      const int i = g * 64 + c * 4;
+      if (i < dv)
+        *reinterpret_cast<float4*>(orow + i) = make_float4(acc[r][2 * g].x * inv, acc[r][2 * g].y * inv, acc[r][2 * g + 1].x * inv, acc[r][2 * g + 1].y * inv);
+    }
+  }
+}
+
+template <int DMAX>
+int launch_attention_tiles(const TileParams& p, int n, cudaStream_t stream) {
+  static DeviceOnce once;
+  const int status = configure_once(once, paged_attention_tile_kernel<DMAX>, attention_tile_smem(DMAX));
+  if (status) return status;
+  const dim3 grid(n / p.per_tile + p.entries, p.nkv);                  // at least as many as there are tiles; the others return
+  if (grid.y > 65535) return B200_ERR_TOO_LARGE;
+  launch(paged_attention_tile_kernel<DMAX>, grid, dim3(kTileThreads), attention_tile_smem(DMAX), stream, p);
+  return launch_status();
 }
 
 }  // namespace b200
@@ -182,4 +438,26 @@ extern "C" int b200_paged_attention_simt(
     int nq, int nkv, int d, float scale, int window, int dtype, cudaStream_t stream) {
   return b200_paged_attention_simt_rules(q, k_pool, v_pool, out, positions, token_entry, block_table, table_stride,
                                          page_size, n, nq, nkv, d, d, scale, window, 0.f, nullptr, 0, dtype, stream);
+}
+
+// float32, rows of 16-byte multiples, head sizes up to 128, at most 32 query heads a key head: the tiles of a prompt portion.  The
+// same results, bit for bit, as the entry points above give.  q_start [entries + 1]: the tokens of entry e are q_start[e] ..
+// q_start[e + 1] - 1, at consecutive positions; block_table [entries, table_stride].
+extern "C" int b200_paged_attention_tiles(
+    const float* q, const float* k_pool, const float* v_pool, float* out, const int* positions, const int* q_start,
+    const int* block_table, int entries, int table_stride, int page_size, int n, int nq, int nkv, int d, int dv, float scale,
+    int window, float softcap, const float* slopes, int sink, int chunk, const float* log_r1, const float* log_r2,
+    const float* sinks, cudaStream_t stream) {
+  using namespace b200;
+  if (n <= 0 || entries <= 0) return 0;
+  if (d <= 0 || dv <= 0 || d % 4 || dv % 4 || nq <= 0 || nkv <= 0 || nq % nkv != 0 || page_size <= 0 ||
+      (log_r1 == nullptr) != (log_r2 == nullptr))
+    return B200_ERR_BAD_SIZE;
+  if (d > 128 || dv > 128 || nq / nkv > kTileRows) return B200_ERR_TOO_LARGE;
+  const TileParams p{q, k_pool, v_pool, out, positions, q_start, block_table, entries, table_stride, page_size, nq, nkv, d, dv,
+                     kTileRows / (nq / nkv), window, chunk, sink, scale, softcap, slopes, log_r1, log_r2, sinks};
+  const int widest = d > dv ? d : dv;
+  if (widest <= 32) return launch_attention_tiles<32>(p, n, stream);
+  if (widest <= 64) return launch_attention_tiles<64>(p, n, stream);
+  return launch_attention_tiles<128>(p, n, stream);
 }

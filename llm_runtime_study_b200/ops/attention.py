@@ -9,6 +9,12 @@ import torch
 from . import functional as F
 
 
+def portions_start(ctx: Any) -> "torch.Tensor | None":
+    """The first token of every entry, for the kernels that tile prompt portions; ``None`` for batches of single tokens."""
+
+    return None if ctx.all_decode else getattr(ctx, "q_start", None)
+
+
 def paged_attention(q: torch.Tensor, cache: Any, ctx: Any, *, scale: float, window: int = 0) -> torch.Tensor:
     """Causal attention of the batch's query tokens over their requests' pages.
 
@@ -28,5 +34,5 @@ def paged_attention(q: torch.Tensor, cache: Any, ctx: Any, *, scale: float, wind
             return out
     return F.paged_attention_simt(
         q, cache.keys, cache.values, positions=ctx.positions, token_entry=ctx.token_entry,
-        block_table=table, scale=scale, window=window,
+        block_table=table, scale=scale, window=window, q_start=portions_start(ctx),
     )

@@ -9,6 +9,7 @@ import torch
 
 from . import attention_bf16, native
 from . import functional as F
+from .attention import portions_start
 
 # "tcgen05": the tensor-core kernels wherever they take the shape (tcgen05 for prompt portions of head size 64 and
 # 128, mma.sync otherwise); "mma": mma.sync only; "simt": the CUDA-core kernel everywhere
@@ -87,7 +88,7 @@ def paged_attention_rules(q: torch.Tensor, cache: Any, ctx: Any, table: torch.Te
         return out
     return F.paged_attention_simt_rules(
         q, cache.keys, cache.values, positions=ctx.positions, token_entry=ctx.token_entry, block_table=table,
-        scale=scale, window=window, softcap=softcap, slopes=slopes, sink=sink,
+        scale=scale, window=window, softcap=softcap, slopes=slopes, sink=sink, q_start=portions_start(ctx),
     )
 
 
@@ -130,4 +131,5 @@ def _masked(q: torch.Tensor, cache: Any, ctx: Any, table: torch.Tensor, *, scale
     return F.paged_attention_simt_rules(
         q, cache.keys, cache.values, positions=ctx.positions, token_entry=ctx.token_entry, block_table=table,
         scale=scale, window=window, softcap=softcap, slopes=slopes, sink=sink, chunk=chunk, log_bias=log_bias,
+        q_start=portions_start(ctx),
     )

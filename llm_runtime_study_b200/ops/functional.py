@@ -150,12 +150,25 @@ def qk_norm_rope_write(
     return q_out
 
 
+def attention_tiles_take(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor) -> bool:
+    """Whether the tiled float32 kernel takes these tensors: rows that start on 16-byte boundaries, head sizes up to 128, up to 32
+    query heads a key head (its CTAs hold 32 rows)."""
+
+    _, nq, d = q.shape
+    nkv, dv = v_pool.shape[1], v_pool.shape[3]
+    return (q.dtype == torch.float32 and d % 4 == 0 and dv % 4 == 0 and max(d, dv) <= 128 and nq % nkv == 0 and nq // nkv <= 32
+            and all(t.data_ptr() % 16 == 0 for t in (q, k_pool, v_pool)))
+
+
 def paged_attention_simt(
     q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, *, positions: torch.Tensor,
-    token_entry: torch.Tensor, block_table: torch.Tensor, scale: float, window: int = 0,
+    token_entry: torch.Tensor, block_table: torch.Tensor, scale: float, window: int = 0, q_start: torch.Tensor | None = None,
 ) -> torch.Tensor:
     """Causal attention of every query token over keys ``0..position`` of its request,
-    32-bit arithmetic, reduction order fixed by the token's position alone."""
+    32-bit arithmetic, reduction order fixed by the token's position alone.  ``q_start`` (int32
+    ``[entries + 1]``): the tokens of entry ``e`` are rows ``q_start[e] .. q_start[e + 1] - 1``, at
+    consecutive positions; given for batches that hold prompt portions, whose rows then share their
+    keys in tiles where the sizes allow it (the same bits)."""
 
     require(q, "q", dims=3)
     n, nq, d = q.shape
@@ -169,10 +182,25 @@ def paged_attention_simt(
     require(positions, "positions", dtype=torch.int32, shape=(n,))
     require(token_entry, "token_entry", dtype=torch.int32, shape=(n,))
     require(block_table, "block_table", dtype=torch.int32, dims=2)
+    if q_start is not None and attention_tiles_take(q, k_pool, v_pool):
+        return _attention_tiles(q, k_pool, v_pool, positions, q_start, block_table, scale, window)
     out = torch.empty_like(q)
     call("b200_paged_attention_simt", ptr(q), ptr(k_pool), ptr(v_pool), ptr(out), ptr(positions),
          ptr(token_entry), ptr(block_table), block_table.shape[1], page_size, n, nq, nkv, d,
          float(scale), int(window), tag(q.dtype), stream_ptr())
+    return out
+
+
+def _attention_tiles(q, k_pool, v_pool, positions, q_start, block_table, scale, window, softcap=0.0, slopes=None, sink=False, chunk=0,
+                     r1=None, r2=None, sinks=None) -> torch.Tensor:
+    n, nq, d = q.shape
+    _, nkv, page_size, dv = v_pool.shape
+    entries = block_table.shape[0]
+    require(q_start, "q_start", dtype=torch.int32, shape=(entries + 1,))
+    out = torch.empty((n, nq, dv), dtype=q.dtype, device=q.device)
+    call("b200_paged_attention_tiles", ptr(q), ptr(k_pool), ptr(v_pool), ptr(out), ptr(positions), ptr(q_start), ptr(block_table), entries,
+         block_table.shape[1], page_size, n, nq, nkv, d, dv, float(scale), int(window), float(softcap), ptr(slopes), 1 if sink else 0,
+         int(chunk), ptr(r1), ptr(r2), ptr(sinks), stream_ptr())
     return out
 
 
@@ -215,6 +243,7 @@ def paged_attention_simt_rules(
     q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, *, positions: torch.Tensor, token_entry: torch.Tensor,
     block_table: torch.Tensor, scale: float, window: int = 0, softcap: float = 0.0, slopes: torch.Tensor | None = None,
     sink: "bool | torch.Tensor" = False, chunk: int = 0, log_bias: tuple[torch.Tensor, torch.Tensor] | None = None,
+    q_start: torch.Tensor | None = None,
 ) -> torch.Tensor:
     """``paged_attention_simt`` with rules on the scores: ``S <- cap * tanh(S / cap)`` (``softcap > 0``), then
     ``S <- S - slopes[head] * (p - t)``, ``S <- S - r1[head] * ln(1 + r2[head] * (p - t))`` (``log_bias = (r1, r2)``), and with
@@ -246,6 +275,8 @@ def paged_attention_simt_rules(
         sinks, sink = require(sink, "sink", dtype=torch.float32, shape=(nq,)), False
     if d > 256 or dv > 256:
         raise KernelError(f"head sizes {d} and {dv} must be at most 256")
+    if q_start is not None and attention_tiles_take(q, k_pool, v_pool):
+        return _attention_tiles(q, k_pool, v_pool, positions, q_start, block_table, scale, window, softcap, slopes, sink, chunk, r1, r2, sinks)
     out = torch.empty((n, nq, dv), dtype=q.dtype, device=q.device)
     call("b200_paged_attention_simt_masked", ptr(q), ptr(k_pool), ptr(v_pool), ptr(out), ptr(positions), ptr(token_entry),
          ptr(block_table), block_table.shape[1], page_size, n, nq, nkv, d, dv, dv, float(scale), int(window), float(softcap),

@@ -275,6 +275,48 @@ def test_paged_attention_simt(dtype, nq, nkv, d, page):
     torch.testing.assert_close(out.cpu().double(), want, **tol(dtype) if dtype == torch.float32 else dict(atol=2e-2, rtol=2e-2))
 
 
+# (query heads, key heads, d, dv, page): groups that do and do not divide the 32 rows of a tile, columns that fill no vector of
+# threads, pages that tiles of 32 keys do not align with; then every rule alone and together
+@pytest.mark.parametrize("nq,nkv,d,dv,page", [(4, 2, 16, 16, 4), (6, 1, 32, 32, 8), (5, 5, 48, 36, 16), (16, 8, 128, 128, 16), (10, 2, 100, 64, 16),
+                                              (32, 1, 32, 48, 8), (21, 3, 64, 64, 32), (34, 1, 32, 32, 8)])
+@pytest.mark.parametrize("rules", [{}, {"window": 33}, {"softcap": 5.0, "slopes": True}, {"chunk": 48, "log_bias": True}, {"sink": "each", "window": 7},
+                                   {"sink": "zero", "softcap": 20.0}])
+def test_attention_tiles_give_the_bits_of_single_tokens(nq, nkv, d, dv, page, rules):
+    g = torch.Generator().manual_seed(nq * 7 + d)
+    spans = [(1, 1), (33, 33), (70, 5), (131, 1), (64, 2), (200, 150), (97, 64)]         # (length after the step, tokens in it)
+    lens = [n for _, n in spans]
+    pages = [-(-length // page) for length, _ in spans]
+    ids = torch.randperm(sum(pages), generator=g).to(torch.int32)
+    table = torch.full((len(spans), max(pages)), -1, dtype=torch.int32)
+    for i, n in enumerate(pages):
+        table[i, :n] = ids[sum(pages[:i]) : sum(pages[:i]) + n]
+    k_pool = torch.randn(sum(pages), nkv, page, d, generator=g)
+    v_pool = torch.randn(sum(pages), nkv, page, dv, generator=g)
+    pos = torch.tensor([t for length, n in spans for t in range(length - n, length)], dtype=torch.int32)
+    entry = torch.repeat_interleave(torch.arange(len(spans), dtype=torch.int32), torch.tensor(lens))
+    for i, (length, _) in enumerate(spans):           # what lies behind a request's last token is nobody's: it may be anything
+        if length % page:
+            k_pool[table[i, pages[i] - 1], :, length % page :] = float("nan")
+            v_pool[table[i, pages[i] - 1], :, length % page :] = float("inf")
+    q_start = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32)
+    q = dev(torch.randn(sum(lens), nq, d, generator=g))
+    options = {key: value for key, value in rules.items() if key in ("window", "softcap", "chunk")}
+    if "slopes" in rules:
+        options["slopes"] = dev(torch.rand(nq, generator=g))
+    if "log_bias" in rules:
+        options["log_bias"] = (dev(torch.rand(nq, generator=g)), dev(torch.rand(nq, generator=g)))
+    if "sink" in rules:
+        options["sink"] = True if rules["sink"] == "zero" else dev(torch.randn(nq, generator=g))
+
+    def run(**more):
+        return F().paged_attention_simt_rules(q, dev(k_pool), dev(v_pool), positions=dev(pos), token_entry=dev(entry), block_table=dev(table),
+                                              scale=1 / math.sqrt(d), **options, **more)
+
+    alone, tiled = run(), run(q_start=dev(q_start))
+    assert bool(torch.isfinite(alone).all())
+    assert torch.equal(alone, tiled)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("window", [1, 7, 32, 33])
 def test_paged_attention_simt_window(dtype, window):
