@@ -61,42 +61,38 @@ __device__ __forceinline__ float uniform23(uint64_t stream, uint32_t index) {
   return (static_cast<float>(static_cast<uint32_t>(z >> 41)) + 0.5f) * (1.0f / 8388608.0f);
 }
 
-// A CTA's share of a row: elements [begin, end), begin a multiple of four.
+// A CTA's share of a row: `count` elements from the row's element `base` (a multiple of four) on.
 struct Slice {
-  const float* x;      // the row
-  int begin, end;
+  const float* x;        // the share: the logits themselves, or the scaled ones staged in shared memory
+  int count, base;
+  float temperature;     // what x is still to be divided by (1: nothing)
 };
 
-// Calls f(x[i] / temperature, i) for every i of the slice: 16-byte loads, two in flight per thread,
+// Calls f(scaled logit, vocabulary index) for every element of the slice: 16-byte loads, two in flight per thread,
 // then the ragged end.  The order in which a thread sees its elements is fixed by the block size.
 template <typename F>
-__device__ __forceinline__ void for_each_scaled(const Slice& sl, float temperature, F&& f) {
+__device__ __forceinline__ void for_each_scaled(const Slice& sl, F&& f) {
   const bool aligned = (reinterpret_cast<uintptr_t>(sl.x) & 15) == 0;
-  const int first = sl.begin >> 2;
-  const int vec = aligned ? sl.end >> 2 : first;          // whole groups of four up to here
+  const int vec = aligned ? sl.count >> 2 : 0;            // whole groups of four
   const float4* x4 = reinterpret_cast<const float4*>(sl.x);
-  const float* x = sl.x;
   const int step = blockDim.x;
-  int i = first + threadIdx.x;
+  const float t = sl.temperature;
+  const bool divides = t != 1.f;
+  auto four = [&](float4 a, int i) {
+    if (divides) { a.x /= t; a.y /= t; a.z /= t; a.w /= t; }
+    f(a.x, sl.base + 4 * i);
+    f(a.y, sl.base + 4 * i + 1);
+    f(a.z, sl.base + 4 * i + 2);
+    f(a.w, sl.base + 4 * i + 3);
+  };
+  int i = threadIdx.x;
   for (; i + step < vec; i += 2 * step) {
     const float4 a = x4[i], b = x4[i + step];
-    f(a.x / temperature, 4 * i);
-    f(a.y / temperature, 4 * i + 1);
-    f(a.z / temperature, 4 * i + 2);
-    f(a.w / temperature, 4 * i + 3);
-    f(b.x / temperature, 4 * (i + step));
-    f(b.y / temperature, 4 * (i + step) + 1);
-    f(b.z / temperature, 4 * (i + step) + 2);
-    f(b.w / temperature, 4 * (i + step) + 3);
+    four(a, i);
+    four(b, i + step);
   }
-  for (; i < vec; i += step) {
-    const float4 a = x4[i];
-    f(a.x / temperature, 4 * i);
-    f(a.y / temperature, 4 * i + 1);
-    f(a.z / temperature, 4 * i + 2);
-    f(a.w / temperature, 4 * i + 3);
-  }
-  for (int j = 4 * vec + threadIdx.x; j < sl.end; j += step) f(x[j] / temperature, j);
+  for (; i < vec; i += step) four(x4[i], i);
+  for (int j = 4 * vec + threadIdx.x; j < sl.count; j += step) f(divides ? sl.x[j] / t : sl.x[j], sl.base + j);
 }
 
 // ---- reductions over the CTAs of a cluster (a cluster of one is the plain block) ----
@@ -127,86 +123,99 @@ __device__ __forceinline__ float load_from_rank(const float* local, uint32_t ran
 struct ClusterSlots {
   float (*slots)[16];      // [2][16] in shared memory: what this CTA contributes
   float (*gathered)[16];   // [16 ranks][16]: the contributions of all ranks, fetched by one thread each
+  float* totals;           // [16]: their sums
   int which;
 };
 constexpr int kMaxClusterRanks = 16;
-template <int N>
-__device__ void cluster_sum_n(float (&v)[N], ClusterSlots& cs, uint32_t ranks) {
-  static_assert(N <= 16, "slots hold sixteen values");
-  if (ranks == 1) return;
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int n = 0; n < N; ++n) cs.slots[cs.which][n] = v[n];
-  }
-  cluster_barrier();
-  // one remote load per thread, all in flight together; then every thread adds them up in rank order
-  if (threadIdx.x < ranks * N) {
-    const uint32_t r = threadIdx.x / N, n = threadIdx.x % N;
-    cs.gathered[r][n] = load_from_rank(&cs.slots[cs.which][n], r);
+// Sums of the ranks' values, in rank order, into `totals`: every CTA holds the same bits.  slots[which][0 .. n) hold this
+// CTA's values and have been written by the threads below `n` of a warp or by one thread; all threads call.
+__device__ __forceinline__ void cluster_totals(ClusterSlots& cs, uint32_t ranks, uint32_t n) {
+  if (ranks == 1) {
+    __syncthreads();
+    if (threadIdx.x < n) cs.totals[threadIdx.x] = cs.slots[cs.which][threadIdx.x];
+  } else {
+    cluster_barrier();
+    // one remote load per thread, all in flight together; then a thread per value adds them up
+    if (threadIdx.x < ranks * n) cs.gathered[threadIdx.x / n][threadIdx.x % n] = load_from_rank(&cs.slots[cs.which][threadIdx.x % n], threadIdx.x / n);
+    __syncthreads();
+    if (threadIdx.x < n) {
+      float total = 0.f;
+      for (uint32_t r = 0; r < ranks; ++r) total += cs.gathered[r][threadIdx.x];
+      cs.totals[threadIdx.x] = total;
+    }
   }
   __syncthreads();
-#pragma unroll
-  for (int n = 0; n < N; ++n) {
-    float total = 0.f;
-    for (uint32_t r = 0; r < ranks; ++r) total += cs.gathered[r][n];
-    v[n] = total;
-  }
-  __syncthreads();          // the gathered values are read before the next reduction overwrites them
-  cs.which ^= 1;
+  cs.which ^= 1;           // two sets of slots alternate: one barrier per reduction is enough
+}
+__device__ float cluster_sum(float v, float* scratch, ClusterSlots& cs, uint32_t ranks) {
+  v = block_sum(v, scratch);
+  if (threadIdx.x == 0) cs.slots[cs.which][0] = v;
+  cluster_totals(cs, ranks, 1);
+  const float total = cs.totals[0];
+  __syncthreads();         // read before the next reduction overwrites it
+  return total;
 }
 
-// Sums of N per-thread values over the block, in a fixed order; every thread gets all N results.
-template <int N>
-__device__ void block_sum_n(float (&v)[N], float (*scratch)[32]) {
+// Sums of sixteen per-thread values over the block and the cluster, in a fixed order, into cs.totals.  Within a warp each
+// exchange halves the values a lane answers for (16 shuffles instead of 5 a value); a warp then finishes one value.
+__device__ void sum_sixteen(float (&v)[16], float (*scratch)[32], ClusterSlots& cs, uint32_t ranks) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
 #pragma unroll
-  for (int n = 0; n < N; ++n) {
+  for (int o = 16, keep = 8; o > 1; o >>= 1, keep >>= 1) {
+    const bool upper = (lane & o) != 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[n] += __shfl_xor_sync(0xffffffffu, v[n], o);
+    for (int i = 0; i < 8; ++i) {
+      if (i < keep) {
+        const float send = upper ? v[i] : v[i + keep];
+        v[i] = (upper ? v[i + keep] : v[i]) + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
   }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  if ((lane & 1) == 0) scratch[lane >> 1][warp] = v[0];      // lane 2 n holds value n (its bits chose the halves from the top)
   __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int n = 0; n < N; ++n) scratch[n][warp] = v[n];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int n = 0; n < N; ++n) {
+  for (int n = warp; n < 16; n += nwarps) {
     float t = lane < nwarps ? scratch[n][lane] : 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    v[n] = t;
+    if (lane == 0) cs.slots[cs.which][n] = t;
   }
+  cluster_totals(cs, ranks, 16);
 }
 
 // The largest key k such that weight(keys >= k) >= target, searched four bits a pass over the whole row
 // (every CTA of the cluster scans its slice; the partial weights are added in rank order).  The weight of
 // an element is 1 (MASS = false: a count) or exp(v - mx) (MASS = true); elements below `floor_key`
-// weigh nothing.  0 when even the whole row does not reach the target.
+// weigh nothing.  0 when even the whole row does not reach the target.  Elements whose leading bits lie above
+// those found so far count in every later pass alike: their weight is carried, and a pass weighs only the
+// elements that share the bits found (from the third pass on, few).
 template <bool MASS>
-__device__ uint32_t find_threshold(const Slice& sl, float temperature, uint32_t floor_key, float mx, float target,
-                                   float (*scratch)[32], ClusterSlots& cs, uint32_t ranks) {
+__device__ uint32_t find_threshold(const Slice& sl, uint32_t floor_key, float mx, float target, float (*scratch)[32],
+                                   ClusterSlots& cs, uint32_t ranks) {
   uint32_t k = 0;
+  float above = 0.f;
   for (int shift = 28; shift >= 0; shift -= 4) {
-    float w[15];
+    float w[16];
 #pragma unroll
-    for (int j = 0; j < 15; ++j) w[j] = 0.f;
-    for_each_scaled(sl, temperature, [&](float v, int) {
+    for (int j = 0; j < 16; ++j) w[j] = 0.f;
+    const uint32_t found = shift == 28 ? 0u : k >> (shift + 4);
+    for_each_scaled(sl, [&](float v, int) {
       const uint32_t key = ordered_key(v);
-      if (key < floor_key || key < k) return;
-      // among the keys that share the bits found so far, the next four bits say how many candidates it reaches
-      const uint32_t reach = (key >> shift) >= (k >> shift) + 16u ? 15u : ((key >> shift) & 15u);
+      if (key < floor_key || (shift != 28 && (key >> (shift + 4)) != found)) return;
+      const uint32_t digit = (key >> shift) & 15u;      // how many of the fifteen candidates the element reaches
       const float weight = MASS ? expf(v - mx) : 1.f;
 #pragma unroll
-      for (int j = 0; j < 15; ++j) w[j] += static_cast<uint32_t>(j) < reach ? weight : 0.f;
+      for (int j = 0; j < 15; ++j)
+        if (static_cast<uint32_t>(j) < digit) w[j] += weight;
     });
-    block_sum_n<15>(w, scratch);
-    cluster_sum_n<15>(w, cs, ranks);
+    sum_sixteen(w, scratch, cs, ranks);
     uint32_t best = 0;
 #pragma unroll
     for (int j = 0; j < 15; ++j)
-      if (w[j] >= target) best = j + 1;       // weights fall with j: the last one that still reaches the target
+      if (above + cs.totals[j] >= target) best = j + 1;       // weights fall with j: the last one that still reaches the target
     k |= best << shift;
+    if (best < 15) above += cs.totals[best];
+    __syncthreads();                                          // the totals have been read
   }
   return k;
 }
@@ -242,15 +251,21 @@ __device__ ArgMax block_argmax(ArgMax v, ArgMax* scratch) {
 }
 
 // One cluster of CTAs per row (gridDim.x = rows * cluster size): each CTA scans its slice of the row and
-// the CTAs combine their results through distributed shared memory.
+// the CTAs combine their results through distributed shared memory.  STAGED: the slice is read from memory and divided by
+// the temperature once and kept in shared memory for the twenty passes over it (`staged`: room for it).  Bound by the passes'
+// arithmetic: 32 rows of 151,936 entries, 19 of them filtered, 104 us (228 when every pass read and divided the logits and
+// weighed each element against all fifteen candidates in all of its eight passes).
+template <bool STAGED>
 __global__ void __launch_bounds__(1024)
 sample_kernel(const float* __restrict__ logits, int ld, int vocab, RowParams params,
               int* __restrict__ out, int filtered_only) {
   __shared__ ArgMax arg_scratch[32];
   __shared__ float sum_scratch[32];
-  __shared__ float multi_scratch[15][32];
+  __shared__ float multi_scratch[16][32];
   __shared__ float slot_memory[2][16];
   __shared__ float gathered_memory[kMaxClusterRanks][16];
+  __shared__ float totals[16];
+  extern __shared__ __align__(16) float staged[];
   pdl_trigger();
   pdl_wait();
   const uint32_t ranks = cluster_size(), rank = cluster_rank();
@@ -264,13 +279,9 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab, RowParams par
   const uint64_t seed = (static_cast<uint64_t>(static_cast<uint32_t>(p[4])) << 32) | static_cast<uint32_t>(p[3]);
   const uint32_t counter = static_cast<uint32_t>(p[5]);
   const int per = ((vocab + static_cast<int>(ranks) - 1) / static_cast<int>(ranks) + 3) & ~3;
-  Slice sl{logits + static_cast<size_t>(row) * ld, min(vocab, static_cast<int>(rank) * per), min(vocab, static_cast<int>(rank + 1) * per)};
-  ClusterSlots cs{slot_memory, gathered_memory, 0};
-  auto cluster_sum = [&](float v) {
-    float one[1] = {block_sum(v, sum_scratch)};
-    cluster_sum_n<1>(one, cs, ranks);
-    return one[0];
-  };
+  const int begin = min(vocab, static_cast<int>(rank) * per), end = min(vocab, static_cast<int>(rank + 1) * per);
+  Slice sl{logits + static_cast<size_t>(row) * ld + begin, end - begin, begin, 1.f};
+  ClusterSlots cs{slot_memory, gathered_memory, totals, 0};
   auto cluster_argmax = [&](ArgMax v) {
     v = block_argmax(v, arg_scratch);
     if (ranks == 1) return v;
@@ -292,32 +303,38 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab, RowParams par
   };
 
   // non-finite logits are an error (mini_llm/sampling.py:104-113): report -1
-  float bad = 0.f;
-  for_each_scaled(sl, 1.f, [&](float v, int) { bad += isfinite(v) ? 0.f : 1.f; });
-  const bool any_bad = cluster_sum(bad) > 0.f;
+  float bad = 0.f, mx = -INFINITY;
+  const float scale = temperature == 0.f ? 1.f : temperature;
+  for_each_scaled(sl, [&](float raw, int i) {
+    bad += isfinite(raw) ? 0.f : 1.f;
+    const float v = raw / scale;
+    mx = fmaxf(mx, v);
+    if (STAGED) staged[i - begin] = v;
+  });
+  if (STAGED) sl.x = staged;
+  else sl.temperature = scale;
+  const bool any_bad = cluster_sum(bad, sum_scratch, cs, ranks) > 0.f;     // (a block-wide barrier: the staged values are there)
   int result = -1;
   if (!any_bad && temperature == 0.f) {
     ArgMax best{-INFINITY, 0x7fffffff};
-    for_each_scaled(sl, 1.f, [&](float v, int i) { best = better(best, ArgMax{v, i}); });
+    for_each_scaled(sl, [&](float v, int i) { best = better(best, ArgMax{v, i}); });
     result = cluster_argmax(best).index;
   } else if (!any_bad) {
     uint32_t low_key = 0;  // tokens with key >= low_key stay
     if (top_k > 0 && top_k < vocab)
-      low_key = find_threshold<false>(sl, temperature, 0u, 0.f, static_cast<float>(top_k), multi_scratch, cs, ranks);
+      low_key = find_threshold<false>(sl, 0u, 0.f, static_cast<float>(top_k), multi_scratch, cs, ranks);
     if (top_p < 1.f) {
-      float mx = -INFINITY;
-      for_each_scaled(sl, temperature, [&](float v, int) { mx = fmaxf(mx, v); });
       mx = cluster_argmax(ArgMax{mx, 0}).value;
       float z = 0.f;
-      for_each_scaled(sl, temperature, [&](float v, int) {
+      for_each_scaled(sl, [&](float v, int) {
         if (ordered_key(v) >= low_key) z += expf(v - mx);
       });
-      const float target = top_p * cluster_sum(z);
-      low_key = max(low_key, find_threshold<true>(sl, temperature, low_key, mx, target, multi_scratch, cs, ranks));
+      const float target = top_p * cluster_sum(z, sum_scratch, cs, ranks);
+      low_key = max(low_key, find_threshold<true>(sl, low_key, mx, target, multi_scratch, cs, ranks));
     }
     const uint64_t stream = splitmix64(seed ^ splitmix64(static_cast<uint64_t>(counter)));
     ArgMax best{-INFINITY, 0x7fffffff};
-    for_each_scaled(sl, temperature, [&](float v, int i) {
+    for_each_scaled(sl, [&](float v, int i) {
       if (ordered_key(v) < low_key) return;
       const float u = uniform23(stream, static_cast<uint32_t>(i));
       best = better(best, ArgMax{v - logf(-logf(u)), i});
@@ -404,17 +421,22 @@ __global__ void sample_final_kernel(const float* __restrict__ part_value, const 
 
 }  // namespace b200
 
-// The single-kernel path: a cluster of up to eight CTAs per row for vocabularies of 32,768 entries and
-// more, one CTA otherwise.
+// The single-kernel path: a cluster of eight CTAs per row for vocabularies of 32,768 entries and more, one CTA
+// otherwise.  151,936 entries: a share is 76 KB, so two CTAs of 512 threads are resident on an SM and 32 rows run at once.
+constexpr size_t kMostStaged = 200 * 1024;
 static int launch_sample(const float* logits, int ld, int vocab, b200::RowParams params, int* out, int rows, int filtered_only,
                          cudaStream_t stream) {
-  const int threads = vocab >= 8192 ? 1024 : (vocab >= 1024 ? 256 : 128);
-  // a cluster of CTAs per row for large vocabularies, as long as all clusters fit on the GPU at once
-  const int cluster = vocab < 32768 ? 1 : (rows <= 16 ? 8 : (rows <= 32 ? 4 : (rows <= 64 ? 2 : 1)));
+  const int cluster = vocab < 32768 ? 1 : 8;
+  const int threads = cluster > 1 ? 512 : (vocab >= 8192 ? 1024 : (vocab >= 1024 ? 256 : 128));
+  const size_t share = sizeof(float) * static_cast<size_t>(((vocab + cluster - 1) / cluster + 3) & ~3);
+  const bool staged = share <= kMostStaged;
+  static b200::DeviceOnce once;
+  if (staged)
+    if (int e = b200::configure_once(once, b200::sample_kernel<true>, kMostStaged)) return e;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(rows * cluster);
   config.blockDim = dim3(threads);
-  config.dynamicSmemBytes = 0;
+  config.dynamicSmemBytes = staged ? share : 0;
   config.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -425,7 +447,8 @@ static int launch_sample(const float* logits, int ld, int vocab, b200::RowParams
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = b200::pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&config, b200::sample_kernel, logits, ld, vocab, params, out, filtered_only);
+  cudaError_t e = staged ? cudaLaunchKernelEx(&config, b200::sample_kernel<true>, logits, ld, vocab, params, out, filtered_only)
+                         : cudaLaunchKernelEx(&config, b200::sample_kernel<false>, logits, ld, vocab, params, out, filtered_only);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 

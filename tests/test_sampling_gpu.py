@@ -66,6 +66,23 @@ def test_large_odd_vocabulary_every_cluster_size(sampler, rows):
         assert got[r] == want or abs(float(scores[got[r]] - scores[want])) < 1e-4
 
 
+# the smallest vocabulary that clusters share, the one below it, one whose shares leave most of the last CTA idle, and one whose
+# shares do not fit in shared memory
+@pytest.mark.parametrize("vocab", [32767, 32768, 32793, 1_700_003])
+@pytest.mark.parametrize("opts", [dict(temperature=0.9, top_k=40), dict(temperature=1.2, top_p=0.8), dict(temperature=0.7, top_k=1000, top_p=0.9)])
+def test_thresholds_at_the_edges_of_the_shares(sampler, vocab, opts):
+    torch.manual_seed(6)
+    logits = torch.randn(2, vocab) * 3
+    logits[1, -3:] += 20.0                                        # the row's last elements decide it
+    specs = [(cfg(**opts), 55 + r, r) for r in range(2)]
+    got = sampler.sample(logits.cuda(), specs)
+    for r in range(2):
+        want, scores = plain.sample(logits[r], opts["temperature"], opts.get("top_k"), opts.get("top_p", 1.0), 55 + r, r)
+        keep = plain.kept_mask(logits[r], opts["temperature"], opts.get("top_k"), opts.get("top_p", 1.0))
+        assert keep[got[r]]
+        assert got[r] == want or abs(float(scores[got[r]] - scores[want])) < 1e-4
+
+
 def test_rows_are_independent_of_the_batch(sampler):
     torch.manual_seed(2)
     logits = torch.randn(8, 503).cuda()
