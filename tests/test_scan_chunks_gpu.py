@@ -1,0 +1,120 @@
+"""The scan of prompt portions sixteen tokens at a time against the token-by-token kernel and 64-bit arithmetic."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _reference(q, k, v, lens, state, slots, *, decay, gain, beta):
+    """The recurrence in 64 bits: q, k [N, H, d], v [N, H, dv], decay [N, H, d], gain [N, H] or None, beta [N, H] or None."""
+
+    out, end = torch.empty_like(v), state.clone()
+    first = 0
+    for n, slot in zip(lens, slots):
+        S = end[slot]
+        for t in range(first, first + n):
+            S = decay[t][..., None] * S
+            u = v[t] if gain is None else gain[t][:, None] * v[t]
+            if beta is not None:
+                u = beta[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+            S = S + k[t][:, :, None] * u[:, None, :]
+            out[t] = torch.einsum("hdv,hd->hv", S, q[t])
+        end[slot] = S
+        first += n
+    return out, end
+
+
+FORMS = ["head", "head_float_qk", "channel", "row", "delta_channel", "delta_token"]
+
+
+# portions around a chunk's edges, key sizes that fill 2, 4 and 8 warps and none, value columns around a block of 32
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("heads,qk_heads,d,dv,lens", [(2, 2, 128, 128, [257]), (4, 2, 40, 33, [1, 15, 16, 17, 64]), (3, 3, 16, 8, [100, 31]),
+                                                      (1, 1, 72, 64, [49, 1])])
+def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens):
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    if form == "row":
+        qk_heads = heads
+    g = torch.Generator().manual_seed(len(form) + d)
+    n, slots = sum(lens), [2 * i + 1 for i in range(len(lens))]
+    delta = form.startswith("delta")
+    narrow = torch.float32 if delta or form == "head_float_qk" else torch.bfloat16
+    q, k = (torch.randn(n, qk_heads * d, generator=g).to(narrow) for _ in range(2))
+    v = torch.randn(n, heads * dv, generator=g).to(torch.float32 if delta else torch.bfloat16)
+    if delta:
+        q, k = (torch.nn.functional.normalize(x.view(n, qk_heads, d), dim=-1).reshape(n, -1) for x in (q, k))
+    state = 0.3 * torch.randn(2 * len(lens) + 2, heads, d, dv, generator=g)
+    norm_state = 0.3 * torch.randn(2 * len(lens) + 2, heads, d, generator=g)
+    options, gain, beta = {}, None, None
+    if form.startswith("head"):
+        decay = torch.linspace(0.7, 1.0, heads)
+        options["decay"] = decay
+        wide = decay[None, :, None].expand(n, heads, d)
+    elif form in ("channel", "delta_channel"):
+        gate = torch.sigmoid(3.0 * torch.randn(n, heads, d, generator=g) + 2.0)
+        gate[n // 2] *= 1e-30                        # a decay that empties the state, as strong gates do
+        options["gate"] = gate.reshape(n, -1)
+        wide = gate
+    else:
+        token = torch.sigmoid(torch.randn(n, heads, generator=g) + 2.0)
+        options["row_decay" if delta else "decay"] = token
+        wide = token[..., None].expand(n, heads, d)
+        if form == "row":
+            gain = torch.rand(n, heads, generator=g)
+            options["gain"] = gain
+    if delta:
+        beta = torch.sigmoid(torch.randn(n, heads, generator=g))
+        options["beta"] = beta
+    q_start = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+    dev = lambda x: x.to(DEV)
+
+    def run(fixed_order):
+        s, ns = dev(state), dev(norm_state)
+        common = dict(heads=heads, dim=d, vdim=dv, state=s, q_start=q_start, slots=torch.tensor(slots, dtype=torch.int32, device=DEV),
+                      fixed_order=fixed_order, q_scale=0.5, **{key: dev(x) for key, x in options.items()})
+        # rows of a wider projection: strides of their own
+        rows = [dev(torch.cat((x, x), dim=1))[:, : x.shape[1]] for x in (q, k, v)]
+        if form == "row":
+            out, norm_out = S.linear_scan_row_gates(*rows, norm_state=ns, **common)
+            return out, s, norm_out, ns
+        return S.linear_scan(*rows, qk_heads=qk_heads, silu=form == "head", **common), s, None, None
+
+    act = (lambda x: x * torch.sigmoid(x)) if form == "head" else (lambda x: x)
+    group = heads // qk_heads
+    wq, wk = (act(x.double()).view(n, qk_heads, d).repeat_interleave(group, dim=1) for x in (q, k))
+    wv = act(v.double()).view(n, heads, dv)
+    wide = wide.double()
+    want, end = _reference(0.5 * wq, wk, wv, lens, state.double(), slots, decay=wide, gain=None if gain is None else gain.double(),
+                           beta=None if beta is None else beta.double())
+    assert S.scans_in_chunks(n, len(lens), d, False)
+    chunked, chained = run(False), run(True)
+
+    def error(got, ref):
+        return float((got.double().cpu() - ref).norm() / ref.norm())
+
+    pairs = [(0, want.reshape(n, -1)), (1, end)]
+    if form == "row":
+        ones = torch.ones(n, heads, 1, dtype=torch.float64)
+        nwant, nend = _reference(0.5 * wq, wk, ones, lens, norm_state.double()[..., None], slots, decay=wide, gain=gain.double(), beta=None)
+        pairs += [(2, nwant[..., 0]), (3, nend[..., 0])]
+    for i, ref in pairs:
+        # products of up to 16 decays and sums of up to 16 + 128 terms, a rounding of 6e-8 each, sizes adding up like their roots; SiLU
+        # of 16-bit rows takes the hardware's exponential (2 units in the last place), in either kernel
+        assert error(chunked[i], ref) < 2e-6, (i, error(chunked[i], ref), error(chained[i], ref))
+        assert error(chunked[i], ref) < 1.5 * error(chained[i], ref) + 1e-7
+
+
+def test_a_bad_row_reaches_later_tokens_only():
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    n, heads, d = 64, 2, 32
+    g = torch.Generator().manual_seed(1)
+    q, k, v = (torch.randn(n, heads * d, generator=g).bfloat16().to(DEV) for _ in range(3))
+    v[37], k[41] = float("nan"), float("inf")
+    out = S.linear_scan(q, k, v, heads=heads, qk_heads=heads, dim=d, vdim=d, state=torch.zeros(1, heads, d, d, device=DEV),
+                        q_start=torch.tensor([0, n], dtype=torch.int32, device=DEV), slots=torch.zeros(1, dtype=torch.int32, device=DEV),
+                        decay=torch.full((heads,), 0.9, device=DEV))
+    assert bool(torch.isfinite(out[:37]).all()) and not bool(torch.isfinite(out[37:]).any())
