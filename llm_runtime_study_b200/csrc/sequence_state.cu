@@ -398,6 +398,153 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const DeltaPreparePa
   }
 }
 
+// The same for key and value sizes up to 128 and up to four taps: a thread owns one channel of each kind for TOKENS tokens,
+// so that a row of the projection is read once (the taps' window is in registers) and the low-rank map's column once for
+// all of them, and the sums of squares of all the tokens' q and k are finished together: each exchange within a warp halves
+// the sums a lane answers for.  One CTA per head and TOKENS tokens; 16 where that fills the GPU, else 1.  The order of every
+// sum is the same in both.  2,048 tokens of 32 heads of 128: 100 us for 184 MB; 32 single tokens of
+// 16 heads: 14 us.  (A token at a time, four reads of a row and two block-wide sums in a row: 395 and 29 us.)
+constexpr int kPrepareTaps = 4;
+template <typename T, int TOKENS>
+__global__ void __launch_bounds__(128) delta_prepare_tokens_kernel(const DeltaPrepareParams p, int n) {
+  constexpr int W = kPrepareTaps - 1;        // inputs before a token that its taps reach
+  extern __shared__ __align__(16) float low[];              // [rank][TOKENS]
+  __shared__ float partial[4][2 * TOKENS];
+  pdl_trigger();
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, t0 = blockIdx.x * TOKENS;
+  const int d = p.d, dv = p.dv, qk = p.G * d, C = 2 * qk + p.H * dv, K = p.ntaps;
+  const int group = p.H / p.G, gq = h / group, count = min(TOKENS, n - t0);
+  const bool does_qk = h % group == 0;
+  const T* proj = static_cast<const T*>(p.proj);
+  const size_t hv = static_cast<size_t>(p.H) * dv, hd = static_cast<size_t>(p.H) * d;
+  const int entry = p.token_entry[t0];
+  const int first = p.q_start[entry], local0 = t0 - first, slot0 = p.slots[entry];
+  const bool together = t0 + count <= p.q_start[entry + 1];     // the tokens are one request's, one behind the other
+
+  for (int idx = tid; idx < p.rank * TOKENS; idx += 128) {
+    const int t = idx % TOKENS, j = idx / TOKENS;
+    low[idx] = t < count ? to_float(proj[static_cast<size_t>(t0 + t) * p.ld + p.a_off + j]) : 0.f;
+  }
+  if (tid < count) {
+    p.beta[static_cast<size_t>(t0 + tid) * p.H + h] = sigmoid_f(to_float(proj[static_cast<size_t>(t0 + tid) * p.ld + p.b_off + h]));
+    if (p.rank == 0) {
+      const float a = to_float(proj[static_cast<size_t>(t0 + tid) * p.ld + p.a_off + h]);
+      p.g[static_cast<size_t>(t0 + tid) * p.H + h] = expf(-expf(p.a_log[h]) * softplus_f(a + p.dt_bias[h]));
+    }
+  }
+  // the convolution and SiLU of channel c for all the tokens
+  auto convolve = [&](int c, float (&y)[TOKENS]) {
+    float tap[kPrepareTaps];           // the last K of them; those before are zero and meet nothing
+#pragma unroll
+    for (int j = 0; j < kPrepareTaps; ++j) tap[j] = j + K >= kPrepareTaps ? p.taps[static_cast<size_t>(c) * K + j + K - kPrepareTaps] : 0.f;
+    auto input = [&](int from, int at, int slot) -> float {     // the request's input number `at` of this step (negative: kept ones)
+      if (at >= 0) return to_float(proj[static_cast<size_t>(from + at) * p.ld + c]);
+      return at + K - 1 >= 0 ? p.conv_state[(static_cast<size_t>(slot) * (K - 1) + (K - 1 + at)) * C + c] : 0.f;
+    };
+    if (together) {
+      // the step's own rows without a branch, so that all are on their way at once (one past the last is the last again, and
+      // nothing is made of it); rows before the tile may be kept ones
+      T own[TOKENS];
+#pragma unroll
+      for (int t = 0; t < TOKENS; ++t) own[t] = proj[static_cast<size_t>(t0 + min(t, count - 1)) * p.ld + c];
+      float x[TOKENS + W];
+#pragma unroll
+      for (int i = 0; i < W; ++i) x[i] = i + K >= kPrepareTaps ? input(first, local0 + i - W, slot0) : 0.f;
+#pragma unroll
+      for (int t = 0; t < TOKENS; ++t) x[W + t] = to_float(own[t]);
+#pragma unroll
+      for (int t = 0; t < TOKENS; ++t) {
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < kPrepareTaps; ++j) acc = fmaf(tap[j], x[t + j], acc);
+        y[t] = silu_of<T>(acc);
+      }
+    } else {
+#pragma unroll
+      for (int t = 0; t < TOKENS; ++t) {
+        y[t] = 0.f;
+        if (t >= count) continue;
+        const int e = p.token_entry[t0 + t], from = p.q_start[e], slot = p.slots[e];
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < kPrepareTaps; ++j)
+          if (j + K >= kPrepareTaps) acc = fmaf(tap[j], input(from, t0 + t - from - (W - j), slot), acc);
+        y[t] = silu_of<T>(acc);
+      }
+    }
+  };
+  if (does_qk) {                       // the same for every thread of the CTA
+    float q[TOKENS], k[TOKENS], ss[2 * TOKENS];
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t) q[t] = k[t] = 0.f;
+    if (tid < d) {
+      convolve(gq * d + tid, q);
+      convolve(qk + gq * d + tid, k);
+    }
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t) {
+      ss[t] = q[t] * q[t];
+      ss[TOKENS + t] = k[t] * k[t];
+    }
+    // sums over the warp, by xor of 16, 8, 4, 2, 1 whether or not lanes share the values out
+    int held = 0;                      // the value this lane ends up with
+#pragma unroll
+    for (int o = 16, keep = TOKENS; o > 0; o >>= 1, keep >>= 1) {
+      if (keep >= 1) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < TOKENS; ++i) {
+          if (i < keep) {
+            const float send = upper ? ss[i] : ss[i + keep];
+            ss[i] = (upper ? ss[i + keep] : ss[i]) + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+        }
+        held += upper ? keep : 0;
+      } else {
+        ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+      }
+    }
+    partial[warp][held] = ss[0];       // lanes that hold the same value hold the same bits
+    __syncthreads();
+    if (tid < d) {
+#pragma unroll
+      for (int t = 0; t < TOKENS; ++t) {
+        if (t >= count) break;
+        const float sq = ((partial[0][t] + partial[1][t]) + partial[2][t]) + partial[3][t];
+        const float sk = ((partial[0][TOKENS + t] + partial[1][TOKENS + t]) + partial[2][TOKENS + t]) + partial[3][TOKENS + t];
+        p.q[static_cast<size_t>(t0 + t) * qk + gq * d + tid] = q[t] * (rsqrtf(sq + p.unit_eps) * p.q_scale);
+        p.k[static_cast<size_t>(t0 + t) * qk + gq * d + tid] = k[t] * rsqrtf(sk + p.unit_eps);
+      }
+    }
+  } else {
+    __syncthreads();                   // low[] is complete
+  }
+  if (tid < dv) {
+    float v[TOKENS];
+    convolve(2 * qk + h * dv + tid, v);
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t)
+      if (t < count) p.v[(t0 + t) * hv + h * dv + tid] = v[t];
+  }
+  if (p.rank > 0 && tid < d) {
+    const T* up = static_cast<const T*>(p.a_up) + static_cast<size_t>(h) * d + tid;
+    float a[TOKENS];
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t) a[t] = 0.f;
+#pragma unroll 8
+    for (int j = 0; j < p.rank; ++j) {
+      const float u = to_float(up[j * hd]);
+#pragma unroll
+      for (int t = 0; t < TOKENS; ++t) a[t] = fmaf(u, low[j * TOKENS + t], a[t]);
+    }
+    const float rate = expf(p.a_log[h]), bias = p.dt_bias[static_cast<size_t>(h) * d + tid];
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t)
+      if (t < count) p.g[(t0 + t) * hd + static_cast<size_t>(h) * d + tid] = expf(-rate * softplus_f(a[t] + bias));
+  }
+}
+
 // ------------------------------------------------------------- exponential gates of a matrix memory
 // Per request and head, token after token: with i = cap tanh((zi + bi) / cap) and f = ln sigmoid(cap tanh((zf + bf) / cap)),
 //   m_t = max(f + m_(t-1), i),  decay = exp(f + m_(t-1) - m_t),  gain = exp(i - m_t),  floor = exp(-m_t)
@@ -559,6 +706,140 @@ __global__ void group_norm_gate_kernel(const float* __restrict__ x, int width, i
   }
 }
 
+// The same with 16-byte reads, in two forms; the order of a group's sum of squares is a function of the group's size.
+// Small groups (one head, up to 128 columns): a warp owns a group of TOKENS rows, a lane four columns; a low-rank map's
+// columns are read once for all the rows.  2,048 rows of 32 groups of 128 with a map of rank 32: 44 us, 28 us a
+// launch for 1,733 rows without one (75 and 49 us with a CTA per row and group, two bytes at a time, a read of the map per row).
+template <typename T> struct Quad;            // four neighbouring elements of the storage type
+template <> struct Quad<float> {
+  using type = float4;
+  __device__ static float4 widen(const type& v) { return v; }
+  __device__ static type narrow(const float4& v) { return v; }
+};
+template <> struct Quad<__nv_bfloat16> {
+  using type = uint2;
+  __device__ static float4 widen(const type& v) {
+    const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&v)[0]);
+    const float2 b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&v)[1]);
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+  __device__ static type narrow(const float4& v) {
+    type r;
+    reinterpret_cast<__nv_bfloat162*>(&r)[0] = __floats2bfloat162_rn(v.x, v.y);
+    reinterpret_cast<__nv_bfloat162*>(&r)[1] = __floats2bfloat162_rn(v.z, v.w);
+    return r;
+  }
+};
+struct GroupNormParams {
+  const float* x; int n, width, group; const float* w; int w_len; float eps;
+  const float* den; const float* floor_; float den_eps;
+  const void* gate_in; int gate_ld, rank; const void* gate_up; int gate_silu; void* out;
+};
+__device__ __forceinline__ float gated(float x, float f, float w, float logit, int silu) {
+  return x * f * w * (silu ? silu_f(logit) : sigmoid_f(logit));
+}
+
+template <typename T, int TOKENS>
+__global__ void __launch_bounds__(128) group_norm_gate_warp_kernel(const GroupNormParams p) {
+  using Q = Quad<T>;
+  extern __shared__ __align__(16) float low[];     // [rank][TOKENS]: the rows' low-rank input
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, groups = p.width / p.group;
+  const int g = blockIdx.y * 4 + warp, t0 = blockIdx.x * TOKENS, count = min(TOKENS, p.n - t0);
+  for (int idx = threadIdx.x; idx < p.rank * TOKENS; idx += 128) {
+    const int t = idx / p.rank, j = idx % p.rank;
+    low[j * TOKENS + t] = t < count ? to_float(static_cast<const T*>(p.gate_in)[static_cast<size_t>(t0 + t) * p.gate_ld + j]) : 0.f;
+  }
+  __syncthreads();
+  if (g >= groups) return;
+  const int c = g * p.group + lane * 4;
+  const bool on = lane * 4 < p.group;
+  float4 x[TOKENS], z[TOKENS];
+  float factor[TOKENS];
+#pragma unroll
+  for (int t = 0; t < TOKENS; ++t)
+    x[t] = on && t < count ? *reinterpret_cast<const float4*>(p.x + static_cast<size_t>(t0 + t) * p.width + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (p.rank == 0) {
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t) {
+      z[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (on && t < count)
+        z[t] = Q::widen(*reinterpret_cast<const typename Q::type*>(static_cast<const T*>(p.gate_in) + static_cast<size_t>(t0 + t) * p.gate_ld + c));
+    }
+  } else {
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t) z[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const T* up = static_cast<const T*>(p.gate_up) + (on ? c : 0);
+#pragma unroll 8
+    for (int j = 0; j < p.rank; ++j) {
+      const float4 u = Q::widen(*reinterpret_cast<const typename Q::type*>(up + static_cast<size_t>(j) * p.width));
+#pragma unroll
+      for (int t = 0; t < TOKENS; ++t) {
+        const float l = low[j * TOKENS + t];
+        z[t].x = fmaf(u.x, l, z[t].x);
+        z[t].y = fmaf(u.y, l, z[t].y);
+        z[t].z = fmaf(u.z, l, z[t].z);
+        z[t].w = fmaf(u.w, l, z[t].w);
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < TOKENS; ++t) {
+    const float4 v = x[t];
+    const float ss = warp_sum(fmaf(v.x, v.x, v.y * v.y) + fmaf(v.z, v.z, v.w * v.w));
+    float inv = 1.f;
+    if (p.den != nullptr && t < count) {
+      const size_t at = static_cast<size_t>(t0 + t) * groups + g;
+      inv = 1.f / (fmaxf(fabsf(p.den[at]), p.floor_[at]) + p.den_eps);
+    }
+    factor[t] = inv * rsqrtf(ss / static_cast<float>(p.group) * inv * inv + p.eps);
+  }
+  if (!on) return;
+  float4 w = make_float4(1.f, 1.f, 1.f, 1.f);
+  if (p.w != nullptr) w = *reinterpret_cast<const float4*>(p.w + (p.w_len == p.group ? lane * 4 : c));
+#pragma unroll
+  for (int t = 0; t < TOKENS; ++t) {
+    if (t >= count) break;
+    const float f = factor[t];
+    const float4 y = make_float4(gated(x[t].x, f, w.x, z[t].x, p.gate_silu), gated(x[t].y, f, w.y, z[t].y, p.gate_silu),
+                                 gated(x[t].z, f, w.z, z[t].z, p.gate_silu), gated(x[t].w, f, w.w, z[t].w, p.gate_silu));
+    *reinterpret_cast<typename Q::type*>(static_cast<T*>(p.out) + static_cast<size_t>(t0 + t) * p.width + c) = Q::narrow(y);
+  }
+}
+
+// Large groups (the whole row) whose gate is read directly: a CTA per row and group, the row read twice, the second time from
+// the caches: 17 us for 2,048 rows of 4,096 (70 with two-byte reads).
+template <typename T>
+__global__ void __launch_bounds__(256) group_norm_gate_row_kernel(const GroupNormParams p) {
+  using Q = Quad<T>;
+  __shared__ float scratch[32];
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x, base = blockIdx.y * p.group, quads = p.group / 4;
+  const float4* row = reinterpret_cast<const float4*>(p.x + static_cast<size_t>(t) * p.width + base);
+  const auto* gate = reinterpret_cast<const typename Q::type*>(static_cast<const T*>(p.gate_in) + static_cast<size_t>(t) * p.gate_ld + base);
+  auto* out = reinterpret_cast<typename Q::type*>(static_cast<T*>(p.out) + static_cast<size_t>(t) * p.width + base);
+  float ss = 0.f;
+  for (int i = threadIdx.x; i < quads; i += 256) {
+    const float4 v = row[i];
+    ss += fmaf(v.x, v.x, v.y * v.y) + fmaf(v.z, v.z, v.w * v.w);
+  }
+  float inv = 1.f;
+  if (p.den != nullptr) {
+    const size_t at = static_cast<size_t>(t) * gridDim.y + blockIdx.y;
+    inv = 1.f / (fmaxf(fabsf(p.den[at]), p.floor_[at]) + p.den_eps);
+  }
+  const float f = inv * rsqrtf(block_sum(ss, scratch) / static_cast<float>(p.group) * inv * inv + p.eps);
+  const float4* weight = p.w == nullptr ? nullptr : reinterpret_cast<const float4*>(p.w_len == p.group ? p.w : p.w + base);
+  for (int i = threadIdx.x; i < quads; i += 256) {
+    const float4 v = row[i], z = Q::widen(gate[i]);
+    const float4 w = weight ? weight[i] : make_float4(1.f, 1.f, 1.f, 1.f);
+    out[i] = Q::narrow(make_float4(gated(v.x, f, w.x, z.x, p.gate_silu), gated(v.y, f, w.y, z.y, p.gate_silu),
+                                   gated(v.z, f, w.z, z.z, p.gate_silu), gated(v.w, f, w.w, z.w, p.gate_silu)));
+  }
+}
+
 }  // namespace b200
 
 // `tokens`: rows in the batch (with `entries` it tells a batch of single tokens from one that holds portions).
@@ -656,8 +937,21 @@ extern "C" int b200_delta_prepare(const void* proj, int ld, int b_off, int a_off
   if (H <= 0 || G <= 0 || H % G != 0 || d <= 0 || dv <= 0 || ntaps <= 0 || rank < 0) return B200_ERR_BAD_SIZE;
   DeltaPrepareParams p{proj, ld, b_off, a_off, rank, taps, ntaps, conv_state, a_log, dt_bias, a_up, q, k, v, g, beta,
                        q_start, slots, token_entry, H, G, d, dv, unit_eps, q_scale};
+  if (H > 65535) return B200_ERR_TOO_LARGE;
+  if (d <= 128 && dv <= 128 && ntaps <= kPrepareTaps && rank <= 512) {
+    // sixteen tokens a CTA as soon as that gives every SM two
+    const int tokens = static_cast<long long>(n) * H >= 16 * 2 * 148 ? 16 : 1;
+    const dim3 grid((n + tokens - 1) / tokens, H);
+    const size_t smem = sizeof(float) * tokens * rank;
+    if (tokens == 16) {
+      B200_DISPATCH_DTYPE(dtype, T, launch(delta_prepare_tokens_kernel<T, 16>, grid, dim3(128), smem, stream, p, n));
+    } else {
+      B200_DISPATCH_DTYPE(dtype, T, launch(delta_prepare_tokens_kernel<T, 1>, grid, dim3(128), smem, stream, p, n));
+    }
+    return launch_status();
+  }
   const size_t smem = sizeof(float) * (static_cast<size_t>(2) * d + rank + static_cast<size_t>(rank) * d + (static_cast<size_t>(2) * d + dv) * ntaps);
-  if (smem > 200 * 1024 || H > 65535) return B200_ERR_TOO_LARGE;
+  if (smem > 200 * 1024) return B200_ERR_TOO_LARGE;
   // small batches: a CTA per token and head; prompt portions: eight tokens share a CTA's copy of the head's weights
   const int tokens_per_cta = n * H >= 8 * 2 * 148 ? 8 : 1;
   dim3 grid((n + tokens_per_cta - 1) / tokens_per_cta, H);
@@ -693,6 +987,22 @@ extern "C" int b200_group_norm_gate(const float* x, int n, int width, int group,
   if (width <= 0 || group <= 0 || width % group != 0 || rank < 0 || rank > 4096 || (w != nullptr && w_len != group && w_len != width) ||
       (den == nullptr) != (floor_ == nullptr))
     return B200_ERR_BAD_SIZE;
+  // whole groups of four columns on 16- and 8-byte boundaries in every operand
+  const size_t four = dtype == kBF16 ? 8 : 16;
+  auto at = [](const void* ptr, size_t bytes) { return reinterpret_cast<uintptr_t>(ptr) % bytes == 0; };
+  const bool quads = group % 4 == 0 && at(x, 16) && at(out, four) && (w == nullptr || at(w, 16)) &&
+                     (rank > 0 ? at(gate_up, four) : gate_ld % 4 == 0 && at(gate_in, four));
+  if (quads && (group <= 128 ? rank <= 1024 : rank == 0) && (width / group + 3) / 4 <= 65535 && (group <= 128 || width / group <= 65535)) {
+    const GroupNormParams p{x, n, width, group, w, w_len, eps, den, floor_, den_eps, gate_in, gate_ld, rank, gate_up, gate_silu, out};
+    if (group > 128) {
+      B200_DISPATCH_DTYPE(dtype, T, launch(group_norm_gate_row_kernel<T>, dim3(n, width / group), dim3(256), 0, stream, p));
+    } else if (static_cast<long long>(n) * (width / group) >= 8 * 4 * 2 * 148) {
+      B200_DISPATCH_DTYPE(dtype, T, launch(group_norm_gate_warp_kernel<T, 8>, dim3((n + 7) / 8, (width / group + 3) / 4), dim3(128), sizeof(float) * 8 * rank, stream, p));
+    } else {
+      B200_DISPATCH_DTYPE(dtype, T, launch(group_norm_gate_warp_kernel<T, 1>, dim3(n, (width / group + 3) / 4), dim3(128), sizeof(float) * rank, stream, p));
+    }
+    return launch_status();
+  }
   dim3 grid(n, width / group);
   if (grid.y > 65535) return B200_ERR_TOO_LARGE;
   const int threads = group >= 256 ? 256 : (group + 31) / 32 * 32;
