@@ -756,6 +756,85 @@ __global__ void qk_rownorm_write_kernel(const T* __restrict__ qkv, int ld, T* __
   }
 }
 
+// The same with 16-byte accesses: the row's vectors are in registers (up to kRowVecs of q and of k a thread), everything is
+// read before anything waits, and both sums share one pass over the block.  36 us with two-byte accesses for 2,048 rows of
+// 4,096 + 1,024 + 1,024 columns.
+constexpr int kRowVecs = 4;
+template <typename T>
+__global__ void __launch_bounds__(256)
+qk_rownorm_write_vec_kernel(const T* __restrict__ qkv, int ld, T* __restrict__ q_out, const float* __restrict__ q_w,
+                            const float* __restrict__ k_w, float eps, float temp_coef, int temp_every,
+                            const int* __restrict__ positions, const int* __restrict__ token_entry,
+                            const int* __restrict__ block_table, int table_stride, int page_size, T* __restrict__ k_pool,
+                            T* __restrict__ v_pool, int nq, int nkv, int d, int dv) {
+  constexpr int VN = Vec<T>::n;
+  using V = typename Vec<T>::type;
+  __shared__ float2 scratch[8];
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x, tid = threadIdx.x;
+  const int qv = nq * d / VN, kv = nkv * d / VN, vv = nkv * dv / VN;
+  const V* row = reinterpret_cast<const V*>(qkv + static_cast<size_t>(t) * ld);
+  V xq[kRowVecs], xk[kRowVecs];
+#pragma unroll
+  for (int i = 0; i < kRowVecs; ++i) {
+    if (tid + 256 * i < qv) xq[i] = row[tid + 256 * i];
+    if (tid + 256 * i < kv) xk[i] = row[qv + tid + 256 * i];
+  }
+  const int p = positions[t];
+  const int page = block_table[static_cast<size_t>(token_entry[t]) * table_stride + p / page_size];
+  const size_t at = static_cast<size_t>(max(page, 0)) * nkv * page_size + p % page_size;
+  if (page >= 0) {                    // a padding row has no pages
+    for (int i = tid; i < vv; i += 256) {
+      const int g = i * VN / dv, c = i * VN % dv;
+      *reinterpret_cast<V*>(v_pool + (at + static_cast<size_t>(g) * page_size) * dv + c) = row[qv + kv + i];
+    }
+  }
+  float2 ss = make_float2(0.f, 0.f);
+  float f[VN];
+#pragma unroll
+  for (int i = 0; i < kRowVecs; ++i) {
+    if (tid + 256 * i < qv) {
+      Vec<T>::unpack(xq[i], f);
+#pragma unroll
+      for (int e = 0; e < VN; ++e) ss.x = fmaf(f[e], f[e], ss.x);
+    }
+    if (tid + 256 * i < kv) {
+      Vec<T>::unpack(xk[i], f);
+#pragma unroll
+      for (int e = 0; e < VN; ++e) ss.y = fmaf(f[e], f[e], ss.y);
+    }
+  }
+  ss = make_float2(warp_sum(ss.x), warp_sum(ss.y));
+  if ((tid & 31) == 0) scratch[tid >> 5] = ss;
+  __syncthreads();
+  ss = scratch[0];
+#pragma unroll
+  for (int w = 1; w < 8; ++w) { ss.x += scratch[w].x; ss.y += scratch[w].y; }
+  const float fq = q_w ? rsqrtf(ss.x / static_cast<float>(nq * d) + eps) : 1.f;
+  const float fk = k_w ? rsqrtf(ss.y / static_cast<float>(nkv * d) + eps) : 1.f;
+  const float temp = temp_every > 0 ? 1.f + temp_coef * logf(static_cast<float>((p + 1) / temp_every) + 1.f) : 1.f;
+  auto scaled = [&](const V& x, float factor, const float* w, float last) {
+    Vec<T>::unpack(x, f);
+#pragma unroll
+    for (int e = 0; e < VN; e += 4) {
+      const float4 g = w ? *reinterpret_cast<const float4*>(w + e) : make_float4(1.f, 1.f, 1.f, 1.f);
+      f[e] = f[e] * factor * g.x * last; f[e + 1] = f[e + 1] * factor * g.y * last;
+      f[e + 2] = f[e + 2] * factor * g.z * last; f[e + 3] = f[e + 3] * factor * g.w * last;
+    }
+    return Vec<T>::pack(f);
+  };
+#pragma unroll
+  for (int i = 0; i < kRowVecs; ++i) {
+    const int j = tid + 256 * i;
+    if (j < qv) reinterpret_cast<V*>(q_out)[static_cast<size_t>(t) * qv + j] = scaled(xq[i], fq, q_w ? q_w + j * VN : nullptr, temp);
+    if (j < kv && page >= 0) {
+      const int g = j * VN / d, c = j * VN % d;
+      *reinterpret_cast<V*>(k_pool + (at + static_cast<size_t>(g) * page_size) * d + c) = scaled(xk[i], fk, k_w ? k_w + j * VN : nullptr, 1.f);
+    }
+  }
+}
+
 // rows [gate | up], each `inter` wide: g = min(gate, limit), u = clamp(up, -limit, limit),
 // out = g * sigmoid(alpha * g) * (u + 1)
 template <typename T>
@@ -900,6 +979,16 @@ extern "C" int b200_qk_rownorm_write(const void* qkv, int ld, void* q_out, const
   using namespace b200;
   if (n <= 0) return 0;
   if (nq <= 0 || nkv <= 0 || d <= 0 || dv <= 0 || page_size <= 0 || ld < nq * d + nkv * (d + dv)) return B200_ERR_BAD_SIZE;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_pool) |
+                         reinterpret_cast<uintptr_t>(v_pool) | reinterpret_cast<uintptr_t>(q_w) | reinterpret_cast<uintptr_t>(k_w)) & 15) == 0;
+  const int vn = dtype == kBF16 ? 8 : 4;        // whole 16-byte vectors in every row and head
+  if (aligned && (ld | d | dv) % vn == 0 && nq * d <= 256 * kRowVecs * vn && nkv * d <= 256 * kRowVecs * vn) {
+    B200_DISPATCH_DTYPE(dtype, T, launch(qk_rownorm_write_vec_kernel<T>, dim3(n), dim3(256), 0, stream, static_cast<const T*>(qkv), ld,
+                                         static_cast<T*>(q_out), q_w, k_w, eps, temp_coef, temp_every, positions, token_entry,
+                                         block_table, table_stride, page_size, static_cast<T*>(k_pool), static_cast<T*>(v_pool),
+                                         nq, nkv, d, dv));
+    return launch_status();
+  }
   B200_DISPATCH_DTYPE(dtype, T, launch(qk_rownorm_write_kernel<T>, dim3(n), dim3(256), 0, stream, static_cast<const T*>(qkv), ld,
                                        static_cast<T*>(q_out), q_w, k_w, eps, temp_coef, temp_every, positions, token_entry,
                                        block_table, table_stride, page_size, static_cast<T*>(k_pool), static_cast<T*>(v_pool),

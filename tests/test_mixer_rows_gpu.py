@@ -1,6 +1,8 @@
 """Kernels that prepare or finish rows of mixers, at the edges of what their vectors, warps and tiles of tokens hold, against
 64-bit arithmetic."""
 
+import math
+
 import pytest
 import torch
 
@@ -100,3 +102,79 @@ def test_group_norm_gate(dtype, n, groups, group, rank, act, divided):
     if rank:
         logits = logits @ up.double()
     close(out, y * (torch.sigmoid(logits) if act == "sigmoid" else logits * torch.sigmoid(logits)), tolerance(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,groups,group", [(1, 3, 8), (5, 300, 16), (3, 7, 6), (2, 32, 128)])
+def test_sigmoid_gate(dtype, n, groups, group):
+    from llm_runtime_study_b200.ops import mixer_steps as M
+
+    g = torch.Generator().manual_seed(n)
+    x, gate = torch.randn(n, groups * group, generator=g).to(dtype), torch.randn(n, groups + 5, generator=g).to(dtype)
+    out = M.sigmoid_gate(x.to(DEV), gate.to(DEV), gate_offset=3, group=group)
+    close(out, x.double() * torch.sigmoid(gate.double()[:, 3 : 3 + groups]).repeat_interleave(group, dim=1), tolerance(dtype))
+
+
+# rows of one vector a thread, of several with a ragged end, of more than the registers hold, heads that no vector divides; a row without pages
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq,nkv,d,dv", [(32, 8, 128, 128), (3, 1, 8, 16), (5, 5, 24, 40), (2, 1, 10, 8), (80, 4, 128, 64)])
+def test_qk_rownorm_write(dtype, nq, nkv, d, dv):
+    from llm_runtime_study_b200.ops import functional as F
+
+    g = torch.Generator().manual_seed(nq)
+    n, page = 5, 4
+    width = nq * d + nkv * (d + dv)
+    rows = torch.randn(n, width + (-width % 8), generator=g).to(dtype)
+    qw, kw = torch.randn(nq * d, generator=g), torch.randn(nkv * d, generator=g)
+    positions, entry = [0, 3, 4, 11, 2], [0, 0, 0, 1, 2]
+    table = torch.tensor([[2, 5, -1], [1, 0, 4], [-1, -1, -1]], dtype=torch.int32)
+    k_pool, v_pool = torch.zeros(6, nkv, page, d, dtype=dtype, device=DEV), torch.zeros(6, nkv, page, dv, dtype=dtype, device=DEV)
+    q = F.qk_rownorm_write(rows.to(DEV), num_q_heads=nq, num_kv_heads=nkv, head_dim=d, value_dim=dv, q_weight=qw.to(DEV), k_weight=kw.to(DEV),
+                           eps=1e-5, temp_coef=0.3, temp_every=4, positions=ints(positions), token_entry=ints(entry), block_table=table.to(DEV),
+                           page_size=page, k_pool=k_pool, v_pool=v_pool)
+    x = rows.double()
+    norm = lambda a, w: a / torch.sqrt(a.square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    temp = torch.tensor([1 + 0.3 * math.log((p + 1) // 4 + 1) for p in positions], dtype=torch.float64)
+    close(q.view(n, -1), norm(x[:, : nq * d], qw) * temp[:, None], tolerance(dtype))
+    keys, values = torch.zeros(6, nkv, page, d, dtype=torch.float64), torch.zeros(6, nkv, page, dv, dtype=torch.float64)
+    for t in range(4):
+        at = int(table[entry[t], positions[t] // page])
+        keys[at, :, positions[t] % page] = norm(x[t, nq * d : (nq + nkv) * d], kw).view(nkv, d)
+        values[at, :, positions[t] % page] = x[t, (nq + nkv) * d : width].view(nkv, dv)
+    close(k_pool, keys, tolerance(dtype))
+    assert torch.equal(v_pool.double().cpu(), values)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("q_rank,kv_rank,rot,dims", [(2048, 512, 64, 64), (8, 16, 8, 4), (1000, 40, 16, 0), (12, 6, 4, 2), (8200, 64, 0, 0), (520, 0, 0, 0)])
+def test_latent_prepare(dtype, q_rank, kv_rank, rot, dims):
+    from llm_runtime_study_b200.ops import mixer_steps as M
+
+    g = torch.Generator().manual_seed(q_rank)
+    n, page, q_off = 3, 4, 8
+    kv_off = q_off + q_rank + (-q_rank % 8)
+    width = kv_off + kv_rank + rot
+    rows = torch.randn(n, width + (-width % 8), generator=g).to(dtype)
+    qw, kw = torch.randn(q_rank, generator=g), torch.randn(max(kv_rank, 1), generator=g)
+    positions, entry = [1, 6, 3], [0, 0, 1]
+    table = torch.tensor([[2, 3], [-1, -1]], dtype=torch.int32)
+    freq = torch.rand(max(dims // 2, 1), generator=g)
+    pool = torch.zeros(4, page, max(kv_rank + rot, 1), dtype=dtype, device=DEV)
+    options = dict(kv_offset=kv_off, kv_rank=kv_rank, kv_weight=kw.to(DEV), rot=rot, pool=pool, block_table=table.to(DEV), page_size=page, rot_dims=dims,
+                   inv_freq=freq.to(DEV) if dims else None, interleaved=True, rot_factor=1.25) if kv_rank else {}
+    cq = M.latent_prepare(rows.to(DEV), q_offset=q_off, q_rank=q_rank, q_weight=qw.to(DEV), eps=1e-5, positions=ints(positions),
+                          token_entry=ints(entry), **options)
+    x = rows.double()
+    norm = lambda a, w: a / torch.sqrt(a.square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    close(cq, norm(x[:, q_off : q_off + q_rank], qw), tolerance(dtype))
+    if not kv_rank:
+        return
+    want = torch.zeros(4, page, kv_rank + rot, dtype=torch.float64)
+    for t in range(2):
+        turned = x[t, kv_off + kv_rank : kv_off + kv_rank + rot].clone()
+        for i in range(dims // 2):
+            a = positions[t] * float(freq[i])
+            u, v = float(turned[2 * i]), float(turned[2 * i + 1])
+            turned[2 * i], turned[2 * i + 1] = 1.25 * (u * math.cos(a) - v * math.sin(a)), 1.25 * (v * math.cos(a) + u * math.sin(a))
+        want[int(table[0, positions[t] // page]), positions[t] % page] = torch.cat((norm(x[t, kv_off : kv_off + kv_rank], kw), turned))
+    close(pool, want, tolerance(dtype))
