@@ -13,20 +13,31 @@ from .native import c_float, c_int, c_void_p, call, ptr, require, stream_ptr, ta
 native.register_library(
     "b200_scan_chunks", ("scan_chunks.cu",),
     {"b200_scan_chunks": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, *[c_void_p] * 12, *[c_int] * 7, c_float, c_int, c_int, c_void_p],
-     "b200_scan_chunks_record_floats": [c_int, c_int]},
+     "b200_scan_chunks_record_floats": [c_int, c_int],
+     "b200_scan_single": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, *[c_void_p] * 11, *[c_int] * 6, c_float, c_int, c_int, c_void_p]},
 )
 
 CHUNK_TOKENS, CHUNK_MAX_DIM = 16, 128     # tokens a chunk, largest key size of the chunked kernel
 CHUNK_MIN_TOKENS = 48                     # tokens beyond one per request from which a batch is scanned in chunks
+CHUNK_MAX_BYTES = 1 << 30                 # records of a launch at most (2,048 tokens of 32 heads of 128: 0.11 GB)
 
 
-def scans_in_chunks(n: int, entries: int, dim: int, fixed_order: bool) -> bool:
+def _record_bytes(n: int, entries: int, heads: int, dim: int) -> int:
+    """What the records of a batch take (the larger form, the delta rule's)."""
+
+    dim = 32 if dim <= 32 else (64 if dim <= 64 else 128)
+    return (n // CHUNK_TOKENS + entries) * heads * 4 * (3 * CHUNK_TOKENS * dim + 2 * CHUNK_TOKENS * CHUNK_TOKENS + dim)
+
+
+def scans_in_chunks(n: int, entries: int, heads: int, dim: int, fixed_order: bool) -> bool:
     """Whether a batch of ``n`` tokens of ``entries`` requests is scanned sixteen tokens at a time (``csrc/scan_chunks.cu``): batches
     with portions of prompts beside 16-bit activations.  With ``fixed_order`` a token's sums must not depend on where a step's
     chunks begin; single tokens have no chunk to share.  A chain takes 0.27 to 0.47 us a token, a chunk of sixteen 2.2 to 3 us behind
-    some 8 us for the records: from about 48 tokens on the chunks are ahead."""
+    some 8 us for the records: from about 48 tokens on the chunks are ahead.  Batches whose records would take more than a gigabyte
+    of memory are scanned token by token too."""
 
-    return not fixed_order and dim <= CHUNK_MAX_DIM and n - entries >= CHUNK_MIN_TOKENS
+    return (not fixed_order and dim <= CHUNK_MAX_DIM and n - entries >= CHUNK_MIN_TOKENS
+            and _record_bytes(n, entries, heads, dim) <= CHUNK_MAX_BYTES)
 
 
 def _scan_chunks(q, k, v, *, heads, qk_heads, dim, vdim, state, q_start, slots, out, gate=None, decay=None, row_decay=None, row_gain=None,
@@ -40,8 +51,23 @@ def _scan_chunks(q, k, v, *, heads, qk_heads, dim, vdim, state, q_start, slots, 
          heads, qk_heads, dim, vdim, 1 if silu else 0, float(q_scale), tag(q.dtype), tag(v.dtype), stream_ptr(), launches=2)
 
 
+def scans_single(n: int, entries: int, dim: int, vdim: int, fixed_order: bool) -> bool:
+    """Whether a batch of one token a request goes to the kernel that holds a head's state in a CTA's registers: whole 16-byte
+    columns, key sizes up to 128; faster at every batch from one request on (8 requests of 32 heads of 128: 7.9 us against 13.4).  (With
+    ``fixed_order`` a token's sums are those of the token-by-token kernel.)"""
+
+    return not fixed_order and n == entries and dim <= CHUNK_MAX_DIM and vdim % 4 == 0
+
+
+def _scan_single(q, k, v, *, heads, qk_heads, dim, vdim, state, q_start, slots, out, gate=None, decay=None, row_decay=None, row_gain=None,
+                 beta=None, norm_state=None, norm_out=None, silu=False, q_scale=1.0) -> None:
+    call("b200_scan_single", ptr(q), ptr(k), ptr(v), q.stride(0), k.stride(0), v.stride(0), ptr(gate), ptr(decay), ptr(row_decay),
+         ptr(row_gain), ptr(beta), ptr(state), ptr(norm_state), ptr(norm_out), ptr(out), ptr(q_start), ptr(slots), slots.shape[0], heads, qk_heads,
+         dim, vdim, 1 if silu else 0, float(q_scale), tag(q.dtype), tag(v.dtype), stream_ptr())
+
+
 def _chunk_form(q: torch.Tensor, v: torch.Tensor, gate, decay, beta) -> bool:
-    """Whether the chunked kernel has this form of the scan: what bfloat16 models run on prompts."""
+    """Whether the kernels for chunks and for single tokens have this form of the scan: what bfloat16 models run."""
 
     if beta is not None:
         return decay is None and q.dtype == v.dtype == torch.float32
@@ -90,7 +116,11 @@ def linear_scan(
     if beta is not None:
         require(beta, "beta", dtype=torch.float32, shape=(n, heads))
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
-    if scans_in_chunks(n, entries, dim, fixed_order) and _chunk_form(q, v, gate, decay, beta):
+    if _chunk_form(q, v, gate, decay, beta) and scans_single(n, entries, dim, vdim, fixed_order) and state.data_ptr() % 16 == 0:
+        _scan_single(q, k, v, heads=heads, qk_heads=qk_heads, dim=dim, vdim=vdim, state=state, q_start=q_start, slots=slots, out=out, gate=gate,
+                     decay=decay, row_decay=row_decay, beta=beta, silu=silu, q_scale=q_scale)
+        return out
+    if scans_in_chunks(n, entries, heads, dim, fixed_order) and _chunk_form(q, v, gate, decay, beta):
         _scan_chunks(q, k, v, heads=heads, qk_heads=qk_heads, dim=dim, vdim=vdim, state=state, q_start=q_start, slots=slots, out=out, gate=gate,
                      decay=decay, row_decay=row_decay, beta=beta, silu=silu, q_scale=q_scale)
         return out
@@ -126,7 +156,11 @@ def linear_scan_row_gates(
     require(slots, "slots", dtype=torch.int32, shape=(entries,))
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
     norm_out = torch.empty((n, heads), dtype=torch.float32, device=q.device)
-    if scans_in_chunks(n, entries, dim, fixed_order) and q.dtype == torch.bfloat16:
+    if q.dtype == torch.bfloat16 and scans_single(n, entries, dim, vdim, fixed_order) and state.data_ptr() % 16 == 0:
+        _scan_single(q, k, v, heads=heads, qk_heads=heads, dim=dim, vdim=vdim, state=state, q_start=q_start, slots=slots, out=out,
+                     row_decay=decay, row_gain=gain, norm_state=norm_state, norm_out=norm_out, q_scale=q_scale)
+        return out, norm_out
+    if scans_in_chunks(n, entries, heads, dim, fixed_order) and q.dtype == torch.bfloat16:
         _scan_chunks(q, k, v, heads=heads, qk_heads=heads, dim=dim, vdim=vdim, state=state, q_start=q_start, slots=slots, out=out,
                      row_decay=decay, row_gain=gain, norm_state=norm_state, norm_out=norm_out, q_scale=q_scale)
         return out, norm_out

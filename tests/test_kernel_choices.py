@@ -25,6 +25,12 @@ def test_projection_kernel_choice_at_the_benchmark_shapes():
     assert gemm_bf16.pick_kernel(384, 4096, 12288) == ("streamk", 256)
 
 
+def test_projections_to_few_columns():
+    for k in (2048, 3072, 4096):
+        assert gemm_bf16.pick_kernel(257, 1024, k) == gemm_bf16.pick_kernel(512, 1024, k) == ("splitk", 0)
+        assert gemm_bf16.pick_kernel(513, 1024, k) == gemm_bf16.pick_kernel(2048, 264, k) == ("persistent", 128)
+
+
 def test_decode_parts_are_bounded_and_use_the_gpu():
     for requests, kv_heads, longest, slots in itertools.product((1, 3, 8, 64, 500), (1, 8), (1, 100, 2048, 32768, 1 << 20), (296, 592)):
         parts = attention_bf16.decode_splits(requests, kv_heads, 1, longest, slots)
@@ -65,3 +71,14 @@ def test_split_k_shape_fills_the_sms_and_keeps_tiles_wide():
         assert width % 32 == 0 and 96 <= width <= 256 and splits in (1, 2, 4)
         assert -(-n // width) * splits <= 148 or splits == 1
         assert shape(128, n, k) == (width, splits)     # the choice does not depend on the rows that came along
+
+
+def test_which_scans_go_in_chunks():
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    assert S.scans_in_chunks(2048, 1, 32, 128, False) and S.scans_in_chunks(405, 25, 32, 128, False)
+    assert not S.scans_in_chunks(2048, 1, 32, 128, True)          # float32: sums that no cut changes
+    assert not S.scans_in_chunks(2048, 1, 32, 136, False) and not S.scans_in_chunks(40, 1, 32, 128, False)
+    assert not S.scans_in_chunks(1 << 20, 1, 32, 128, False)      # records of 57 GB
+    assert S.scans_single(8, 8, 128, 64, False) and not S.scans_single(9, 8, 128, 64, False)
+    assert not S.scans_single(8, 8, 128, 33, False) and not S.scans_single(8, 8, 129, 64, False) and not S.scans_single(8, 8, 128, 64, True)

@@ -1,4 +1,5 @@
-"""The scan of prompt portions sixteen tokens at a time against the token-by-token kernel and 64-bit arithmetic."""
+"""The scan of prompt portions sixteen tokens at a time, and of single tokens with a head's state in one CTA, against the
+token-by-token kernel and 64-bit arithmetic."""
 
 import pytest
 import torch
@@ -29,10 +30,12 @@ def _reference(q, k, v, lens, state, slots, *, decay, gain, beta):
 FORMS = ["head", "head_float_qk", "channel", "row", "delta_channel", "delta_token"]
 
 
-# portions around a chunk's edges, key sizes that fill 2, 4 and 8 warps and none, value columns around a block of 32
+# portions around a chunk's edges, key sizes that fill 2, 4 and 8 warps and none, value columns around a block of 32; single tokens
+# with value columns below, at and above the 128 that a CTA holds
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("heads,qk_heads,d,dv,lens", [(2, 2, 128, 128, [257]), (4, 2, 40, 33, [1, 15, 16, 17, 64]), (3, 3, 16, 8, [100, 31]),
-                                                      (1, 1, 72, 64, [49, 1])])
+                                                      (1, 1, 72, 64, [49, 1]),
+                                                      (4, 2, 128, 128, [1] * 5), (3, 3, 40, 36, [1]), (2, 1, 17, 132, [1, 1])])
 def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens):
     from llm_runtime_study_b200.ops import sequence_state as S
 
@@ -89,7 +92,7 @@ def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens):
     wide = wide.double()
     want, end = _reference(0.5 * wq, wk, wv, lens, state.double(), slots, decay=wide, gain=None if gain is None else gain.double(),
                            beta=None if beta is None else beta.double())
-    assert S.scans_in_chunks(n, len(lens), d, False)
+    assert S.scans_in_chunks(n, len(lens), heads, d, False) or S.scans_single(n, len(lens), d, dv, False)
     chunked, chained = run(False), run(True)
 
     def error(got, ref):
