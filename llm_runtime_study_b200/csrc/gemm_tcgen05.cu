@@ -327,11 +327,11 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_rows, con
 }
 
 // ------------------------------------------------------------------------ 2-CTA kernel
-// A pair of CTAs (a cluster of two, on neighbouring SMs) computes one 256 x 256 tile with
-// tcgen05.mma.cta_group::2.  Each CTA brings in 128 rows of A and 128 of the 256 weight rows per
-// 64-wide K block (32 KB instead of the 48 KB a CTA of the one-CTA kernel needs for the same
-// 128 x 256 outputs) and keeps its 128 x 256 half of the accumulator in its own TMEM; the tensor
-// core of the pair reads both halves of B.  Only the even CTA (the leader) issues MMAs.  Protocol
+// A pair of CTAs (a cluster of two, on neighbouring SMs) computes one 256 x BN tile with
+// tcgen05.mma.cta_group::2 (BN 256, or narrower where that fills the last round of tiles better: pair_width).
+// Each CTA brings in 128 rows of A and half of the BN weight rows per 64-wide K block (at BN = 256 32 KB instead
+// of the 48 KB a CTA of the one-CTA kernel needs for the same 128 x 256 outputs) and keeps its 128 x BN half of the
+// accumulator in its own TMEM; the tensor core of the pair reads both halves of B.  Only the even CTA (the leader) issues MMAs.  Protocol
 // per stage: both CTAs' TMA copies complete on the leader's `full` barrier (armed by the leader
 // for the bytes of both); the leader's commit arrives on `empty` in both CTAs.  Per tile: the
 // leader's commit arrives on `acc_full` in both CTAs; the eight epilogue warps of the pair arrive
@@ -380,10 +380,12 @@ __host__ __device__ constexpr uint32_t umma_idesc_pair(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
 }
 
-template <int STAGES, bool SWIGLU, typename OutT>
+template <int BN, int STAGES, bool SWIGLU, typename OutT>
 __global__ void __launch_bounds__(kThreads)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, GemmParams p) {
-  constexpr int BN = 256, HALF_N = 128, PAIR_M = 256;
+  // cta_group::2 with 256 rows takes widths in steps of 32; half a tile's weight rows are whole 8-row groups of the swizzle
+  static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "widths the pair's instruction takes");
+  constexpr int HALF_N = BN / 2, PAIR_M = 256, ACC = 256;      // ACC: columns of tensor memory a buffered accumulator starts after
   constexpr uint32_t ROW_BYTES = BM * BK * 2, COL_BYTES = HALF_N * BK * 2, STAGE_BYTES = ROW_BYTES + COL_BYTES;
   constexpr uint32_t TMEM_COLS = 512;
   extern __shared__ unsigned char smem_raw[];
@@ -456,7 +458,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __g
       const uint32_t acc_phase = (local >> 1) & 1;
       if (!mbar_wait_warp(acc_empty + buf, acc_phase ^ 1)) { atomicExch(&g_gemm_error, 4); ok = false; break; }
       tcgen05_fence_after();
-      const uint32_t tmem_d = tmem_base + buf * BN;
+      const uint32_t tmem_d = tmem_base + buf * ACC;
       for (int kb = 0; kb < num_kb; ++kb) {
         if (!mbar_wait_warp(full + s, phase)) { atomicExch(&g_gemm_error, 2); ok = false; break; }
         tcgen05_fence_after();
@@ -485,7 +487,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __g
       const bool ok = mbar_wait(acc_full + buf, acc_phase);
       if (!ok) atomicExch(&g_gemm_error, 3);
       tcgen05_fence_after();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * ACC;
       const int m = row0 + row;
       OutT* crow = static_cast<OutT*>(p.c) + static_cast<size_t>(m) * p.ldc;
 #pragma unroll 1
@@ -1097,14 +1099,35 @@ static int launch_splitk(const CUtensorMap& rows, const CUtensorMap& cols, GemmP
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 
-template <int STAGES, bool SWIGLU, typename OutT>
-static int launch_pair(const CUtensorMap& rows, const CUtensorMap& cols, const GemmParams& p, cudaStream_t stream) {
-  constexpr size_t smem = STAGES * (BM * BK * 2 + 128 * BK * 2) + 1024 + 256;
-  auto kernel = gemm_tcgen05_pair_kernel<STAGES, SWIGLU, OutT>;
+// Width of the pairs' tiles.  All pairs work on tiles of one width in rounds, and a round takes about as long as width + 64
+// columns would (192 K blocks of 405 x 4,096: 378 ns each at 256 columns).  256 unless a narrower width is at least 5 % ahead:
+// 405 x 24,576: 192 tiles of 256 columns are 2.6 rounds of 74 pairs, 220 of 224 columns 2.97; 405 x 4,096: 32 tiles of 256
+// columns leave most pairs idle, 64 of 128 do not.  Measured at the width chosen and at 256 columns: 405 x 24,576 x 4,096 73.6
+// and 76.4 us, 405 x 6,144 x 4,096 22.8 and 27.6, 405 x 4,096 x 12,288 52.2 and 72.5, 700 x 4,096 x 12,288 64.4 and 73.4,
+// 1,024 x 6,144 x 4,096 40.2 and 48.4, 1,024 x 24,576 x 4,096 137 and 154.  Shorter K ranges keep 256 columns: there a tile's start
+// and epilogue weigh more than the rounds that these widths save.
+static int pair_width(int M, int N, int K, int sm_count) {
+  if (K < 4096) return 256;
+  const int pairs = sm_count / 2 > 0 ? sm_count / 2 : 1, m_tiles = (M + 255) / 256;
+  auto cost = [&](int width) {
+    const long tiles = static_cast<long>(m_tiles) * ((N + width - 1) / width);
+    return (tiles + pairs - 1) / pairs * (width + 64);
+  };
+  int best = 256;
+  for (const int width : {224, 192, 128})
+    if (100 * cost(width) <= 95 * cost(256) && cost(width) < cost(best)) best = width;
+  return best;
+}
+
+template <int BN, bool SWIGLU, typename OutT>
+static int launch_pair_width(const CUtensorMap& rows, const CUtensorMap& cols, const GemmParams& p, cudaStream_t stream) {
+  constexpr int STAGES = BN == 128 ? 8 : (BN == 192 ? 7 : 6);      // 180 to 196 KB of operands in flight
+  constexpr size_t smem = STAGES * (BM * BK * 2 + BN / 2 * BK * 2) + 1024 + 256;
+  auto kernel = gemm_tcgen05_pair_kernel<BN, STAGES, SWIGLU, OutT>;
   static b200::DeviceOnce once;
   int sm_count = 0;
   if (int e = b200::configure_once(once, kernel, smem, &sm_count)) return e;
-  const int tiles = ((p.M + 255) / 256) * ((p.N + 255) / 256);
+  const int tiles = ((p.M + 255) / 256) * ((p.N + BN - 1) / BN);
   int pairs = sm_count / 2;
   if (tiles < pairs) pairs = tiles;
   cudaLaunchConfig_t config{};
@@ -1123,6 +1146,16 @@ static int launch_pair(const CUtensorMap& rows, const CUtensorMap& cols, const G
   config.numAttrs = pdl_enabled() ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&config, kernel, rows, cols, p);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+template <bool SWIGLU, typename OutT>
+static int launch_pair(const CUtensorMap& rows, const CUtensorMap& cols, const GemmParams& p, cudaStream_t stream) {
+  switch (p.bn) {
+    case 128: return launch_pair_width<128, SWIGLU, OutT>(rows, cols, p, stream);
+    case 192: return launch_pair_width<192, SWIGLU, OutT>(rows, cols, p, stream);
+    case 224: return launch_pair_width<224, SWIGLU, OutT>(rows, cols, p, stream);
+    default: return launch_pair_width<256, SWIGLU, OutT>(rows, cols, p, stream);
+  }
 }
 
 }  // namespace b200
@@ -1149,8 +1182,9 @@ extern "C" int b200_gemm_tcgen05_error() {
 //               128 x tile_n tile shared by a cluster of `splits` <= 8 CTAs; tile_n a multiple of 32 up to
 //               256; 0 for either: chosen from N and K so that the SMs are filled once; `stages`: depth of
 //               the operand ring, 0 = as deep as shared memory allows)
-//   tile_n      128 or 256 columns per tile (kind 0; the others take 256): narrower tiles put a product
-//               with few rows on more SMs
+//   tile_n      128 or 256 columns per tile (kind 0; kind 2 takes 256): narrower tiles put a product
+//               with few rows on more SMs; kind 1: 128, 192, 224 or 256, 0: chosen from M, N and K so that the
+//               rounds of tiles are full (b200_gemm_tcgen05_pair_width)
 //   partials, flags  stream-K only: b200_gemm_tcgen05_streamk_partial_floats() floats and
 //               b200_gemm_tcgen05_streamk_flags() 32-bit words that are zero before the first launch
 //               (the kernel leaves them zero); launches that share them must not overlap
@@ -1167,11 +1201,16 @@ extern "C" int b200_gemm_tcgen05_splitk_shape(int M, int N, int K, int sm_count,
   return 0;
 }
 
+// The width the pairs' tiles get for a product of M x N x K on a GPU with `sm_count` SMs (callable without a GPU).
+extern "C" int b200_gemm_tcgen05_pair_width(int M, int N, int K, int sm_count) {
+  return M > 0 && N > 0 && K > 0 ? pair_width(M, N, K, sm_count) : 0;
+}
+
 template <int KIND, int BN, bool SWIGLU, typename OutT>
 static int launch_kind(const CUtensorMap& rows, const CUtensorMap& cols, const GemmParams& p, cudaStream_t stream) {
   constexpr int STAGES = BN == 256 ? 4 : (BN == 128 ? 6 : 8);      // 192 KB of stages in every case
   if constexpr (KIND == 0) return launch_persistent<BN, STAGES, SWIGLU, OutT>(rows, cols, p, stream);
-  else if constexpr (KIND == 1) return launch_pair<6, SWIGLU, OutT>(rows, cols, p, stream);
+  else if constexpr (KIND == 1) return launch_pair<SWIGLU, OutT>(rows, cols, p, stream);
   else if constexpr (KIND == 3) return launch_splitk<SWIGLU, OutT>(rows, cols, p, stream);
   else return launch_streamk<BN, STAGES, SWIGLU, OutT>(rows, cols, p, stream);
 }
@@ -1190,17 +1229,24 @@ extern "C" int b200_gemm_tcgen05(const void* A, const void* W, const float* bias
                                  float* partials, unsigned* flags, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || K % 8 != 0 || ldc < (swiglu ? N / 2 : N) || (swiglu && N % 16 != 0) || swiglu < 0 || swiglu > ACT_GELU_TANH || kind < 0 || kind > 3) return B200_ERR_BAD_SIZE;
-  if (kind == 1) tile_n = 256;
-  if (kind != 3 && tile_n != 128 && tile_n != 256) return B200_ERR_BAD_SIZE;
+  if (kind == 1 ? (tile_n != 0 && tile_n != 128 && tile_n != 192 && tile_n != 224 && tile_n != 256)
+                : (kind != 3 && tile_n != 128 && tile_n != 256))
+    return B200_ERR_BAD_SIZE;
   if (accumulate && (!out_f32 || swiglu)) return B200_ERR_BAD_SIZE;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) return B200_ERR_BAD_SIZE;
   if (kind == 2 && (!partials || !flags || (reinterpret_cast<uintptr_t>(partials) & 15))) return 10004;
   GemmParams p{C, bias, M, N, K, ldc, (ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) ? 1 : 0, accumulate, partials, flags, splits, BM, tile_n, 0};
   p.gate_act = swiglu;
+  if (kind == 1 && tile_n == 0) {
+    int device = 0, sm_count = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
+    tile_n = p.bn = pair_width(M, N, K, sm_count);
+  }
   CUtensorMap rows, cols;
   if (int e = make_map(&rows, A, M, K, BM)) return e;
   if (kind != 3)
-    if (int e = make_map(&cols, W, N, K, kind == 1 ? 128 : tile_n)) return e;
+    if (int e = make_map(&cols, W, N, K, kind == 1 ? tile_n / 2 : tile_n)) return e;
   if (kind == 1) return launch_variant<1, 256>(rows, cols, p, out_f32, swiglu, stream);
   if (kind == 3) {
     int device = 0, sm_count = 0;

@@ -19,6 +19,7 @@ native.register_library(
         "b200_gemm_tcgen05_grouped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
                                       c_void_p],
         "b200_gemm_tcgen05_error": [],
+        "b200_gemm_tcgen05_pair_width": [c_int, c_int, c_int, c_int],
         "b200_gemm_tcgen05_splitk_shape": [c_int, c_int, c_int, c_int, c_void_p, c_void_p],
         "b200_gemm_tcgen05_streamk_partial_floats": [],
         "b200_gemm_tcgen05_streamk_flags": [],
@@ -68,8 +69,10 @@ def supported(m: int, n: int, k: int) -> bool:
 
 def pick_kernel(m: int, n: int, k: int) -> tuple[str, int]:
     """Which kernel and which tile width take a product of this shape (chosen from timings at the
-    Qwen3-8B layer widths with 128 to 4,096 rows).  Pairs of SMs on 256 x 256 tiles when those fill
-    most of the 74 pairs; one CTA per 128 x 256 tile when those cover half the SMs or more; up to
+    Qwen3-8B layer widths with 128 to 4,096 rows).  Pairs of SMs when 256 x 256 tiles fill
+    most of the 74 pairs, or 128 x 256 tiles half the SMs (their tiles are narrower where that fills the pairs better; with fewer
+    than 256 rows or K below 4,096 one CTA per 128 x 256 tile; 405 x 6,144 x 4,096: 22.8 us against 29.8, 700 x 4,096 x 4,096: 28.6 against 37.1), and
+    for a long K range that no kernel below shares (405 x 4,096 x 12,288: 52.2 us against 58.4 with 128-column tiles); up to
     256 rows and a third of the SMs: clusters that share a tile's K range (split-K, which chooses
     its own width); stream-K when a third of the SMs or fewer would have a tile and the K range is
     long enough to share; else one CTA per 128 x 128 tile.  A product with few tiles is as slow as
@@ -85,11 +88,13 @@ def pick_kernel(m: int, n: int, k: int) -> tuple[str, int]:
         return "pair", 256
     tiles = -(-m // 128) * -(-n // 256)
     if 2 * tiles >= sms:
-        return "persistent", 256
+        return ("pair" if m >= PAIR_MIN_ROWS and k >= 4096 and PAIR_ENABLED else "persistent"), 256
     if m <= 256 and 3 * tiles <= sms:
         return "splitk", 0
     if 3 * tiles <= sms + 2 and k >= 48 * 64:
         return "streamk", 256
+    if m > 384 and k >= 8192 and PAIR_ENABLED:
+        return "pair", 256
     return "persistent", 128
 
 
@@ -129,14 +134,15 @@ def gated_unit(swiglu: "bool | str") -> int:
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None,
            out_dtype: torch.dtype = torch.bfloat16, *, swiglu: "bool | str" = False, add_to: torch.Tensor | None = None,
-           kernel: str | None = None, tile_n: int | None = None, splits: int = 0, stages: int = 0) -> torch.Tensor:
+           kernel: str | None = None, tile_n: int | None = None, splits: int = 0, stages: int = 0, pair_width: int = 0) -> torch.Tensor:
     """``x @ weight.T (+ bias)`` on the tcgen05 tensor cores; float32 accumulation; bfloat16 or
     float32 output.
 
     ``swiglu``: the weight holds gate and up rows interleaved in blocks of eight and the result is
     ``silu(gate) * up``, half as wide (``"gelu_tanh"``: with that gate).  ``add_to`` (float32 ``[M, N]``): the product is added to it
     in place and it is returned.  ``kernel``: "persistent" (one CTA per tile of 128 rows and
-    ``tile_n`` = 128 or 256 columns), "pair" (two CTAs per 256 x 256 tile), "streamk" (few
+    ``tile_n`` = 128 or 256 columns), "pair" (two CTAs per tile of 256 rows and
+    ``pair_width`` = 128, 192, 224 or 256 columns; 0 lets the kernel choose so that its rounds of tiles are full), "streamk" (few
     tiles: up to three SMs share a tile's K range) or "splitk" (few rows: a cluster of ``splits``
     <= 8 CTAs shares the K range of every 128 x ``tile_n`` tile, ``tile_n`` a multiple of 32; 0 for either
     lets the kernel choose so that the SMs are filled once; ``stages``: depth of its operand ring, 0 = as
@@ -172,6 +178,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         if kernel not in KERNELS or tile_n not in (128, 256) or (tile_n == 128 and kernel != "persistent"):
             raise KernelError(f"unknown projection kernel {kernel!r} or tile width {tile_n}: expected one of {sorted(KERNELS)}, "
                               "256 columns, or 128 with the persistent kernel")
+    if kernel == "pair":
+        tile_n = pair_width
     partials, flags = _streamk_workspace(x.device) if kernel == "streamk" else (None, None)
     native.call("b200_gemm_tcgen05", x.data_ptr(), weight.data_ptr(), native.ptr(bias), out.data_ptr(), m, n, k,
                 out.shape[1], 1 if out_dtype == torch.float32 else 0, gated_unit(swiglu), 0 if add_to is None else 1,

@@ -25,6 +25,21 @@ def test_projection_kernel_choice_at_the_benchmark_shapes():
     assert gemm_bf16.pick_kernel(384, 4096, 12288) == ("streamk", 256)
 
 
+def test_widths_of_the_pairs_tiles():
+    """Rounds of tiles that are full or nearly so; 256 columns unless a narrower width is clearly ahead (host arithmetic)."""
+
+    from llm_runtime_study_b200.ops import native
+
+    width = lambda m, n, k=4096: native.query("b200_gemm_tcgen05_pair_width", m, n, k, 148)
+    assert all(width(2048, n) == 256 for n in (4096, 6144, 24576)) and width(8192, 12288) == 256
+    assert width(405, 24576) == 224 and width(405, 6144) == 192 and width(405, 4096) == 128 and width(1024, 6144) == 192
+    for m in (256, 300, 700, 1500):
+        for n in (16, 264, 5000, 151936):
+            assert width(m, n) in (128, 192, 224, 256) and width(m, n, 4088) == 256
+    assert gemm_bf16.pick_kernel(405, 6144, 4096) == gemm_bf16.pick_kernel(405, 4096, 12288) == ("pair", 256)
+    assert gemm_bf16.pick_kernel(405, 6144, 4088) == ("persistent", 256)
+
+
 def test_projections_to_few_columns():
     for k in (2048, 3072, 4096):
         assert gemm_bf16.pick_kernel(257, 1024, k) == gemm_bf16.pick_kernel(512, 1024, k) == ("splitk", 0)

@@ -704,6 +704,29 @@ def test_tcgen05_pair_projection(m, n, k, bias, out):
     assert torch.equal(got, again)
 
 
+# one tile, ragged edges in every dimension, a last tile of a few columns, several rounds of tiles
+@pytest.mark.parametrize("width", [128, 192, 224, 256])
+@pytest.mark.parametrize("m,n,k", [(256, 224, 64), (130, 464, 72), (405, 4112, 520), (700, 6160, 1000)])
+@pytest.mark.parametrize("form", ["bf16", "float", "add", "swiglu"])
+def test_tcgen05_pair_widths_give_the_same_bits(m, n, k, width, form):
+    """An output's sum runs over K in the same order whatever the tile's width: all widths give the bits of 256 columns."""
+
+    x, w, b, want = _gemm_case(m, n, k, True)
+    resid = torch.randn(m, n, generator=torch.Generator().manual_seed(5))
+
+    def run(columns):
+        if form == "add":
+            return _gemm().linear(dev(x), dev(w), dev(b), add_to=dev(resid.clone()), kernel="pair", pair_width=columns)
+        return _gemm().linear(dev(x), dev(w), dev(b), torch.float32 if form == "float" else torch.bfloat16, swiglu=form == "swiglu", kernel="pair",
+                              pair_width=columns)
+
+    got, wide = run(width), run(256)
+    _gemm().check_error()
+    assert torch.equal(got, wide) and bool(torch.isfinite(got).all())
+    if form == "float":
+        torch.testing.assert_close(got.cpu().double(), want, atol=2e-5 * float(want.abs().max()), rtol=0)
+
+
 @pytest.mark.parametrize("kernel", ["pair", "persistent"])
 @pytest.mark.parametrize("m,n,k", [(256, 256, 64), (300, 1000, 520), (2048, 4096, 4096)])
 def test_tcgen05_adds_to_the_residual(m, n, k, kernel):
