@@ -1104,10 +1104,11 @@ static int launch_splitk(const CUtensorMap& rows, const CUtensorMap& cols, GemmP
 // 405 x 24,576: 192 tiles of 256 columns are 2.6 rounds of 74 pairs, 220 of 224 columns 2.97; 405 x 4,096: 32 tiles of 256
 // columns leave most pairs idle, 64 of 128 do not.  Measured at the width chosen and at 256 columns: 405 x 24,576 x 4,096 73.6
 // and 76.4 us, 405 x 6,144 x 4,096 22.8 and 27.6, 405 x 4,096 x 12,288 52.2 and 72.5, 700 x 4,096 x 12,288 64.4 and 73.4,
-// 1,024 x 6,144 x 4,096 40.2 and 48.4, 1,024 x 24,576 x 4,096 137 and 154.  Shorter K ranges keep 256 columns: there a tile's start
-// and epilogue weigh more than the rounds that these widths save.
+// 1,024 x 6,144 x 4,096 40.2 and 48.4, 1,024 x 24,576 x 4,096 137 and 154.  640 x 8,192 x 2,048 22.3 and 26.6, 1,024 x 8,192 x 2,048
+// 26.4 and 28.1, 405 x 6,144 x 1,024 11.3 and 13.2, 1,024 x 6,144 x 1,024 15.4 and 18.0; 1,024 and 2,048 x 4,096 x 1,024 the same to
+// 1 %.  Shorter K ranges, not measured, keep 256 columns: there a tile's start and epilogue are most of its time.
 static int pair_width(int M, int N, int K, int sm_count) {
-  if (K < 4096) return 256;
+  if (K < 1024) return 256;
   const int pairs = sm_count / 2 > 0 ? sm_count / 2 : 1, m_tiles = (M + 255) / 256;
   auto cost = [&](int width) {
     const long tiles = static_cast<long>(m_tiles) * ((N + width - 1) / width);

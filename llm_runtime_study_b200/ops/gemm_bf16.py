@@ -71,7 +71,7 @@ def pick_kernel(m: int, n: int, k: int) -> tuple[str, int]:
     """Which kernel and which tile width take a product of this shape (chosen from timings at the
     Qwen3-8B layer widths with 128 to 4,096 rows).  Pairs of SMs when 256 x 256 tiles fill
     most of the 74 pairs, or 128 x 256 tiles half the SMs (their tiles are narrower where that fills the pairs better; with fewer
-    than 256 rows or K below 4,096 one CTA per 128 x 256 tile; 405 x 6,144 x 4,096: 22.8 us against 29.8, 700 x 4,096 x 4,096: 28.6 against 37.1), and
+    than 256 rows or K below 1,024 one CTA per 128 x 256 tile; 405 x 6,144 x 4,096: 22.8 us against 29.8, 700 x 4,096 x 4,096: 28.6 against 37.1), and
     for a long K range that no kernel below shares (405 x 4,096 x 12,288: 52.2 us against 58.4 with 128-column tiles); up to
     256 rows and a third of the SMs: clusters that share a tile's K range (split-K, which chooses
     its own width); stream-K when a third of the SMs or fewer would have a tile and the K range is
@@ -88,7 +88,7 @@ def pick_kernel(m: int, n: int, k: int) -> tuple[str, int]:
         return "pair", 256
     tiles = -(-m // 128) * -(-n // 256)
     if 2 * tiles >= sms:
-        return ("pair" if m >= PAIR_MIN_ROWS and k >= 4096 and PAIR_ENABLED else "persistent"), 256
+        return ("pair" if m >= PAIR_MIN_ROWS and k >= 1024 and PAIR_ENABLED else "persistent"), 256
     if m <= 256 and 3 * tiles <= sms:
         return "splitk", 0
     if 3 * tiles <= sms + 2 and k >= 48 * 64:

@@ -35,9 +35,9 @@ def test_widths_of_the_pairs_tiles():
     assert width(405, 24576) == 224 and width(405, 6144) == 192 and width(405, 4096) == 128 and width(1024, 6144) == 192
     for m in (256, 300, 700, 1500):
         for n in (16, 264, 5000, 151936):
-            assert width(m, n) in (128, 192, 224, 256) and width(m, n, 4088) == 256
+            assert width(m, n) in (128, 192, 224, 256) and width(m, n, 1016) == 256
     assert gemm_bf16.pick_kernel(405, 6144, 4096) == gemm_bf16.pick_kernel(405, 4096, 12288) == ("pair", 256)
-    assert gemm_bf16.pick_kernel(405, 6144, 4088) == ("persistent", 256)
+    assert gemm_bf16.pick_kernel(405, 6144, 1016) == ("persistent", 256)
 
 
 def test_projections_to_few_columns():
