@@ -4,9 +4,12 @@
 //
 // A CTA takes up to BM = 64 rows: consecutive query tokens of one request times the heads of one group of at most 64
 // heads.  Keys are streamed in tiles of 32 rows through shared memory (cp.async, two stages) from the request's pages.
-// Eight warps: warp w owns rows 16 (w & 3) .. + 15 and the value columns of half (w >> 2); both warps of a row group
-// form the same scores S = Q K^T (mma.sync m16n8k16, float accumulation), run the same online softmax in float32, round
-// P to bfloat16 and multiply it with their half of the value columns, read transposed out of the key tile.
+// Eight warps: warp w owns rows 16 (w & 3) .. + 15 and the value columns of half (w >> 2); the two warps of a row group
+// each form the scores S = Q K^T (mma.sync m16n8k16, float accumulation) of half of the tile's keys and exchange them through
+// shared memory (both forming all of them made that 70 % of a warp's products; rows of more than 868 columns leave no room for
+// the exchange and still do), run the same online softmax in float32, round P to bfloat16 and multiply it with their half of
+// the value columns, read transposed out of the key tile.  32 heads over rows of 576 columns, before the exchange and with it:
+// a prompt of 1,733 tokens 633 and 541 us, of 300 tokens 49.3 and 43.0, single tokens of 100 requests over 2,049 rows 264 and 213.
 // Key t is visible to a query at position p iff t <= p and (window == 0 or t > p - window).  With a sink every head's sum has
 // one more term exp(sink[head]), which belongs to no key.
 #include "common.cuh"
@@ -27,7 +30,9 @@ constexpr int LDS = DK + 8;                 // padded row: ldmatrix rows fall in
 constexpr int KSTEPS = DK / 16;
 constexpr int DVH = DV / 2;                 // value columns of one warp
 constexpr int OTILES = DVH / 8;
-constexpr int kSmemBytes = (BM + 2 * BN) * LDS * 2;
+constexpr int kTileBytes = (BM + 2 * BN) * LDS * 2, kExchangeBytes = NT * 32;    // eight scores a thread
+constexpr bool kShareScores = kTileBytes + kExchangeBytes <= 227 * 1024;        // else both warps form all scores
+constexpr int kSmemBytes = kTileBytes + (kShareScores ? kExchangeBytes : 0);
 
 struct LatentParams {
   const bf16* q;            // [n, heads, DK]
@@ -67,6 +72,7 @@ latent_attention_kernel(const LatentParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* qs = reinterpret_cast<bf16*>(smem_raw);
   bf16* ks = qs + BM * LDS;
+  float4* exchange = reinterpret_cast<float4*>(smem_raw + kTileBytes);      // [row group][half][2][lane]
   pdl_trigger();
   pdl_wait();
   const int tile = blockIdx.x, hgroup = blockIdx.y;
@@ -143,15 +149,41 @@ latent_attention_kernel(const LatentParams p) {
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
+    if constexpr (kShareScores) {
 #pragma unroll 4
-    for (int kk = 0; kk < KSTEPS; ++kk) {
-      uint32_t a[4], b[2][4];
-      ldmatrix_x4(a, qs + (rg * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDS + kk * 16 + (lane >> 4) * 8);
+      for (int kk = 0; kk < KSTEPS; ++kk) {          // s[0], s[1]: this warp's sixteen keys
+        uint32_t a[4], b[4];
+        ldmatrix_x4(a, qs + (rg * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDS + kk * 16 + (lane >> 4) * 8);
+        ldmatrix_x4(b, kcur + (half * 16 + (lane & 7) + (lane >> 4) * 8) * LDS + kk * 16 + ((lane >> 3) & 1) * 8);
+        mma_bf16(s[0], a, b[0], b[1]);
+        mma_bf16(s[1], a, b[2], b[3]);
+      }
+      float4* mine = exchange + (rg * 2 + half) * 64 + lane;
+      mine[0] = make_float4(s[0][0], s[0][1], s[0][2], s[0][3]);
+      mine[32] = make_float4(s[1][0], s[1][1], s[1][2], s[1][3]);
+      asm volatile("bar.sync %0, 64;\n" ::"r"(1 + rg) : "memory");       // the two warps of the row group
+      const float4* theirs = exchange + (rg * 2 + (half ^ 1)) * 64 + lane;
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
-        ldmatrix_x4(b[j], kcur + (j * 16 + (lane & 7) + (lane >> 4) * 8) * LDS + kk * 16 + ((lane >> 3) & 1) * 8);
+      for (int j = 0; j < 2; ++j) {
+        const float4 t = theirs[32 * j];
+        const float other[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) mma_bf16(s[j], a, b[j >> 1][(j & 1) * 2], b[j >> 1][(j & 1) * 2 + 1]);
+        for (int e = 0; e < 4; ++e) {
+          s[2 + j][e] = half ? s[j][e] : other[e];
+          s[j][e] = half ? other[e] : s[j][e];
+        }
+      }
+    } else {
+#pragma unroll 4
+      for (int kk = 0; kk < KSTEPS; ++kk) {
+        uint32_t a[4], b[2][4];
+        ldmatrix_x4(a, qs + (rg * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDS + kk * 16 + (lane >> 4) * 8);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          ldmatrix_x4(b[j], kcur + (j * 16 + (lane & 7) + (lane >> 4) * 8) * LDS + kk * 16 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_bf16(s[j], a, b[j >> 1][(j & 1) * 2], b[j >> 1][(j & 1) * 2 + 1]);
+      }
     }
     // mask, online softmax (base 2)
     float m_new[2] = {m[0], m[1]};

@@ -76,7 +76,7 @@ def latent_attention(q: torch.Tensor, pool: torch.Tensor, ctx: Any, table: torch
     out = torch.empty((n, heads, value_dim), dtype=q.dtype, device=q.device)
     splits, scratch, floats = 1, None, 0
     if decode:
-        splits = decode_splits(n, heads, min(window, ctx.max_kv_len) if window else ctx.max_kv_len)
+        splits = decode_splits(n, heads, min(window, ctx.max_kv_len) if window else ctx.max_kv_len, d)
         if splits > 1:
             floats = n * heads * splits * (value_dim + 2)
             scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
@@ -104,10 +104,15 @@ def _single_token_tiles(n: int, device) -> tuple[torch.Tensor, torch.Tensor, tor
     return kept[0][:n], kept[0][:n], kept[1][:n]
 
 
-def decode_splits(requests: int, heads: int, keys: int) -> int:
+def decode_splits(requests: int, heads: int, keys: int, width: int = 0) -> int:
     """Into how many parts a single token's keys are cut: enough CTAs for two a multiprocessor, no part shorter than four
-    tiles of 32 keys, at most 32 parts."""
+    tiles of 32 keys, at most 32 parts.  Rows of ``width`` columns whose tiles take more than half of the shared memory leave room for
+    one CTA: then no more CTAs than multiprocessors, since a second round costs as much as the first (32 requests of 32 heads over
+    777 rows of 576 columns: six parts were 192 CTAs in two rounds, four take one: 57.4 and 36.9 us with the merge)."""
 
     ctas = requests * -(-heads // ROWS_PER_TILE)
-    wanted = -(-2 * native.sm_count() // max(ctas, 1))
+    if (ROWS_PER_TILE + 64) * (width + 8) * 2 > MAX_SHARED_BYTES // 2:
+        wanted = native.sm_count() // max(ctas, 1)
+    else:
+        wanted = -(-2 * native.sm_count() // max(ctas, 1))
     return max(1, min(wanted, keys // 128, 32))

@@ -97,3 +97,21 @@ def test_which_scans_go_in_chunks():
     assert not S.scans_in_chunks(1 << 20, 1, 32, 128, False)      # records of 57 GB
     assert S.scans_single(8, 8, 128, 64, False) and not S.scans_single(9, 8, 128, 64, False)
     assert not S.scans_single(8, 8, 128, 33, False) and not S.scans_single(8, 8, 129, 64, False) and not S.scans_single(8, 8, 128, 64, True)
+
+
+def test_parts_of_a_single_tokens_keys_over_shared_rows(monkeypatch):
+    """Rows too wide for two CTAs a multiprocessor are cut into at most one round of CTAs, narrow ones into two."""
+
+    from llm_runtime_study_b200.ops import attention_latent
+
+    monkeypatch.setattr(attention_latent.native, "sm_count", lambda: 148)
+    for requests in (1, 2, 7, 8, 74, 75, 148, 149, 300):
+        for heads in (1, 32, 64, 65):
+            ctas = requests * -(-heads // 64)
+            wide = attention_latent.decode_splits(requests, heads, 1 << 20, 576)
+            narrow = attention_latent.decode_splits(requests, heads, 1 << 20, 80)
+            assert wide == 1 or wide == 32 or ctas * wide <= 148 < ctas * (wide + 1)
+            assert narrow == 32 or ctas * narrow >= 296 > ctas * (narrow - 1)
+            assert wide <= narrow
+    assert attention_latent.decode_splits(8, 32, 2049, 576) == 16
+    assert attention_latent.decode_splits(1, 32, 511, 576) == 3 and attention_latent.decode_splits(1, 32, 100, 576) == 1

@@ -194,6 +194,37 @@ def test_tensor_core_latent_attention(heads, rank, rot, page, window, q_lens):
         at += k
 
 
+@pytest.mark.parametrize("heads,rank,rot", [(7, 64, 16), (33, 512, 64), (3, 512, 384)])
+@pytest.mark.parametrize("single", [False, True])
+def test_latent_scores_formed_by_two_warps(heads, rank, rot, single):
+    """Sequences that end at every edge of a tile's two halves of 16 keys, with the widest rows (no room for the exchange of
+    scores) beside narrow ones.  A weight and a result are each rounded to bfloat16 once: 2^-9 of the largest value twice; the float32
+    sums over at most 896 columns add less than a tenth of that."""
+
+    from llm_runtime_study_b200.ops import attention_latent
+
+    torch.manual_seed(rank + rot)
+    lengths, d, page = [1, 15, 16, 17, 31, 32, 33, 49], rank + rot, 16
+    table, pages = _pages(rank, page, lengths)
+    rows = [(0.5 * torch.randn(m, d)).bfloat16() for m in lengths]
+    pool = torch.zeros(pages, page, d, dtype=torch.bfloat16)
+    for e, m in enumerate(lengths):
+        for t in range(m):
+            pool[table[e, t // page], t % page] = rows[e][t]
+    q_lens = [1] * len(lengths) if single else lengths
+    ctx, _, _ = _latent_ctx(lengths, q_lens)
+    q = (0.5 * torch.randn(sum(q_lens), heads, d)).bfloat16()
+    got = attention_latent.latent_attention(dev(q), dev(pool), ctx, dev(table), value_dim=rank, scale=0.1).cpu().double()
+    at = 0
+    for e, (m, k) in enumerate(zip(lengths, q_lens)):
+        full_q = torch.zeros(m, heads, d, dtype=torch.float64)
+        full_q[m - k:] = q[at:at + k].double()
+        keys = rows[e].double()[:, None, :]
+        want = plain.softmax_attention(full_q, keys, keys[:, :, :rank], scale=0.1, window=None)[m - k:]
+        assert (got[at:at + k] - want).abs().max() <= 1.1 * 2.0 ** -8 * float(rows[e].double().abs().max()), e
+        at += k
+
+
 def test_single_tokens_whose_keys_are_cut_into_parts():
     """Three requests of unequal length, one token each: the longest is cut into several parts and merged; a part may
     hold no visible key at all (the short request)."""
