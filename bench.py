@@ -1420,10 +1420,11 @@ def _fumolorn_kernels(peak, timed) -> dict:
         decay, gain, const = torch.rand(n, heads, device=dev), torch.rand(n, heads, device=dev), torch.full((heads,), 0.97, device=dev)
         gate, beta = 0.9 + 0.1 * torch.rand(n, vw, device=dev), torch.rand(n, heads, device=dev)
         moved = 2.0 * entries * heads * d * d * 4 + n * vw * 10
-        sizes = dict(heads=heads, qk_heads=heads, dim=d, vdim=d, state=state, q_start=q_start, slots=slots)
+        lens = [n // entries] * entries
+        sizes = dict(heads=heads, qk_heads=heads, dim=d, vdim=d, state=state, q_start=q_start, slots=slots, lens=lens)
         out[f"scan_row_gates_{n}_tokens_{entries}_requests"] = beside(
             lambda: S.linear_scan_row_gates(q, k, v, heads=heads, dim=d, vdim=d, decay=decay, gain=gain, state=state, norm_state=norm_state,
-                                            q_start=q_start, slots=slots, q_scale=d ** -0.5),
+                                            q_start=q_start, slots=slots, q_scale=d ** -0.5, lens=lens),
             lambda: S.linear_scan(q, k, v, **sizes, decay=const), moved + 8.0 * entries * heads * d, moved)
         out[f"scan_channel_decay_{n}_tokens_{entries}_requests"] = beside(
             lambda: S.linear_scan(q, k, v, **sizes, gate=gate, q_scale=d ** -0.5),
@@ -1629,7 +1630,7 @@ def _refolix_kernels(peak, timed) -> dict:
         const, row_decay = torch.full((heads,), 0.97, device=dev), 0.9 + 0.1 * torch.rand(n, heads, device=dev)
         gate, beta = 0.9 + 0.1 * torch.rand(n, vw, device=dev), torch.rand(n, heads, device=dev)
         states = 2.0 * entries * heads * d * d * 4
-        sizes = dict(heads=heads, qk_heads=heads, dim=d, vdim=d, state=state, q_start=q_start, slots=slots)
+        sizes = dict(heads=heads, qk_heads=heads, dim=d, vdim=d, state=state, q_start=q_start, slots=slots, lens=[n // entries] * entries)
         name = f"{n}_tokens_{entries}_requests"
         out[f"scan_retention_{name}"] = beside(
             lambda: S.linear_scan(q32, k32, v, **sizes, decay=const), lambda: S.linear_scan(q, k, v, **sizes, decay=const),

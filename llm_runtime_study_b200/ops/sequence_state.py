@@ -4,6 +4,8 @@ the read-out.  The state and everything that enters the recurrence are float32."
 
 from __future__ import annotations
 
+from typing import Sequence
+
 import torch
 
 from ..errors import KernelError
@@ -20,6 +22,16 @@ native.register_library(
 CHUNK_TOKENS, CHUNK_MAX_DIM = 16, 128     # tokens a chunk, largest key size of the chunked kernel
 CHUNK_MIN_TOKENS = 48                     # tokens beyond one per request from which a batch is scanned in chunks
 CHUNK_MAX_BYTES = 1 << 30                 # records of a launch at most (2,048 tokens of 32 heads of 128: 0.11 GB)
+
+
+def _lengths(lens: "Sequence[int] | None", n: int, entries: int) -> "Sequence[int] | None":
+    """The entries' lengths, checked; those of a single entry are known without being told."""
+
+    if lens is None:
+        return [n] if entries == 1 else None
+    if len(lens) != entries or sum(lens) != n or min(lens, default=0) < 0:
+        raise KernelError(f"{len(lens)} lengths that add up to {sum(lens)} do not describe {n} rows of {entries} entries")
+    return lens
 
 
 def _record_bytes(n: int, entries: int, heads: int, dim: int) -> int:
@@ -51,12 +63,14 @@ def _scan_chunks(q, k, v, *, heads, qk_heads, dim, vdim, state, q_start, slots, 
          heads, qk_heads, dim, vdim, 1 if silu else 0, float(q_scale), tag(q.dtype), tag(v.dtype), stream_ptr(), launches=2)
 
 
-def scans_single(n: int, entries: int, dim: int, vdim: int, fixed_order: bool) -> bool:
+def scans_single(n: int, entries: int, dim: int, vdim: int, fixed_order: bool, lens: "Sequence[int] | None" = None) -> bool:
     """Whether a batch of one token a request goes to the kernel that holds a head's state in a CTA's registers: whole 16-byte
     columns, key sizes up to 128; faster at every batch from one request on (8 requests of 32 heads of 128: 7.9 us against 13.4).  (With
-    ``fixed_order`` a token's sums are those of the token-by-token kernel.)"""
+    ``fixed_order`` a token's sums are those of the token-by-token kernel.)  The kernel takes row ``q_start[e]`` of every entry and
+    looks at no other, so as many tokens as requests is not enough: ``lens`` (the entries' lengths) must all be one."""
 
-    return not fixed_order and n == entries and dim <= CHUNK_MAX_DIM and vdim % 4 == 0
+    return (not fixed_order and n == entries and (lens is None or all(m == 1 for m in lens)) and dim <= CHUNK_MAX_DIM
+            and vdim % 4 == 0)
 
 
 def _scan_single(q, k, v, *, heads, qk_heads, dim, vdim, state, q_start, slots, out, gate=None, decay=None, row_decay=None, row_gain=None,
@@ -78,7 +92,7 @@ def linear_scan(
     q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, heads: int, qk_heads: int, dim: int, vdim: int,
     state: torch.Tensor, q_start: torch.Tensor, slots: torch.Tensor, gate: torch.Tensor | None = None,
     decay: torch.Tensor | None = None, beta: torch.Tensor | None = None, silu: bool = False, q_scale: float = 1.0,
-    fixed_order: bool = False, row_decay: torch.Tensor | None = None,
+    fixed_order: bool = False, row_decay: torch.Tensor | None = None, lens: "Sequence[int] | None" = None,
 ) -> torch.Tensor:
     """Per request (entry ``e`` owns rows ``q_start[e] .. q_start[e+1]-1`` and the state row ``slots[e]``) and head,
     token after token: ``S <- D S + k u^T``, ``o = S^T q`` with ``D`` the head's constant ``decay`` or the row's
@@ -89,7 +103,9 @@ def linear_scan(
     q is multiplied by ``q_scale`` then.  ``v`` may be bfloat16 beside float32 ``q`` and ``k`` (constant decay, no ``beta``).
     ``state`` is ``[slots, heads, dim, vdim]`` float32 and is updated in place.  ``fixed_order``: every sum is formed in
     an order that does not depend on the shape of the batch (the kernel otherwise spreads a column over more lanes when few
-    requests bring long portions), so a token's bits do not depend on the cut.  Returns float32 ``[N, heads * vdim]``."""
+    requests bring long portions), so a token's bits do not depend on the cut.  ``lens``: the entries' numbers of rows on the host
+    (what ``q_start`` holds on the device); known, they send batches of single tokens to a kernel of their own.  Returns
+    float32 ``[N, heads * vdim]``."""
 
     n = q.shape[0]
     for t, name, width in ((q, "q", qk_heads * dim), (k, "k", qk_heads * dim), (v, "v", heads * vdim)):
@@ -103,6 +119,7 @@ def linear_scan(
     require(q_start, "q_start", dtype=torch.int32, dims=1)
     entries = q_start.shape[0] - 1
     require(slots, "slots", dtype=torch.int32, shape=(entries,))
+    lens = _lengths(lens, n, entries)
     if sum(t is not None for t in (gate, decay, row_decay)) != 1:
         raise KernelError("linear_scan takes one of: gate factors per row and channel, one decay per row and head, one decay per head")
     if row_decay is not None:
@@ -116,7 +133,8 @@ def linear_scan(
     if beta is not None:
         require(beta, "beta", dtype=torch.float32, shape=(n, heads))
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
-    if _chunk_form(q, v, gate, decay, beta) and scans_single(n, entries, dim, vdim, fixed_order) and state.data_ptr() % 16 == 0:
+    if (lens and _chunk_form(q, v, gate, decay, beta) and scans_single(n, entries, dim, vdim, fixed_order, lens)
+            and state.data_ptr() % 16 == 0):
         _scan_single(q, k, v, heads=heads, qk_heads=qk_heads, dim=dim, vdim=vdim, state=state, q_start=q_start, slots=slots, out=out, gate=gate,
                      decay=decay, row_decay=row_decay, beta=beta, silu=silu, q_scale=q_scale)
         return out
@@ -133,12 +151,13 @@ def linear_scan(
 def linear_scan_row_gates(
     q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, heads: int, dim: int, vdim: int, decay: torch.Tensor, gain: torch.Tensor,
     state: torch.Tensor, norm_state: torch.Tensor, q_start: torch.Tensor, slots: torch.Tensor, q_scale: float = 1.0,
-    fixed_order: bool = False,
+    fixed_order: bool = False, lens: "Sequence[int] | None" = None,
 ) -> tuple[torch.Tensor, torch.Tensor]:
     """``linear_scan`` with one decay and one input gain per row and head, and a normaliser: ``S <- decay S + gain k v^T``,
     ``n <- decay n + gain k``; returns ``S^T q`` float32 ``[N, heads * vdim]`` and ``n . q`` float32 ``[N, heads]`` (q times
     ``q_scale`` as it is read).  ``state`` ``[slots, heads, dim, vdim]`` and ``norm_state`` ``[slots, heads, dim]`` float32 are
-    updated in place; ``decay`` and ``gain`` are float32 ``[N, heads]``.  ``fixed_order`` as for ``linear_scan``."""
+    updated in place; ``decay`` and ``gain`` are float32 ``[N, heads]``.  ``fixed_order`` and ``lens`` as for
+    ``linear_scan``."""
 
     n = q.shape[0]
     for t, name, width in ((q, "q", heads * dim), (k, "k", heads * dim), (v, "v", heads * vdim)):
@@ -154,9 +173,10 @@ def linear_scan_row_gates(
     require(q_start, "q_start", dtype=torch.int32, dims=1)
     entries = q_start.shape[0] - 1
     require(slots, "slots", dtype=torch.int32, shape=(entries,))
+    lens = _lengths(lens, n, entries)
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
     norm_out = torch.empty((n, heads), dtype=torch.float32, device=q.device)
-    if q.dtype == torch.bfloat16 and scans_single(n, entries, dim, vdim, fixed_order) and state.data_ptr() % 16 == 0:
+    if lens and q.dtype == torch.bfloat16 and scans_single(n, entries, dim, vdim, fixed_order, lens) and state.data_ptr() % 16 == 0:
         _scan_single(q, k, v, heads=heads, qk_heads=heads, dim=dim, vdim=vdim, state=state, q_start=q_start, slots=slots, out=out,
                      row_decay=decay, row_gain=gain, norm_state=norm_state, norm_out=norm_out, q_scale=q_scale)
         return out, norm_out

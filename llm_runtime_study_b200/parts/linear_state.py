@@ -67,7 +67,7 @@ class DecayedLinearAttention(Mixer):
         out = S.linear_scan(
             proj[:, :qk], proj[:, qk : 2 * qk], proj[:, 2 * qk : 2 * qk + vw], heads=self.num_heads, qk_heads=self.num_heads,
             dim=self.head_dim, vdim=self.value_dim, state=cache.state, q_start=ctx.q_start, slots=ctx.slots, decay=self.decays,
-            silu=True, fixed_order=self.runtime.dtype == torch.float32,
+            silu=True, fixed_order=self.runtime.dtype == torch.float32, lens=ctx.q_lens,
         )
         gated = S.group_norm_gate(out, self.norm_weight, self.eps, proj, gate_offset=2 * qk + vw, out_dtype=self.runtime.dtype)
         return self.o_proj(gated, torch.float32)
@@ -166,6 +166,7 @@ class GatedDeltaRule(Mixer):
             q, k, v, heads=self.num_heads, qk_heads=self.num_qk_heads, dim=self.head_dim, vdim=self.value_dim,
             state=cache.states["state"], q_start=ctx.q_start, slots=ctx.slots, gate=None if per_head else g,
             row_decay=g if per_head else None, beta=beta, fixed_order=self.runtime.dtype == torch.float32,
+            lens=ctx.q_lens,
         )
         gated = S.group_norm_gate(out, self.norm_weight, self.eps, proj, gate_offset=gate_offset, gate_up=self.g_up,
                                   act=self.gate_act, out_dtype=self.runtime.dtype)
@@ -219,7 +220,7 @@ class Retention(Mixer):
                            rotary=self.position.rotary_layout() if self.position is not None else None)
         out = S.linear_scan(
             q, k, proj[:, 2 * H * d : H * (2 * d + dv)], heads=H, qk_heads=H, dim=d, vdim=dv, state=cache.state, q_start=ctx.q_start,
-            slots=ctx.slots, decay=self.decays, fixed_order=self.runtime.dtype == torch.float32,
+            slots=ctx.slots, decay=self.decays, fixed_order=self.runtime.dtype == torch.float32, lens=ctx.q_lens,
         )
         gated = S.group_norm_gate(out, None, self.eps, proj, gate_offset=H * (2 * d + dv), group=dv, act="silu", out_dtype=self.runtime.dtype)
         return self.o_proj(gated, torch.float32)
@@ -270,7 +271,7 @@ class GatedLinearAttention(Mixer):
         out = S.linear_scan(
             proj[:, :qk], proj[:, qk : 2 * qk], proj[:, 2 * qk : 2 * qk + vw], heads=self.num_heads, qk_heads=self.num_heads,
             dim=self.head_dim, vdim=self.value_dim, state=cache.state, q_start=ctx.q_start, slots=ctx.slots, gate=alpha,
-            q_scale=self.head_dim ** -0.5, fixed_order=self.runtime.dtype == torch.float32,
+            q_scale=self.head_dim ** -0.5, fixed_order=self.runtime.dtype == torch.float32, lens=ctx.q_lens,
         )
         gated = S.group_norm_gate(out, self.norm_weight, self.eps, proj, gate_offset=2 * qk + vw, act="silu", out_dtype=self.runtime.dtype)
         return self.o_proj(gated, torch.float32)
@@ -330,7 +331,7 @@ class MatrixMemory(Mixer):
         out, den = S.linear_scan_row_gates(
             proj[:, :qk], proj[:, qk : 2 * qk], proj[:, 2 * qk : 2 * qk + vw], heads=H, dim=self.head_dim, vdim=self.value_dim,
             decay=decay, gain=gain, state=cache.states["state"], norm_state=cache.states["normaliser"], q_start=ctx.q_start,
-            slots=ctx.slots, q_scale=self.head_dim ** -0.5, fixed_order=self.runtime.dtype == torch.float32,
+            slots=ctx.slots, q_scale=self.head_dim ** -0.5, fixed_order=self.runtime.dtype == torch.float32, lens=ctx.q_lens,
         )
         gated = S.group_norm_gate(out, self.norm_weight, self.eps, proj, gate_offset=2 * qk + vw, group=self.value_dim,
                                   divisor=(den, floor, self.NORMALISER_EPS), out_dtype=self.runtime.dtype)

@@ -96,6 +96,7 @@ def test_which_scans_go_in_chunks():
     assert not S.scans_in_chunks(2048, 1, 32, 136, False) and not S.scans_in_chunks(40, 1, 32, 128, False)
     assert not S.scans_in_chunks(1 << 20, 1, 32, 128, False)      # records of 57 GB
     assert S.scans_single(8, 8, 128, 64, False) and not S.scans_single(9, 8, 128, 64, False)
+    assert S.scans_single(3, 3, 128, 64, False, [1, 1, 1]) and not S.scans_single(3, 3, 128, 64, False, [0, 2, 1])   # as many rows, another cut
     assert not S.scans_single(8, 8, 128, 33, False) and not S.scans_single(8, 8, 129, 64, False) and not S.scans_single(8, 8, 128, 64, True)
 
 

@@ -31,11 +31,12 @@ FORMS = ["head", "head_float_qk", "channel", "row", "delta_channel", "delta_toke
 
 
 # portions around a chunk's edges, key sizes that fill 2, 4 and 8 warps and none, value columns around a block of 32; single tokens
-# with value columns below, at and above the 128 that a CTA holds
+# with value columns below, at and above the 128 that a CTA holds; as many tokens as requests, but not one each
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("heads,qk_heads,d,dv,lens", [(2, 2, 128, 128, [257]), (4, 2, 40, 33, [1, 15, 16, 17, 64]), (3, 3, 16, 8, [100, 31]),
                                                       (1, 1, 72, 64, [49, 1]),
-                                                      (4, 2, 128, 128, [1] * 5), (3, 3, 40, 36, [1]), (2, 1, 17, 132, [1, 1])])
+                                                      (4, 2, 128, 128, [1] * 5), (3, 3, 40, 36, [1]), (2, 1, 17, 132, [1, 1]),
+                                                      (2, 2, 128, 128, [2, 0]), (4, 2, 40, 36, [0, 3, 0]), (2, 1, 17, 132, [1, 0, 0, 3])])
 def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens):
     from llm_runtime_study_b200.ops import sequence_state as S
 
@@ -77,7 +78,7 @@ def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens):
     def run(fixed_order):
         s, ns = dev(state), dev(norm_state)
         common = dict(heads=heads, dim=d, vdim=dv, state=s, q_start=q_start, slots=torch.tensor(slots, dtype=torch.int32, device=DEV),
-                      fixed_order=fixed_order, q_scale=0.5, **{key: dev(x) for key, x in options.items()})
+                      fixed_order=fixed_order, q_scale=0.5, lens=lens, **{key: dev(x) for key, x in options.items()})
         # rows of a wider projection: strides of their own
         rows = [dev(torch.cat((x, x), dim=1))[:, : x.shape[1]] for x in (q, k, v)]
         if form == "row":
@@ -92,7 +93,8 @@ def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens):
     wide = wide.double()
     want, end = _reference(0.5 * wq, wk, wv, lens, state.double(), slots, decay=wide, gain=None if gain is None else gain.double(),
                            beta=None if beta is None else beta.double())
-    assert S.scans_in_chunks(n, len(lens), heads, d, False) or S.scans_single(n, len(lens), d, dv, False)
+    one_each = all(m == 1 for m in lens)
+    assert S.scans_in_chunks(n, len(lens), heads, d, False) or S.scans_single(n, len(lens), d, dv, False, lens) == one_each
     chunked, chained = run(False), run(True)
 
     def error(got, ref):
@@ -108,6 +110,31 @@ def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens):
         # of 16-bit rows takes the hardware's exponential (2 units in the last place), in either kernel
         assert error(chunked[i], ref) < 2e-6, (i, error(chunked[i], ref), error(chained[i], ref))
         assert error(chunked[i], ref) < 1.5 * error(chained[i], ref) + 1e-7
+
+
+def test_as_many_rows_as_requests_are_single_tokens_only_when_the_lengths_say_so():
+    """Without lengths any cut of ``q_start`` is served, empty requests included; lengths that do not fit are refused."""
+
+    from llm_runtime_study_b200.errors import KernelError
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    heads, d = 2, 32
+    g = torch.Generator().manual_seed(3)
+    q, k, v = (torch.randn(3, heads * d, generator=g).bfloat16() for _ in range(3))
+    begin = 0.3 * torch.randn(3, heads, d, d, generator=g)
+    decay = torch.tensor([0.9, 0.8])
+    for lens in ([0, 2, 1], [3, 0, 0], [1, 1, 1]):
+        state = begin.to(DEV)
+        first = [sum(lens[:i]) for i in range(4)]
+        args = dict(heads=heads, qk_heads=heads, dim=d, vdim=d, q_start=torch.tensor(first, dtype=torch.int32, device=DEV),
+                    slots=torch.arange(3, dtype=torch.int32, device=DEV), decay=decay.to(DEV))
+        out = S.linear_scan(q.to(DEV), k.to(DEV), v.to(DEV), state=state, **args)
+        rows = [x.double().view(3, heads, d) for x in (q, k, v)]
+        want, end = _reference(*rows, lens, begin.double(), range(3), decay=decay.double()[None, :, None].expand(3, heads, d), gain=None, beta=None)
+        assert float((out.double().cpu() - want.reshape(3, -1)).norm() / want.norm()) < 1e-6       # a few float32 roundings
+        assert float((state.double().cpu() - end).norm() / end.norm()) < 1e-6
+        with pytest.raises(KernelError, match="lengths"):
+            S.linear_scan(q.to(DEV), k.to(DEV), v.to(DEV), state=state, lens=lens[:2], **args)
 
 
 def test_a_bad_row_reaches_later_tokens_only():
