@@ -81,6 +81,33 @@ def test_delta_prepare_tiles_of_tokens(dtype, heads, qk_heads, d, dv, taps, rank
 
 # groups a warp holds (whole, partly idle lanes, many and few rows), whole rows, and groups no vector divides
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+def test_delta_prepare_keeps_bad_rows_within_the_taps_reach(dtype, taps):
+    """An infinite or NaN row reaches the tokens whose taps meet it and no others, wherever it lies in a tile of tokens."""
+
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    heads, d, n = 32, 16, 200
+    g = torch.Generator().manual_seed(taps)
+    channels, bad = 3 * heads * d, {0: math.inf, 35: math.nan, 64: -math.inf, 110: math.inf, 199: math.nan}
+    proj = torch.randn(n, channels + 2 * heads, generator=g)
+    for row, value in bad.items():
+        proj[row, :channels] = value
+    q, k, v, decay, beta = S.delta_prepare(
+        proj.to(dtype).to(DEV), heads=heads, qk_heads=heads, dim=d, vdim=d, beta_offset=channels, low_offset=channels + heads, rank=0,
+        taps=torch.randn(channels, taps, generator=g).to(DEV), conv_state=torch.zeros(1, taps - 1, channels, device=DEV),
+        a_log=torch.zeros(heads, device=DEV), dt_bias=torch.zeros(heads, device=DEV), a_up=None, q_start=ints([0, n]), slots=ints([0]),
+        token_entry=ints([0] * n), unit_eps=1e-6, q_scale=1.0)
+    assert n * heads >= 16 * 2 * 148                # sixteen tokens a CTA
+    reached = torch.zeros(n, dtype=torch.bool)
+    for row in bad:
+        reached[row : row + taps] = True
+    for name, x in (("q", q), ("k", k), ("v", v)):
+        assert torch.equal(torch.isfinite(x).all(dim=1).cpu(), ~reached), name
+    assert not bool(torch.isfinite(v[reached.to(DEV)]).any()) and bool(torch.isfinite(decay).all()) and bool(torch.isfinite(beta).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("n,groups,group,rank", [(300, 32, 128, 32), (3, 5, 128, 7), (257, 40, 36, 0), (2, 1, 4096, 0), (5, 3, 260, 0), (4, 2, 30, 3), (1, 4, 4, 1)])
 @pytest.mark.parametrize("act,divided", [("sigmoid", False), ("silu", True)])
 def test_group_norm_gate(dtype, n, groups, group, rank, act, divided):
