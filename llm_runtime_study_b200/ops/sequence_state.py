@@ -20,8 +20,9 @@ native.register_library(
 )
 
 CHUNK_TOKENS, CHUNK_MAX_DIM = 16, 128     # tokens a chunk, largest key size of the chunked kernel
-CHUNK_MIN_TOKENS = 48                     # tokens beyond one per request from which a batch is scanned in chunks
+CHUNK_MIN_TOKENS = 48                     # tokens beyond one per request from which a batch may be scanned in chunks
 CHUNK_MAX_BYTES = 1 << 30                 # records of a launch at most (2,048 tokens of 32 heads of 128: 0.11 GB)
+MOST_RUNS = 4                             # launches a batch of long and short portions is cut into at most
 
 
 def _lengths(lens: "Sequence[int] | None", n: int, entries: int) -> "Sequence[int] | None":
@@ -42,20 +43,96 @@ def _record_bytes(n: int, entries: int, heads: int, dim: int) -> int:
 
 
 def scans_in_chunks(n: int, entries: int, heads: int, dim: int, fixed_order: bool) -> bool:
-    """Whether a batch of ``n`` tokens of ``entries`` requests is scanned sixteen tokens at a time (``csrc/scan_chunks.cu``): batches
-    with portions of prompts beside 16-bit activations.  With ``fixed_order`` a token's sums must not depend on where a step's
-    chunks begin; single tokens have no chunk to share.  A chain takes 0.27 to 0.47 us a token, a chunk of sixteen 2.2 to 3 us behind
-    some 8 us for the records: from about 48 tokens on the chunks are ahead.  Batches whose records would take more than a gigabyte
-    of memory are scanned token by token too."""
+    """Whether a batch of ``n`` tokens of ``entries`` requests can hold portions that are scanned sixteen tokens at a time
+    (``csrc/scan_chunks.cu``; ``portion_in_chunks`` says which): batches with portions of prompts beside 16-bit activations.  With
+    ``fixed_order`` a token's sums must not depend on where a step's chunks begin.  Batches whose records would take more than a
+    gigabyte of memory are scanned token by token."""
 
     return (not fixed_order and dim <= CHUNK_MAX_DIM and n - entries >= CHUNK_MIN_TOKENS
             and _record_bytes(n, entries, heads, dim) <= CHUNK_MAX_BYTES)
 
 
-def _scan_chunks(q, k, v, *, heads, qk_heads, dim, vdim, state, q_start, slots, out, gate=None, decay=None, row_decay=None, row_gain=None,
+def portion_in_chunks(lens: "Sequence[int]", heads: int, dim: int, columns: int, delta: bool) -> int:
+    """The number of tokens from which a portion of a batch is scanned in chunks (0: none is); ``columns``: of a head's state.
+
+    A chunk costs about 2.2 us behind some 8 us for the records; a token of a chain 0.2 us as long as the chains' CTAs of 8 columns
+    all run at once, two an SM, and 0.3 to 0.5 us beyond that.  A chunk takes the same 0.06 us a head (0.13 with the
+    delta rule) whether it holds sixteen tokens or one.  So what counts is the portion's own length, not the batch's.  Microseconds in
+    chunks and as a chain, 128 x 128: 4 heads, one portion of 64 tokens 21.6, 22.8 (delta rule, a decay per channel 28.3, 24.6), of 96
+    26.4, 31.3 (34.4, 32.8); 16 heads, 64 tokens 23.5, 24.8 (29.6, 28.7), 96 tokens 27.6, 34.8 (35.8, 39.6); 32 heads, eight of 24 48, 55 (83, 74), two of
+    48 25.8, 42.3 (39.9, 57.3), eight of 48 60.4, 98.3 (112, 129), 64 of 2 206, 90 (404, 107).  With key sizes up to 64 and enough chains to
+    fill the GPU with CTAs of 32 columns a chain is as fast or faster at any length (8 heads of 64, 64 portions of 64: 62.4, 53.3;
+    96.2, 65.5).  Few chains beside requests of another kernel pay for that launch too (4 heads, 64 tokens beside one token: 26, 23)."""
+
+    sms = native.sm_count()
+    if not delta and dim > 64:                 # many portions, each as long as two chunks or nearly
+        short = sum(m >= 24 for m in lens)
+        if short >= 4 and short * heads * -(-columns // 8) > 4 * sms:
+            return 24
+    long = sum(m >= 48 for m in lens)
+    if not long or (dim <= 64 and long * heads * -(-columns // 32) >= 2 * sms):
+        return 0
+    ctas = long * heads * -(-columns // 8)
+    if ctas > 2 * sms:
+        return 48
+    if ctas <= sms and long < len(lens):
+        return 128 if delta else 96
+    return 96 if delta else 64
+
+
+def scan_runs(lens: "Sequence[int]", least: int) -> "list[tuple[str, int, int]]":
+    """A batch as runs of neighbouring requests, ``(kind, first, last + 1)``: "chunks" for portions of ``least`` tokens and more,
+    "single" for requests of one token each, "chain" for all others.  More than two runs are for portions of 128 tokens and more only
+    (16 heads, requests of 1, 1, 1, 1, 60, 3 and 60 tokens: 49 us in four launches, 45 in one), and more than four are one chain."""
+
+    runs: list[tuple[str, int, int]] = []
+    at = 0
+
+    def others(last: int) -> None:
+        if at < last:
+            runs.append(("single" if min(lens[at:last]) == max(lens[at:last]) == 1 else "chain", at, last))
+
+    for i in [i for i, m in enumerate(lens) if m >= least] if least else ():
+        if runs and runs[-1][0] == "chunks" and at == i:
+            runs[-1] = ("chunks", runs[-1][1], i + 1)
+        else:
+            others(i)
+            runs.append(("chunks", i, i + 1))
+        at = i + 1
+    others(len(lens))
+    if len(runs) > 2 and least < 128:
+        return scan_runs(lens, 128)
+    return runs if len(runs) <= MOST_RUNS else [("chain", 0, len(lens))]
+
+
+def _scan_plan(lens, n: int, entries: int, heads: int, dim: int, vdim: int, columns: int, delta: bool, fixed_order: bool):
+    """The kernels of a batch, as ``scan_runs`` names them, with what is left of its choice: single tokens whose sizes their kernel
+    does not take are chains.  Lengths that are not known are taken for equal ones, none of them for single tokens."""
+
+    least = 0
+    if scans_in_chunks(n, entries, heads, dim, fixed_order):
+        least = portion_in_chunks(lens if lens else [n // entries] * entries, heads, dim, columns, delta)
+    if not lens:
+        return [("chunks" if least and n >= least * entries else "chain", 0, entries)]
+    singles = scans_single(1, 1, dim, vdim, fixed_order)
+    return [("chain" if kind == "single" and not singles else kind, first, last) for kind, first, last in scan_runs(lens, least)]
+
+
+def _parts(plan, lens, n: int):
+    """The runs of a plan with their numbers of rows and of chunks (without lengths: at most so many, every request's last chunk
+    may be short)."""
+
+    for kind, first, last in plan:
+        if lens:
+            mine = lens[first:last]
+            yield kind, first, last, sum(mine), sum(-(-m // CHUNK_TOKENS) for m in mine)
+        else:
+            yield kind, first, last, n, n // CHUNK_TOKENS + last - first
+
+
+def _scan_chunks(q, k, v, *, chunks, heads, qk_heads, dim, vdim, state, q_start, slots, out, gate=None, decay=None, row_decay=None, row_gain=None,
                  beta=None, norm_state=None, norm_out=None, silu=False, q_scale=1.0) -> None:
-    n, entries = q.shape[0], slots.shape[0]
-    chunks = n // CHUNK_TOKENS + entries          # every request's last chunk may be short
+    entries = slots.shape[0]
     floats = native.query("b200_scan_chunks_record_floats", dim, 0 if beta is None else 1)
     records = torch.empty(chunks * heads * floats, dtype=torch.float32, device=q.device)
     call("b200_scan_chunks", ptr(q), ptr(k), ptr(v), q.stride(0), k.stride(0), v.stride(0), ptr(gate), ptr(decay), ptr(row_decay),
@@ -64,7 +141,7 @@ def _scan_chunks(q, k, v, *, heads, qk_heads, dim, vdim, state, q_start, slots, 
 
 
 def scans_single(n: int, entries: int, dim: int, vdim: int, fixed_order: bool, lens: "Sequence[int] | None" = None) -> bool:
-    """Whether a batch of one token a request goes to the kernel that holds a head's state in a CTA's registers: whole 16-byte
+    """Whether requests of one token each go to the kernel that holds a head's state in a CTA's registers: whole 16-byte
     columns, key sizes up to 128; faster at every batch from one request on (8 requests of 32 heads of 128: 7.9 us against 13.4).  (With
     ``fixed_order`` a token's sums are those of the token-by-token kernel.)  The kernel takes row ``q_start[e]`` of every entry and
     looks at no other, so as many tokens as requests is not enough: ``lens`` (the entries' lengths) must all be one."""
@@ -104,8 +181,8 @@ def linear_scan(
     ``state`` is ``[slots, heads, dim, vdim]`` float32 and is updated in place.  ``fixed_order``: every sum is formed in
     an order that does not depend on the shape of the batch (the kernel otherwise spreads a column over more lanes when few
     requests bring long portions), so a token's bits do not depend on the cut.  ``lens``: the entries' numbers of rows on the host
-    (what ``q_start`` holds on the device); known, they send batches of single tokens to a kernel of their own.  Returns
-    float32 ``[N, heads * vdim]``."""
+    (what ``q_start`` holds on the device); known, they send single tokens, short and long portions each to a kernel of their
+    own.  Returns float32 ``[N, heads * vdim]``."""
 
     n = q.shape[0]
     for t, name, width in ((q, "q", qk_heads * dim), (k, "k", qk_heads * dim), (v, "v", heads * vdim)):
@@ -133,18 +210,21 @@ def linear_scan(
     if beta is not None:
         require(beta, "beta", dtype=torch.float32, shape=(n, heads))
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
-    if (lens and _chunk_form(q, v, gate, decay, beta) and scans_single(n, entries, dim, vdim, fixed_order, lens)
-            and state.data_ptr() % 16 == 0):
-        _scan_single(q, k, v, heads=heads, qk_heads=qk_heads, dim=dim, vdim=vdim, state=state, q_start=q_start, slots=slots, out=out, gate=gate,
-                     decay=decay, row_decay=row_decay, beta=beta, silu=silu, q_scale=q_scale)
-        return out
-    if scans_in_chunks(n, entries, heads, dim, fixed_order) and _chunk_form(q, v, gate, decay, beta):
-        _scan_chunks(q, k, v, heads=heads, qk_heads=qk_heads, dim=dim, vdim=vdim, state=state, q_start=q_start, slots=slots, out=out, gate=gate,
-                     decay=decay, row_decay=row_decay, beta=beta, silu=silu, q_scale=q_scale)
-        return out
-    call("b200_linear_scan", ptr(q), ptr(k), ptr(v), q.stride(0), k.stride(0), v.stride(0), ptr(gate), heads * dim, ptr(decay),
-         ptr(row_decay), ptr(beta), heads, ptr(state), ptr(out), heads * vdim, ptr(q_start), ptr(slots), entries, n, heads, qk_heads, dim, vdim,
-         1 if silu else 0, float(q_scale), 1 if fixed_order else 0, tag(q.dtype), tag(v.dtype), stream_ptr())
+    plan = [("chain", 0, entries)]
+    if _chunk_form(q, v, gate, decay, beta):
+        plan = _scan_plan(lens, n, entries, heads, dim, vdim, vdim, beta is not None, fixed_order)
+    for kind, first, last, rows, chunks in _parts(plan, lens, n):
+        starts, at = (q_start, slots) if last - first == entries else (q_start[first : last + 1], slots[first:last])
+        shared = dict(heads=heads, qk_heads=qk_heads, dim=dim, vdim=vdim, state=state, q_start=starts, slots=at, out=out, gate=gate, decay=decay,
+                      row_decay=row_decay, beta=beta, silu=silu, q_scale=q_scale)
+        if kind == "single" and state.data_ptr() % 16 == 0:
+            _scan_single(q, k, v, **shared)
+        elif kind == "chunks":
+            _scan_chunks(q, k, v, chunks=chunks, **shared)
+        else:
+            call("b200_linear_scan", ptr(q), ptr(k), ptr(v), q.stride(0), k.stride(0), v.stride(0), ptr(gate), heads * dim, ptr(decay),
+                 ptr(row_decay), ptr(beta), heads, ptr(state), ptr(out), heads * vdim, ptr(starts), ptr(at), last - first, rows, heads, qk_heads, dim, vdim,
+                 1 if silu else 0, float(q_scale), 1 if fixed_order else 0, tag(q.dtype), tag(v.dtype), stream_ptr())
     return out
 
 
@@ -176,17 +256,21 @@ def linear_scan_row_gates(
     lens = _lengths(lens, n, entries)
     out = torch.empty((n, heads * vdim), dtype=torch.float32, device=q.device)
     norm_out = torch.empty((n, heads), dtype=torch.float32, device=q.device)
-    if lens and q.dtype == torch.bfloat16 and scans_single(n, entries, dim, vdim, fixed_order, lens) and state.data_ptr() % 16 == 0:
-        _scan_single(q, k, v, heads=heads, qk_heads=heads, dim=dim, vdim=vdim, state=state, q_start=q_start, slots=slots, out=out,
-                     row_decay=decay, row_gain=gain, norm_state=norm_state, norm_out=norm_out, q_scale=q_scale)
-        return out, norm_out
-    if scans_in_chunks(n, entries, heads, dim, fixed_order) and q.dtype == torch.bfloat16:
-        _scan_chunks(q, k, v, heads=heads, qk_heads=heads, dim=dim, vdim=vdim, state=state, q_start=q_start, slots=slots, out=out,
-                     row_decay=decay, row_gain=gain, norm_state=norm_state, norm_out=norm_out, q_scale=q_scale)
-        return out, norm_out
-    call("b200_linear_scan_row_gates", ptr(q), ptr(k), ptr(v), q.stride(0), k.stride(0), v.stride(0), ptr(decay), ptr(gain), ptr(state),
-         ptr(norm_state), ptr(out), ptr(norm_out), ptr(q_start), ptr(slots), entries, n, heads, dim, vdim, float(q_scale),
-         1 if fixed_order else 0, tag(q.dtype), stream_ptr())
+    plan = [("chain", 0, entries)]
+    if q.dtype == torch.bfloat16:
+        plan = _scan_plan(lens, n, entries, heads, dim, vdim, vdim + 1, False, fixed_order)      # the normaliser is a column of the state
+    for kind, first, last, rows, chunks in _parts(plan, lens, n):
+        starts, at = (q_start, slots) if last - first == entries else (q_start[first : last + 1], slots[first:last])
+        shared = dict(heads=heads, qk_heads=heads, dim=dim, vdim=vdim, state=state, q_start=starts, slots=at, out=out, row_decay=decay,
+                      row_gain=gain, norm_state=norm_state, norm_out=norm_out, q_scale=q_scale)
+        if kind == "single" and state.data_ptr() % 16 == 0:
+            _scan_single(q, k, v, **shared)
+        elif kind == "chunks":
+            _scan_chunks(q, k, v, chunks=chunks, **shared)
+        else:
+            call("b200_linear_scan_row_gates", ptr(q), ptr(k), ptr(v), q.stride(0), k.stride(0), v.stride(0), ptr(decay), ptr(gain), ptr(state),
+                 ptr(norm_state), ptr(out), ptr(norm_out), ptr(starts), ptr(at), last - first, rows, heads, dim, vdim, float(q_scale),
+                 1 if fixed_order else 0, tag(q.dtype), stream_ptr())
     return out, norm_out
 
 

@@ -100,6 +100,30 @@ def test_which_scans_go_in_chunks():
     assert not S.scans_single(8, 8, 128, 33, False) and not S.scans_single(8, 8, 129, 64, False) and not S.scans_single(8, 8, 128, 64, True)
 
 
+def test_which_portions_go_in_chunks(monkeypatch):
+    """By a portion's own length: many short ones beside each other, or single tokens beside a long one, are no reason."""
+
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    monkeypatch.setattr(S.native, "sm_count", lambda: 148)
+    least = lambda lens, heads=32, dim=128, columns=128, delta=False: S.portion_in_chunks(lens, heads, dim, columns, delta)
+    assert least([2] * 64) == least([7] * 8) == least([23] * 100) == least([47] * 100, delta=True) == 0
+    assert least([30] * 8) == 24 and least([30] * 2) == least([30] * 8, heads=4) == 0
+    assert least([1] * 24 + [381]) == least([2048], delta=True) == least([1, 300], delta=True) == 48
+    assert least([300], heads=16) == least([1] * 24 + [300], heads=16) == 64 and least([300], heads=16, delta=True) == 96
+    assert least([300], heads=4) == 64 and least([300, 1], heads=4) == 96 and least([300, 1], heads=4, delta=True) == 128
+    assert least([100] * 64, heads=8, dim=64, columns=64) == 0 and least([100], heads=8, dim=64, columns=64) == 64
+    assert S.scan_runs([1] * 24 + [381], 48) == [("single", 0, 24), ("chunks", 24, 25)]
+    assert S.scan_runs([1, 2, 1, 0], 0) == [("chain", 0, 4)] and S.scan_runs([1, 1], 0) == [("single", 0, 2)]
+    assert S.scan_runs([1, 900, 5, 1, 130, 128], 48) == [("single", 0, 1), ("chunks", 1, 2), ("chain", 2, 4), ("chunks", 4, 6)]
+    assert S.scan_runs([1, 60, 3, 60], 48) == [("chain", 0, 4)] and S.scan_runs([1, 1, 60, 60], 48)[1] == ("chunks", 2, 4)
+    assert S.scan_runs([900, 1] * 3, 48) == [("chain", 0, 6)]              # more launches than it is worth
+    plan = lambda lens, n, entries, fixed=False: S._scan_plan(lens, n, entries, 32, 128, 128, 128, False, fixed)
+    assert plan([1] * 24 + [381], 405, 25) == [("single", 0, 24), ("chunks", 24, 25)]
+    assert plan([1] * 24 + [381], 405, 25, fixed=True) == [("chain", 0, 25)]
+    assert plan(None, 405, 25) == [("chain", 0, 25)] and plan(None, 1200, 25) == [("chunks", 0, 25)] and plan(None, 8, 8) == [("chain", 0, 8)]
+
+
 def test_parts_of_a_single_tokens_keys_over_shared_rows(monkeypatch):
     """Rows too wide for two CTAs a multiprocessor are cut into at most one round of CTAs, narrow ones into two."""
 

@@ -27,6 +27,7 @@ def _reference(q, k, v, lens, state, slots, *, decay, gain, beta):
     return out, end
 
 
+MIXED = [1, 1, 1, 130, 20, 200]         # single tokens, long and short portions: a kernel for each run of them
 FORMS = ["head", "head_float_qk", "channel", "row", "delta_channel", "delta_token"]
 
 
@@ -36,8 +37,9 @@ FORMS = ["head", "head_float_qk", "channel", "row", "delta_channel", "delta_toke
 @pytest.mark.parametrize("heads,qk_heads,d,dv,lens", [(2, 2, 128, 128, [257]), (4, 2, 40, 33, [1, 15, 16, 17, 64]), (3, 3, 16, 8, [100, 31]),
                                                       (1, 1, 72, 64, [49, 1]),
                                                       (4, 2, 128, 128, [1] * 5), (3, 3, 40, 36, [1]), (2, 1, 17, 132, [1, 1]),
-                                                      (2, 2, 128, 128, [2, 0]), (4, 2, 40, 36, [0, 3, 0]), (2, 1, 17, 132, [1, 0, 0, 3])])
-def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens):
+                                                      (2, 2, 128, 128, [2, 0]), (4, 2, 40, 36, [0, 3, 0]), (2, 1, 17, 132, [1, 0, 0, 3]),
+                                                      (2, 2, 128, 64, MIXED), (3, 1, 40, 33, MIXED)])
+def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens, monkeypatch):
     from llm_runtime_study_b200.ops import sequence_state as S
 
     if form == "row":
@@ -93,8 +95,11 @@ def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens):
     wide = wide.double()
     want, end = _reference(0.5 * wq, wk, wv, lens, state.double(), slots, decay=wide, gain=None if gain is None else gain.double(),
                            beta=None if beta is None else beta.double())
-    one_each = all(m == 1 for m in lens)
-    assert S.scans_in_chunks(n, len(lens), heads, d, False) or S.scans_single(n, len(lens), d, dv, False, lens) == one_each
+    if lens != MIXED:                        # every portion in chunks, short ones too
+        monkeypatch.setattr(S, "portion_in_chunks", lambda *sizes: 1)
+    else:
+        runs = S.scan_runs(lens, S.portion_in_chunks(lens, heads, d, dv, delta))
+        assert [kind for kind, _, _ in runs] == ["single", "chunks", "chain", "chunks"]
     chunked, chained = run(False), run(True)
 
     def error(got, ref):
