@@ -175,6 +175,10 @@ inline int configure_once(DeviceOnce& once, Kernel kernel, size_t smem_bytes, in
   return 0;
 }
 
+// Threads for a row of `vecs` 16-byte vectors that a CTA holds in registers, about one or two each: a row that is narrower
+// than its CTA leaves threads idle, and the multiprocessor holds fewer rows.
+inline int row_threads(int vecs) { return vecs <= 64 ? 64 : (vecs <= 192 ? 128 : 256); }
+
 }  // namespace b200
 
 // Error codes of our own, above the CUDA range, for refused sizes.

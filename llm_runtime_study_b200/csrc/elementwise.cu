@@ -758,10 +758,10 @@ __global__ void qk_rownorm_write_kernel(const T* __restrict__ qkv, int ld, T* __
 
 // The same with 16-byte accesses: the row's vectors are in registers (up to kRowVecs of q and of k a thread), everything is
 // read before anything waits, and both sums share one pass over the block.  36 us with two-byte accesses for 2,048 rows of
-// 4,096 + 1,024 + 1,024 columns.
+// 4,096 + 1,024 + 1,024 columns.  THREADS, and with it the order of the sums, follows from the width of q and k alone (row_threads).
 constexpr int kRowVecs = 4;
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 qk_rownorm_write_vec_kernel(const T* __restrict__ qkv, int ld, T* __restrict__ q_out, const float* __restrict__ q_w,
                             const float* __restrict__ k_w, float eps, float temp_coef, int temp_every,
                             const int* __restrict__ positions, const int* __restrict__ token_entry,
@@ -769,7 +769,7 @@ qk_rownorm_write_vec_kernel(const T* __restrict__ qkv, int ld, T* __restrict__ q
                             T* __restrict__ v_pool, int nq, int nkv, int d, int dv) {
   constexpr int VN = Vec<T>::n;
   using V = typename Vec<T>::type;
-  __shared__ float2 scratch[8];
+  __shared__ float2 scratch[THREADS / 32];
   pdl_trigger();
   pdl_wait();
   const int t = blockIdx.x, tid = threadIdx.x;
@@ -778,14 +778,14 @@ qk_rownorm_write_vec_kernel(const T* __restrict__ qkv, int ld, T* __restrict__ q
   V xq[kRowVecs], xk[kRowVecs];
 #pragma unroll
   for (int i = 0; i < kRowVecs; ++i) {
-    if (tid + 256 * i < qv) xq[i] = row[tid + 256 * i];
-    if (tid + 256 * i < kv) xk[i] = row[qv + tid + 256 * i];
+    if (tid + THREADS * i < qv) xq[i] = row[tid + THREADS * i];
+    if (tid + THREADS * i < kv) xk[i] = row[qv + tid + THREADS * i];
   }
   const int p = positions[t];
   const int page = block_table[static_cast<size_t>(token_entry[t]) * table_stride + p / page_size];
   const size_t at = static_cast<size_t>(max(page, 0)) * nkv * page_size + p % page_size;
   if (page >= 0) {                    // a padding row has no pages
-    for (int i = tid; i < vv; i += 256) {
+    for (int i = tid; i < vv; i += THREADS) {
       const int g = i * VN / dv, c = i * VN % dv;
       *reinterpret_cast<V*>(v_pool + (at + static_cast<size_t>(g) * page_size) * dv + c) = row[qv + kv + i];
     }
@@ -794,12 +794,12 @@ qk_rownorm_write_vec_kernel(const T* __restrict__ qkv, int ld, T* __restrict__ q
   float f[VN];
 #pragma unroll
   for (int i = 0; i < kRowVecs; ++i) {
-    if (tid + 256 * i < qv) {
+    if (tid + THREADS * i < qv) {
       Vec<T>::unpack(xq[i], f);
 #pragma unroll
       for (int e = 0; e < VN; ++e) ss.x = fmaf(f[e], f[e], ss.x);
     }
-    if (tid + 256 * i < kv) {
+    if (tid + THREADS * i < kv) {
       Vec<T>::unpack(xk[i], f);
 #pragma unroll
       for (int e = 0; e < VN; ++e) ss.y = fmaf(f[e], f[e], ss.y);
@@ -810,7 +810,7 @@ qk_rownorm_write_vec_kernel(const T* __restrict__ qkv, int ld, T* __restrict__ q
   __syncthreads();
   ss = scratch[0];
 #pragma unroll
-  for (int w = 1; w < 8; ++w) { ss.x += scratch[w].x; ss.y += scratch[w].y; }
+  for (int w = 1; w < THREADS / 32; ++w) { ss.x += scratch[w].x; ss.y += scratch[w].y; }
   const float fq = q_w ? rsqrtf(ss.x / static_cast<float>(nq * d) + eps) : 1.f;
   const float fk = k_w ? rsqrtf(ss.y / static_cast<float>(nkv * d) + eps) : 1.f;
   const float temp = temp_every > 0 ? 1.f + temp_coef * logf(static_cast<float>((p + 1) / temp_every) + 1.f) : 1.f;
@@ -826,7 +826,7 @@ qk_rownorm_write_vec_kernel(const T* __restrict__ qkv, int ld, T* __restrict__ q
   };
 #pragma unroll
   for (int i = 0; i < kRowVecs; ++i) {
-    const int j = tid + 256 * i;
+    const int j = tid + THREADS * i;
     if (j < qv) reinterpret_cast<V*>(q_out)[static_cast<size_t>(t) * qv + j] = scaled(xq[i], fq, q_w ? q_w + j * VN : nullptr, temp);
     if (j < kv && page >= 0) {
       const int g = j * VN / d, c = j * VN % d;
@@ -983,10 +983,16 @@ extern "C" int b200_qk_rownorm_write(const void* qkv, int ld, void* q_out, const
                          reinterpret_cast<uintptr_t>(v_pool) | reinterpret_cast<uintptr_t>(q_w) | reinterpret_cast<uintptr_t>(k_w)) & 15) == 0;
   const int vn = dtype == kBF16 ? 8 : 4;        // whole 16-byte vectors in every row and head
   if (aligned && (ld | d | dv) % vn == 0 && nq * d <= 256 * kRowVecs * vn && nkv * d <= 256 * kRowVecs * vn) {
-    B200_DISPATCH_DTYPE(dtype, T, launch(qk_rownorm_write_vec_kernel<T>, dim3(n), dim3(256), 0, stream, static_cast<const T*>(qkv), ld,
-                                         static_cast<T*>(q_out), q_w, k_w, eps, temp_coef, temp_every, positions, token_entry,
-                                         block_table, table_stride, page_size, static_cast<T*>(k_pool), static_cast<T*>(v_pool),
-                                         nq, nkv, d, dv));
+#define B200_QK_ROWS(THREADS)                                                                                                        \
+  B200_DISPATCH_DTYPE(dtype, T, launch(qk_rownorm_write_vec_kernel<T, THREADS>, dim3(n), dim3(THREADS), 0, stream,                     \
+                                       static_cast<const T*>(qkv), ld, static_cast<T*>(q_out), q_w, k_w, eps, temp_coef, temp_every,   \
+                                       positions, token_entry, block_table, table_stride, page_size, static_cast<T*>(k_pool),          \
+                                       static_cast<T*>(v_pool), nq, nkv, d, dv))
+    const int threads = row_threads((nq > nkv ? nq : nkv) * d / vn);
+    if (threads == 64) { B200_QK_ROWS(64); }
+    else if (threads == 128) { B200_QK_ROWS(128); }
+    else { B200_QK_ROWS(256); }
+#undef B200_QK_ROWS
     return launch_status();
   }
   B200_DISPATCH_DTYPE(dtype, T, launch(qk_rownorm_write_kernel<T>, dim3(n), dim3(256), 0, stream, static_cast<const T*>(qkv), ld,

@@ -144,7 +144,8 @@ def test_sigmoid_gate(dtype, n, groups, group):
 
 # rows of one vector a thread, of several with a ragged end, of more than the registers hold, heads that no vector divides; a row without pages
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("nq,nkv,d,dv", [(32, 8, 128, 128), (3, 1, 8, 16), (5, 5, 24, 40), (2, 1, 10, 8), (80, 4, 128, 64)])
+@pytest.mark.parametrize("nq,nkv,d,dv", [(32, 8, 128, 128), (3, 1, 8, 16), (5, 5, 24, 40), (2, 1, 10, 8), (80, 4, 128, 64), (16, 2, 64, 64),
+                                         (9, 1, 64, 72)])
 def test_qk_rownorm_write(dtype, nq, nkv, d, dv):
     from llm_runtime_study_b200.ops import functional as F
 
