@@ -167,10 +167,11 @@ latent_prepare_kernel(const T* __restrict__ rows, int ld, int q_off, int q_rank,
 }
 
 // The same with 16-byte accesses: the row's vectors are in registers (up to kLatentVecs of the query latent and one of the
-// kept latent a thread), everything is read before anything waits, and both sums share one pass over the block.
+// kept latent a thread), everything is read before anything waits, and both sums share one pass over the block.  THREADS, and with
+// it the order of the sums, follows from the widths alone (row_threads).
 constexpr int kLatentVecs = 4;
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 latent_prepare_vec_kernel(const T* __restrict__ rows, int ld, int q_off, int q_rank, const float* __restrict__ q_w,
                           T* __restrict__ cq_out, int kv_off, int kv_rank, const float* __restrict__ kv_w, int rot,
                           const Rotation rotation, float eps, const int* __restrict__ positions,
@@ -178,7 +179,7 @@ latent_prepare_vec_kernel(const T* __restrict__ rows, int ld, int q_off, int q_r
                           int page_size, T* __restrict__ pool) {
   constexpr int VN = Vec<T>::n;
   using V = typename Vec<T>::type;
-  __shared__ float2 scratch[8];
+  __shared__ float2 scratch[THREADS / 32];
   pdl_trigger();
   pdl_wait();
   const int token = blockIdx.x, tid = threadIdx.x, qv = q_rank / VN, kv = kv_rank / VN;
@@ -186,7 +187,7 @@ latent_prepare_vec_kernel(const T* __restrict__ rows, int ld, int q_off, int q_r
   V xq[kLatentVecs], xk;
 #pragma unroll
   for (int i = 0; i < kLatentVecs; ++i)
-    if (tid + 256 * i < qv) xq[i] = reinterpret_cast<const V*>(row + q_off)[tid + 256 * i];
+    if (tid + THREADS * i < qv) xq[i] = reinterpret_cast<const V*>(row + q_off)[tid + THREADS * i];
   if (tid < kv) xk = reinterpret_cast<const V*>(row + kv_off)[tid];
   int p = 0, page = -1;
   if (kv_rank > 0) {
@@ -196,14 +197,14 @@ latent_prepare_vec_kernel(const T* __restrict__ rows, int ld, int q_off, int q_r
   T* dst = pool + (static_cast<size_t>(max(page, 0)) * page_size + (kv_rank > 0 ? p % page_size : 0)) * (kv_rank + rot);
   if (page >= 0) {                 // the rotated part waits for no sum
     const T* src = row + kv_off + kv_rank;
-    for (int i = 255 - tid; i < rotation.dims / 2; i += 256) rotate_pair(src, dst + kv_rank, i, static_cast<float>(p), rotation);
-    for (int i = rotation.dims + tid; i < rot; i += 256) dst[kv_rank + i] = src[i];
+    for (int i = THREADS - 1 - tid; i < rotation.dims / 2; i += THREADS) rotate_pair(src, dst + kv_rank, i, static_cast<float>(p), rotation);
+    for (int i = rotation.dims + tid; i < rot; i += THREADS) dst[kv_rank + i] = src[i];
   }
   float2 ss = make_float2(0.f, 0.f);
   float f[VN];
 #pragma unroll
   for (int i = 0; i < kLatentVecs; ++i) {
-    if (tid + 256 * i >= qv) break;
+    if (tid + THREADS * i >= qv) break;
     Vec<T>::unpack(xq[i], f);
 #pragma unroll
     for (int e = 0; e < VN; ++e) ss.x = fmaf(f[e], f[e], ss.x);
@@ -218,7 +219,7 @@ latent_prepare_vec_kernel(const T* __restrict__ rows, int ld, int q_off, int q_r
   __syncthreads();
   ss = scratch[0];
 #pragma unroll
-  for (int w = 1; w < 8; ++w) { ss.x += scratch[w].x; ss.y += scratch[w].y; }
+  for (int w = 1; w < THREADS / 32; ++w) { ss.x += scratch[w].x; ss.y += scratch[w].y; }
   const float fq = rsqrtf(ss.x / static_cast<float>(q_rank) + eps);
   auto scaled = [&](const V& x, float factor, const float* w) {
     Vec<T>::unpack(x, f);
@@ -231,7 +232,7 @@ latent_prepare_vec_kernel(const T* __restrict__ rows, int ld, int q_off, int q_r
   };
 #pragma unroll
   for (int i = 0; i < kLatentVecs; ++i) {
-    const int at = tid + 256 * i;
+    const int at = tid + THREADS * i;
     if (at >= qv) break;
     reinterpret_cast<V*>(cq_out + static_cast<size_t>(token) * q_rank)[at] = scaled(xq[i], fq, q_w + at * VN);
   }
@@ -462,10 +463,16 @@ extern "C" int b200_latent_prepare(const void* rows, int ld, int q_off, int q_ra
   const int vn = dtype == kBF16 ? 8 : 4;        // whole 16-byte vectors in every row and part
   if (aligned && (ld | q_off | q_rank | kv_off | kv_rank | (kv_rank > 0 ? kv_rank + rot : 0)) % vn == 0 && q_rank <= 256 * kLatentVecs * vn &&
       kv_rank <= 256 * vn) {
-    B200_DISPATCH_DTYPE(dtype, T, launch(latent_prepare_vec_kernel<T>, dim3(n), dim3(256), 0, stream, static_cast<const T*>(rows), ld, q_off,
-                                         q_rank, q_w, static_cast<T*>(cq_out), kv_off, kv_rank, kv_w, rot,
-                                         Rotation{inv_freq, rot_dims, interleaved, rot_factor}, eps,
-                                         positions, token_entry, block_table, table_stride, page_size, static_cast<T*>(pool)));
+#define B200_LATENT_ROWS(THREADS)                                                                                                    \
+  B200_DISPATCH_DTYPE(dtype, T, launch(latent_prepare_vec_kernel<T, THREADS>, dim3(n), dim3(THREADS), 0, stream,                       \
+                                       static_cast<const T*>(rows), ld, q_off, q_rank, q_w, static_cast<T*>(cq_out), kv_off, kv_rank,  \
+                                       kv_w, rot, Rotation{inv_freq, rot_dims, interleaved, rot_factor}, eps, positions, token_entry,  \
+                                       block_table, table_stride, page_size, static_cast<T*>(pool)))
+    const int threads = row_threads((q_rank > kv_rank ? q_rank : kv_rank) / vn);      // (at least one for every vector of the kept latent)
+    if (threads == 64) { B200_LATENT_ROWS(64); }
+    else if (threads == 128 && kv_rank <= 128 * vn) { B200_LATENT_ROWS(128); }
+    else { B200_LATENT_ROWS(256); }
+#undef B200_LATENT_ROWS
     return launch_status();
   }
   B200_DISPATCH_DTYPE(dtype, T, launch(latent_prepare_kernel<T>, dim3(n), dim3(256), 0, stream, static_cast<const T*>(rows), ld, q_off,

@@ -174,7 +174,8 @@ def test_qk_rownorm_write(dtype, nq, nkv, d, dv):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("q_rank,kv_rank,rot,dims", [(2048, 512, 64, 64), (8, 16, 8, 4), (1000, 40, 16, 0), (12, 6, 4, 2), (8200, 64, 0, 0), (520, 0, 0, 0)])
+@pytest.mark.parametrize("q_rank,kv_rank,rot,dims", [(2048, 512, 64, 64), (8, 16, 8, 4), (1000, 40, 16, 0), (12, 6, 4, 2), (8200, 64, 0, 0), (520, 0, 0, 0),
+                                                      (768, 264, 8, 8), (512, 1040, 16, 16)])
 def test_latent_prepare(dtype, q_rank, kv_rank, rot, dims):
     from llm_runtime_study_b200.ops import mixer_steps as M
 
