@@ -715,17 +715,29 @@ __global__ void group_norm_gate_kernel(const float* __restrict__ x, int width, i
 }
 
 // The same with 16-byte reads, in two forms; the order of a group's sum of squares is a function of the group's size.
-// Small groups (one head, up to 128 columns): a warp owns a group of TOKENS rows, a lane four columns; a low-rank map's
-// columns are read once for all the rows.  2,048 rows of 32 groups of 128 with a map of rank 32: 44 us, 28 us a
-// launch for 1,733 rows without one (75 and 49 us with a CTA per row and group, two bytes at a time, a read of the map per row).
+// Small groups (one head, up to 128 columns): a warp owns a group of TOKENS rows, a lane four columns; a low-rank map's (MAP)
+// columns are read once for all the rows.  2,048 rows of 32 groups of 128 with a map of rank 32: 44 us (106 with a CTA per row and group,
+// two bytes at a time, a read of the map per row).  Without a map rows have nothing to share: 19 us for the same rows with one a
+// warp, 32 with eight (53).
 template <typename T> struct Quad;            // four neighbouring elements of the storage type
 template <> struct Quad<float> {
   using type = float4;
+  // a load that stays where it is written: the compiler otherwise moves a batch's loads down to their uses
+  __device__ static type ask(const void* p) {
+    type v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+  }
   __device__ static float4 widen(const type& v) { return v; }
   __device__ static type narrow(const float4& v) { return v; }
 };
 template <> struct Quad<__nv_bfloat16> {
   using type = uint2;
+  __device__ static type ask(const void* p) {
+    type v;
+    asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+  }
   __device__ static float4 widen(const type& v) {
     const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&v)[0]);
     const float2 b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&v)[1]);
@@ -747,7 +759,7 @@ __device__ __forceinline__ float gated(float x, float f, float w, float logit, i
   return x * f * w * (silu ? silu_f(logit) : sigmoid_f(logit));
 }
 
-template <typename T, int TOKENS>
+template <typename T, int TOKENS, bool MAP>
 __global__ void __launch_bounds__(128) group_norm_gate_warp_kernel(const GroupNormParams p) {
   using Q = Quad<T>;
   extern __shared__ __align__(16) float low[];     // [rank][TOKENS]: the rows' low-rank input
@@ -755,11 +767,13 @@ __global__ void __launch_bounds__(128) group_norm_gate_warp_kernel(const GroupNo
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, groups = p.width / p.group;
   const int g = blockIdx.y * 4 + warp, t0 = blockIdx.x * TOKENS, count = min(TOKENS, p.n - t0);
-  for (int idx = threadIdx.x; idx < p.rank * TOKENS; idx += 128) {
-    const int t = idx / p.rank, j = idx % p.rank;
-    low[j * TOKENS + t] = t < count ? to_float(static_cast<const T*>(p.gate_in)[static_cast<size_t>(t0 + t) * p.gate_ld + j]) : 0.f;
+  if constexpr (MAP) {
+    for (int idx = threadIdx.x; idx < p.rank * TOKENS; idx += 128) {
+      const int t = idx / p.rank, j = idx % p.rank;
+      low[j * TOKENS + t] = t < count ? to_float(static_cast<const T*>(p.gate_in)[static_cast<size_t>(t0 + t) * p.gate_ld + j]) : 0.f;
+    }
+    __syncthreads();
   }
-  __syncthreads();
   if (g >= groups) return;
   const int c = g * p.group + lane * 4;
   const bool on = lane * 4 < p.group;
@@ -768,7 +782,7 @@ __global__ void __launch_bounds__(128) group_norm_gate_warp_kernel(const GroupNo
 #pragma unroll
   for (int t = 0; t < TOKENS; ++t)
     x[t] = on && t < count ? *reinterpret_cast<const float4*>(p.x + static_cast<size_t>(t0 + t) * p.width + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-  if (p.rank == 0) {
+  if constexpr (!MAP) {
 #pragma unroll
     for (int t = 0; t < TOKENS; ++t) {
       z[t] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -779,9 +793,8 @@ __global__ void __launch_bounds__(128) group_norm_gate_warp_kernel(const GroupNo
 #pragma unroll
     for (int t = 0; t < TOKENS; ++t) z[t] = make_float4(0.f, 0.f, 0.f, 0.f);
     const T* up = static_cast<const T*>(p.gate_up) + (on ? c : 0);
-#pragma unroll 8
-    for (int j = 0; j < p.rank; ++j) {
-      const float4 u = Q::widen(*reinterpret_cast<const typename Q::type*>(up + static_cast<size_t>(j) * p.width));
+    auto add = [&](const typename Q::type& row, int j) {
+      const float4 u = Q::widen(row);
 #pragma unroll
       for (int t = 0; t < TOKENS; ++t) {
         const float l = low[j * TOKENS + t];
@@ -790,7 +803,20 @@ __global__ void __launch_bounds__(128) group_norm_gate_warp_kernel(const GroupNo
         z[t].z = fmaf(u.z, l, z[t].z);
         z[t].w = fmaf(u.w, l, z[t].w);
       }
+    };
+    int j = 0;
+    if constexpr (TOKENS == 1) {      // a single row a warp has nothing to do while the map's rows are on their way: sixteen at a time
+      constexpr int N = 16;
+      for (; j + N <= p.rank; j += N) {
+        typename Q::type row[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) row[i] = Q::ask(up + static_cast<size_t>(j + i) * p.width);
+#pragma unroll
+        for (int i = 0; i < N; ++i) add(row[i], j + i);
+      }
     }
+#pragma unroll 8
+    for (; j < p.rank; ++j) add(*reinterpret_cast<const typename Q::type*>(up + static_cast<size_t>(j) * p.width), j);
   }
 #pragma unroll
   for (int t = 0; t < TOKENS; ++t) {
@@ -1000,14 +1026,21 @@ extern "C" int b200_group_norm_gate(const float* x, int n, int width, int group,
   auto at = [](const void* ptr, size_t bytes) { return reinterpret_cast<uintptr_t>(ptr) % bytes == 0; };
   const bool quads = group % 4 == 0 && at(x, 16) && at(out, four) && (w == nullptr || at(w, 16)) &&
                      (rank > 0 ? at(gate_up, four) : gate_ld % 4 == 0 && at(gate_in, four));
-  if (quads && (group <= 128 ? rank <= 1024 : rank == 0) && (width / group + 3) / 4 <= 65535 && (group <= 128 || width / group <= 65535)) {
+  // Few bfloat16 rows with a low-rank map stay with the CTA per row and group below: a thread a column has four times the threads for
+  // the chain of loads that the map is (32 rows of 16 groups, rank 128: 5.5 us against 6.4 with a warp a group, rank 32 3.0 against 3.3; 64
+  // rows of 32 groups 11.6 against 7.9 and 5.0 against 3.7).  In float32 a row's bits must not depend on how many others there are.
+  const long long row_groups = static_cast<long long>(n) * (width / group);
+  const bool few = dtype == kBF16 && rank > 0 && row_groups < 1500;
+  if (quads && !few && (group <= 128 ? rank <= 1024 : rank == 0) && (width / group + 3) / 4 <= 65535 && (group <= 128 || width / group <= 65535)) {
     const GroupNormParams p{x, n, width, group, w, w_len, eps, den, floor_, den_eps, gate_in, gate_ld, rank, gate_up, gate_silu, out};
     if (group > 128) {
       B200_DISPATCH_DTYPE(dtype, T, launch(group_norm_gate_row_kernel<T>, dim3(n, width / group), dim3(256), 0, stream, p));
-    } else if (static_cast<long long>(n) * (width / group) >= 8 * 4 * 2 * 148) {
-      B200_DISPATCH_DTYPE(dtype, T, launch(group_norm_gate_warp_kernel<T, 8>, dim3((n + 7) / 8, (width / group + 3) / 4), dim3(128), sizeof(float) * 8 * rank, stream, p));
+    } else if (rank == 0) {
+      B200_DISPATCH_DTYPE(dtype, T, launch(group_norm_gate_warp_kernel<T, 1, false>, dim3(n, (width / group + 3) / 4), dim3(128), 0, stream, p));
+    } else if (row_groups >= 8 * 4 * 2 * 148) {      // eight rows share what a warp reads of the map
+      B200_DISPATCH_DTYPE(dtype, T, launch(group_norm_gate_warp_kernel<T, 8, true>, dim3((n + 7) / 8, (width / group + 3) / 4), dim3(128), sizeof(float) * 8 * rank, stream, p));
     } else {
-      B200_DISPATCH_DTYPE(dtype, T, launch(group_norm_gate_warp_kernel<T, 1>, dim3(n, (width / group + 3) / 4), dim3(128), sizeof(float) * rank, stream, p));
+      B200_DISPATCH_DTYPE(dtype, T, launch(group_norm_gate_warp_kernel<T, 1, true>, dim3(n, (width / group + 3) / 4), dim3(128), sizeof(float) * rank, stream, p));
     }
     return launch_status();
   }

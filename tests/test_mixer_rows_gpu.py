@@ -108,7 +108,8 @@ def test_delta_prepare_keeps_bad_rows_within_the_taps_reach(dtype, taps):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("n,groups,group,rank", [(300, 32, 128, 32), (3, 5, 128, 7), (257, 40, 36, 0), (2, 1, 4096, 0), (5, 3, 260, 0), (4, 2, 30, 3), (1, 4, 4, 1)])
+@pytest.mark.parametrize("n,groups,group,rank", [(300, 32, 128, 32), (3, 5, 128, 7), (257, 40, 36, 0), (2, 1, 4096, 0), (5, 3, 260, 0), (4, 2, 30, 3), (1, 4, 4, 1),
+                                                  (50, 32, 96, 33), (47, 32, 128, 16)])
 @pytest.mark.parametrize("act,divided", [("sigmoid", False), ("silu", True)])
 def test_group_norm_gate(dtype, n, groups, group, rank, act, divided):
     from llm_runtime_study_b200.ops import sequence_state as S
@@ -129,6 +130,23 @@ def test_group_norm_gate(dtype, n, groups, group, rank, act, divided):
     if rank:
         logits = logits @ up.double()
     close(out, y * (torch.sigmoid(logits) if act == "sigmoid" else logits * torch.sigmoid(logits)), tolerance(dtype))
+
+
+@pytest.mark.parametrize("rank", [0, 5, 40])
+def test_group_norm_gate_in_float32_gives_a_row_the_same_bits_in_any_batch(rank):
+    """One row, few rows and rows that share what is read of the map."""
+
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    g = torch.Generator().manual_seed(rank)
+    n, groups, group = 300, 32, 64
+    x, gate = torch.randn(n, groups * group, generator=g).to(DEV), torch.randn(n, rank or groups * group, generator=g).to(DEV)
+    up = torch.randn(rank, groups * group, generator=g).to(DEV) if rank else None
+    weight = torch.randn(group, generator=g).to(DEV)
+    run = lambda k: S.group_norm_gate(x[:k].contiguous(), weight, 1e-5, gate[:k].contiguous(), gate_up=up, out_dtype=torch.float32)
+    together = run(n)
+    for k in (1, 40, 60):
+        assert torch.equal(run(k), together[:k])
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
