@@ -353,7 +353,7 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab, RowParams par
 // Rows without top_k / top_p need one pass only (argmax of the logits, or of the logits
 // plus Gumbel noise), so the vocabulary is cut into `chunks` parts handled by different
 // CTAs; the second stage picks the best of the partial results.  Rows with filters take
-// the single-CTA kernel above.
+// the kernel above.
 __device__ __forceinline__ bool row_is_filtered(const int* p, int vocab) {
   const float temperature = __int_as_float(p[0]);
   return temperature != 0.f && ((p[1] > 0 && p[1] < vocab) || __int_as_float(p[2]) < 1.f);
@@ -423,12 +423,16 @@ __global__ void sample_final_kernel(const float* __restrict__ part_value, const 
 
 // The single-kernel path: a cluster of eight CTAs per row for vocabularies of 32,768 entries and more, one CTA
 // otherwise.  151,936 entries: a share is 76 KB, so two CTAs of 512 threads are resident on an SM and 32 rows run at once.
-constexpr size_t kMostStaged = 200 * 1024;
+// Shares of up to 32 KB leave room for more CTAs than 512 threads each do, and rows beyond 64 want them resident at once: 256 threads then.
+// 128 rows, all with top-k, 32,768 and 50,257 entries: 77 and 99 us (118 and 149 with 512 threads; 82 and 116 with one CTA a row that reads
+// the logits in every pass); 256 rows 137 and 179 us (223 and 283; 162 and 228).  For fewer rows 512 threads are as fast or faster (64 rows, half of
+// them filtered: 52 and 66 us against 59 and 80).
+constexpr size_t kMostStaged = 200 * 1024, kSmallShare = 32 * 1024;
 static int launch_sample(const float* logits, int ld, int vocab, b200::RowParams params, int* out, int rows, int filtered_only,
                          cudaStream_t stream) {
   const int cluster = vocab < 32768 ? 1 : 8;
-  const int threads = cluster > 1 ? 512 : (vocab >= 8192 ? 1024 : (vocab >= 1024 ? 256 : 128));
   const size_t share = sizeof(float) * static_cast<size_t>(((vocab + cluster - 1) / cluster + 3) & ~3);
+  const int threads = cluster > 1 ? (rows > 64 && share <= kSmallShare ? 256 : 512) : (vocab >= 8192 ? 1024 : (vocab >= 1024 ? 256 : 128));
   const bool staged = share <= kMostStaged;
   static b200::DeviceOnce once;
   if (staged)
@@ -460,8 +464,8 @@ extern "C" int b200_sample(const float* logits, int ld, int vocab, const int* pa
 }
 
 // Two-stage variant.  `scratch` holds rows * chunks floats followed by rows * chunks ints;
-// `any_filtered` tells whether some row uses top_k / top_p (then the single-CTA kernel also
-// runs, for those rows only).
+// `any_filtered` tells whether some row uses top_k / top_p (then the kernel with a cluster per row
+// also runs, for those rows only).
 static int sample_chunked(const float* logits, int ld, int vocab, b200::RowParams params, int* out, int rows,
                           int chunks, void* scratch, int any_filtered, cudaStream_t stream) {
   if (rows <= 0) return 0;

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 def sampler():
     from llm_runtime_study_b200.sampling import Sampler
 
-    return Sampler(torch.device("cuda:0"), max_rows=64)
+    return Sampler(torch.device("cuda:0"), max_rows=130)
 
 
 def cfg(**kw):
@@ -49,17 +49,22 @@ def test_matches_the_plain_sampler(sampler, vocab, opts):
         assert got[r] == want or abs(float(scores[got[r]] - scores[want])) < 1e-4
 
 
-@pytest.mark.parametrize("rows", [3, 20, 40, 64])
-def test_large_odd_vocabulary_every_cluster_size(sampler, rows):
-    """40,003 entries (rows after the first are not 16-byte aligned) with 3, 20, 40 and 64 rows: clusters
-    of eight, four and two CTAs a row and the single CTA."""
+@pytest.mark.parametrize("rows", [3, 20, 64, 65, 130])
+def test_large_odd_vocabulary_with_more_rows_than_fit_at_once(sampler, rows):
+    """40,003 entries (rows after the first are not 16-byte aligned), clusters of eight CTAs a row: up to 64 rows with 512 threads each,
+    beyond that with 256; all rows filtered, and rows with filters between rows without."""
 
     torch.manual_seed(5)
     vocab, opts = 40003, dict(temperature=0.9, top_k=40, top_p=0.7)
     logits = torch.randn(rows, vocab) * 2
+    device_logits = logits.cuda()
     specs = [(cfg(**opts), 77 + r, r) for r in range(rows)]
-    got = sampler.sample(logits.cuda(), specs)
-    for r in range(0, rows, max(1, rows // 8)):
+    others = [dict(), dict(temperature=0.8), opts]
+    got = sampler.sample(device_logits, specs)
+    mixed = sampler.sample(device_logits, [(cfg(**others[r % 3]), 77 + r, r) for r in range(rows)])
+    assert [mixed[r] for r in range(2, rows, 3)] == [got[r] for r in range(2, rows, 3)]
+    assert [mixed[r] for r in range(0, rows, 3)] == logits.argmax(dim=-1)[::3].tolist()
+    for r in sorted({*range(0, rows, max(1, rows // 8)), rows - 1}):
         want, scores = plain.sample(logits[r], opts["temperature"], opts["top_k"], opts["top_p"], 77 + r, r)
         keep = plain.kept_mask(logits[r], opts["temperature"], opts["top_k"], opts["top_p"])
         assert keep[got[r]], f"row {r}: token {got[r]} is outside the kept set"
