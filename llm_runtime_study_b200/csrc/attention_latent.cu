@@ -6,10 +6,12 @@
 // heads.  Keys are streamed in tiles of 32 rows through shared memory (cp.async, two stages) from the request's pages.
 // Eight warps: warp w owns rows 16 (w & 3) .. + 15 and the value columns of half (w >> 2); the two warps of a row group
 // each form the scores S = Q K^T (mma.sync m16n8k16, float accumulation) of half of the tile's keys and exchange them through
-// shared memory (both forming all of them made that 70 % of a warp's products; rows of more than 868 columns leave no room for
-// the exchange and still do), run the same online softmax in float32, round P to bfloat16 and multiply it with their half of
-// the value columns, read transposed out of the key tile.  32 heads over rows of 576 columns, before the exchange and with it:
-// a prompt of 1,733 tokens 633 and 541 us, of 300 tokens 49.3 and 43.0, single tokens of 100 requests over 2,049 rows 264 and 213.
+// shared memory, run the same online softmax in float32, round P to bfloat16 and multiply it with their half of the value
+// columns, read transposed out of the key tile.  Both forming all scores made that 70 % of a warp's products.  Rows of more than 868
+// columns leave no room for the exchange and still do; so do rows of less than 80, whose few products cost less than it.
+// Before the exchange and with it: 32 heads over rows of 576 columns, one prompt of 1,733 tokens 633 and 541 us, of 300 tokens 49.3
+// and 43.0, single tokens of 100 requests over 2,049 rows 264 and 213; 4 heads over rows of 32 columns, a prompt of 300 tokens beside
+// 24 single tokens over 1,500 rows 38.7 and 47.2.
 // Key t is visible to a query at position p iff t <= p and (window == 0 or t > p - window).  With a sink every head's sum has
 // one more term exp(sink[head]), which belongs to no key.
 #include "common.cuh"
@@ -31,7 +33,8 @@ constexpr int KSTEPS = DK / 16;
 constexpr int DVH = DV / 2;                 // value columns of one warp
 constexpr int OTILES = DVH / 8;
 constexpr int kTileBytes = (BM + 2 * BN) * LDS * 2, kExchangeBytes = NT * 32;    // eight scores a thread
-constexpr bool kShareScores = kTileBytes + kExchangeBytes <= 227 * 1024;        // else both warps form all scores
+// else both warps form all scores: there is no room, or a warp's few products cost less than the exchange
+constexpr bool kShareScores = DK >= 80 && kTileBytes + kExchangeBytes <= 227 * 1024;
 constexpr int kSmemBytes = kTileBytes + (kShareScores ? kExchangeBytes : 0);
 
 struct LatentParams {
@@ -53,18 +56,22 @@ struct LatentParams {
   float* part_ml;   // [rows][splits][2]
 };
 
-// Eight threads copy a key row: its page is looked up once for all of them, a tile ahead of the copies (looked up before every
-// 16-byte copy a launch for 1,733 tokens of 32 heads took 323 us, so 247; single tokens of 8 requests 40.7 and 32.9 us).
-constexpr int kRowThreads = NT / BN;
-__device__ __forceinline__ int key_page(const LatentParams& p, const int* table, int t, int lo, int hi) {
-  return t >= lo && t <= hi ? table[t / p.page_size] : -1;
+// Several threads copy a key row: its page is looked up once for all of them, a tile ahead of the copies (three prompts of 1,733 tokens in
+// all, 32 heads over rows of 576 columns: 323 us with a lookup before every 16-byte copy, so 247; single tokens of 8 requests 40.7
+// and 32.9 us).  Rows of less than 64 columns have fewer copies than a row has threads: the others look up nothing.
+constexpr int kRowThreads = DK >= 64 ? NT / BN : (DK >= 32 ? 4 : 2);
+__device__ __forceinline__ const bf16* key_row(const LatentParams& p, const int* table, int t, int lo, int hi) {
+  if (t < lo || t > hi || threadIdx.x >= BN * kRowThreads) return nullptr;
+  const int page = table[t / p.page_size];
+  return page >= 0 ? p.pool + (static_cast<size_t>(page) * p.page_size + t % p.page_size) * DK : nullptr;
 }
-__device__ __forceinline__ void load_key_tile(bf16* ks, const LatentParams& p, int page, int t) {
-  const int r = threadIdx.x / kRowThreads;
-  const bf16* src = page >= 0 ? p.pool + (static_cast<size_t>(page) * p.page_size + t % p.page_size) * DK : p.pool;
-  const int bytes = page >= 0 ? 16 : 0;
+__device__ __forceinline__ void load_key_tile(bf16* ks, const LatentParams& p, const bf16* row) {
+  if (kRowThreads * BN < NT && threadIdx.x >= BN * kRowThreads) return;
+  const bf16* src = row != nullptr ? row : p.pool;
+  const int bytes = row != nullptr ? 16 : 0;
+  ks += threadIdx.x / kRowThreads * LDS;
 #pragma unroll
-  for (int ch = threadIdx.x % kRowThreads; ch < DK / 8; ch += kRowThreads) cp_async_16(ks + r * LDS + ch * 8, src + ch * 8, bytes);
+  for (int ch = threadIdx.x % kRowThreads; ch < DK / 8; ch += kRowThreads) cp_async_16(ks + ch * 8, src + ch * 8, bytes);
 }
 
 __global__ void __launch_bounds__(NT, 1)
@@ -115,9 +122,9 @@ latent_attention_kernel(const LatentParams p) {
     tiles = min(tiles - first_tile, per);
     t_begin += first_tile * BN;
   }
-  const int key_row = threadIdx.x / kRowThreads;
-  if (tiles > 0) load_key_tile(ks, p, key_page(p, table, t_begin + key_row, lo, hi), t_begin + key_row);
-  int next_page = tiles > 1 ? key_page(p, table, t_begin + BN + key_row, lo, hi) : -1;
+  const int in_tile = threadIdx.x / kRowThreads;             // which of a tile's rows this thread copies
+  if (tiles > 0) load_key_tile(ks, p, key_row(p, table, t_begin + in_tile, lo, hi));
+  const bf16* next_row = tiles > 1 ? key_row(p, table, t_begin + BN + in_tile, lo, hi) : nullptr;
   cp_async_commit();
 
   float o[OTILES][4];
@@ -138,8 +145,8 @@ latent_attention_kernel(const LatentParams p) {
   for (int kt = 0; kt < tiles; ++kt) {
     const int t0 = t_begin + kt * BN;
     bf16* kcur = ks + (kt & 1) * BN * LDS;
-    if (kt + 1 < tiles) load_key_tile(ks + ((kt + 1) & 1) * BN * LDS, p, next_page, t0 + BN + key_row);
-    next_page = kt + 2 < tiles ? key_page(p, table, t0 + 2 * BN + key_row, lo, hi) : -1;
+    if (kt + 1 < tiles) load_key_tile(ks + ((kt + 1) & 1) * BN * LDS, p, next_row);
+    next_row = kt + 2 < tiles ? key_row(p, table, t0 + 2 * BN + in_tile, lo, hi) : nullptr;
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
