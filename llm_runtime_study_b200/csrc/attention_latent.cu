@@ -36,6 +36,8 @@ constexpr int kTileBytes = (BM + 2 * BN) * LDS * 2, kExchangeBytes = NT * 32;   
 // else both warps form all scores: there is no room, or a warp's few products cost less than the exchange
 constexpr bool kShareScores = DK >= 80 && kTileBytes + kExchangeBytes <= 227 * 1024;
 constexpr int kSmemBytes = kTileBytes + (kShareScores ? kExchangeBytes : 0);
+// CTAs that a multiprocessor holds: what the cut of single tokens' keys into parts counts on (two_fit in ops/attention_latent.py)
+constexpr int kResident = DV <= 144 && 2 * (kSmemBytes + 1024) <= 228 * 1024 ? 2 : 1;
 
 struct LatentParams {
   const bf16* q;            // [n, heads, DK]
@@ -74,7 +76,7 @@ __device__ __forceinline__ void load_key_tile(bf16* ks, const LatentParams& p, c
   for (int ch = threadIdx.x % kRowThreads; ch < DK / 8; ch += kRowThreads) cp_async_16(ks + ch * 8, src + ch * 8, bytes);
 }
 
-__global__ void __launch_bounds__(NT, 1)
+__global__ void __launch_bounds__(NT, kResident)
 latent_attention_kernel(const LatentParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* qs = reinterpret_cast<bf16*>(smem_raw);

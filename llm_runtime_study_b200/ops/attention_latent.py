@@ -17,6 +17,7 @@ from .native import c_float, c_int, c_void_p
 BACKEND = os.environ.get("LLM_RUNTIME_STUDY_B200_ATTENTION_LATENT", "mma")
 ROWS_PER_TILE = 64
 MAX_SHARED_BYTES = 227 * 1024
+EXCHANGE_BYTES = 8 * 1024       # scores that two warps exchange
 
 _TABLE = {
     "b200_attention_latent_rank": [],
@@ -76,7 +77,7 @@ def latent_attention(q: torch.Tensor, pool: torch.Tensor, ctx: Any, table: torch
     out = torch.empty((n, heads, value_dim), dtype=q.dtype, device=q.device)
     splits, scratch, floats = 1, None, 0
     if decode:
-        splits = decode_splits(n, heads, min(window, ctx.max_kv_len) if window else ctx.max_kv_len, d)
+        splits = decode_splits(n, heads, min(window, ctx.max_kv_len) if window else ctx.max_kv_len, d, value_dim)
         if splits > 1:
             floats = n * heads * splits * (value_dim + 2)
             scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
@@ -104,15 +105,27 @@ def _single_token_tiles(n: int, device) -> tuple[torch.Tensor, torch.Tensor, tor
     return kept[0][:n], kept[0][:n], kept[1][:n]
 
 
-def decode_splits(requests: int, heads: int, keys: int, width: int = 0) -> int:
+def two_fit(width: int, values: int) -> bool:
+    """Whether two CTAs of the kernel for rows of ``width`` columns, ``values`` of them values, fit a multiprocessor: their tiles and
+    the exchange of scores beside them (none below 80 columns or without room) in its 228 KB, a kilobyte of which each CTA takes for
+    itself, and their sums in its registers (beyond 144 value columns a thread needs more than 128)."""
+
+    shared = (ROWS_PER_TILE + 64) * (width + 8) * 2
+    if width >= 80 and shared + EXCHANGE_BYTES <= MAX_SHARED_BYTES:
+        shared += EXCHANGE_BYTES
+    return values <= 144 and 2 * (shared + 1024) <= 228 * 1024
+
+
+def decode_splits(requests: int, heads: int, keys: int, width: int = 0, values: int = 0) -> int:
     """Into how many parts a single token's keys are cut: enough CTAs for two a multiprocessor, no part shorter than four
-    tiles of 32 keys, at most 32 parts.  Rows of ``width`` columns whose tiles take more than half of the shared memory leave room for
-    one CTA: then no more CTAs than multiprocessors, since a second round costs as much as the first (32 requests of 32 heads over
-    777 rows of 576 columns: six parts were 192 CTAs in two rounds, four take one: 57.4 and 36.9 us with the merge)."""
+    tiles of 32 keys, at most 32 parts.  Where only one CTA fits (``two_fit``) no more CTAs than multiprocessors, since a second round costs
+    as much as the first: 32 requests of 32 heads over 777 rows of 576 columns were 192 CTAs in two rounds with six parts and
+    take one with four, 57.4 and 36.9 us with the merge; of 16 heads over rows of 320 columns, 256 of them values, 28.0 and 20.0, over 8,000
+    rows 166 and 137."""
 
     ctas = requests * -(-heads // ROWS_PER_TILE)
-    if (ROWS_PER_TILE + 64) * (width + 8) * 2 > MAX_SHARED_BYTES // 2:
-        wanted = native.sm_count() // max(ctas, 1)
-    else:
+    if two_fit(width, values):
         wanted = -(-2 * native.sm_count() // max(ctas, 1))
+    else:
+        wanted = native.sm_count() // max(ctas, 1)
     return max(1, min(wanted, keys // 128, 32))

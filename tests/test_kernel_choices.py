@@ -138,5 +138,9 @@ def test_parts_of_a_single_tokens_keys_over_shared_rows(monkeypatch):
             assert wide == 1 or wide == 32 or ctas * wide <= 148 < ctas * (wide + 1)
             assert narrow == 32 or ctas * narrow >= 296 > ctas * (narrow - 1)
             assert wide <= narrow
+    # the exchange of scores counts (rows of 416 columns do not fit twice because of it), and so do the registers of many value columns
+    assert attention_latent.two_fit(400, 128) and not attention_latent.two_fit(416, 128) and attention_latent.two_fit(80, 64)
+    assert attention_latent.two_fit(208, 144) and not attention_latent.two_fit(208, 160)
+    assert attention_latent.decode_splits(32, 16, 777, 320, 256) == 4 and attention_latent.decode_splits(32, 16, 777, 192, 128) == 6
     assert attention_latent.decode_splits(8, 32, 2049, 576) == 16
     assert attention_latent.decode_splits(1, 32, 511, 576) == 3 and attention_latent.decode_splits(1, 32, 100, 576) == 1
