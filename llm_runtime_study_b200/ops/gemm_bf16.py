@@ -39,6 +39,7 @@ native.register_library(
 )
 
 PAIR_MIN_ROWS = 256   # from here on pairs of SMs work on 256 x 256 tiles (tcgen05 cta_group::2)
+PAIR_WIDTHS = (128, 192, 224, 256)
 PAIR_ENABLED = os.environ.get("LLM_RUNTIME_STUDY_B200_GEMM_PAIR", "1") != "0"
 SKINNY_M = 16         # up to here weights are streamed straight into mma.sync fragments
 KERNELS = {"persistent": 0, "pair": 1, "streamk": 2, "splitk": 3}
@@ -79,7 +80,12 @@ def pick_kernel(m: int, n: int, k: int) -> tuple[str, int]:
     the SM that has most to pull in, so it pays to spread the bytes over more SMs.  Up to 1,024 columns that
     holds up to 512 rows: 405 x 1024 x 3072 takes 12.9 us with split-K, 20.1 with 128-column tiles and 27.0 with
     stream-K; 405 x 1024 x 2048 12.5 against 17.4.  With more rows split-K's clusters no longer fit at once (600 x 1024 x
-    3072: 23.8 us) and 128-column tiles (20.2) stay ahead of stream-K (27.3)."""
+    3072: 23.8 us) and 128-column tiles (20.2) stay ahead of stream-K (27.3).
+    ("pair", 256) names the kernel's rows of tiles; their width is the kernel's own choice (``b200_gemm_tcgen05_pair_width``).  Against the
+    rules before the pairs' narrower tiles (256 columns only, 128 x 256 tiles one CTA each, long K ranges in 128-column tiles) the choice
+    differs for 1,093 of the products of 130 to 4,096 rows, 128 to 24,576 columns and K of 1,024 to 12,288 that were timed both ways; it takes 0.86 of their
+    time in the mean (405 x 6,144 x 1,024 from cold caches 16.4 us, 18.4 with one CTA a tile).  Two of them are slower, 450 and 1,024 x 8,192 x 4,104 by 5
+    and 7 %: their rows are not whole 128-byte lines.  Up to 384 rows a K range of 8,192 and more keeps the kernels it had."""
 
     sms = native.sm_count()
     if n <= 1024 and 256 < m <= 2048 and 2048 <= k <= 4096:
@@ -142,7 +148,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     ``silu(gate) * up``, half as wide (``"gelu_tanh"``: with that gate).  ``add_to`` (float32 ``[M, N]``): the product is added to it
     in place and it is returned.  ``kernel``: "persistent" (one CTA per tile of 128 rows and
     ``tile_n`` = 128 or 256 columns), "pair" (two CTAs per tile of 256 rows and
-    ``pair_width`` = 128, 192, 224 or 256 columns; 0 lets the kernel choose so that its rounds of tiles are full), "streamk" (few
+    ``pair_width`` = 128, 192, 224 or 256 columns, or ``tile_n`` = 256; neither lets the kernel choose so that its rounds of tiles are full), "streamk" (few
     tiles: up to three SMs share a tile's K range) or "splitk" (few rows: a cluster of ``splits``
     <= 8 CTAs shares the K range of every 128 x ``tile_n`` tile, ``tile_n`` a multiple of 32; 0 for either
     lets the kernel choose so that the SMs are filled once; ``stages``: depth of its operand ring, 0 = as
@@ -169,6 +175,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         out = torch.empty((m, n // 2 if swiglu else n), dtype=out_dtype, device=x.device)
     picked_kernel, picked_width = pick_kernel(m, n, k)
     kernel = kernel or picked_kernel
+    if pair_width and (kernel != "pair" or pair_width not in PAIR_WIDTHS):
+        raise KernelError(f"pair_width {pair_width} is for the pair kernel, and one of {PAIR_WIDTHS}")
+    asked = tile_n
     if kernel == "splitk":
         tile_n = tile_n or 0                        # 0: the kernel chooses
         if tile_n % 32 or not 0 <= tile_n <= 256 or not 0 <= splits <= 8:
@@ -179,7 +188,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
             raise KernelError(f"unknown projection kernel {kernel!r} or tile width {tile_n}: expected one of {sorted(KERNELS)}, "
                               "256 columns, or 128 with the persistent kernel")
     if kernel == "pair":
-        tile_n = pair_width
+        tile_n = pair_width or asked or 0               # 0: the kernel chooses
     partials, flags = _streamk_workspace(x.device) if kernel == "streamk" else (None, None)
     native.call("b200_gemm_tcgen05", x.data_ptr(), weight.data_ptr(), native.ptr(bias), out.data_ptr(), m, n, k,
                 out.shape[1], 1 if out_dtype == torch.float32 else 0, gated_unit(swiglu), 0 if add_to is None else 1,

@@ -727,6 +727,21 @@ def test_tcgen05_pair_widths_give_the_same_bits(m, n, k, width, form):
         torch.testing.assert_close(got.cpu().double(), want, atol=2e-5 * float(want.abs().max()), rtol=0)
 
 
+def test_tcgen05_pair_width_is_asked_for_by_either_name_and_only_of_the_pairs():
+    from llm_runtime_study_b200.errors import KernelError
+
+    x, w, b, want = _gemm_case(300, 1000, 520, True)
+    args = (dev(x), dev(w), dev(b), torch.float32)
+    wide = _gemm().linear(*args, kernel="pair", pair_width=256)
+    for options in ({}, {"tile_n": 256}, {"tile_n": 256, "pair_width": 128}):
+        assert torch.equal(_gemm().linear(*args, kernel="pair", **options), wide)
+    _gemm().check_error()
+    for options in ({"kernel": "persistent", "pair_width": 128}, {"kernel": "splitk", "pair_width": 256}, {"kernel": "pair", "pair_width": 160},
+                    {"kernel": "pair", "tile_n": 128}):
+        with pytest.raises(KernelError, match="width"):
+            _gemm().linear(*args, **options)
+
+
 @pytest.mark.parametrize("kernel", ["pair", "persistent"])
 @pytest.mark.parametrize("m,n,k", [(256, 256, 64), (300, 1000, 520), (2048, 4096, 4096)])
 def test_tcgen05_adds_to_the_residual(m, n, k, kernel):
