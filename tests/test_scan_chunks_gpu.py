@@ -117,6 +117,46 @@ def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens, monke
         assert error(chunked[i], ref) < 1.5 * error(chained[i], ref) + 1e-7
 
 
+def test_the_normalised_read_out_of_every_token():
+    """The matrix memory's read-out over its normaliser, token by token: a token whose normaliser cancels weighs as much as any other.
+    Either sum is off by at most a few float32 roundings of its terms' absolute values (16-bit q, k, v; products of up to 300 decays), and the
+    chunks are no further off than the chain."""
+
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    n, heads, d, dv = 300, 3, 128, 64
+    g = torch.Generator().manual_seed(11)
+    q, k, v = (torch.randn(n, heads, w, generator=g).bfloat16() for w in (d, d, dv))
+    decay, gain = torch.sigmoid(torch.randn(n, heads, generator=g) + 3.0), torch.rand(n, heads, generator=g)
+    dev = lambda x: x.to(DEV).reshape(n, -1)
+    q_start = torch.tensor([0, n], dtype=torch.int32, device=DEV)
+
+    def run(fixed_order):
+        return S.linear_scan_row_gates(dev(q), dev(k), dev(v), heads=heads, dim=d, vdim=dv, decay=dev(decay), gain=dev(gain),
+                                       state=torch.zeros(1, heads, d, dv, device=DEV), norm_state=torch.zeros(1, heads, d, device=DEV),
+                                       q_start=q_start, slots=torch.zeros(1, dtype=torch.int32, device=DEV), fixed_order=fixed_order, lens=[n])
+
+    def reference(q, k, v):
+        wide = decay.double()[..., None].expand(n, heads, d)
+        ones = torch.ones(n, heads, 1, dtype=torch.float64)
+        sums = [_reference(q, k, x, [n], torch.zeros(1, heads, d, x.shape[2], dtype=torch.float64), [0], decay=wide, gain=gain.double(), beta=None)[0]
+                for x in (v, ones)]
+        return sums[0], sums[1][..., 0]
+
+    (out, den), (size, den_size) = (reference(*(f(x.double()) for x in (q, k, v))) for f in (lambda x: x, torch.abs))
+    assert float((den.abs() / den_size).min()) < 1e-3             # some normalisers all but vanish
+    worst = []
+    for fixed in (False, True):
+        got, got_den = (x.double().cpu() for x in run(fixed))
+        off = ((got.view(n, heads, dv) - out).abs() / size).amax(), ((got_den - den).abs() / den_size).amax()
+        ratio, want = got.view(n, heads, dv) / got_den[..., None], out / den[..., None]
+        # the ratio's error in units of what the two sums' roundings make of it
+        scale = (size + want.abs() * den_size[..., None]) / den.abs()[..., None]
+        worst.append(max(*map(float, off), float(((ratio - want).abs() / scale).amax())))
+    # a decay's product over 300 tokens is off by 300 roundings at most, the terms that count by those of the last few dozen tokens
+    assert worst[0] < 5e-6 and worst[0] < 2 * worst[1], worst
+
+
 def test_as_many_rows_as_requests_are_single_tokens_only_when_the_lengths_say_so():
     """Without lengths any cut of ``q_start`` is served, empty requests included; lengths that do not fit are refused."""
 
