@@ -39,7 +39,15 @@ struct ChunkParams {
   const int* q_start; const int* slots;
   int entries, H, Hqk, d, dp, dv, act;             // dp: d rounded up to 32, 64 or 128
   float q_scale;
+  int skip, most;                                  // of every request: tokens before this launch's, tokens in it at most
 };
+
+// The rows of a request that a launch scans.
+struct Portion { int first, count; };
+__device__ __forceinline__ Portion portion_of(const ChunkParams& p, int entry) {
+  const int first = p.q_start[entry], count = p.q_start[entry + 1] - first, skip = min(p.skip, count);
+  return {first + skip, min(p.most, count - skip)};
+}
 
 // A record: Q [16][dp], K [16][dp], (KF [16][dp],) A [16][16], (T [16][16],) whole [dp].
 __host__ __device__ constexpr int record_floats(int dp, bool delta) {
@@ -69,8 +77,9 @@ __global__ void __launch_bounds__(128) scan_chunk_records_kernel(const ChunkPara
   int entry = 0, chunk = blockIdx.x, first = 0, count = 0;
   for (;; ++entry) {
     if (entry == p.entries) return;
-    first = p.q_start[entry];
-    count = p.q_start[entry + 1] - first;
+    const Portion portion = portion_of(p, entry);
+    first = portion.first;
+    count = portion.count;
     const int chunks = (count + C - 1) / C;
     if (chunk < chunks) break;
     chunk -= chunks;
@@ -281,10 +290,11 @@ __global__ void __launch_bounds__(WARPS * 32) scan_chunk_kernel(const ChunkParam
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int d = p.d, dv = p.dv, columns = dv + (ROW ? 1 : 0), col_blocks = (columns + NC - 1) / NC;
   const int h = blockIdx.x / col_blocks, col0 = blockIdx.x % col_blocks * NC, col = col0 + lane, entry = blockIdx.y;
-  const int t_begin = p.q_start[entry], t_end = p.q_start[entry + 1];
+  const Portion portion = portion_of(p, entry);
+  const int t_begin = portion.first, t_end = t_begin + portion.count;
   if (t_begin >= t_end) return;
   int slot0 = 0;                                        // this request's first record
-  for (int e = 0; e < entry; ++e) slot0 += (p.q_start[e + 1] - p.q_start[e] + C - 1) / C;
+  for (int e = 0; e < entry; ++e) slot0 += (portion_of(p, e).count + C - 1) / C;
   const int chunks = (t_end - t_begin + C - 1) / C;
   const bool is_norm = ROW && col == dv, live = col < dv || is_norm;
   const size_t head = static_cast<size_t>(p.slots[entry]) * p.H + h;
@@ -622,18 +632,21 @@ int scan_form(const ChunkParams& p, int chunks, int dtype, int v_dtype, cudaStre
 // The forms of the scan that portions of prompts meet beside 16-bit activations: float32 q, k, v with the delta rule (a decay per
 // channel: gate, or per token: row_decay), float32 q, k beside bfloat16 v or bfloat16 rows with one decay a head (decay), bfloat16
 // rows with a decay per channel (gate) or with row gates (row_decay and row_gain; norm_state, norm_out).  Key sizes up to 128.
-// `chunks`: at least the number of chunks of 16 tokens of all requests; records: chunks * H * b200_scan_chunks_record_floats(d, delta)
-// floats, 16-byte aligned.
+// Of every request's tokens the launch takes those from `skip` on, `most` at most (both multiples of 16 where a request goes on behind
+// them): a long portion's records need not all be there at once, its state goes from launch to launch in the request's slot.
+// `chunks`: at least the number of chunks of 16 tokens of all requests in it; records: chunks * H * b200_scan_chunks_record_floats(d,
+// delta) floats, 16-byte aligned.
 extern "C" long b200_scan_chunks_record_floats(int d, int delta) { return b200::record_floats(b200::padded_dim(d), delta != 0); }
 
 extern "C" int b200_scan_chunks(const void* q, const void* k, const void* v, int ldq, int ldk, int ldv, const float* gate,
                                 const float* decay, const float* row_decay, const float* row_gain, const float* beta, float* state,
                                 float* norm_state, float* norm_out, float* out, float* records, const int* q_start, const int* slots,
-                                int entries, int chunks, int H, int Hqk, int d, int dv, int act, float q_scale, int dtype, int v_dtype,
-                                cudaStream_t stream) {
+                                int entries, int chunks, int skip, int most, int H, int Hqk, int d, int dv, int act, float q_scale,
+                                int dtype, int v_dtype, cudaStream_t stream) {
   using namespace b200;
+  if (skip < 0 || most <= 0 || skip % kChunkTokens != 0) return B200_ERR_BAD_SIZE;
   const ChunkParams p{q, k, v, ldq, ldk, ldv, gate, decay, row_decay, row_gain, beta, state, norm_state, norm_out, out, records,
-                      q_start, slots, entries, H, Hqk, d, 0, dv, act, q_scale};
+                      q_start, slots, entries, H, Hqk, d, 0, dv, act, q_scale, skip, most};
   return scan_form<true>(p, chunks, dtype, v_dtype, stream);
 }
 
@@ -647,6 +660,6 @@ extern "C" int b200_scan_single(const void* q, const void* k, const void* v, int
   using namespace b200;
   if (dv % 4 != 0 || ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(out)) & 15)) return B200_ERR_BAD_SIZE;
   const ChunkParams p{q, k, v, ldq, ldk, ldv, gate, decay, row_decay, row_gain, beta, state, norm_state, norm_out, out, nullptr,
-                      q_start, slots, entries, H, Hqk, d, 0, dv, act, q_scale};
+                      q_start, slots, entries, H, Hqk, d, 0, dv, act, q_scale, 0, 1};
   return scan_form<false>(p, 1, dtype, v_dtype, stream);
 }

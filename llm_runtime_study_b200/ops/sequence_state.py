@@ -14,14 +14,15 @@ from .native import c_float, c_int, c_void_p, call, ptr, require, stream_ptr, ta
 
 native.register_library(
     "b200_scan_chunks", ("scan_chunks.cu",),
-    {"b200_scan_chunks": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, *[c_void_p] * 12, *[c_int] * 7, c_float, c_int, c_int, c_void_p],
+    {"b200_scan_chunks": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, *[c_void_p] * 12, *[c_int] * 9, c_float, c_int, c_int, c_void_p],
      "b200_scan_chunks_record_floats": [c_int, c_int],
      "b200_scan_single": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, *[c_void_p] * 11, *[c_int] * 6, c_float, c_int, c_int, c_void_p]},
 )
 
 CHUNK_TOKENS, CHUNK_MAX_DIM = 16, 128     # tokens a chunk, largest key size of the chunked kernel
 CHUNK_MIN_TOKENS = 48                     # tokens beyond one per request from which a batch may be scanned in chunks
-CHUNK_MAX_BYTES = 1 << 30                 # records of a launch at most (2,048 tokens of 32 heads of 128: 0.11 GB)
+CHUNK_MAX_BYTES = 1 << 30                 # records of a batch at most (2,048 tokens of 32 heads of 128: 0.11 GB)
+CHUNK_SLICE_BYTES = 1 << 27               # of which at most so much is there at once
 MOST_RUNS = 4                             # launches a batch of long and short portions is cut into at most
 
 
@@ -130,14 +131,30 @@ def _parts(plan, lens, n: int):
             yield kind, first, last, n, n // CHUNK_TOKENS + last - first
 
 
-def _scan_chunks(q, k, v, *, chunks, heads, qk_heads, dim, vdim, state, q_start, slots, out, gate=None, decay=None, row_decay=None, row_gain=None,
+def chunk_slices(lens: "Sequence[int] | None", n: int, entries: int, chunks: int, chunk_bytes: int) -> "list[tuple[int, int, int]]":
+    """The launches of portions scanned in chunks, ``(skip, most, chunks)``: of every request the tokens from ``skip`` on, ``most`` at
+    most, ``chunks`` of them in all.  One launch as long as the records of all chunks take no more than ``CHUNK_SLICE_BYTES``, else as many
+    tokens of every request at a time as fit (a chunk of each at least)."""
+
+    fit = CHUNK_SLICE_BYTES // chunk_bytes
+    if chunks <= fit:
+        return [(0, max(n, 1), chunks)]
+    most = CHUNK_TOKENS * max(1, fit // entries)
+    longest = max(lens) if lens else n
+    return [(skip, most, sum(-(-min(most, max(0, m - skip)) // CHUNK_TOKENS) for m in lens) if lens else most // CHUNK_TOKENS * entries)
+            for skip in range(0, longest, most)]
+
+
+def _scan_chunks(q, k, v, *, chunks, lens, heads, qk_heads, dim, vdim, state, q_start, slots, out, gate=None, decay=None, row_decay=None, row_gain=None,
                  beta=None, norm_state=None, norm_out=None, silu=False, q_scale=1.0) -> None:
     entries = slots.shape[0]
     floats = native.query("b200_scan_chunks_record_floats", dim, 0 if beta is None else 1)
-    records = torch.empty(chunks * heads * floats, dtype=torch.float32, device=q.device)
-    call("b200_scan_chunks", ptr(q), ptr(k), ptr(v), q.stride(0), k.stride(0), v.stride(0), ptr(gate), ptr(decay), ptr(row_decay),
-         ptr(row_gain), ptr(beta), ptr(state), ptr(norm_state), ptr(norm_out), ptr(out), ptr(records), ptr(q_start), ptr(slots), entries, chunks,
-         heads, qk_heads, dim, vdim, 1 if silu else 0, float(q_scale), tag(q.dtype), tag(v.dtype), stream_ptr(), launches=2)
+    slices = chunk_slices(lens, q.shape[0], entries, chunks, heads * floats * 4)
+    records = torch.empty(max(held for _, _, held in slices) * heads * floats, dtype=torch.float32, device=q.device)
+    for skip, most, held in slices:
+        call("b200_scan_chunks", ptr(q), ptr(k), ptr(v), q.stride(0), k.stride(0), v.stride(0), ptr(gate), ptr(decay), ptr(row_decay),
+             ptr(row_gain), ptr(beta), ptr(state), ptr(norm_state), ptr(norm_out), ptr(out), ptr(records), ptr(q_start), ptr(slots), entries, held,
+             skip, most, heads, qk_heads, dim, vdim, 1 if silu else 0, float(q_scale), tag(q.dtype), tag(v.dtype), stream_ptr(), launches=2)
 
 
 def scans_single(n: int, entries: int, dim: int, vdim: int, fixed_order: bool, lens: "Sequence[int] | None" = None) -> bool:
@@ -220,7 +237,7 @@ def linear_scan(
         if kind == "single" and state.data_ptr() % 16 == 0:
             _scan_single(q, k, v, **shared)
         elif kind == "chunks":
-            _scan_chunks(q, k, v, chunks=chunks, **shared)
+            _scan_chunks(q, k, v, chunks=chunks, lens=lens[first:last] if lens else None, **shared)
         else:
             call("b200_linear_scan", ptr(q), ptr(k), ptr(v), q.stride(0), k.stride(0), v.stride(0), ptr(gate), heads * dim, ptr(decay),
                  ptr(row_decay), ptr(beta), heads, ptr(state), ptr(out), heads * vdim, ptr(starts), ptr(at), last - first, rows, heads, qk_heads, dim, vdim,
@@ -266,7 +283,7 @@ def linear_scan_row_gates(
         if kind == "single" and state.data_ptr() % 16 == 0:
             _scan_single(q, k, v, **shared)
         elif kind == "chunks":
-            _scan_chunks(q, k, v, chunks=chunks, **shared)
+            _scan_chunks(q, k, v, chunks=chunks, lens=lens[first:last] if lens else None, **shared)
         else:
             call("b200_linear_scan_row_gates", ptr(q), ptr(k), ptr(v), q.stride(0), k.stride(0), v.stride(0), ptr(decay), ptr(gain), ptr(state),
                  ptr(norm_state), ptr(out), ptr(norm_out), ptr(starts), ptr(at), last - first, rows, heads, dim, vdim, float(q_scale),

@@ -100,6 +100,23 @@ def test_which_scans_go_in_chunks():
     assert not S.scans_single(8, 8, 128, 33, False) and not S.scans_single(8, 8, 129, 64, False) and not S.scans_single(8, 8, 128, 64, True)
 
 
+def test_records_of_long_portions_come_in_slices():
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    chunk = 32 * 27_136                      # 32 heads of 128, the delta rule
+    fit = S.CHUNK_SLICE_BYTES // chunk
+    assert S.chunk_slices([2048], 2048, 1, 128, chunk) == [(0, 2048, 128)]
+    for lens in ([16_000], [5_000, 300, 9_001], [17_000, 1]):
+        whole = sum(-(-m // 16) for m in lens)
+        for known in (lens, None):
+            slices = S.chunk_slices(known, sum(lens), len(lens), whole if known else sum(lens) // 16 + len(lens), chunk)
+            assert max(held for _, _, held in slices) <= fit
+            assert all(skip % 16 == most % 16 == 0 for skip, most, _ in slices)
+            assert slices[-1][0] + slices[-1][1] >= max(lens) and [s[0] for s in slices[1:]] == [s[0] + s[1] for s in slices[:-1]]
+            if known:
+                assert sum(held for _, _, held in slices) == whole
+
+
 def test_which_portions_go_in_chunks(monkeypatch):
     """By a portion's own length: many short ones beside each other, or single tokens beside a long one, are no reason."""
 

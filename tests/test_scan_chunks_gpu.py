@@ -117,6 +117,38 @@ def test_chunks_against_the_recurrence(form, heads, qk_heads, d, dv, lens, monke
         assert error(chunked[i], ref) < 1.5 * error(chained[i], ref) + 1e-7
 
 
+@pytest.mark.parametrize("form", ["row", "delta"])
+@pytest.mark.parametrize("known", [True, False])
+def test_records_in_slices_give_the_same_bits(form, known, monkeypatch):
+    """Portions whose records do not fit at once, in launches that follow each other: the state goes through the request's slot as the
+    same float32 numbers, so nothing changes.  Portions that end inside a slice, at its end and behind it, empty ones among them."""
+
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    heads, d, dv, lens = 2, 40, 33, [130, 64, 63, 65] if known else [130, 64, 0, 63, 65]
+    n, entries = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(3)
+    rand = lambda *shape: torch.rand(*shape, generator=g).to(DEV)
+    q, k, v = (rand(n, heads * w) - 0.5 for w in (d, d, dv))
+    token, other, state, norm_state = rand(n, heads), rand(n, heads), rand(entries, heads, d, dv), rand(entries, heads, d)
+    q_start = torch.tensor([sum(lens[:i]) for i in range(entries + 1)], dtype=torch.int32, device=DEV)
+    common = dict(heads=heads, dim=d, vdim=dv, q_start=q_start, slots=torch.arange(entries, dtype=torch.int32, device=DEV),
+                  lens=lens if known else None)
+    monkeypatch.setattr(S, "portion_in_chunks", lambda *sizes: 1)
+
+    def run():
+        s, ns = state.clone(), norm_state.clone()
+        if form == "row":
+            return *S.linear_scan_row_gates(*(x.bfloat16() for x in (q, k, v)), decay=token, gain=other, state=s, norm_state=ns, **common), s, ns
+        return S.linear_scan(q, k, v, qk_heads=heads, row_decay=token, beta=other, state=s, **common), s
+
+    whole = run()
+    for slice_bytes in (1, 1 << 18):         # a chunk of every request a launch; about two
+        monkeypatch.setattr(S, "CHUNK_SLICE_BYTES", slice_bytes)
+        for a, b in zip(run(), whole):
+            assert torch.equal(a, b)
+
+
 def test_the_normalised_read_out_of_every_token():
     """The matrix memory's read-out over its normaliser, token by token: a token whose normaliser cancels weighs as much as any other.
     Either sum is off by at most a few float32 roundings of its terms' absolute values (16-bit q, k, v; products of up to 300 decays), and the
