@@ -80,7 +80,8 @@ def pick_kernel(m: int, n: int, k: int) -> tuple[str, int]:
     the SM that has most to pull in, so it pays to spread the bytes over more SMs.  Up to 1,024 columns that
     holds up to 512 rows: 405 x 1024 x 3072 takes 12.9 us with split-K, 20.1 with 128-column tiles and 27.0 with
     stream-K; 405 x 1024 x 2048 12.5 against 17.4.  With more rows split-K's clusters no longer fit at once (600 x 1024 x
-    3072: 23.8 us) and 128-column tiles (20.2) stay ahead of stream-K (27.3).
+    3072: 23.8 us) and 128-column tiles (20.2) stay ahead of stream-K (27.3).  Up to 96 columns its tiles are narrow
+    and a short K range is not worth sharing (300 x 64 x 2048: 12.9 us against 11.8; x 2560: 13.5 against 13.6).
     ("pair", 256) names the kernel's rows of tiles; their width is the kernel's own choice (``b200_gemm_tcgen05_pair_width``).  Against the
     rules before the pairs' narrower tiles (256 columns only, 128 x 256 tiles one CTA each, long K ranges in 128-column tiles) the choice
     differs for 1,093 of the products of 130 to 4,096 rows, 128 to 24,576 columns and K of 1,024 to 12,288 that were timed both ways; it takes 0.86 of their
@@ -89,7 +90,7 @@ def pick_kernel(m: int, n: int, k: int) -> tuple[str, int]:
 
     sms = native.sm_count()
     if n <= 1024 and 256 < m <= 2048 and 2048 <= k <= 4096:
-        return ("splitk", 0) if m <= 512 else ("persistent", 128)
+        return ("splitk", 0) if m <= 512 and (n > 96 or k >= 2560) else ("persistent", 128)
     if m >= PAIR_MIN_ROWS and PAIR_ENABLED and 5 * -(-m // 256) * -(-n // 256) >= 2 * sms:   # 60 of a B200's 74 pairs
         return "pair", 256
     tiles = -(-m // 128) * -(-n // 256)

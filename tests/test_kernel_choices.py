@@ -46,6 +46,12 @@ def test_projections_to_few_columns():
         assert gemm_bf16.pick_kernel(513, 1024, k) == gemm_bf16.pick_kernel(2048, 264, k) == ("persistent", 128)
 
 
+def test_projections_to_very_few_columns_share_only_long_k_ranges():
+    for m in (257, 512):
+        assert gemm_bf16.pick_kernel(m, 64, 2304) == gemm_bf16.pick_kernel(m, 96, 2048) == ("persistent", 128)
+        assert gemm_bf16.pick_kernel(m, 64, 2560) == gemm_bf16.pick_kernel(m, 104, 2048) == ("splitk", 0)
+
+
 def test_decode_parts_are_bounded_and_use_the_gpu():
     for requests, kv_heads, longest, slots in itertools.product((1, 3, 8, 64, 500), (1, 8), (1, 100, 2048, 32768, 1 << 20), (296, 592)):
         parts = attention_bf16.decode_splits(requests, kv_heads, 1, longest, slots)
