@@ -242,6 +242,54 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, co
   }
 }
 
+// ------------------------------------------------------------------------------------------ short rows
+// K of at most one segment: 64 x 64 tiles, 4 x 4 outputs a thread, one buffer.  The tiles above prepare for long K (two steps of
+// loads ahead, sums of segments in shared memory), which costs more than it saves in a few steps of kBK columns: 24 x 39 x 19 3.1 us
+// against 4.8, 509 x 753 x 35 4.9 against 6.1, 8 x 1441 x 95 6.8 against 7.3.
+__global__ void __launch_bounds__(256)
+gemm_f32_short_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                      float* __restrict__ C, int M, int N, int K, int lda, int ldc) {
+  constexpr int BM = 64, BN = 64, BK = kBK;
+  __shared__ float As[BK][BM + 4], Ws[BK][BN + 4];
+  pdl_trigger();
+  pdl_wait();
+  const int tid = threadIdx.x, m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int tx = tid & 15, ty = tid >> 4, lrow = tid >> 2, lk = (tid & 3) * 4;
+  float acc[4][4] = {};
+  for (int k0 = 0; k0 < K; k0 += BK) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = k0 + lk + i, am = m0 + lrow, wn = n0 + lrow;
+      As[lk + i][lrow] = am < M && k < K ? A[static_cast<size_t>(am) * lda + k] : 0.f;
+      Ws[lk + i][lrow] = wn < N && k < K ? W[static_cast<size_t>(wn) * K + k] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      float a[4], w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = Ws[k][tx * 4 + j];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + ty * 4 + i;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int n = n0 + tx * 4 + j;
+      if (n < N) C[static_cast<size_t>(m) * ldc + n] = acc[i][j] + (bias ? bias[n] : 0.f);
+    }
+  }
+}
+
 template <int BM, int BN, int TM, int TN, bool VEC>
 int launch_tiles(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, cudaStream_t stream) {
   static DeviceOnce once;
@@ -279,7 +327,7 @@ int launch_few(const float* A, const float* W, const float* bias, float* C, int 
 
 }  // namespace b200
 
-// `kernel`: 0 chooses by size; 1: few rows, 2: tiles of 64 x 64, 3: tiles of 128 x 64 (for tests and measurements).
+// `kernel`: 0 chooses by size; 1: few rows, 2: tiles of 64 x 64, 3: tiles of 128 x 64, 4: short rows (for tests and measurements).
 extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,
                                      int ldc, int kernel, cudaStream_t stream) {
   using namespace b200;
@@ -295,7 +343,16 @@ extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float
     // x 1024 37.5 against 39.0, 24 x 1024 x 3072 25.6 against 37.8, 64 x 6144 x 1024 83 against 40.
     // Tiles of 128 rows do a third more arithmetic per byte of shared memory read; where they would be fewer than about
     // 1.7 an SM, tiles of 64 fill the SMs better (509 x 4096 x 1024: 109 us against 116; 509 x 1024 x 3072: 109 against 89).
-    if (vec && (M <= 8 || (M <= 24 && small < 148))) kernel = 1;
+    // Few rows: up to about seven CTAs an SM at once (ten up to four rows), 8 us a round of them from K of 128 on (K beyond 512: as the weights
+    // stream), where tiles take 3 us and 0.034 a column.  So beyond one round a short K goes to tiles (9 x 6400 x 256: 15.6 us against
+    // 12.2, 24 x 9400 x 1024: 48 against 38), and so does K up to 160 beyond four rows (8 x 6400 x 64: 6.1 against 5.6, 20 x 2880 x 64: 9.0 against 5.4).
+    // Short rows: up to 112 columns that are not whole 16-byte vectors and up to 32 that are, while the tiles are few.
+    const long long ctas = static_cast<long long>((N + kRowsW - 1) / kRowsW) * ((M + 7) / 8), rounds = (ctas + 7 * 148 - 1) / (7 * 148);
+    const float few_us = rounds * (8.f + (K > 512 ? (K - 512) / 128.f : 0.f)), tiles_us = 3.f + 0.034f * (K < 1024 ? K : 1024);
+    const bool few = M <= 2 || (M <= 4 && (K > 160 || ctas <= 10 * 148)) || (M <= 8 && K >= 512) ||
+                     (K > 160 && (M <= 8 || (M <= 24 && small < 148)) && few_us <= tiles_us);
+    if (vec && few) kernel = 1;
+    else if (K <= (vec ? 32 : 112) && small <= 512) kernel = 4;
     else kernel = large >= 250 && M > 64 ? 3 : 2;
   }
   if ((M + 63) / 64 > 65535) return B200_ERR_TOO_LARGE;
@@ -305,6 +362,11 @@ extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float
     if (M == 2) return launch_few<2>(A, W, bias, C, M, N, K, lda, ldc, stream);
     if (M <= 4) return launch_few<4>(A, W, bias, C, M, N, K, lda, ldc, stream);
     return launch_few<8>(A, W, bias, C, M, N, K, lda, ldc, stream);
+  }
+  if (kernel == 4) {
+    if (K > kSegment) return B200_ERR_BAD_SIZE;
+    launch(gemm_f32_short_kernel, dim3((N + 63) / 64, (M + 63) / 64), dim3(256), 0, stream, A, W, bias, C, M, N, K, lda, ldc);
+    return launch_status();
   }
   if (kernel == 3)
     return vec ? launch_tiles<128, 64, 8, 8, true>(A, W, bias, C, M, N, K, lda, ldc, stream)

@@ -121,6 +121,21 @@ def test_gemm_f32_kernels_agree_bit_for_bit(m, n, k):
     assert float((results[0].double() - want).abs().max()) < 6e-8 * 200 * math.sqrt(k)
 
 
+# one column, a step of 16 and its edges, the longest K that the choice sends there and the longest it takes, one tile and parts of further ones
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (64, 64, 16), (65, 63, 17), (100, 130, 112), (3, 70, 127), (9, 5, 128)])
+def test_gemm_f32_of_short_rows_gives_the_bits_of_the_tiles(m, n, k):
+    from llm_runtime_study_b200.ops import native
+
+    torch.manual_seed(5)
+    x, w, b = dev(torch.randn(m, k)), dev(torch.randn(n, k)), dev(torch.randn(n))
+    results = [F().linear_f32(x, w, b)]
+    for kernel in (4, 2, 3):
+        out = torch.full((m, n), float("nan"), device=x.device)
+        native.call("b200_gemm_f32_variant", x.data_ptr(), w.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, k, n, kernel, native.stream_ptr())
+        results.append(out)
+    assert all(torch.equal(out, results[0]) for out in results[1:])
+
+
 def _scatter_to_pages(k, v, page_size, nkv, d, dtype, seed=0, extra_pages=3):
     """Put contiguous k, v [T, nkv, d] into shuffled pages; return pools + table row."""
 
