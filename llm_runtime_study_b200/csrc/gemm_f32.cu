@@ -345,11 +345,12 @@ extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float
     // 1.7 an SM, tiles of 64 fill the SMs better (509 x 4096 x 1024: 109 us against 116; 509 x 1024 x 3072: 109 against 89).
     // Few rows: up to about seven CTAs an SM at once (ten up to four rows), 8 us a round of them from K of 128 on (K beyond 512: as the weights
     // stream), where tiles take 3 us and 0.034 a column.  So beyond one round a short K goes to tiles (9 x 6400 x 256: 15.6 us against
-    // 12.2, 24 x 9400 x 1024: 48 against 38), and so does K up to 160 beyond four rows (8 x 6400 x 64: 6.1 against 5.6, 20 x 2880 x 64: 9.0 against 5.4).
+    // 12.2, 24 x 9400 x 1024: 48 against 38), and so does K up to 160 beyond four rows (8 x 6400 x 64: 6.1 against 5.6, 20 x 2880 x 64: 9.0 against 5.4)
+    // except K up to 64 in a third of a round (8 x 64 x 64: 4.9 against 5.4, 24 x 512 x 64: 5.4 both).
     // Short rows: up to 112 columns that are not whole 16-byte vectors and up to 32 that are, while the tiles are few.
     const long long ctas = static_cast<long long>((N + kRowsW - 1) / kRowsW) * ((M + 7) / 8), rounds = (ctas + 7 * 148 - 1) / (7 * 148);
     const float few_us = rounds * (8.f + (K > 512 ? (K - 512) / 128.f : 0.f)), tiles_us = 3.f + 0.034f * (K < 1024 ? K : 1024);
-    const bool few = M <= 2 || (M <= 4 && (K > 160 || ctas <= 10 * 148)) || (M <= 8 && K >= 512) ||
+    const bool few = M <= 2 || (M <= 24 && K <= 64 && ctas <= 400) || (M <= 4 && (K > 160 || ctas <= 10 * 148)) || (M <= 8 && K >= 512) ||
                      (K > 160 && (M <= 8 || (M <= 24 && small < 148)) && few_us <= tiles_us);
     if (vec && few) kernel = 1;
     else if (K <= (vec ? 32 : 112) && small <= 512) kernel = 4;
