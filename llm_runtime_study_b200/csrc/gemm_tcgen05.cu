@@ -35,10 +35,6 @@ __device__ int g_gemm_error = 0;
 // ------------------------------------------------------------------ the shared wrappers, as this file names them
 // (mbarrier, TMA, fences, descriptors and tcgen05.ld live in tcgen05.cuh, shared with the attention kernels)
 
-// The wait as a converged warp runs it: every lane waits, and all lanes get the same answer.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity) ? 1 : 0) != 0;
-}
 // shared-memory matrix descriptor: K-major tile, 128-byte swizzle, 8-row groups 1024 bytes apart
 __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_byte_addr) { return umma_desc_sw128(smem_byte_addr, 16, 1024); }
 // instruction descriptor, kind::f16: D = f32, A = B = bf16, both K-major, M = 128, N = n
@@ -112,11 +108,31 @@ struct GemmParams {
   int gate_act;       // SWIGLU: ACT_SILU or ACT_GELU_TANH
 };
 
+// What C holds in 32 columns of a row of it from column nb on, asked for a chunk ahead of its use (from L2 or HBM it takes
+// as long as the chunk before it: 2,048 x 4,096 x 4,096 59.1 us without, 56.4 with it and the shorter set-up).
+template <bool SWIGLU, typename OutT>
+__device__ __forceinline__ void held_chunk(float (&have)[32], const GemmParams& p, const OutT* crow, int m, int nb) {
+  if constexpr (!SWIGLU && sizeof(OutT) == 4) {
+    if (!p.accumulate || m >= p.M) return;
+    if (p.vector_ok && nb + 32 <= p.N) {
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) {
+        const float4 e = *reinterpret_cast<const float4*>(crow + nb + j);
+        have[j] = e.x; have[j + 1] = e.y; have[j + 2] = e.z; have[j + 3] = e.w;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) have[j] = nb + j < p.N ? crow[nb + j] : 0.f;
+    }
+  }
+}
+
 // What the epilogue does with 32 consecutive accumulator columns of one row, starting at column nb of
 // the product: bias, then either SiLU(gate) * up (or another gate) on interleaved blocks of eight, or the optional sum
 // with what C holds, then conversion and 16-byte stores where the row allows them.
+// `have`: what C holds there (held_chunk), where the product is added to it.
 template <bool SWIGLU, typename OutT>
-__device__ __forceinline__ void finish_chunk(float (&v)[32], const GemmParams& p, OutT* crow, int nb) {
+__device__ __forceinline__ void finish_chunk(float (&v)[32], const float (&have)[32], const GemmParams& p, OutT* crow, int nb) {
   if (p.bias) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] += nb + j < p.N ? p.bias[nb + j] : 0.f;
@@ -153,18 +169,8 @@ __device__ __forceinline__ void finish_chunk(float (&v)[32], const GemmParams& p
     const bool whole = p.vector_ok && nb + 32 <= p.N;
     if constexpr (sizeof(OutT) == 4) {
       if (p.accumulate) {
-        const float* have = reinterpret_cast<const float*>(crow) + nb;
-        if (whole) {
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const float4 e = *reinterpret_cast<const float4*>(have + j);
-            v[j] += e.x; v[j + 1] += e.y; v[j + 2] += e.z; v[j + 3] += e.w;
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (nb + j < p.N) v[j] += have[j];
-        }
+        for (int j = 0; j < 32; ++j) v[j] += have[j];
       }
     }
     if (whole) {
@@ -204,17 +210,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_rows, con
   const int tiles = m_tiles * n_tiles;
   const int num_kb = (p.K + BK - 1) / BK;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full + s, 1);
-      mbar_init(empty + s, 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(acc_full + b, 1);
-      mbar_init(acc_empty + b, 4);     // one arrival per epilogue warp
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
+  if (warp == 0) mbar_init_warp(full, 2 * STAGES + 4, 2, 4);    // acc_empty: one arrival per epilogue warp
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(tmem_slot)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -292,22 +288,27 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_rows, con
       const uint32_t acc_phase = (local >> 1) & 1;
       ++local;
       const int row0 = (tile % m_tiles) * BM, col0 = (tile / m_tiles) * BN;
+      const int m = row0 + row;
+      OutT* crow = static_cast<OutT*>(p.c) + static_cast<size_t>(m) * p.ldc;
+      float next[32];
+      held_chunk<SWIGLU, OutT>(next, p, crow, m, col0);
       const bool ok = mbar_wait(acc_full + buf, acc_phase);
       if (!ok) atomicExch(&g_gemm_error, 3);
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN;
-      const int m = row0 + row;
-      OutT* crow = static_cast<OutT*>(p.c) + static_cast<size_t>(m) * p.ldc;
 #pragma unroll 1
       for (int c = 0; c < BN; c += 32) {
-        float v[32];
+        float v[32], have[32];
         if (ok) {
           tmem_load_32(taddr + c, v);
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = 0.f;
         }
-        if (m < p.M) finish_chunk<SWIGLU, OutT>(v, p, crow, col0 + c);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) have[j] = next[j];
+        if (c + 32 < BN) held_chunk<SWIGLU, OutT>(next, p, crow, m, col0 + c + 32);
+        if (m < p.M) finish_chunk<SWIGLU, OutT>(v, have, p, crow, col0 + c);
       }
       tcgen05_fence_before();
       __syncwarp();
@@ -336,50 +337,6 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_rows, con
 // for the bytes of both); the leader's commit arrives on `empty` in both CTAs.  Per tile: the
 // leader's commit arrives on `acc_full` in both CTAs; the eight epilogue warps of the pair arrive
 // on the leader's `acc_empty`.
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_address, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(out) : "r"(smem_address), "r"(rank));
-  return out;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-// TMA copy into this CTA's shared memory whose bytes are counted on a barrier of the pair's leader
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t leader_bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n" ::"r"(
-          smem_addr(dst)),
-      "l"(map), "r"(leader_bar), "r"(x), "r"(y)
-      : "memory");
-}
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// arrives, once the MMAs issued so far have finished, on the barrier at this address in both CTAs of the pair
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  const uint16_t both = 3;
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(
-                   smem_addr(bar)),
-               "h"(both)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_address) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_address) : "memory");
-}
-// instruction descriptor for the pair: M = 256 (128 rows per CTA)
-__host__ __device__ constexpr uint32_t umma_idesc_pair(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
-}
-
 template <int BN, int STAGES, bool SWIGLU, typename OutT>
 __global__ void __launch_bounds__(kThreads)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, GemmParams p) {
@@ -404,17 +361,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __g
   const int tiles = m_tiles * n_tiles;
   const int num_kb = (p.K + BK - 1) / BK;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full + s, 1);
-      mbar_init(empty + s, 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(acc_full + b, 1);
-      mbar_init(acc_empty + b, 8);     // one arrival per epilogue warp of the pair
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
+  if (warp == 0) mbar_init_warp(full, 2 * STAGES + 4, 2, 8);    // acc_empty: one arrival per epilogue warp of the pair
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(tmem_slot)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
@@ -484,22 +431,27 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __g
       const int buf = local & 1;
       const uint32_t acc_phase = (local >> 1) & 1;
       const int row0 = (tile % m_tiles) * PAIR_M + static_cast<int>(rank) * BM, col0 = (tile / m_tiles) * BN;
+      const int m = row0 + row;
+      OutT* crow = static_cast<OutT*>(p.c) + static_cast<size_t>(m) * p.ldc;
+      float next[32];
+      held_chunk<SWIGLU, OutT>(next, p, crow, m, col0);
       const bool ok = mbar_wait(acc_full + buf, acc_phase);
       if (!ok) atomicExch(&g_gemm_error, 3);
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * ACC;
-      const int m = row0 + row;
-      OutT* crow = static_cast<OutT*>(p.c) + static_cast<size_t>(m) * p.ldc;
 #pragma unroll 1
       for (int c = 0; c < BN; c += 32) {
-        float v[32];
+        float v[32], have[32];
         if (ok) {
           tmem_load_32(taddr + c, v);
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = 0.f;
         }
-        if (m < p.M) finish_chunk<SWIGLU, OutT>(v, p, crow, col0 + c);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) have[j] = next[j];
+        if (c + 32 < BN) held_chunk<SWIGLU, OutT>(next, p, crow, m, col0 + c + 32);
+        if (m < p.M) finish_chunk<SWIGLU, OutT>(v, have, p, crow, col0 + c);
       }
       tcgen05_fence_before();
       __syncwarp();
@@ -510,7 +462,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __g
   __syncwarp();
   tcgen05_fence_before();
   __syncthreads();
-  cluster_sync_all();                     // the leader's MMAs read this CTA's shared memory until its last commit
+  cluster_sync_relaxed();                 // the leader's MMAs read this CTA's shared memory until its last commit
   if (warp == 1) {
     __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
@@ -600,17 +552,7 @@ gemm_tcgen05_streamk_kernel(const __grid_constant__ CUtensorMap map_rows, const 
   plan.sharers = static_cast<int>(min(static_cast<long long>(min(plan.ctas, 3 * left)), plan.left_units));
   const int cta = blockIdx.x;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full + s, 1);
-      mbar_init(empty + s, 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(acc_full + b, 1);
-      mbar_init(acc_empty + b, 4);     // one arrival per epilogue warp
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
+  if (warp == 0) mbar_init_warp(full, 2 * STAGES + 4, 2, 4);    // acc_empty: one arrival per epilogue warp
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(tmem_slot)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -721,8 +663,9 @@ gemm_tcgen05_streamk_kernel(const __grid_constant__ CUtensorMap map_rows, const 
       OutT* crow = static_cast<OutT*>(p.c) + static_cast<size_t>(m) * p.ldc;
 #pragma unroll 1
       for (int c = 0; c < BN; c += 32) {
-        float v[32];
+        float v[32], have[32];
         float4 t[2][8];
+        held_chunk<SWIGLU, OutT>(have, p, crow, m, col0 + c);
         const int partners = last_partner - cta;
         // the loads of up to two partners are in flight while the accumulator comes out of TMEM
 #pragma unroll
@@ -752,7 +695,7 @@ gemm_tcgen05_streamk_kernel(const __grid_constant__ CUtensorMap map_rows, const 
             v[4 * j] += e.x; v[4 * j + 1] += e.y; v[4 * j + 2] += e.z; v[4 * j + 3] += e.w;
           }
         }
-        if (m < p.M) finish_chunk<SWIGLU, OutT>(v, p, crow, col0 + c);
+        if (m < p.M) finish_chunk<SWIGLU, OutT>(v, have, p, crow, col0 + c);
       }
       tcgen05_fence_before();
       __syncwarp();
@@ -817,14 +760,7 @@ gemm_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_rows, const _
   const int kb0 = static_cast<int>(static_cast<long long>(num_kb) * part / splits);
   const int kb1 = static_cast<int>(static_cast<long long>(num_kb) * (part + 1) / splits);
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) {
-      mbar_init(full + s, 1);
-      mbar_init(empty + s, 1);
-    }
-    mbar_init(acc_full, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
+  if (warp == 0) mbar_init_warp(full, 2 * stages + 1, 0, 1);
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(tmem_slot)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -899,14 +835,15 @@ gemm_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_rows, const _
       if (quarter * 32 < rows) {
 #pragma unroll 1
         for (int c = 0; c < bn; c += 32) {
-          float v[32];
+          float v[32], have[32];
+          held_chunk<SWIGLU, OutT>(have, p, crow, m, col0 + c);
           if (ok) {
             tmem_load_32(taddr + c, v);
           } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = 0.f;
           }
-          if (m < p.M) finish_chunk<SWIGLU, OutT>(v, p, crow, col0 + c);
+          if (m < p.M) finish_chunk<SWIGLU, OutT>(v, have, p, crow, col0 + c);
         }
       }
     } else if (quarter * 32 < rows) {     // warps whose 32 rows all lie below the matrix have nothing to hand over
@@ -928,13 +865,17 @@ gemm_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_rows, const _
     }
   }
   if (splits > 1) {
+    const int pieces = rows * (bn / 32);
+    const int begin = static_cast<int>(static_cast<long long>(pieces) * part / splits);
+    const int end = static_cast<int>(static_cast<long long>(pieces) * (part + 1) / splits);
+    auto c_row = [&](int u) { return static_cast<OutT*>(p.c) + static_cast<size_t>(row0 + u % rows) * p.ldc; };
+    float have[32];
+    if (const int u = begin + static_cast<int>(threadIdx.x) - 64; warp >= 2 && u < end)
+      held_chunk<SWIGLU, OutT>(have, p, c_row(u), row0, col0 + u / rows * 32);
     __syncwarp();
     cluster_sync_all();                   // every CTA's partial accumulator is in its shared memory
     if (warp >= 2) {
       const uint32_t base = smem_addr(smem);
-      const int pieces = rows * (bn / 32);
-      const int begin = static_cast<int>(static_cast<long long>(pieces) * part / splits);
-      const int end = static_cast<int>(static_cast<long long>(pieces) * (part + 1) / splits);
 #pragma unroll 1
       for (int u = begin + static_cast<int>(threadIdx.x) - 64; u < end; u += 128) {
         const int chunk = u / rows, r = u - chunk * rows;
@@ -961,12 +902,12 @@ gemm_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_rows, const _
               }
             }
         }
-        const int m = row0 + r;
-        finish_chunk<SWIGLU, OutT>(v, p, static_cast<OutT*>(p.c) + static_cast<size_t>(m) * p.ldc, col0 + chunk * 32);
+        finish_chunk<SWIGLU, OutT>(v, have, p, c_row(u), col0 + chunk * 32);
+        if (u + 128 < end) held_chunk<SWIGLU, OutT>(have, p, c_row(u + 128), row0, col0 + (u + 128) / rows * 32);
       }
     }
     __syncwarp();
-    cluster_sync_all();                   // nobody leaves while another CTA still reads its shared memory
+    cluster_sync_relaxed();               // nobody leaves while another CTA still reads its shared memory
   }
   __syncwarp();
   tcgen05_fence_before();
