@@ -38,6 +38,16 @@ native.register_library(
     },
 )
 
+native.register_library(
+    "b200_gemm_features", ("gemm_features.cu",),
+    {
+        "b200_gemm_features": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                               c_void_p],
+        "b200_gemm_features_error": [],
+        "b200_gemm_features_shape": [c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
+    },
+)
+
 PAIR_MIN_ROWS = 256   # from here on pairs of SMs work on 256 x 256 tiles (tcgen05 cta_group::2)
 PAIR_WIDTHS = (128, 192, 224, 256)
 PAIR_ENABLED = os.environ.get("LLM_RUNTIME_STUDY_B200_GEMM_PAIR", "1") != "0"
@@ -105,6 +115,27 @@ def pick_kernel(m: int, n: int, k: int) -> tuple[str, int]:
     return "persistent", 128
 
 
+def by_features(m: int, n: int, k: int, out_float32: bool) -> bool:
+    """Whether a product of this shape goes to the kernel that has the weight as its row operand (``linear_features``) and not to the one that
+    ``pick_kernel`` names.  Timed both ways at 18 numbers of rows (17 to 2,048), 11 of columns (256 to 12,288) and 8 of K (512 to
+    12,288), float32 sums and bfloat16 results.  Float32 rows are what it writes best: it is ahead from 129 rows on (0.40 to 0.97 of the time, 0.75
+    in the mean) but where other kernels fill the GPU better: around 2,048 columns up to 256 rows (1.05 to 1.14), 8,192
+    and more columns beyond 1,024 rows (0.97 to 1.05), short K with many rows (1.06 to 1.17).  Of the bfloat16 results those with few tiles
+    and a long K range (257 to 512 rows up to 4,096 columns 0.48 to 1.07, mean 0.73; to 1,024 rows up to 2,048 columns 0.51 to 0.99), 129
+    to 256 rows whose 128-row tiles are half empty (3,072 to 6,144 columns: 0.65 to 1.03), and 513 to 896 rows of wide products, whose
+    256-row tiles are (0.73 to 1.05, mean 0.92)."""
+
+    if not (PAIR_ENABLED and 128 < m <= 2048):
+        return False
+    if out_float32:
+        return not ((176 < m <= 256 and 1536 < n <= 2560) or (m > 1024 and (n >= 8192 or k < 1024)))
+    if m <= 256:
+        return 3072 <= n <= 4096 or (m <= 208 and 4096 < n <= 6144)
+    if m <= 512:
+        return n <= 4096 and k >= 3072
+    return (m <= 1024 and n <= 2048 and k >= 3072) or (m <= 896 and n >= 5120)
+
+
 # weight elements from which 9 to 16 rows go to the tcgen05 split-K kernel
 SKINNY_LARGE = int(os.environ.get("LLM_RUNTIME_STUDY_B200_SKINNY_LARGE", 52_000_000))
 
@@ -153,7 +184,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     tiles: up to three SMs share a tile's K range) or "splitk" (few rows: a cluster of ``splits``
     <= 8 CTAs shares the K range of every 128 x ``tile_n`` tile, ``tile_n`` a multiple of 32; 0 for either
     lets the kernel choose so that the SMs are filled once; ``stages``: depth of its operand ring, 0 = as
-    deep as shared memory allows); chosen by shape when not given."""
+    deep as shared memory allows); chosen by shape when not given, the kernel of ``linear_features`` among them."""
 
     native.require(x, "x", dtype=torch.bfloat16, dims=2)
     native.require(weight, "weight", dtype=torch.bfloat16, dims=2)
@@ -174,6 +205,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         if out_dtype not in (torch.bfloat16, torch.float32):
             raise KernelError(f"unsupported output type {out_dtype}")
         out = torch.empty((m, n // 2 if swiglu else n), dtype=out_dtype, device=x.device)
+    if not (kernel or tile_n or splits or stages or pair_width or swiglu) and by_features(m, n, k, out_dtype == torch.float32):
+        _by_features(x, weight, bias, out, add_to is not None, (0, 0), 0)
+        return out
     picked_kernel, picked_width = pick_kernel(m, n, k)
     kernel = kernel or picked_kernel
     if pair_width and (kernel != "pair" or pair_width not in PAIR_WIDTHS):
@@ -197,7 +231,53 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     return out
 
 
+def _by_features(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, out: torch.Tensor, add: bool, tokens: tuple[int, int],
+                 splits: int) -> None:
+    (m, k), n = x.shape, weight.shape[0]
+    native.call("b200_gemm_features", x.data_ptr(), weight.data_ptr(), native.ptr(bias), out.data_ptr(), m, n, k, n,
+                1 if out.dtype == torch.float32 else 0, 1 if add else 0, tokens[0], tokens[1], splits, native.stream_ptr())
+
+
+def linear_features(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None, out_dtype: torch.dtype = torch.bfloat16, *,
+                    add_to: torch.Tensor | None = None, tokens: tuple[int, int] = (0, 0), splits: int = 0) -> torch.Tensor:
+    """As ``linear``, with the weight as the tensor cores' row operand: pairs of SMs on tiles of 256 features and ``tokens`` rows of
+    ``x`` (the two numbers' sum, each a multiple of 32 up to 256, the second may be 0), ``splits`` (1, 2 or 4) pairs to a tile's K range;
+    chosen by shape when not given."""
+
+    native.require(x, "x", dtype=torch.bfloat16, dims=2)
+    native.require(weight, "weight", dtype=torch.bfloat16, dims=2)
+    m, k = x.shape
+    n = weight.shape[0]
+    if weight.shape[1] != k:
+        raise KernelError(f"linear: x has width {k}, weight expects {weight.shape[1]}")
+    if not supported(m, n, k):
+        raise KernelError(f"tcgen05 projection needs K to be a multiple of 8, got {k}")
+    if bias is not None:
+        native.require(bias, "bias", dtype=torch.float32, shape=(n,))
+    if add_to is not None:
+        native.require(add_to, "add_to", dtype=torch.float32, shape=(m, n))
+        out, out_dtype = add_to, torch.float32
+    else:
+        if out_dtype not in (torch.bfloat16, torch.float32):
+            raise KernelError(f"unsupported output type {out_dtype}")
+        out = torch.empty((m, n), dtype=out_dtype, device=x.device)
+    _by_features(x, weight, bias, out, add_to is not None, tokens, splits)
+    return out
+
+
+def features_shape(m: int, n: int, k: int, sm_count: int = 0) -> tuple[int, int, int]:
+    """(tokens of a tile's first and second product, pairs to a tile's K range) that are chosen for this product."""
+
+    import ctypes
+
+    got = (ctypes.c_int * 3)()
+    at = ctypes.addressof(got)
+    native.call("b200_gemm_features_shape", m, n, k, sm_count or native.sm_count(), at, at + 4, at + 8, launches=0)
+    return got[0], got[1], got[2]
+
+
 native.register_error_probe("b200_gemm_tcgen05", "b200_gemm_tcgen05_error", "tcgen05 projection")
+native.register_error_probe("b200_gemm_features", "b200_gemm_features_error", "tcgen05 projection by features")
 
 
 def check_error() -> None:

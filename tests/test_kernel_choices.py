@@ -52,6 +52,24 @@ def test_projections_to_very_few_columns_share_only_long_k_ranges():
         assert gemm_bf16.pick_kernel(m, 64, 2560) == gemm_bf16.pick_kernel(m, 104, 2048) == ("splitk", 0)
 
 
+def test_tiles_of_the_projections_by_features():
+    """Whatever is chosen, the kernel takes it: widths in steps of 32 up to 256 each, shared K ranges only where they hold as many blocks."""
+
+    for m, n, k in itertools.product((1, 32, 33, 129, 256, 257, 405, 512, 513, 1024, 1025, 2048, 16384), (8, 264, 1024, 4096, 6144, 12288), (8, 72, 200, 1024, 4096, 12288)):
+        first, second, splits = gemm_bf16.features_shape(m, n, k, 148)
+        assert first % 32 == 0 and 32 <= first <= 256 and second % 32 == 0 and 0 <= second <= first and splits in (1, 2, 4)
+        assert splits <= -(-k // 64) and (splits == 1 or second == 0)
+    assert gemm_bf16.features_shape(405, 4096, 4096, 148) == (224, 0, 2) and gemm_bf16.features_shape(1024, 4096, 4096, 148) == (256, 0, 1)
+    assert gemm_bf16.features_shape(160, 1024, 2048, 148)[2] == 4
+
+
+def test_which_projections_go_by_features():
+    takes = gemm_bf16.by_features
+    assert takes(405, 4096, 12288, True) and takes(129, 1024, 1024, True) and takes(1024, 4096, 4096, True) and takes(405, 4096, 4096, False)
+    assert not takes(128, 4096, 4096, True) and not takes(2049, 4096, 4096, True) and not takes(256, 2048, 8192, True)
+    assert not takes(405, 6144, 4096, False) and takes(640, 6144, 4096, False) and not takes(1024, 6144, 4096, False)
+
+
 def test_decode_parts_are_bounded_and_use_the_gpu():
     for requests, kv_heads, longest, slots in itertools.product((1, 3, 8, 64, 500), (1, 8), (1, 100, 2048, 32768, 1 << 20), (296, 592)):
         parts = attention_bf16.decode_splits(requests, kv_heads, 1, longest, slots)

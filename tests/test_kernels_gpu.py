@@ -757,6 +757,42 @@ def test_tcgen05_pair_width_is_asked_for_by_either_name_and_only_of_the_pairs():
             _gemm().linear(*args, **options)
 
 
+# one tile of one product and of two, ragged edges in every dimension, two accumulators in turn, tiles behind the last full round
+# whose products are items of their own, a K range shared by two and four pairs (fewer K blocks than shares of them are even), and
+# what is chosen by size
+@pytest.mark.parametrize("m,n,k,tokens,splits", [
+    (17, 256, 64, (32, 0), 1), (33, 100, 72, (64, 0), 1), (129, 256, 520, (96, 64), 1), (405, 24576, 72, (224, 0), 1),
+    (405, 20000, 192, (224, 192), 1), (1000, 9000, 256, (256, 256), 1), (100, 1000, 520, (128, 0), 2), (405, 4112, 1000, (224, 192), 2),
+    (200, 520, 264, (224, 0), 4), (512, 1024, 3072, (128, 0), 4), (405, 4096, 4096, (0, 0), 0), (1025, 1040, 200, (0, 0), 0), (130, 8, 8, (0, 0), 0),
+])
+@pytest.mark.parametrize("form", ["bf16", "float", "add"])
+def test_tcgen05_projection_by_features(m, n, k, tokens, splits, form):
+    x, w, b, want = _gemm_case(m, n, k, True)
+    resid = torch.randn(m, n, generator=torch.Generator().manual_seed(5))
+    scale = float(want.abs().max())
+
+    def run():
+        add_to = dev(resid.clone()) if form == "add" else None
+        return _gemm().linear_features(dev(x), dev(w), dev(b), torch.bfloat16 if form == "bf16" else torch.float32, add_to=add_to, tokens=tokens,
+                                       splits=splits)
+
+    got = run()
+    _gemm().check_error()
+    assert torch.equal(got, run()) and _gemm().native.query("b200_gemm_features_error") == 0
+    torch.testing.assert_close(got.cpu().double(), want + (resid.double() if form == "add" else 0), atol=(1e-2 if form == "bf16" else 2e-5) * scale, rtol=0)
+
+
+def test_tcgen05_projection_by_features_refuses_what_it_cannot_take():
+    from llm_runtime_study_b200.errors import KernelError
+
+    x, w = torch.zeros(32, 128, device="cuda").bfloat16(), torch.zeros(64, 128, device="cuda").bfloat16()
+    for tokens, splits in (((48, 0), 1), ((288, 0), 1), ((64, 16), 1), ((32, 0), 3), ((32, 0), 4), ((0, 32), 1)):     # 4: only two K blocks
+        with pytest.raises(KernelError):
+            _gemm().linear_features(x, w, tokens=tokens, splits=splits)
+    with pytest.raises(KernelError):                                  # the exchange of such a tile finds no room
+        _gemm().linear_features(torch.zeros(512, 512, device="cuda").bfloat16(), torch.zeros(64, 512, device="cuda").bfloat16(), tokens=(256, 256), splits=4)
+
+
 @pytest.mark.parametrize("kernel", ["pair", "persistent"])
 @pytest.mark.parametrize("m,n,k", [(256, 256, 64), (300, 1000, 520), (2048, 4096, 4096)])
 def test_tcgen05_adds_to_the_residual(m, n, k, kernel):
