@@ -8,11 +8,12 @@
 // The draw is Gumbel-max: argmax(x_i + g_i), g_i = -log(-log(u_i)), which samples
 // softmax(x) exactly.  u_i comes from a counter-based generator keyed by (request
 // seed, index of the token being generated, vocabulary index), so a request's draws
-// do not depend on what else is in the batch.  The thresholds for top_k and top_p
-// are found by a search over the 32 bits of an order-preserving integer key of x, four
-// bits a pass (fifteen candidate thresholds are counted at once), which needs no sort and
-// no scratch memory; the passes over the row use 16-byte loads, two in flight per thread.
-// Every sum is taken in an order fixed by the launch shape: the same bits every run.
+// do not depend on what else is in the batch.  The thresholds for top_k and top_p are found in three
+// passes over the row (narrow_threshold): how many elements lie in each of 1,024 (256) equal steps below the
+// row's maximum, the same within the steps that can hold the threshold, and the few elements left after that
+// exactly; rows of which too many elements are left (equal values, a threshold far below the maximum) by a search over the 32 bits of an
+// order-preserving integer key, four bits a pass (find_threshold).  Counts are whole numbers and every sum of weights is taken in an order
+// fixed by the launch shape: the same bits every run.
 //
 // The per-row parameters are six words [temperature bits, top_k, top_p bits, seed low, seed high,
 // counter].  They come either as an array [rows][6], or out of the per-request slot records on the
@@ -220,6 +221,244 @@ __device__ uint32_t find_threshold(const Slice& sl, uint32_t floor_key, float mx
   return k;
 }
 
+// ---- thresholds in three passes
+// An element's place below the maximum is (mx - v) * inv, in steps: a function that never falls as v falls, whatever is rounded, so
+// the elements of a step are neighbours in value.  Counts are exact, and the weights of a step's elements are
+// known to e^-width, so counts alone say between which steps the threshold lies, for a mass too.
+// STEPS: 1,024 for CTAs of 512 threads and more, 256 for smaller ones, whose shares hold fewer elements and whose threads would
+// fetch more counts each (256 rows of 32,768 entries, 256 threads: 417 us with 1,024 steps, 162 with 256; 260 before).
+constexpr int kLeft = 256;                    // elements that may be left for the end
+constexpr float kReach = 32.f;                // the steps reach this far below the maximum (e^-32 of its weight), the last one on from there
+
+template <int STEPS>
+struct NarrowMemory {
+  int counts[2][STEPS];
+  uint32_t left[2][kLeft], gathered[kLeft], sorted[kLeft];   // (left, left_count: a set for each threshold, which other CTAs may still be reading)
+  int left_count[2], kept_count, low, high, above;
+  float warp_sums[2][32];
+  uint32_t result;
+  int warp_counts[32];
+};
+
+__device__ __forceinline__ uint32_t load_word_from_rank(const void* local, uint32_t rank) {
+  uint32_t address = static_cast<uint32_t>(__cvta_generic_to_shared(local)), remote, v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(address), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];\n" : "=r"(v) : "r"(remote) : "memory");
+  return v;
+}
+// The word at this place in the first eight ranks' shared memory, all fetched together (0 from ranks that are not there).
+constexpr int kRanks = 8;                     // CTAs of a cluster, where there is one
+__device__ __forceinline__ void load_from_ranks(const void* local, uint32_t ranks, int (&v)[kRanks]) {
+#pragma unroll
+  for (int r = 0; r < kRanks; ++r) v[r] = r < static_cast<int>(ranks) ? static_cast<int>(load_word_from_rank(local, r)) : 0;
+}
+__device__ __forceinline__ float key_value(uint32_t key) { return __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key); }
+
+// `sum` becomes the sum of the block-wide sums of all ranks, at the barrier that the counts or the elements left are exchanged behind: a
+// meeting of its own would take 2 us.  Two sets of slots alternate, as elsewhere.
+__device__ __forceinline__ void meet(float& sum, ClusterSlots& cs, uint32_t ranks) {
+  if (ranks == 1) {
+    __syncthreads();
+    return;
+  }
+  if (threadIdx.x == 0) cs.slots[cs.which][0] = sum;
+  cluster_barrier();
+  int v[kRanks];
+  load_from_ranks(&cs.slots[cs.which][0], ranks, v);
+  sum = 0.f;
+#pragma unroll
+  for (int r = 0; r < kRanks; ++r) sum += __int_as_float(v[r]);
+  cs.which ^= 1;
+}
+
+// The steps between which the threshold lies, from the counts of all ranks: with MASS the first that reaches the target if every
+// element weighs as much as its step allows, and the first that does if it weighs as little; else the one that reaches it, and the count
+// before it.  Step s holds places origin + s * width .. on.  The last step where it is not reached.  MASS: `sum` comes as the
+// block-wide sum and goes as the cluster's: the whole weight, `part` of which is the target (FIRST), or the weight of the
+// elements before the steps.  All threads call; the counts have been written by atomics of this CTA's threads.
+template <bool MASS, bool FIRST, int STEPS>
+__device__ void bracket(NarrowMemory<STEPS>& nm, int* counts, ClusterSlots& cs, uint32_t ranks, float origin, float width, float inv, bool open_end,
+                        float& sum, float& target, float part, int need) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, each = STEPS / blockDim.x, first = tid * each;
+  meet(sum, cs, ranks);
+  if (MASS && FIRST) target = part * sum;
+  const float before = MASS && !FIRST ? sum : 0.f, slack = FIRST ? 1e-4f : 4e-6f;      // (far beyond what rounding does to the sums)
+  const float target_low = target * (1.f - slack), target_high = target * (1.f + slack);
+  int mine[8], total = 0;
+  float most[8], least[8], sum_most = 0.f, sum_least = 0.f;
+  if (tid == 0) { nm.low = nm.high = STEPS - 1; nm.above = 0; }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    mine[i] = 0;
+    if (i < each) {
+      if (ranks == 1) {
+        mine[i] = counts[first + i];
+      } else {
+        int v[kRanks];
+        load_from_ranks(&counts[first + i], ranks, v);
+#pragma unroll
+        for (int r = 0; r < kRanks; ++r) mine[i] += v[r];
+      }
+    }
+    total += mine[i];
+    if (MASS) {
+      most[i] = least[i] = 0.f;
+      if (mine[i] > 0) {
+        const float at = origin + (first + i) * width;      // rounding of places and exponentials: far below 2e-5
+        most[i] = mine[i] * expf(-at / inv) * 1.00002f;
+        least[i] = open_end && first + i == STEPS - 1 ? 0.f : mine[i] * expf(-(at + width) / inv) * 0.99998f;
+      }
+      sum_most += most[i];
+      sum_least += least[i];
+    }
+  }
+  auto scan = [&](auto v, auto* scratch) {                  // what the threads before this one hold
+    auto x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const auto y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) scratch[warp] = x;
+    __syncthreads();
+    decltype(v) base = 0;
+    for (int w = 0; w < warp; ++w) base += scratch[w];
+    return base + x - v;
+  };
+  if (MASS) {
+    float upper = before + scan(sum_most, nm.warp_sums[0]), lower = before + scan(sum_least, nm.warp_sums[1]);
+    int low = STEPS - 1, high = STEPS - 1;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i >= each) break;
+      upper += most[i];
+      lower += least[i];
+      if (upper >= target_low) low = min(low, first + i);
+      if (lower >= target_high) high = min(high, first + i);
+    }
+    low = __reduce_min_sync(0xffffffffu, low);
+    high = __reduce_min_sync(0xffffffffu, high);
+    if (lane == 0) {
+      atomicMin(&nm.low, low);
+      atomicMin(&nm.high, high);
+    }
+  } else {
+    int count = scan(total, nm.warp_counts);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i >= each) break;
+      if (count < need && count + mine[i] >= need) {
+        nm.low = nm.high = first + i;
+        nm.above = count;
+      }
+      count += mine[i];
+    }
+  }
+  __syncthreads();
+}
+
+// As find_threshold over the elements whose key is at least floor_key: the largest key k such that weight(keys >= k) reaches
+// `need` elements, or `part` of the whole weight (MASS).  ~0u when too many elements are left at the end.
+template <bool MASS, int STEPS>
+__device__ uint32_t narrow_threshold(const Slice& sl, uint32_t floor_key, float mx, float inv, int need, float part, NarrowMemory<STEPS>& nm,
+                                     float* sum_scratch, ClusterSlots& cs, uint32_t ranks) {
+  const int tid = threadIdx.x, set = MASS ? 1 : 0;
+  auto place = [&](float v) { return fminf((mx - v) * inv, 2.f * STEPS); };
+  for (int i = tid; i < STEPS; i += blockDim.x) nm.counts[0][i] = nm.counts[1][i] = 0;
+  if (tid == 0) nm.left_count[set] = 0;
+  __syncthreads();
+  float z = 0.f;
+  for_each_scaled(sl, [&](float v, int) {
+    if (ordered_key(v) < floor_key) return;
+    atomicAdd(&nm.counts[0][min(STEPS - 1, static_cast<int>(place(v)))], 1);
+    if (MASS) z += expf(v - mx);
+  });
+  float target = 0.f;
+  if (MASS) z = block_sum(z, sum_scratch);
+  bracket<MASS, true, STEPS>(nm, nm.counts[0], cs, ranks, 0.f, 1.f, inv, true, z, target, part, need);
+  const int low = nm.low, high = max(nm.high, nm.low), above = nm.above;
+  const float finer = static_cast<float>(STEPS) / static_cast<float>(high - low + 1);
+  auto fine = [&](float at) { return min(STEPS - 1, static_cast<int>(fminf((at - low) * finer, static_cast<float>(STEPS)))); };
+  float m = 0.f;
+  for_each_scaled(sl, [&](float v, int) {
+    if (ordered_key(v) < floor_key) return;
+    const float at = place(v);
+    const int step = min(STEPS - 1, static_cast<int>(at));
+    if (step < low) {
+      if (MASS) m += expf(v - mx);
+    } else if (step <= high) {
+      atomicAdd(&nm.counts[1][fine(at)], 1);
+    }
+  });
+  float before = MASS ? block_sum(m, sum_scratch) : 0.f;
+  bracket<MASS, false, STEPS>(nm, nm.counts[1], cs, ranks, static_cast<float>(low), 1.f / finer, inv, high == STEPS - 1, before, target, part, need - above);
+  const int low2 = nm.low, high2 = max(nm.high, nm.low), above2 = nm.above;
+  m = 0.f;
+  for_each_scaled(sl, [&](float v, int) {
+    const uint32_t key = ordered_key(v);
+    if (key < floor_key) return;
+    const float at = place(v);
+    const int step = min(STEPS - 1, static_cast<int>(at));
+    if (step < low || step > high) return;
+    const int f = fine(at);
+    if (f < low2) {
+      if (MASS) m += expf(v - mx);
+    } else if (f <= high2) {
+      const int slot = atomicAdd(&nm.left_count[set], 1);
+      if (slot < kLeft) nm.left[set][slot] = key;
+    }
+  });
+  m = MASS ? block_sum(m, sum_scratch) : 0.f;
+  meet(m, cs, ranks);
+  before += m;
+  // every rank's elements, in every CTA; in the order of their keys (those of equal ones does not matter)
+  int total = 0, held[kRanks];
+  bool fits = true;
+  if (ranks == 1) held[0] = nm.left_count[set];
+  else load_from_ranks(&nm.left_count[set], ranks, held);
+#pragma unroll
+  for (int r = 0; r < kRanks; ++r) {
+    if (r >= static_cast<int>(ranks)) break;
+    fits = fits && held[r] <= kLeft && total + held[r] <= kLeft;
+    if (fits)
+      for (int i = tid; i < held[r]; i += blockDim.x) nm.gathered[total + i] = ranks == 1 ? nm.left[set][i] : load_word_from_rank(&nm.left[set][i], r);
+    total += held[r];
+  }
+  __syncthreads();
+  if (!fits) return ~0u;
+  for (int i = tid; i < total; i += blockDim.x) {
+    const uint32_t key = nm.gathered[i];
+    int rank = 0;
+    for (int j = 0; j < total; ++j) rank += nm.gathered[j] > key || (nm.gathered[j] == key && j < i);
+    nm.sorted[rank] = key;
+  }
+  __syncthreads();
+  if (tid < 32) {
+    uint32_t found = floor_key;
+    if (MASS) {
+      bool reached = false;
+      for (int i0 = 0; i0 < total && !reached; i0 += 32) {      // thirty-two at a time, from the largest on
+        found = nm.sorted[min(i0 + tid, total - 1)];
+        float mass = i0 + tid < total ? expf(key_value(found) - mx) : 0.f;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const float y = __shfl_up_sync(0xffffffffu, mass, o);
+          if (tid >= o) mass += y;
+        }
+        const unsigned enough = __ballot_sync(0xffffffffu, before + mass >= target);
+        before += __shfl_sync(0xffffffffu, mass, 31);
+        reached = enough != 0u;
+        found = __shfl_sync(0xffffffffu, found, reached ? __ffs(enough) - 1 : 31);
+      }
+    } else if (total > 0) {
+      found = nm.sorted[max(0, min(need - above - above2, total) - 1)];
+    }
+    if (tid == 0) nm.result = found;
+  }
+  __syncthreads();
+  return nm.result;
+}
+
 struct ArgMax {
   float value;
   int index;
@@ -252,10 +491,11 @@ __device__ ArgMax block_argmax(ArgMax v, ArgMax* scratch) {
 
 // One cluster of CTAs per row (gridDim.x = rows * cluster size): each CTA scans its slice of the row and
 // the CTAs combine their results through distributed shared memory.  STAGED: the slice is read from memory and divided by
-// the temperature once and kept in shared memory for the twenty passes over it (`staged`: room for it).  Bound by the passes'
-// arithmetic: 32 rows of 151,936 entries, 19 of them filtered, 104 us (228 when every pass read and divided the logits and
-// weighed each element against all fifteen candidates in all of its eight passes).
-template <bool STAGED>
+// the temperature once and kept in shared memory for the passes over it (`staged`: room for it).  32 rows of 151,936 entries, 19 of
+// them filtered: 58 us, half of it the passes' arithmetic and half the meetings of the clusters (118 us when each threshold took eight passes of
+// find_threshold, which weighs elements against fifteen candidates, and rows without filters two launches of their own); one row with
+// top-k 25 us (40), with top-p 46 (60).
+template <bool STAGED, int STEPS>
 __global__ void __launch_bounds__(1024)
 sample_kernel(const float* __restrict__ logits, int ld, int vocab, RowParams params,
               int* __restrict__ out, int filtered_only) {
@@ -265,6 +505,7 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab, RowParams par
   __shared__ float slot_memory[2][16];
   __shared__ float gathered_memory[kMaxClusterRanks][16];
   __shared__ float totals[16];
+  __shared__ NarrowMemory<STEPS> nm;
   extern __shared__ __align__(16) float staged[];
   pdl_trigger();
   pdl_wait();
@@ -303,17 +544,39 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab, RowParams par
   };
 
   // non-finite logits are an error (mini_llm/sampling.py:104-113): report -1
-  float bad = 0.f, mx = -INFINITY;
+  float bad = 0.f, mx = -INFINITY, mn = INFINITY;
   const float scale = temperature == 0.f ? 1.f : temperature;
   for_each_scaled(sl, [&](float raw, int i) {
     bad += isfinite(raw) ? 0.f : 1.f;
     const float v = raw / scale;
     mx = fmaxf(mx, v);
+    mn = fminf(mn, v);
     if (STAGED) staged[i - begin] = v;
   });
   if (STAGED) sl.x = staged;
   else sl.temperature = scale;
-  const bool any_bad = cluster_sum(bad, sum_scratch, cs, ranks) > 0.f;     // (a block-wide barrier: the staged values are there)
+  // whether any is not finite, the row's largest and its smallest value, in one exchange (a block-wide barrier: the staged values are there)
+  bad = block_sum(bad, sum_scratch);
+  mx = block_argmax(ArgMax{mx, 0}, arg_scratch).value;
+  mn = -block_argmax(ArgMax{-mn, 0}, arg_scratch).value;
+  if (ranks > 1) {
+    if (threadIdx.x == 0) {
+      cs.slots[cs.which][0] = bad;
+      cs.slots[cs.which][1] = mx;
+      cs.slots[cs.which][2] = mn;
+    }
+    cluster_barrier();
+    if (threadIdx.x < ranks * 3) cs.gathered[threadIdx.x / 3][threadIdx.x % 3] = load_from_rank(&cs.slots[cs.which][threadIdx.x % 3], threadIdx.x / 3);
+    __syncthreads();
+    for (uint32_t r = 0; r < ranks; ++r) {
+      bad += cs.gathered[r][0];
+      mx = fmaxf(mx, cs.gathered[r][1]);
+      mn = fminf(mn, cs.gathered[r][2]);
+    }
+    __syncthreads();
+    cs.which ^= 1;
+  }
+  const bool any_bad = bad > 0.f;
   int result = -1;
   if (!any_bad && temperature == 0.f) {
     ArgMax best{-INFINITY, 0x7fffffff};
@@ -321,24 +584,59 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab, RowParams par
     result = cluster_argmax(best).index;
   } else if (!any_bad) {
     uint32_t low_key = 0;  // tokens with key >= low_key stay
-    if (top_k > 0 && top_k < vocab)
-      low_key = find_threshold<false>(sl, 0u, 0.f, static_cast<float>(top_k), multi_scratch, cs, ranks);
-    if (top_p < 1.f) {
-      mx = cluster_argmax(ArgMax{mx, 0}).value;
-      float z = 0.f;
-      for_each_scaled(sl, [&](float v, int) {
-        if (ordered_key(v) >= low_key) z += expf(v - mx);
-      });
-      const float target = top_p * cluster_sum(z, sum_scratch, cs, ranks);
-      low_key = max(low_key, find_threshold<true>(sl, low_key, mx, target, multi_scratch, cs, ranks));
+    const bool cut = top_k > 0 && top_k < vocab;
+    if (cut || top_p < 1.f) {
+      const bool narrow = isfinite(mx);                      // a tiny temperature may have made infinities of the largest logits
+      const float inv = STEPS / fmaxf(fminf(mx - mn, kReach), 1e-20f);
+      if (cut) {
+        uint32_t key = narrow ? narrow_threshold<false, STEPS>(sl, 0u, mx, inv, top_k, 0.f, nm, sum_scratch, cs, ranks) : ~0u;
+        if (key == ~0u) key = find_threshold<false>(sl, 0u, 0.f, static_cast<float>(top_k), multi_scratch, cs, ranks);
+        low_key = key;
+      }
+      if (top_p < 1.f) {
+        uint32_t key = narrow ? narrow_threshold<true, STEPS>(sl, low_key, mx, inv, 0, top_p, nm, sum_scratch, cs, ranks) : ~0u;
+        if (key == ~0u) {
+          float z = 0.f;
+          for_each_scaled(sl, [&](float v, int) {
+            if (ordered_key(v) >= low_key) z += expf(v - mx);
+          });
+          const float target = top_p * cluster_sum(z, sum_scratch, cs, ranks);
+          key = find_threshold<true>(sl, low_key, mx, target, multi_scratch, cs, ranks);
+        }
+        low_key = max(low_key, key);
+      }
     }
     const uint64_t stream = splitmix64(seed ^ splitmix64(static_cast<uint64_t>(counter)));
     ArgMax best{-INFINITY, 0x7fffffff};
-    for_each_scaled(sl, [&](float v, int i) {
-      if (ordered_key(v) < low_key) return;
+    auto noisy = [&](float v, int i) {
       const float u = uniform23(stream, static_cast<uint32_t>(i));
       best = better(best, ArgMax{v - logf(-logf(u)), i});
-    });
+    };
+    if (low_key == 0u) {
+      for_each_scaled(sl, noisy);
+    } else {
+      // the few that stay are put side by side first: one in a warp would have all of its lanes wait for the noise
+      int* kept = &nm.counts[0][0];                          // (the counts have been used)
+      constexpr int kKept = 2 * STEPS;
+      if (threadIdx.x == 0) nm.kept_count = 0;
+      __syncthreads();
+      for_each_scaled(sl, [&](float v, int i) {
+        if (ordered_key(v) < low_key) return;
+        const unsigned together = __activemask();            // the lanes that are here take neighbouring places by one addition
+        const int lane = threadIdx.x & 31, first = __ffs(together) - 1;
+        int slot = lane == first ? atomicAdd(&nm.kept_count, __popc(together)) : 0;
+        slot = __shfl_sync(together, slot, first) + __popc(together & ((1u << lane) - 1u));
+        if (slot < kKept) kept[slot] = i;
+        else noisy(v, i);
+      });
+      __syncthreads();
+      const int count = min(nm.kept_count, kKept);
+      for (int k = threadIdx.x; k < count; k += blockDim.x) {
+        const int i = kept[k];
+        const float raw = sl.x[i - begin];
+        noisy(sl.temperature != 1.f ? raw / sl.temperature : raw, i);
+      }
+    }
     result = cluster_argmax(best).index;
   }
   // every CTA of the cluster has read the row's parameters by now (the reductions above are barriers)
@@ -430,13 +728,15 @@ __global__ void sample_final_kernel(const float* __restrict__ part_value, const 
 constexpr size_t kMostStaged = 200 * 1024, kSmallShare = 32 * 1024;
 static int launch_sample(const float* logits, int ld, int vocab, b200::RowParams params, int* out, int rows, int filtered_only,
                          cudaStream_t stream) {
-  const int cluster = vocab < 32768 ? 1 : 8;
+  const int cluster = vocab < 32768 ? 1 : b200::kRanks;
   const size_t share = sizeof(float) * static_cast<size_t>(((vocab + cluster - 1) / cluster + 3) & ~3);
   const int threads = cluster > 1 ? (rows > 64 && share <= kSmallShare ? 256 : 512) : (vocab >= 8192 ? 1024 : (vocab >= 1024 ? 256 : 128));
   const bool staged = share <= kMostStaged;
-  static b200::DeviceOnce once;
+  auto kernel = threads <= 256 ? (staged ? b200::sample_kernel<true, 256> : b200::sample_kernel<false, 256>)
+                               : (staged ? b200::sample_kernel<true, 1024> : b200::sample_kernel<false, 1024>);
+  static b200::DeviceOnce once[2];
   if (staged)
-    if (int e = b200::configure_once(once, b200::sample_kernel<true>, kMostStaged)) return e;
+    if (int e = b200::configure_once(once[threads > 256], kernel, kMostStaged)) return e;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(rows * cluster);
   config.blockDim = dim3(threads);
@@ -451,8 +751,7 @@ static int launch_sample(const float* logits, int ld, int vocab, b200::RowParams
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = b200::pdl_enabled() ? 2 : 1;
-  cudaError_t e = staged ? cudaLaunchKernelEx(&config, b200::sample_kernel<true>, logits, ld, vocab, params, out, filtered_only)
-                         : cudaLaunchKernelEx(&config, b200::sample_kernel<false>, logits, ld, vocab, params, out, filtered_only);
+  cudaError_t e = cudaLaunchKernelEx(&config, kernel, logits, ld, vocab, params, out, filtered_only);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 
@@ -463,6 +762,10 @@ extern "C" int b200_sample(const float* logits, int ld, int vocab, const int* pa
   return launch_sample(logits, ld, vocab, b200::RowParams{const_cast<int*>(params), nullptr}, out, rows, 0, stream);
 }
 
+// Up to so many rows, if some are filtered, all of them in the one launch: the rows without filters beside the others (32 rows of 151,936 entries: the
+// two launches before it took 17 us).
+constexpr int kRowsTogether = 64;
+
 // Two-stage variant.  `scratch` holds rows * chunks floats followed by rows * chunks ints;
 // `any_filtered` tells whether some row uses top_k / top_p (then the kernel with a cluster per row
 // also runs, for those rows only).
@@ -470,6 +773,7 @@ static int sample_chunked(const float* logits, int ld, int vocab, b200::RowParam
                           int chunks, void* scratch, int any_filtered, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (vocab <= 0 || ld < vocab || chunks <= 0 || rows > 65535) return B200_ERR_BAD_SIZE;
+  if (any_filtered && rows <= kRowsTogether) return launch_sample(logits, ld, vocab, params, out, rows, 0, stream);
   float* part_value = static_cast<float*>(scratch);
   int* part_index = reinterpret_cast<int*>(part_value + static_cast<size_t>(rows) * chunks);
   dim3 grid(chunks, rows);

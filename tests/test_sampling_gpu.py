@@ -88,6 +88,32 @@ def test_thresholds_at_the_edges_of_the_shares(sampler, vocab, opts):
         assert got[r] == want or abs(float(scores[got[r]] - scores[want])) < 1e-4
 
 
+# one CTA of 128, 256 and 1,024 threads a row and clusters of eight; rows whose values are all equal or of two kinds (more elements are left at
+# the end of the search than are gathered: the search over the keys takes over), so close that most share a step, so far apart that a
+# threshold lies in the last step or beyond what the steps reach, beside one value that is far above all others
+@pytest.mark.parametrize("vocab", [5, 503, 1100, 9001, 40003])
+@pytest.mark.parametrize("form", ["equal", "two", "close", "far", "outlier"])
+def test_thresholds_of_awkward_rows(sampler, vocab, form):
+    torch.manual_seed(7)
+    draw = torch.randperm(vocab).float() / vocab                  # no two are equal
+    logits = {"equal": torch.full((vocab,), -3.0), "two": (draw > 0.5).float() * 4, "close": 8 + draw * 1e-2, "far": draw * 4000 - 1000,
+              "outlier": draw.clone()}[form]
+    if form == "outlier":
+        logits[vocab // 3] = 1e30
+    few, most = max(1, vocab // 50), max(1, vocab - 2)
+    options = [dict(temperature=0.9, top_k=few), dict(temperature=1.1, top_k=most), dict(temperature=0.01, top_k=few)]
+    if form not in ("equal", "two"):                              # (of equal values all stay, of the plain sampler's sorted ones some)
+        options += [dict(temperature=0.9, top_p=0.63), dict(temperature=1.3, top_k=most, top_p=0.31), dict(temperature=1.0, top_p=0.999)]
+    specs = [(cfg(**o), 300 + r, r) for r, o in enumerate(options)]
+    got = sampler.sample(logits.repeat(len(options), 1).cuda(), specs)
+    for r, o in enumerate(options):
+        args = (logits, o["temperature"], o.get("top_k"), o.get("top_p", 1.0))
+        want, scores = plain.sample(*args, 300 + r, r)
+        assert plain.kept_mask(*args)[got[r]], (form, o)
+        # the division by the temperature rounds a score to 6e-8 of itself
+        assert got[r] == want or abs(float(scores[got[r]] - scores[want])) < 1e-4 + 2e-7 * abs(float(scores[want]))
+
+
 def test_rows_are_independent_of_the_batch(sampler):
     torch.manual_seed(2)
     logits = torch.randn(8, 503).cuda()
