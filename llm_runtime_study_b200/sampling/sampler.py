@@ -26,9 +26,9 @@ native.register_library(
 )
 
 CHUNKS = 64   # parts a row's vocabulary is cut into for the one-pass selections
+ROWS_TOGETHER = 64   # up to so many rows, if some are filtered, are one launch (csrc/sampling.cu: kRowsTogether)
 
 PARAM_WORDS = 6
-_MASK64 = (1 << 64) - 1
 
 
 def fresh_seed() -> int:
@@ -38,21 +38,13 @@ def fresh_seed() -> int:
     return random.SystemRandom().getrandbits(63)
 
 
-def _float_bits(value: float) -> int:
-    return struct.unpack("<i", struct.pack("<f", value))[0]
+# per row: temperature, top_k (0: off), top_p, seed low, seed high, counter
+_ROW = struct.Struct("<fifIII")
+_MASK32 = (1 << 32) - 1
 
 
-def pack_row(config: SamplingConfig, seed: int, counter: int) -> list[int]:
-    """[temperature bits, top_k (0: off), top_p bits, seed low, seed high, counter] as int32."""
-
-    def s32(v: int) -> int:
-        v &= 0xFFFFFFFF
-        return v - (1 << 32) if v >= (1 << 31) else v
-
-    return [
-        _float_bits(config.temperature), config.top_k or 0, _float_bits(config.top_p),
-        s32(seed), s32(seed >> 32), s32(counter),
-    ]
+def _launches(rows: int, filtered: bool) -> int:
+    return 2 if not filtered else (1 if rows <= ROWS_TOGETHER else 3)
 
 
 class Sampler:
@@ -62,6 +54,7 @@ class Sampler:
     def __init__(self, device: torch.device, max_rows: int = 256) -> None:
         self.device = device
         self._host = torch.empty(max_rows * PARAM_WORDS, dtype=torch.int32, pin_memory=True)
+        self._host_words = self._host.numpy()
         self._dev = torch.empty(max_rows * PARAM_WORDS, dtype=torch.int32, device=device)
         self._out = torch.empty(max_rows, dtype=torch.int32, device=device)
         self._out_host = torch.empty(max_rows, dtype=torch.int32, pin_memory=True)
@@ -78,22 +71,24 @@ class Sampler:
             raise SamplingError(f"{n} rows of logits but {len(rows)} sampling rows")
         if n > self.max_rows:
             raise SamplingError(f"at most {self.max_rows} rows can be sampled at once")
-        for config, _, _ in rows:
-            if config.top_k is not None and config.top_k > vocab:
-                raise SamplingError(f"top_k {config.top_k} exceeds vocabulary size {vocab}")
-        packed = np.asarray([w for config, seed, counter in rows for w in pack_row(config, seed, counter)], dtype=np.int32)
-        self._host[: packed.shape[0]].numpy()[:] = packed
-        self._dev[: packed.shape[0]].copy_(self._host[: packed.shape[0]], non_blocking=True)
-        filtered = any(c.temperature > 0 and ((c.top_k is not None and c.top_k < vocab) or c.top_p < 1.0)
-                       for c, _, _ in rows)
+        packed, filtered = bytearray(), False
+        for config, seed, counter in rows:
+            top_k, top_p = config.top_k or 0, config.top_p
+            if top_k > vocab:
+                raise SamplingError(f"top_k {top_k} exceeds vocabulary size {vocab}")
+            packed += _ROW.pack(config.temperature, top_k, top_p, seed & _MASK32, (seed >> 32) & _MASK32, counter & _MASK32)
+            filtered = filtered or (config.temperature > 0 and (0 < top_k < vocab or top_p < 1.0))
+        words = n * PARAM_WORDS
+        self._host_words[:words] = np.frombuffer(packed, dtype=np.int32)
+        self._dev[:words].copy_(self._host[:words], non_blocking=True)
         chunks = CHUNKS if vocab >= 4096 else 1
         native.call("b200_sample_chunked", logits.data_ptr(), logits.stride(0), vocab, self._dev.data_ptr(),
                     self._out.data_ptr(), n, chunks, self._scratch.data_ptr(), 1 if filtered else 0,
-                    native.stream_ptr(), launches=3 if filtered else 2)
+                    native.stream_ptr(), launches=_launches(n, filtered))
         self._out_host[:n].copy_(self._out[:n], non_blocking=True)
         torch.cuda.current_stream(self.device).synchronize()
         tokens = self._out_host[:n].tolist()
-        if any(t < 0 for t in tokens):
+        if min(tokens, default=0) < 0:
             raise SamplingError("logits must contain only finite values")
         return tokens
 
@@ -115,4 +110,4 @@ class Sampler:
         chunks = CHUNKS if vocab >= 4096 else 1
         native.call("b200_sample_slots", logits.data_ptr(), logits.stride(0), vocab, records.data_ptr(), row_slots.data_ptr(),
                     out.data_ptr(), n, chunks, self._scratch.data_ptr(), 1 if filtered else 0, native.stream_ptr(),
-                    launches=3 if filtered else 2)
+                    launches=_launches(n, filtered))
