@@ -265,6 +265,19 @@ def linear_features(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | 
     return out
 
 
+def linear_with_bias(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
+    """``x @ weight.T + bias`` in bfloat16 for 17 to 127 rows.  Without a bias such products are the library's; behind one of those
+    the sum is two launches more (the bias in bfloat16, the addition) and rounds twice.  With a K range or a number of columns up to 2,048 by
+    features, else split-K, microseconds with 17, 64 and 127 rows against the library and the sum: 16,384 x 2,048 16.2, 17.1, 17.8
+    (17.6, 19.9, 23.2), 2,048 x 8,192 14.3, 14.4, 15.6 (18.0, 18.4, 18.9), 24,576 x 4,096 40.5, 42.4, 46.4 (42.7, 47.3, 49.9), 4,096 x 12,288
+    23.4, 25.2, 26.8 (27.6, 28.3, 28.6), 1,024 x 1,024 6.5, 6.5, 6.7 (8.1, 7.9, 8.0).  (A float32 sum is one launch and
+    added in place: as fast as these, so it stays.)"""
+
+    if PAIR_ENABLED and (x.shape[1] <= 2048 or weight.shape[0] <= 2048):
+        return linear_features(x, weight, bias, torch.bfloat16)
+    return linear(x, weight, bias, torch.bfloat16, kernel="splitk")
+
+
 def features_shape(m: int, n: int, k: int, sm_count: int = 0) -> tuple[int, int, int]:
     """(tokens of a tile's first and second product, pairs to a tile's K range) that are chosen for this product."""
 

@@ -137,6 +137,8 @@ class Projection:
                     gemm_bf16.linear(x, self.weight, self.bias, torch.float32, add_to=add_to, kernel="splitk")
                     return None
                 return gemm_bf16.linear(x, self.weight, self.bias, out_dtype, kernel="splitk")
+            if self.GEMM_BACKEND == "tcgen05" and self.bias is not None and out_dtype == torch.bfloat16:
+                return gemm_bf16.linear_with_bias(x, self.weight, self.bias)
         if out_dtype == torch.bfloat16:
             y = torch.mm(x, self.weight.t())
         else:

@@ -782,6 +782,16 @@ def test_tcgen05_projection_by_features(m, n, k, tokens, splits, form):
     torch.testing.assert_close(got.cpu().double(), want + (resid.double() if form == "add" else 0), atol=(1e-2 if form == "bf16" else 2e-5) * scale, rtol=0)
 
 
+# by features (few columns, a short K range) and split-K; the fewest and the most rows that come here
+@pytest.mark.parametrize("m", [17, 64, 127])
+@pytest.mark.parametrize("n,k", [(300, 520), (2056, 2056), (2064, 96)])
+def test_few_rows_with_a_bias(m, n, k):
+    x, w, b, want = _gemm_case(m, n, k, True)
+    got = _gemm().linear_with_bias(dev(x), dev(w), dev(b))
+    _gemm().check_error()
+    torch.testing.assert_close(got.cpu().double(), want, atol=1e-2 * float(want.abs().max()), rtol=0)
+
+
 def test_tcgen05_projection_by_features_refuses_what_it_cannot_take():
     from llm_runtime_study_b200.errors import KernelError
 
