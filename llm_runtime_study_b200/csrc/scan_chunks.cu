@@ -16,6 +16,8 @@
 // state is made for all chunks at once by a first kernel: per chunk and head a record of G_t q_t, E_s k_s, (G_t k_t,) A, (T)
 // and G_C, in float32.  The second walks the chunks.
 #include "common.cuh"
+#include "mma.cuh"
+#include "tcgen05.cuh"
 
 namespace b200 {
 
@@ -35,7 +37,7 @@ struct ChunkParams {
   float* state;                                    // [slots, H, d, dv]
   float* norm_state; float* norm_out;              // [slots, H, d], [n, H] (row)
   float* out;                                      // [n, H * dv]
-  float* records;                                  // [chunks][H][record_floats]
+  void* records;                                   // [chunks][H][record_bytes]
   const int* q_start; const int* slots;
   int entries, H, Hqk, d, dp, dv, act;             // dp: d rounded up to 32, 64 or 128
   float q_scale;
@@ -49,9 +51,21 @@ __device__ __forceinline__ Portion portion_of(const ChunkParams& p, int entry) {
   return {first + skip, min(p.most, count - skip)};
 }
 
-// A record: Q [16][dp], K [16][dp], (KF [16][dp],) A [16][16], (T [16][16],) whole [dp].
-__host__ __device__ constexpr int record_floats(int dp, bool delta) {
-  return (delta ? 3 : 2) * kChunkTokens * dp + (delta ? 2 : 1) * kChunkTokens * kChunkTokens + dp;
+// A record: Q, K, (KF,) each three planes of bfloat16 [16][dp + 8] that add up to the float32 numbers, A, (T,) each three planes
+// [16][24] (rows 16 bytes longer than their numbers: ldmatrix then reads eight of them from different banks), whole [dp] floats.
+__host__ __device__ constexpr int record_pitch(int dp) { return dp + 8; }
+constexpr int kSmallPitch = kChunkTokens + 8;
+__host__ __device__ constexpr int record_bytes(int dp, bool delta) {
+  return (delta ? 9 : 6) * kChunkTokens * record_pitch(dp) * 2 + (delta ? 6 : 3) * kChunkTokens * kSmallPitch * 2 + dp * 4;
+}
+// x as the sum of three bfloat16, `plane` numbers apart
+__device__ __forceinline__ void store_parts(__nv_bfloat16* to, int plane, float x) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat16 part = __float2bfloat16_rn(x);
+    to[i * plane] = part;
+    x -= __bfloat162float(part);
+  }
 }
 
 // (as in sequence_state.cu: SiLU of a value that was stored in 16 bits with the hardware's exponential and reciprocal)
@@ -90,7 +104,8 @@ __global__ void __launch_bounds__(128) scan_chunk_records_kernel(const ChunkPara
   const T* qg = static_cast<const T*>(p.q) + static_cast<size_t>(first) * p.ldq + hqk * d + tid;
   const T* kg = static_cast<const T*>(p.k) + static_cast<size_t>(first) * p.ldk + hqk * d + tid;
   const float* gg = p.gate + static_cast<size_t>(first) * p.H * d + h * d + tid;
-  float* record = p.records + (static_cast<size_t>(blockIdx.x) * p.H + h) * record_floats(dp, DELTA);
+  unsigned char* record = reinterpret_cast<unsigned char*>(p.records) + (static_cast<size_t>(blockIdx.x) * p.H + h) * record_bytes(dp, DELTA);
+  const int pitch = record_pitch(dp), plane = C * pitch;
   if (tid < C) {
     const size_t at = static_cast<size_t>(first + tid) * p.H + h;
     alpha[tid] = tid >= count ? 1.f : (GATE == CHUNK_HEAD ? p.decay[h] : GATE == CHUNK_CHANNEL ? 1.f : p.row_decay[at]);
@@ -130,19 +145,19 @@ __global__ void __launch_bounds__(128) scan_chunk_records_kernel(const ChunkPara
   }
   __syncthreads();
   if (tid < dp) {                   // the decays up to a token on q (and k), those behind it on k
-    float* to = record + tid;
+    __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(record) + tid;
     float f = 1.f;
 #pragma unroll
     for (int t = 0; t < C; ++t) {
       f *= GATE == CHUNK_CHANNEL ? g[GATE == CHUNK_CHANNEL ? t : 0] : alpha[t];
-      to[t * dp] = q[t] * f;
-      if (DELTA) to[(2 * C + t) * dp] = k[t] * f;
+      store_parts(to + t * pitch, plane, q[t] * f);
+      if (DELTA) store_parts(to + 6 * plane + t * pitch, plane, k[t] * f);
     }
-    record[record_floats(dp, DELTA) - dp + tid] = f;
+    reinterpret_cast<float*>(record + record_bytes(dp, DELTA))[tid - dp] = f;
     f = 1.f;
 #pragma unroll
     for (int t = C - 1; t >= 0; --t) {
-      to[(C + t) * dp] = k[t] * (GATE == CHUNK_ROW ? f * gain[t] : f);
+      store_parts(to + 3 * plane + t * pitch, plane, k[t] * (GATE == CHUNK_ROW ? f * gain[t] : f));
       f *= GATE == CHUNK_CHANNEL ? g[GATE == CHUNK_CHANNEL ? t : 0] : alpha[t];
     }
   }
@@ -254,232 +269,364 @@ __global__ void __launch_bounds__(128) scan_chunk_records_kernel(const ChunkPara
     }
   }
   __syncthreads();
-  float* to = record + (DELTA ? 3 : 2) * C * dp;
+  __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(record) + (DELTA ? 9 : 6) * plane;
   for (int idx = tid; idx < C * C; idx += 128) {
-    to[idx] = as[idx / C][idx % C];
-    if (DELTA) to[C * C + idx] = ts[idx / C][idx % C];
+    const int at = idx / C * kSmallPitch + idx % C;
+    store_parts(to + at, C * kSmallPitch, as[idx / C][idx % C]);
+    if (DELTA) store_parts(to + 3 * C * kSmallPitch + at, C * kSmallPitch, ts[idx / C][idx % C]);
   }
 }
 
 // ---------------------------------------------------------------------------------------------------- the chunks
-// One CTA per request, head and 32 value columns.  Warp w holds rows 16 w .. 16 w + 15 of the state, a lane four rows and
-// four columns of them, in registers for the whole portion.  Records come two chunks ahead by asynchronous copies into a ring
-// of three.  Per chunk:
-//   every warp multiplies its rows of the state with all sixteen q (k); the lanes that share columns exchange sums, the
-//   warps' sums meet in shared memory;
-//   o and u are finished with A and T, a warp a token, a lane a column; the state takes its sixteen updates.
-// Bound by the latency of a chunk's steps (two to four barriers; 2.2 us a chunk) and by the reads of shared memory beside
-// them, where a value that all lanes read alike costs as much as one each: it meets four columns a lane.  With rows that
-// this kernel's threads fetched and scaled themselves a chunk took 3.9 us.  2,048 tokens of 32 heads of 128 x 128, records and
-// chunks: 39 + 280 us with one decay a head (685 token by token), 80 + 390 with the delta rule and decays per channel (958);
-// three portions of 578 tokens: 46 + 164 with decays per channel (542), 33 + 212 with row gates (438).
+// One CTA per request, head and 32 value columns; two warps hold 16 columns of the state, transposed, half of the rows each, in registers
+// for the whole portion, laid out as the accumulators of mma.sync m16n8k16 (16 columns x 8 rows a tile).  So the state is the row operand
+// of S^T q (k) as it stands and its update is accumulated in its own layout; the two warps exchange their halves' sums.  A chunk's
+// record arrives by one bulk copy, one or two chunks ahead.
+// Float32 factors are sums of three bfloat16 (24 bits); of the nine products of two, the six that reach 2^-24 of the whole are formed on the
+// tensor cores.  Those truncate the sums they accumulate, so every leading product (largest part with largest part) is summed by itself from zero
+// and added in float32, and so is what a chunk adds to the state.  Errors against 64 bits over 400 to 2,000 tokens of 8 to 32 heads, all forms:
+// 0.80 to 1.00 of the FMA kernel's that this one replaced in the read-outs, 0.76 to 1.00 in the states.
+// Bound by the issue of the two warps' instructions: 102 (VSPLIT) or 75 matrix instructions a chunk and warp, 156 with the delta rule, 8.2 clocks each,
+// and about as many others.  With records, 2,048 tokens of 32 heads of 128 x 128: one decay a head 262 us (317 with the FMA kernel, whose warps held
+// 16 rows x 32 columns each and exchanged every sum), delta rule with decays per channel 352 (460); 16 heads 232 and 300 (299, 424); three portions of
+// 578 tokens, 32 heads: decays per channel 159 (217), row gates 172 (250); one of 1,733 with row gates 213 (354).
 // ROW: the normaliser is one more column, behind the last value column, whose value is 1 for every token.
-constexpr int kRing = 3;
-template <typename TV, bool DELTA, bool ROW, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) scan_chunk_kernel(const ChunkParams p) {
-  constexpr int C = kChunkTokens, NC = kChunkCols, DP = WARPS * 16, THREADS = WARPS * 32, RECORD = record_floats(DP, DELTA);
-  constexpr int VPT = C / WARPS;                        // value elements a thread stages, tokens it finishes
-  extern __shared__ __align__(16) float smem[];
-  float* ring = smem;                                   // [kRing][RECORD]
-  float* vs = ring + kRing * RECORD;                    // [2][C][NC]
-  float* us = vs + 2 * C * NC;                          // [C][NC] (delta rule)
-  float* red = us + (DELTA ? C * NC : 0);               // [WARPS][C][NC]
-  float* redk = red + WARPS * C * NC;                   // [WARPS][C][NC] (delta rule)
+// A value that is not finite must not reach the tokens before its own, whose weight for it is 0: where a warp meets one, the sums over
+// a chunk's tokens are formed one by one (up_to_now).
+struct Triple { uint32_t part[3]; };        // two neighbouring values: three bfloat16 pairs that add up to them, largest first
+__device__ __forceinline__ Triple split_pair(float x, float y) {
+  Triple s;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    s.part[i] = pack_bf16(x, y);
+    x -= __uint_as_float(s.part[i] << 16);
+    y -= __uint_as_float(s.part[i] & 0xffff0000u);
+  }
+  return s;
+}
+// the accumulators of two neighbouring tiles (16 columns x 16 rows or tokens) as three row operands of 16 x 16
+__device__ __forceinline__ void split_tiles(const float (&lo)[4], const float (&hi)[4], uint32_t (&a)[3][4]) {
+  const Triple x[4] = {split_pair(lo[0], lo[1]), split_pair(lo[2], lo[3]), split_pair(hi[0], hi[1]), split_pair(hi[2], hi[3])};
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) a[i][j] = x[j].part[i];
+}
+// (as mma_bf16, but free to be moved among other instructions: nothing but registers go in and out)
+__device__ __forceinline__ void mma_free(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// which parts of the two factors make the six products, smallest first; with one part only of the first factor, three
+__device__ constexpr int kPartA[6] = {2, 0, 1, 1, 0, 0}, kPartB[6] = {0, 2, 1, 0, 1, 0};
+
+constexpr int kChunkTiles = kChunkCols / 16, kChunkThreads = kChunkTiles * 64;
+// records in shared memory: as many as leave room for two CTAs an SM
+__host__ __device__ constexpr int record_ring(bool delta) { return delta ? 2 : 3; }
+__device__ int g_scan_error = 0;
+template <typename TV, bool DELTA, bool ROW, bool VSPLIT, int DT>
+__global__ void __launch_bounds__(kChunkThreads) scan_chunk_kernel(const ChunkParams p) {
+  constexpr int C = kChunkTokens, DP = DT * 16, RECORD = record_bytes(DP, DELTA), RING = record_ring(DELTA), PITCH = record_pitch(DP) * 2, HT = DT / 2;
+  constexpr int PLANE = C * PITCH, SMALL = C * kSmallPitch * 2, UPARTS = VSPLIT || DELTA ? 3 : 1;
+  extern __shared__ __align__(16) unsigned char ring[];   // [RING][RECORD]
+  __shared__ __align__(8) uint64_t full[RING];
+  __shared__ float4 handed[DELTA ? 3 : 1][kChunkTiles][2][32];     // sums over half of the rows for the other half's warp: of a read-out, of w
   pdl_trigger();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, tile = warp >> 1, half = warp & 1;
+  if (tid == 0) {
+    for (int i = 0; i < RING; ++i) mbar_init(full + i, 1);
+    fence_barrier_init();
+  }
   pdl_wait();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int d = p.d, dv = p.dv, columns = dv + (ROW ? 1 : 0), col_blocks = (columns + NC - 1) / NC;
-  const int h = blockIdx.x / col_blocks, col0 = blockIdx.x % col_blocks * NC, col = col0 + lane, entry = blockIdx.y;
+  const int d = p.d, dv = p.dv, columns = dv + (ROW ? 1 : 0), col_blocks = (columns + kChunkCols - 1) / kChunkCols;
+  const int h = blockIdx.x / col_blocks, col0 = blockIdx.x % col_blocks * kChunkCols + tile * 16, entry = blockIdx.y;
   const Portion portion = portion_of(p, entry);
   const int t_begin = portion.first, t_end = t_begin + portion.count;
   if (t_begin >= t_end) return;
   int slot0 = 0;                                        // this request's first record
   for (int e = 0; e < entry; ++e) slot0 += (portion_of(p, e).count + C - 1) / C;
   const int chunks = (t_end - t_begin + C - 1) / C;
-  const bool is_norm = ROW && col == dv, live = col < dv || is_norm;
   const size_t head = static_cast<size_t>(p.slots[entry]) * p.H + h;
+  __syncthreads();                                      // the barriers are there
 
-  auto ask = [&](int chunk) {                           // a group of copies per call, empty past the last chunk
-    if (chunk < chunks) {
-      const float* src = p.records + (static_cast<size_t>(slot0 + chunk) * p.H + h) * RECORD;
-      const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(ring + chunk % kRing * RECORD));
-#pragma unroll
-      for (int i = 0; i < (RECORD / 4 + THREADS - 1) / THREADS; ++i) {
-        const int at = tid + i * THREADS;
-        if (at < RECORD / 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + at * 16), "l"(src + at * 4) : "memory");
-      }
+  const unsigned char* next_record = static_cast<const unsigned char*>(p.records) + (static_cast<size_t>(slot0) * p.H + h) * RECORD;
+  int next_slot = 0, left = chunks;                     // of the records still to be asked for
+  auto ask = [&]() {                                    // one thread
+    if (left > 0) {
+      mbar_expect_tx(full + next_slot, RECORD);
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(smem_addr(ring + next_slot * RECORD)),
+                   "l"(next_record), "r"(RECORD), "r"(smem_addr(full + next_slot))
+                   : "memory");
+      next_record += static_cast<size_t>(p.H) * RECORD;
+      next_slot = next_slot + 1 == RING ? 0 : next_slot + 1;
+      --left;
     }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  ask(0);
-  ask(1);
-  const TV* vg = static_cast<const TV*>(p.v) + static_cast<size_t>(h) * dv + col;
-  TV rv[VPT];                       // kept in the storage type: a conversion right behind the load would wait for it
+  if (tid == 0)
+    for (int i = 1; i < RING; ++i) ask();
+  // this lane's columns: col0 + g and 8 further on; its tokens of a chunk: 2 t, 2 t + 1 and 8 further on; its rows of tile j: row0 + 8 j + 2 t, + 1
+  const bool working = col0 < columns;
+  const int row0 = half * (DP / 2);
+  TV rv[2][4];                      // kept in the storage type: a conversion right behind the load would wait for it
+  const TV* vg = static_cast<const TV*>(p.v) + static_cast<size_t>(h) * dv + col0 + g;
   auto fetch_values = [&](int t0) {
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int t = t0 + warp + i * WARPS;
-      rv[i] = t < t_end && col < dv ? vg[static_cast<size_t>(t) * p.ldv] : from_float<TV>(t < t_end && is_norm ? 1.f : 0.f);
+    for (int i = 0; i < 8; ++i) {
+      const int tok = t0 + (i >> 2) * 8 + 2 * t + (i & 1), c = ((i >> 1) & 1) * 8;
+      rv[i >> 2][i & 3] = tok < t_end && col0 + g + c < dv ? vg[static_cast<size_t>(tok) * p.ldv + c]
+                                                           : from_float<TV>(ROW && tok < t_end && col0 + g + c == dv ? 1.f : 0.f);
     }
   };
   fetch_values(t_begin);
-
-  // the lane's part of the state: rows row0 .. row0 + 3, columns col0 + cl .. + 3
-  const int cl = lane % 8 * 4, row0 = warp * 16 + lane / 8 * 4;
   auto cell = [&](int r, int c) -> float* {             // null where there is none
     if (r >= d) return nullptr;
     if (ROW && c == dv) return p.norm_state + head * d + r;
     return c < dv ? p.state + (head * d + r) * dv + c : nullptr;
   };
-  float2 S[4][2];                                       // [column][pair of rows]
+  float S[2 * HT][4];
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
+  for (int j = 0; j < 2 * HT; ++j)
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float* x = cell(row0 + 2 * i, col0 + cl + c);
-      const float* y = cell(row0 + 2 * i + 1, col0 + cl + c);
-      S[c][i] = make_float2(x ? *x : 0.f, y ? *y : 0.f);
+    for (int e = 0; e < 4; ++e) {
+      const float* x = cell(row0 + 8 * j + 2 * t + (e & 1), col0 + g + (e >> 1) * 8);
+      S[j][e] = x ? *x : 0.f;
     }
-
-  // x[t] . S over the warp's rows for the sixteen t, into to[warp][t][column]
-  auto times_state = [&](const float* x, float* to) {
-    const bool upper2 = (lane & 16) != 0, upper1 = (lane & 8) != 0;
-#pragma unroll
-    for (int t0 = 0; t0 < C; t0 += 4) {
-      float part[4][4];                                 // [token][column]
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float4 v = *reinterpret_cast<const float4*>(x + (t0 + t) * DP + row0);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float2 a = __ffma2_rn(make_float2(v.z, v.w), S[c][1], __fmul2_rn(make_float2(v.x, v.y), S[c][0]));
-          part[t][c] = a.x + a.y;
-        }
-      }
-      // the four lanes of a column share the four tokens out: the lane of rows 4 r keeps token r
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float send = upper2 ? part[t][c] : part[t + 2][c];
-          part[t][c] = (upper2 ? part[t + 2][c] : part[t][c]) + __shfl_xor_sync(0xffffffffu, send, 16);
-        }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float send = upper1 ? part[0][c] : part[1][c];
-        part[0][c] = (upper1 ? part[1][c] : part[0][c]) + __shfl_xor_sync(0xffffffffu, send, 8);
-      }
-      *reinterpret_cast<float4*>(to + (warp * C + t0 + lane / 8) * NC + cl) = make_float4(part[0][0], part[0][1], part[0][2], part[0][3]);
-    }
+  // ldmatrix: rows of column operands whose K runs along them (q, k: tokens; A, T: tokens), and of k as rows of K, which it transposes
+  const int row_n = (lane >> 4) * 8 + (lane & 7), half_n = ((lane >> 3) & 1) * 16;
+  const int row_k = ((lane >> 3) & 1) * 8 + (lane & 7), half_k = (lane >> 4) * 16;
+  auto load_n = [&](uint32_t (&r)[4], uint32_t base, int pitch, int step) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(base + row_n * pitch + step * 32 + half_n));
   };
-  auto update_state = [&](const float* kt, const float* whole, const float* u) {
-    const float4 f = *reinterpret_cast<const float4*>(whole + row0);
+  auto load_k = [&](uint32_t (&r)[4], uint32_t base, int step) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(base + row_k * PITCH + step * 32 + half_k));
+  };
+  auto pair_barrier = [&]() { asm volatile("bar.sync %0, 64;\n" ::"r"(tile + 1) : "memory"); };
+
+  // S^T x over this warp's rows for the sixteen rows of x (three planes from `planes` on): [tile of tokens][accumulator]
+  auto times_state = [&](uint32_t planes, float (&out)[2][4]) {
+    float lead[HT][2][4] = {}, rest[2][2][4] = {};      // (a leading product's sum is truncated once, not again by those behind it)
+    uint32_t ahead[3][4];                               // the next step's rows: asked for under this one's products
+    planes += row0 * 2;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      S[c][0] = __fmul2_rn(S[c][0], make_float2(f.x, f.y));
-      S[c][1] = __fmul2_rn(S[c][1], make_float2(f.z, f.w));
+    for (int i = 0; i < 3; ++i) load_n(ahead[i], planes + i * PLANE, PITCH, 0);
+#pragma unroll
+    for (int ks = 0; ks < HT; ++ks) {
+      uint32_t a[3][4], b[3][4];
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[i][j] = ahead[i][j];
+      if (ks + 1 < HT) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) load_n(ahead[i], planes + i * PLANE, PITCH, ks + 1);
+      }
+      split_tiles(S[2 * ks], S[2 * ks + 1], a);
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) mma_free(i == 5 ? lead[ks][nt] : rest[i & 1][nt], a[kPartA[i]], b[kPartB[i]][2 * nt], b[kPartB[i]][2 * nt + 1]);
     }
 #pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+#pragma unroll
+        for (int n = 1; n < HT; n *= 2)
+#pragma unroll
+          for (int ks = 0; ks + n < HT; ks += 2 * n) lead[ks][nt][e] += lead[ks + n][nt][e];
+        out[nt][e] = (rest[0][nt][e] + rest[1][nt][e]) + lead[0][nt][e];
+      }
+  };
+  auto finite = [&](const float (&x)[2][4]) {           // of all lanes
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) bad |= !isfinite(x[i >> 2][i & 3]);
+    return !__any_sync(0xffffffffu, bad);
+  };
+  // out[t] += sum over s <= t of M[t][s] x[s] for eight tokens from `first` on, M in three planes; x also as row operands in `parts` planes
+  auto up_to_now = [&](uint32_t m, int first, const float (&x)[2][4], bool all_finite, const uint32_t (&a)[3][4], int parts, float (&out)[4]) {
+    if (all_finite) {
+      uint32_t b[3][2];
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n"
+                     : "=r"(b[i][0]), "=r"(b[i][1])
+                     : "r"(m + i * SMALL + (first + (lane & 7)) * (kSmallPitch * 2) + half_n));
+      float lead[4] = {}, rest[2][4] = {};
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        if (kPartA[i] >= parts) continue;
+        mma_free(i == 5 ? lead : rest[i & 1], a[kPartA[i]], b[kPartB[i]][0], b[kPartB[i]][1]);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) out[e] += (rest[0][e] + rest[1][e]) + lead[e];
+      return;
+    }
+#pragma unroll 1
     for (int s = 0; s < C; ++s) {
-      const float4 k = *reinterpret_cast<const float4*>(kt + s * DP + row0);
-      const float4 x = *reinterpret_cast<const float4*>(u + s * NC + cl);
-      const float xs[4] = {x.x, x.y, x.z, x.w};
+      const int from = (lane & ~3) | ((s & 7) >> 1);
+      float x0 = 0.f, x1 = 0.f;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        S[c][0] = __ffma2_rn(make_float2(k.x, k.y), make_float2(xs[c], xs[c]), S[c][0]);
-        S[c][1] = __ffma2_rn(make_float2(k.z, k.w), make_float2(xs[c], xs[c]), S[c][1]);
+      for (int i = 0; i < 4; ++i) {                     // (tile, parity) of token s
+        const float y0 = __shfl_sync(0xffffffffu, x[i >> 1][i & 1], from), y1 = __shfl_sync(0xffffffffu, x[i >> 1][2 + (i & 1)], from);
+        if ((s >> 3) * 2 + (s & 1) == i) { x0 = y0; x1 = y1; }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int tok = first + 2 * t + i;
+        if (s > tok) continue;
+        float f = 0.f;
+#pragma unroll
+        for (int part = 2; part >= 0; --part) {
+          uint16_t bits;
+          asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(bits) : "r"(m + part * SMALL + (tok * kSmallPitch + s) * 2));
+          f += __uint_as_float(static_cast<uint32_t>(bits) << 16);
+        }
+        out[i] = fmaf(f, x0, out[i]);
+        out[2 + i] = fmaf(f, x1, out[2 + i]);
       }
     }
   };
 
-  // sum over s <= t of row[s] * u[s][lane], added to x: the row is the same for all lanes
-  auto combine = [&](const float* row, const float* u, int t, float x) {
-#pragma unroll
-    for (int s = 0; s < C; s += 4) {
-      const float4 a = *reinterpret_cast<const float4*>(row + s);
-      if (s <= t) x = fmaf(a.x, u[s * NC + lane], x);            // (later tokens' rows are not touched: they may hold anything)
-      if (s + 1 <= t) x = fmaf(a.y, u[(s + 1) * NC + lane], x);
-      if (s + 2 <= t) x = fmaf(a.z, u[(s + 2) * NC + lane], x);
-      if (s + 3 <= t) x = fmaf(a.w, u[(s + 3) * NC + lane], x);
+  int slot = 0;
+  uint32_t phase = 0;
+  for (int t0 = t_begin; t0 < t_end; t0 += C) {
+    const bool ok = mbar_wait(full + slot, phase);
+    if (!__syncthreads_and(ok)) {                       // (the record is there; the one before has been read)
+      if (tid == 0) {                                   // (copies on their way still get their time)
+        atomicExch(&g_scan_error, 1);
+        for (int i = 0; i < RING; ++i) mbar_wait(full + i, i < slot ? phase ^ 1 : phase);
+      }
+      return;
     }
-    return x;
-  };
-  auto gathered = [&](const float* parts, int t) {
-    float x = 0.f;
+    if (tid == 0) ask();
+    const unsigned char* record_at = ring + slot * RECORD;
+    if (++slot == RING) { slot = 0; phase ^= 1; }
+    if (!working) continue;
+    const uint32_t record = smem_addr(record_at), small = record + (DELTA ? 9 : 6) * PLANE;
+    const float* whole = reinterpret_cast<const float*>(record_at + RECORD - DP * 4) + row0 + 2 * t;
+    float u[2][4], o[2][4];
 #pragma unroll
-    for (int part = 0; part < WARPS; ++part) x += parts[(part * C + t) * NC + lane];
-    return x;
-  };
-
-  for (int chunk = 0; chunk < chunks; ++chunk) {
-    const int t0 = t_begin + chunk * C, count = min(C, t_end - t0);
-    const float* record = ring + chunk % kRing * RECORD;
-    const float* am = record + (DELTA ? 3 : 2) * C * DP;
-    const float* whole = record + RECORD - DP;
-    float* v = vs + (chunk & 1) * C * NC;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      float x = to_float(rv[i]);
-      if (p.act) x = chunk_silu<TV>(x);
-      v[(warp + i * WARPS) * NC + lane] = x;
+    for (int i = 0; i < 8; ++i) {
+      float x = to_float(rv[i >> 2][i & 3]);
+      if (VSPLIT && p.act) x = chunk_silu<TV>(x);
+      u[i >> 2][i & 3] = x;
     }
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    __syncthreads();                                    // the record and the values are there; the chunk before has been read
-    ask(chunk + 2);
     fetch_values(t0 + C);
-    times_state(record, red);
-    if constexpr (DELTA) times_state(record + 2 * C * DP, redk);
-    else update_state(record + C * DP, whole, v);
-    __syncthreads();                                    // the warps' sums are there
+    uint32_t a[3][4];
     if constexpr (DELTA) {
+      float w[2][4];
+      times_state(record + 6 * PLANE, w);
+      handed[1][tile][half][lane] = make_float4(w[0][0], w[0][1], w[0][2], w[0][3]);
+      handed[2][tile][half][lane] = make_float4(w[1][0], w[1][1], w[1][2], w[1][3]);
+      pair_barrier();
+      float sums[2][2][4];                              // both warps add the halves up in their order
 #pragma unroll
-      for (int i = 0; i < VPT; ++i) {
-        const int t = warp + i * WARPS;
-        v[t * NC + lane] -= gathered(redk, t);
+      for (int i = 0; i < 4; ++i) {
+        const float4 x = handed[1 + (i & 1)][tile][i >> 1][lane];
+        sums[i >> 1][i & 1][0] = x.x; sums[i >> 1][i & 1][1] = x.y; sums[i >> 1][i & 1][2] = x.z; sums[i >> 1][i & 1][3] = x.w;
       }
-      __syncthreads();
 #pragma unroll
-      for (int i = 0; i < VPT; ++i) {
-        const int t = warp + i * WARPS;
-        us[t * NC + lane] = combine(am + C * C + t * C, v, t, 0.f);
+      for (int i = 0; i < 8; ++i) {
+        w[i >> 2][i & 3] = u[i >> 2][i & 3] - (sums[0][i >> 2][i & 3] + sums[1][i >> 2][i & 3]);
+        u[i >> 2][i & 3] = 0.f;
       }
-      __syncthreads();
+      split_tiles(w[0], w[1], a);
+      const bool plain = finite(w);
+      up_to_now(small + 3 * SMALL, 0, w, plain, a, 3, u[0]);
+      up_to_now(small + 3 * SMALL, 8, w, plain, a, 3, u[1]);
     }
+    const bool plain = finite(u);
+    if constexpr (UPARTS == 3) {
+      split_tiles(u[0], u[1], a);
+    } else {                                            // the values are bfloat16
+      a[0][0] = pack_bf16(u[0][0], u[0][1]);
+      a[0][1] = pack_bf16(u[0][2], u[0][3]);
+      a[0][2] = pack_bf16(u[1][0], u[1][1]);
+      a[0][3] = pack_bf16(u[1][2], u[1][3]);
+    }
+    times_state(record, o);
+    // each of the two warps finishes eight tokens of the read-out
+    handed[0][tile][half][lane] = half ? make_float4(o[0][0], o[0][1], o[0][2], o[0][3]) : make_float4(o[1][0], o[1][1], o[1][2], o[1][3]);
+    // the state takes its decay and the sixteen tokens' updates, four tiles of eight rows at a time
+    uint32_t ahead[3][2][4];
+    constexpr int GROUP = HT > 1 ? 4 : 2;               // tiles at a time
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int t = warp + i * WARPS;
-      const float o = combine(am + t * C, DELTA ? us : v, t, gathered(red, t));
-      if (live && t < count) {
-        if (is_norm) p.norm_out[static_cast<size_t>(t0 + t) * p.H + h] = o;
-        else p.out[(static_cast<size_t>(t0 + t) * p.H + h) * dv + col] = o;
+    for (int i = 0; i < 3 * GROUP / 2; ++i) load_k(ahead[i / (GROUP / 2)][i % (GROUP / 2)], record + (3 + i / (GROUP / 2)) * PLANE + row0 * 2, i % (GROUP / 2));
+#pragma unroll
+    for (int j = 0; j < 2 * HT; j += GROUP) {
+      float sum[GROUP][4] = {}, top[GROUP][4] = {};
+      uint32_t b[3][2][4];
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) b[i >> 1][i & 1][x] = ahead[i >> 1][i & 1][x];
+      if (j + GROUP < 2 * HT) {
+#pragma unroll
+        for (int i = 0; i < 6; ++i) load_k(ahead[i >> 1][i & 1], record + (3 + (i >> 1)) * PLANE + row0 * 2, j / 2 + 2 + (i & 1));
+      }
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        if (kPartA[i] >= UPARTS) continue;
+#pragma unroll
+        for (int x = 0; x < GROUP; ++x) mma_free(i == 5 ? top[x] : sum[x], a[kPartA[i]], b[kPartB[i]][x >> 1][(x & 1) * 2], b[kPartB[i]][x >> 1][(x & 1) * 2 + 1]);
+      }
+#pragma unroll
+      for (int x = 0; x < GROUP; ++x) {
+        const float2 f = *reinterpret_cast<const float2*>(whole + 8 * (j + x));
+        S[j + x][0] = fmaf(S[j + x][0], f.x, sum[x][0]) + top[x][0];
+        S[j + x][1] = fmaf(S[j + x][1], f.y, sum[x][1]) + top[x][1];
+        S[j + x][2] = fmaf(S[j + x][2], f.x, sum[x][2]) + top[x][2];
+        S[j + x][3] = fmaf(S[j + x][3], f.y, sum[x][3]) + top[x][3];
       }
     }
-    if constexpr (DELTA) update_state(record + C * DP, whole, us);
+    pair_barrier();
+    const float4 other = handed[0][tile][half ^ 1][lane];
+    float mine[4] = {other.x + (half ? o[1][0] : o[0][0]), other.y + (half ? o[1][1] : o[0][1]), other.z + (half ? o[1][2] : o[0][2]),
+                     other.w + (half ? o[1][3] : o[0][3])};
+    up_to_now(small, half * 8, u, plain, a, UPARTS, mine);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int tok = t0 + half * 8 + 2 * t + (i & 1), c = col0 + g + (i >> 1) * 8;
+      if (tok >= t_end) continue;
+      if (c < dv) p.out[(static_cast<size_t>(tok) * p.H + h) * dv + c] = mine[i];
+      else if (ROW && c == dv) p.norm_out[static_cast<size_t>(tok) * p.H + h] = mine[i];
+    }
   }
+  if (!working) return;
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
+  for (int j = 0; j < 2 * HT; ++j)
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      float* x = cell(row0 + 2 * i, col0 + cl + c);
-      float* y = cell(row0 + 2 * i + 1, col0 + cl + c);
-      if (x) *x = S[c][i].x;
-      if (y) *y = S[c][i].y;
+    for (int e = 0; e < 4; ++e) {
+      float* x = cell(row0 + 8 * j + 2 * t + (e & 1), col0 + g + (e >> 1) * 8);
+      if (x) *x = S[j][e];
     }
 }
 
-template <typename TV, bool DELTA, bool ROW, int WARPS>
+template <typename TV, bool DELTA, bool ROW, bool VSPLIT, int DT>
 int launch_chunks(const ChunkParams& p, cudaStream_t stream) {
-  constexpr int C = kChunkTokens, NC = kChunkCols;
-  constexpr size_t smem = sizeof(float) * (kRing * record_floats(WARPS * 16, DELTA) + (DELTA ? 3 : 2) * C * NC + (DELTA ? 2 : 1) * WARPS * C * NC);
+  constexpr size_t smem = record_ring(DELTA) * record_bytes(DT * 16, DELTA);
   static DeviceOnce once;
-  const int status = configure_once(once, scan_chunk_kernel<TV, DELTA, ROW, WARPS>, smem);
+  const int status = configure_once(once, scan_chunk_kernel<TV, DELTA, ROW, VSPLIT, DT>, smem + 8 * 1024);      // (the kernel's own arrays count too)
   if (status) return status;
   const int columns = p.dv + (ROW ? 1 : 0);
-  launch(scan_chunk_kernel<TV, DELTA, ROW, WARPS>, dim3(p.H * ((columns + NC - 1) / NC), p.entries), dim3(WARPS * 32), smem, stream, p);
+  launch(scan_chunk_kernel<TV, DELTA, ROW, VSPLIT, DT>, dim3(p.H * ((columns + kChunkCols - 1) / kChunkCols), p.entries), dim3(kChunkThreads), smem, stream, p);
   return launch_status();
 }
 
 inline int padded_dim(int d) { return d <= 32 ? 32 : (d <= 64 ? 64 : 128); }
+
+template <typename TV, bool DELTA, bool ROW, bool VSPLIT>
+int launch_chunks_of(const ChunkParams& p, cudaStream_t stream) {
+  if (p.dp == 32) return launch_chunks<TV, DELTA, ROW, VSPLIT, 2>(p, stream);
+  if (p.dp == 64) return launch_chunks<TV, DELTA, ROW, VSPLIT, 4>(p, stream);
+  return launch_chunks<TV, DELTA, ROW, VSPLIT, 8>(p, stream);
+}
 
 template <typename T, typename TV, bool DELTA, int GATE>
 int run_chunks(ChunkParams p, int chunks, cudaStream_t stream) {
@@ -487,9 +634,10 @@ int run_chunks(ChunkParams p, int chunks, cudaStream_t stream) {
   p.dp = padded_dim(p.d);
   launch(scan_chunk_records_kernel<T, DELTA, GATE>, dim3(chunks, p.H), dim3(128), 0, stream, p);
   if (int e = launch_status()) return e;
-  if (p.dp == 32) return launch_chunks<TV, DELTA, ROW, 2>(p, stream);
-  if (p.dp == 64) return launch_chunks<TV, DELTA, ROW, 4>(p, stream);
-  return launch_chunks<TV, DELTA, ROW, 8>(p, stream);
+  if constexpr (!DELTA) {
+    if (!p.act) return launch_chunks_of<TV, DELTA, ROW, false>(p, stream);
+  }
+  return launch_chunks_of<TV, DELTA, ROW, true>(p, stream);
 }
 
 // ---------------------------------------------------------------------------------------------------- single tokens
@@ -636,7 +784,7 @@ int scan_form(const ChunkParams& p, int chunks, int dtype, int v_dtype, cudaStre
 // them): a long portion's records need not all be there at once, its state goes from launch to launch in the request's slot.
 // `chunks`: at least the number of chunks of 16 tokens of all requests in it; records: chunks * H * b200_scan_chunks_record_floats(d,
 // delta) floats, 16-byte aligned.
-extern "C" long b200_scan_chunks_record_floats(int d, int delta) { return b200::record_floats(b200::padded_dim(d), delta != 0); }
+extern "C" long b200_scan_chunks_record_floats(int d, int delta) { return b200::record_bytes(b200::padded_dim(d), delta != 0) / 4; }
 
 extern "C" int b200_scan_chunks(const void* q, const void* k, const void* v, int ldq, int ldk, int ldv, const float* gate,
                                 const float* decay, const float* row_decay, const float* row_gain, const float* beta, float* state,
@@ -662,4 +810,13 @@ extern "C" int b200_scan_single(const void* q, const void* k, const void* v, int
   const ChunkParams p{q, k, v, ldq, ldk, ldv, gate, decay, row_decay, row_gain, beta, state, norm_state, norm_out, out, nullptr,
                       q_start, slots, entries, H, Hqk, d, 0, dv, act, q_scale, 0, 1};
   return scan_form<false>(p, 1, dtype, v_dtype, stream);
+}
+
+// Read and clear the error flag set by a bounded wait that ran out.  Synchronises the device.
+extern "C" int b200_scan_chunks_error() {
+  int v = 0, zero = 0;
+  if (cudaDeviceSynchronize() != cudaSuccess) return -1;
+  cudaMemcpyFromSymbol(&v, b200::g_scan_error, sizeof(int));
+  cudaMemcpyToSymbol(b200::g_scan_error, &zero, sizeof(int));
+  return v;
 }

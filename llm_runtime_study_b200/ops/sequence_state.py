@@ -16,8 +16,11 @@ native.register_library(
     "b200_scan_chunks", ("scan_chunks.cu",),
     {"b200_scan_chunks": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, *[c_void_p] * 12, *[c_int] * 9, c_float, c_int, c_int, c_void_p],
      "b200_scan_chunks_record_floats": [c_int, c_int],
+     "b200_scan_chunks_error": [],
      "b200_scan_single": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, *[c_void_p] * 11, *[c_int] * 6, c_float, c_int, c_int, c_void_p]},
 )
+
+native.register_error_probe("b200_scan_chunks", "b200_scan_chunks_error", "linear scan in chunks")
 
 CHUNK_TOKENS, CHUNK_MAX_DIM = 16, 128     # tokens a chunk, largest key size of the chunked kernel
 CHUNK_MIN_TOKENS = 48                     # tokens beyond one per request from which a batch may be scanned in chunks
@@ -37,7 +40,8 @@ def _lengths(lens: "Sequence[int] | None", n: int, entries: int) -> "Sequence[in
 
 
 def _record_bytes(n: int, entries: int, heads: int, dim: int) -> int:
-    """What the records of a batch take (the larger form, the delta rule's)."""
+    """What the numbers of a batch's records take in float32 (the larger form, the delta rule's; the records themselves, whose
+    numbers are three bfloat16 each, half as much again: they are held in slices)."""
 
     dim = 32 if dim <= 32 else (64 if dim <= 64 else 128)
     return (n // CHUNK_TOKENS + entries) * heads * 4 * (3 * CHUNK_TOKENS * dim + 2 * CHUNK_TOKENS * CHUNK_TOKENS + dim)
@@ -56,7 +60,7 @@ def scans_in_chunks(n: int, entries: int, heads: int, dim: int, fixed_order: boo
 def portion_in_chunks(lens: "Sequence[int]", heads: int, dim: int, columns: int, delta: bool) -> int:
     """The number of tokens from which a portion of a batch is scanned in chunks (0: none is); ``columns``: of a head's state.
 
-    A chunk costs about 2.2 us behind some 8 us for the records; a token of a chain 0.2 us as long as the chains' CTAs of 8 columns
+    A chunk costs 1.4 to 1.8 us (2.2 when the sums below were taken: with a kernel of its time) behind some 8 us for the records; a token of a chain 0.2 us as long as the chains' CTAs of 8 columns
     all run at once, two an SM, and 0.3 to 0.5 us beyond that.  A chunk takes the same 0.06 us a head (0.13 with the
     delta rule) whether it holds sixteen tokens or one.  So what counts is the portion's own length, not the batch's.  Microseconds in
     chunks and as a chain, 128 x 128: 4 heads, one portion of 64 tokens 21.6, 22.8 (delta rule, a decay per channel 28.3, 24.6), of 96

@@ -225,3 +225,28 @@ def test_a_bad_row_reaches_later_tokens_only():
                         q_start=torch.tensor([0, n], dtype=torch.int32, device=DEV), slots=torch.zeros(1, dtype=torch.int32, device=DEV),
                         decay=torch.full((heads,), 0.9, device=DEV))
     assert bool(torch.isfinite(out[:37]).all()) and not bool(torch.isfinite(out[37:]).any())
+
+
+@pytest.mark.parametrize("form", ["delta", "row"])
+def test_a_bad_value_in_a_chunk_reaches_its_own_column_and_later_tokens_only(form):
+    """Value columns of two warps' tiles and more; tokens of a chunk before the bad one, which share its products on the tensor cores."""
+
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    n, heads, d, dv, bad = 80, 2, 48, 40, 37
+    g = torch.Generator().manual_seed(2)
+    q, k, v = (torch.randn(n, heads * w, generator=g) for w in (d, d, dv))
+    v[bad, dv + 5] = float("nan")                                    # the second head's
+    common = dict(heads=heads, dim=d, vdim=dv, state=torch.zeros(1, heads, d, dv, device=DEV), lens=[n],
+                  q_start=torch.tensor([0, n], dtype=torch.int32, device=DEV), slots=torch.zeros(1, dtype=torch.int32, device=DEV))
+    token = torch.rand(n, heads, generator=g).to(DEV)
+    if form == "delta":
+        out = S.linear_scan(q.to(DEV), (k / d ** 0.5).to(DEV), v.to(DEV), qk_heads=heads, row_decay=token, beta=token, **common)
+    else:
+        rows = (x.bfloat16().to(DEV) for x in (q, k, v))
+        out, den = S.linear_scan_row_gates(*rows, decay=token, gain=token, norm_state=torch.zeros(1, heads, d, device=DEV), **common)
+        assert bool(torch.isfinite(den).all())
+    fine = torch.isfinite(out).view(n, heads, dv)
+    want = torch.ones(n, heads, dv, dtype=torch.bool)
+    want[bad:, 1, 5] = False
+    assert torch.equal(fine.cpu(), want)
