@@ -19,10 +19,16 @@
 //     behind it adds those up in CTA order and writes the rows' factors rsqrt(mean of squares + eps); it
 //     releases the kernel after it at its first instruction, so the next projection fetches its first
 //     weights meanwhile.  (Adding them up in every CTA of the consuming kernel, or in the producing
-//     kernel's last CTA behind a ticket, cost 4 to 6 us per layer more: measured.)
+//     kernel's last CTA behind a ticket, cost 4 to 6 us per layer more at 4,096 columns and eight rows: measured.)
 //   * SCALED: the rows this kernel multiplies are such weighted, not yet normalised rows.  The factor
 //     is one number per row and commutes with the product, so it is applied to the accumulators.
+//     Of up to kMostSums shares a row (2,048 columns) and eight rows it is formed here (`sums`): a warp a row asks for the shares before its
+//     rows of X and adds them up behind its products, and the one-CTA kernel, which is a link of its own in the chain of a step's launches,
+//     is left out (decode of 28 layers of Qwen3-0.6B, 1 and 8 requests: 826 and
+//     1,050 us with it, 761 and 984 without; nine layers of Qwen3-8B, 4,096 columns, so too: one request 915 -> 909, eight 1,044 -> 1,121).
 // Rounding r * w to bfloat16 before the scale instead of after changes nothing in relative terms.
+#include <type_traits>
+
 #include "common.cuh"
 #include "mma.cuh"
 
@@ -46,9 +52,16 @@ struct NormFusion {
   float eps;                  // EPI_RESIDUAL: its eps
   __nv_bfloat16* weighted;    // EPI_RESIDUAL: out, [M][N] = (residual + product) * next_weight
   float* partials;            // EPI_RESIDUAL: out, [gridDim.x][16] sums of squares of the new residual rows, per CTA
+  const float* sums;          // SCALED, instead of row_scale: such partials of the kernel before, `parts` <= kMostSums of them, rows
+  int parts;                  // of `width` columns, whose norm's eps is `eps`; at most eight rows
+  float width;
 };
+constexpr int kMostSums = 128;
 
-template <int NT, int UNROLL, int kSkinnyWarps, int EPI, bool SCALED, typename OutT>
+// How the rows of X still lack their factors: not at all, as numbers (row_scale), or as shares of their sums of squares (sums).
+enum Scaling : int { SCALE_NONE = 0, SCALE_FACTORS = 1, SCALE_SUMS = 2 };
+
+template <int NT, int UNROLL, int kSkinnyWarps, int EPI, int SCALED, typename OutT>
 __global__ void __launch_bounds__(kSkinnyWarps * 32)
 gemm_skinny_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ X,
                    const float* __restrict__ bias, OutT* __restrict__ C, int M, int N, int K, int ldc, NormFusion fuse) {
@@ -83,6 +96,24 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __r
     }
   }
   pdl_wait();
+  // What the epilogue needs from memory is asked for here: behind the products each would be a wait of its own (0.6 us).
+  float share[SCALED == SCALE_SUMS ? kMostSums / 32 : 1];
+  if constexpr (SCALED == SCALE_SUMS) {
+    if (warp < M) {
+#pragma unroll
+      for (int i = 0; i < kMostSums / 32; ++i) share[i] = lane + 32 * i < fuse.parts ? fuse.sums[(lane + 32 * i) * 16 + warp] : 0.f;
+    }
+  }
+  float have = 0.f, next_w = 0.f, shift = 0.f;
+  if constexpr (EPI == EPI_RESIDUAL) {
+    static_assert(16 * NT * 8 <= kSkinnyWarps * 32, "an output a thread");
+    const int m = threadIdx.x >> 4, n = n0 + (threadIdx.x & 15);
+    if (threadIdx.x < 16 * NT * 8 && m < M && n < N) {
+      have = reinterpret_cast<const float*>(C)[static_cast<size_t>(m) * ldc + n];
+      next_w = fuse.next_weight[n];
+      shift = bias ? bias[n] : 0.f;
+    }
+  }
   for (int k0 = warp * kChunk; k0 < K; k0 += kSkinnyWarps * kChunk) {
 #pragma unroll
     for (int h = 0; h < kChunk / 32; h += UNROLL) {
@@ -117,13 +148,25 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __r
     red[warp][g + 8][j * 8 + 2 * t] = c[j][2];
     red[warp][g + 8][j * 8 + 2 * t + 1] = c[j][3];
   }
+  __shared__ float factors[SCALED == SCALE_SUMS ? 8 : 1];
+  if constexpr (SCALED == SCALE_SUMS) {
+    if (warp < M) {
+      float total = 0.f;
+#pragma unroll
+      for (int i = 0; i < kMostSums / 32; ++i) total += share[i];
+      total = warp_sum(total);
+      if (lane == 0) factors[warp] = rsqrtf(total / fuse.width + fuse.eps);
+    }
+  }
+  // (kept as a plain load where it is used: through shared memory a step of Qwen3-8B size, 8 requests, took 3 % longer)
+  auto factor_of = [&](int m) { return SCALED == SCALE_SUMS ? factors[m] : fuse.row_scale[m]; };
   __syncthreads();
   if constexpr (EPI == EPI_RESIDUAL) {
     // C is the float32 residual stream: add the product in place, write the rows weighted for the next norm,
     // and leave this CTA's share of every row's sum of squares.  All lanes stay in the loop for the shuffles.
     float* resid = reinterpret_cast<float*>(C);
-    for (int idx = threadIdx.x; idx < 16 * NT * 8; idx += kSkinnyWarps * 32) {
-      const int m = idx >> 4, row = idx & 15;
+    if (threadIdx.x < 16 * NT * 8) {
+      const int m = threadIdx.x >> 4, row = threadIdx.x & 15;
       const int n = n0 + row;
       const bool valid = m < M && n < N;
       float r = 0.f;
@@ -131,10 +174,10 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __r
         float acc = 0.f;
 #pragma unroll
         for (int w = 0; w < kSkinnyWarps; ++w) acc += red[w][row][m];
-        acc += bias ? bias[n] : 0.f;
-        r = resid[static_cast<size_t>(m) * ldc + n] + acc;
+        acc += shift;
+        r = have + acc;
         resid[static_cast<size_t>(m) * ldc + n] = r;
-        fuse.weighted[static_cast<size_t>(m) * N + n] = __float2bfloat16_rn(r * fuse.next_weight[n]);
+        fuse.weighted[static_cast<size_t>(m) * N + n] = __float2bfloat16_rn(r * next_w);
       }
       float sq = r * r;
 #pragma unroll
@@ -153,9 +196,9 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __r
         gate += red[w][f][m];
         up += red[w][f + 8][m];
       }
-      if constexpr (SCALED) {
-        gate *= fuse.row_scale[m];
-        up *= fuse.row_scale[m];
+      if constexpr (SCALED != SCALE_NONE) {
+        gate *= factor_of(m);
+        up *= factor_of(m);
       }
       if (bias) {
         gate += bias[n];
@@ -171,7 +214,7 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __r
       float acc = 0.f;
 #pragma unroll
       for (int w = 0; w < kSkinnyWarps; ++w) acc += red[w][row][m];
-      if constexpr (SCALED) acc *= fuse.row_scale[m];
+      if constexpr (SCALED != SCALE_NONE) acc *= factor_of(m);
       acc += bias ? bias[n] : 0.f;
       C[static_cast<size_t>(m) * ldc + n] = from_float<OutT>(acc);
     }
@@ -202,7 +245,7 @@ __global__ void __launch_bounds__(256) rms_finish_kernel(const float* __restrict
 
 using namespace b200;
 
-template <int NT, int UNROLL, int WARPS, int EPI, bool SCALED, typename OutT>
+template <int NT, int UNROLL, int WARPS, int EPI, int SCALED, typename OutT>
 static void launch_one(const __nv_bfloat16* w, const __nv_bfloat16* x, const float* bias, void* C, int M, int N, int K,
                        int ldc, const NormFusion& fuse, cudaStream_t stream) {
   launch(gemm_skinny_kernel<NT, UNROLL, WARPS, EPI, SCALED, OutT>, dim3((N + 15) / 16), dim3(WARPS * 32), 0, stream, w, x,
@@ -213,26 +256,23 @@ static void launch_one(const __nv_bfloat16* w, const __nv_bfloat16* x, const flo
 template <int NT, int UNROLL, int WARPS>
 static void launch_skinny(const __nv_bfloat16* w, const __nv_bfloat16* x, const float* bias, void* C, int M, int N, int K,
                           int ldc, int out_f32, int epi, const NormFusion& fuse, cudaStream_t stream) {
-  const bool scaled = fuse.row_scale != nullptr;
-  if (epi == EPI_RESIDUAL) {
-    launch_one<NT, UNROLL, WARPS, EPI_RESIDUAL, false, float>(w, x, bias, C, M, N, K, ldc, fuse, stream);
-  } else if (epi == EPI_SWIGLU) {
-    if (scaled) {
-      if (out_f32) launch_one<NT, UNROLL, WARPS, EPI_SWIGLU, true, float>(w, x, bias, C, M, N, K, ldc, fuse, stream);
-      else launch_one<NT, UNROLL, WARPS, EPI_SWIGLU, true, __nv_bfloat16>(w, x, bias, C, M, N, K, ldc, fuse, stream);
+  auto of_type = [&](auto epilogue, auto scaling) {
+    constexpr int E = decltype(epilogue)::value, F = decltype(scaling)::value;
+    if (out_f32) launch_one<NT, UNROLL, WARPS, E, F, float>(w, x, bias, C, M, N, K, ldc, fuse, stream);
+    else launch_one<NT, UNROLL, WARPS, E, F, __nv_bfloat16>(w, x, bias, C, M, N, K, ldc, fuse, stream);
+  };
+  auto scaled = [&](auto epilogue) {
+    if (fuse.sums != nullptr) {
+      if constexpr (NT == 1) of_type(epilogue, std::integral_constant<int, SCALE_SUMS>{});     // (at most eight rows)
+    } else if (fuse.row_scale != nullptr) {
+      of_type(epilogue, std::integral_constant<int, SCALE_FACTORS>{});
     } else {
-      if (out_f32) launch_one<NT, UNROLL, WARPS, EPI_SWIGLU, false, float>(w, x, bias, C, M, N, K, ldc, fuse, stream);
-      else launch_one<NT, UNROLL, WARPS, EPI_SWIGLU, false, __nv_bfloat16>(w, x, bias, C, M, N, K, ldc, fuse, stream);
+      of_type(epilogue, std::integral_constant<int, SCALE_NONE>{});
     }
-  } else {
-    if (scaled) {
-      if (out_f32) launch_one<NT, UNROLL, WARPS, EPI_STORE, true, float>(w, x, bias, C, M, N, K, ldc, fuse, stream);
-      else launch_one<NT, UNROLL, WARPS, EPI_STORE, true, __nv_bfloat16>(w, x, bias, C, M, N, K, ldc, fuse, stream);
-    } else {
-      if (out_f32) launch_one<NT, UNROLL, WARPS, EPI_STORE, false, float>(w, x, bias, C, M, N, K, ldc, fuse, stream);
-      else launch_one<NT, UNROLL, WARPS, EPI_STORE, false, __nv_bfloat16>(w, x, bias, C, M, N, K, ldc, fuse, stream);
-    }
-  }
+  };
+  if (epi == EPI_RESIDUAL) launch_one<NT, UNROLL, WARPS, EPI_RESIDUAL, SCALE_NONE, float>(w, x, bias, C, M, N, K, ldc, fuse, stream);
+  else if (epi == EPI_SWIGLU) scaled(std::integral_constant<int, EPI_SWIGLU>{});
+  else scaled(std::integral_constant<int, EPI_STORE>{});
 }
 
 static int skinny(const void* X, const void* W, const float* bias, void* C, int M, int N, int K, int ldc, int out_f32,
@@ -250,7 +290,7 @@ static int skinny(const void* X, const void* W, const float* bias, void* C, int 
     const int ctas = (N + 15) / 16;
     static DeviceOnce once;
     int sms = 0;
-    if (int e = configure_once(once, gemm_skinny_kernel<1, 8, 8, EPI_STORE, false, float>, 0, &sms)) return e;
+    if (int e = configure_once(once, gemm_skinny_kernel<1, 8, 8, EPI_STORE, SCALE_NONE, float>, 0, &sms)) return e;
     if (ctas > 2 * sms && ctas <= 3 * sms) variant = 2;
   }
   if (M <= 8) {
@@ -279,6 +319,21 @@ extern "C" int b200_gemm_skinny_variant(const void* X, const void* W, const floa
   return skinny(X, W, bias, C, M, N, K, ldc, out_f32, variant, swiglu ? EPI_SWIGLU : EPI_STORE, fuse, stream);
 }
 
+// The same with the factors of the rows of X formed here: `sums` [parts][16], `parts` <= 128, what b200_gemm_skinny_residual leaves in its
+// partials for rows of `width` columns, and the eps of their norm.  M <= 8.
+extern "C" int b200_gemm_skinny_summed(const void* X, const void* W, const float* bias, void* C, int M, int N, int K,
+                                       int ldc, int out_f32, int swiglu, const float* sums, int parts, int width, float eps,
+                                       cudaStream_t stream) {
+  if (swiglu < 0 || swiglu > ACT_GELU_TANH || M > 8 || !sums || parts <= 0 || parts > kMostSums || width <= 0) return B200_ERR_BAD_SIZE;
+  NormFusion fuse{};
+  fuse.act = swiglu;
+  fuse.sums = sums;
+  fuse.parts = parts;
+  fuse.width = static_cast<float>(width);
+  fuse.eps = eps;
+  return skinny(X, W, bias, C, M, N, K, ldc, out_f32, 0, swiglu ? EPI_SWIGLU : EPI_STORE, fuse, stream);
+}
+
 extern "C" int b200_gemm_skinny(const void* X, const void* W, const float* bias, void* C, int M, int N, int K,
                                 int ldc, int out_f32, cudaStream_t stream) {
   return b200_gemm_skinny_variant(X, W, bias, C, M, N, K, ldc, out_f32, 0, 0, nullptr, stream);
@@ -286,18 +341,19 @@ extern "C" int b200_gemm_skinny(const void* X, const void* W, const float* bias,
 
 // resid[M][N] (float32, row stride ldc) += X W^T (+ bias); weighted[M][N] (bfloat16) = resid * next_weight;
 // row_scale_out[16] = rsqrt(mean of squares of each new row of resid + eps) (rows from M on: 0).
-// `partials` is scratch of b200_gemm_skinny_partial_floats(N) floats.  Two launches.
+// `partials` is scratch of b200_gemm_skinny_partial_floats(N) floats.  Two launches; without row_scale_out one, and the partials are the
+// result (b200_gemm_skinny_summed).
 extern "C" int b200_gemm_skinny_residual(const void* X, const void* W, const float* bias, float* resid, int M, int N, int K,
                                          int ldc, const float* next_weight, float eps, void* weighted, float* row_scale_out,
                                          float* partials, cudaStream_t stream) {
-  if (!resid || !next_weight || !weighted || !row_scale_out || !partials) return B200_ERR_BAD_SIZE;
+  if (!resid || !next_weight || !weighted || !partials) return B200_ERR_BAD_SIZE;
   NormFusion fuse{};
   fuse.next_weight = next_weight;
   fuse.eps = eps;
   fuse.weighted = static_cast<__nv_bfloat16*>(weighted);
   fuse.partials = partials;
   if (int e = skinny(X, W, bias, resid, M, N, K, ldc, 1, 0, EPI_RESIDUAL, fuse, stream)) return e;
-  if (M <= 0 || N <= 0) return 0;
+  if (M <= 0 || N <= 0 || !row_scale_out) return 0;
   launch(rms_finish_kernel, dim3(1), dim3(256), 0, stream, static_cast<const float*>(partials), (N + 15) / 16, M,
          static_cast<float>(N), eps, row_scale_out);
   return launch_status();

@@ -34,6 +34,8 @@ native.register_library(
                                      c_void_p, c_void_p],
         "b200_gemm_skinny_residual": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                                       native.c_float, c_void_p, c_void_p, c_void_p, c_void_p],
+        "b200_gemm_skinny_summed": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
+                                    native.c_float, c_void_p],
         "b200_gemm_skinny_partial_floats": [c_int],
     },
 )
@@ -307,10 +309,12 @@ def check_error() -> None:
 
 def linear_skinny(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None,
                   out_dtype: torch.dtype = torch.bfloat16, *, variant: int = 0, swiglu: "bool | str" = False,
-                  row_scale: torch.Tensor | None = None) -> torch.Tensor:
+                  row_scale: torch.Tensor | None = None, sums: torch.Tensor | None = None, eps: float = 0.0) -> torch.Tensor:
     """``x @ weight.T (+ bias)`` for at most 16 rows of ``x``: the weight-streaming kernel.
     ``swiglu``: see ``linear``.  ``row_scale`` (float32 ``[16]``): the rows of ``x`` still lack these factors
-    (an RMS norm left half done, see ``linear_skinny_residual``); they are applied to the product, before the bias."""
+    (an RMS norm left half done, see ``linear_skinny_residual``); they are applied to the product, before the bias.
+    ``sums`` (float32 ``[parts, 16]``, with the norm's ``eps``) instead of it: the shares of the rows' sums of squares that make the factors, for at
+    most eight rows."""
 
     native.require(x, "x", dtype=torch.bfloat16, dims=2)
     native.require(weight, "weight", dtype=torch.bfloat16, dims=2)
@@ -328,16 +332,27 @@ def linear_skinny(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | No
         native.require(row_scale, "row_scale", dtype=torch.float32, shape=(16,))
     width = n // 2 if swiglu else n
     out = torch.empty((m, width), dtype=out_dtype, device=x.device)
+    if sums is not None:
+        native.require(sums, "sums", dtype=torch.float32, dims=2)
+        if sums.shape[1] != 16 or row_scale is not None:
+            raise KernelError("a row's factor comes as itself or as 16 columns of shares")
+        native.call("b200_gemm_skinny_summed", x.data_ptr(), weight.data_ptr(), native.ptr(bias), out.data_ptr(), m, n, k, width,
+                    1 if out_dtype == torch.float32 else 0, gated_unit(swiglu), sums.data_ptr(), sums.shape[0], k, float(eps), native.stream_ptr())
+        return out
     native.call("b200_gemm_skinny_variant", x.data_ptr(), weight.data_ptr(), native.ptr(bias), out.data_ptr(), m, n, k, width,
                 1 if out_dtype == torch.float32 else 0, variant, gated_unit(swiglu), native.ptr(row_scale), native.stream_ptr())
     return out
 
 
+SUMMED_ROWS, SUMMED_WIDTH = 8, 2048      # rows, and their columns, up to which the consuming kernel forms the rows' factors itself
+
+
 def linear_skinny_residual(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, resid: torch.Tensor,
-                           next_weight: torch.Tensor, eps: float) -> tuple[torch.Tensor, torch.Tensor]:
+                           next_weight: torch.Tensor, eps: float, *, finish: bool = True) -> tuple[torch.Tensor, torch.Tensor]:
     """``resid += x @ weight.T (+ bias)`` in place (float32 ``[M, N]``, at most 16 rows), and on the way out
     what the RMS norm after it needs: ``resid * next_weight`` rounded to bfloat16, and every row's factor
-    ``rsqrt(mean of squares + eps)`` (``[16]`` floats; rows from ``M`` on hold 0).  Returns (weighted, row_scale)."""
+    ``rsqrt(mean of squares + eps)`` (``[16]`` floats; rows from ``M`` on hold 0).  Returns (weighted, row_scale), or, not to
+    ``finish``, (weighted, sums): the shares ``[N / 16, 16]`` of the rows' sums of squares, which ``linear_skinny`` takes."""
 
     native.require(x, "x", dtype=torch.bfloat16, dims=2)
     native.require(weight, "weight", dtype=torch.bfloat16, dims=2)
@@ -350,9 +365,9 @@ def linear_skinny_residual(x: torch.Tensor, weight: torch.Tensor, bias: torch.Te
     if bias is not None:
         native.require(bias, "bias", dtype=torch.float32, shape=(n,))
     weighted = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
-    row_scale = torch.empty(16, dtype=torch.float32, device=x.device)
-    partials = torch.empty(native.query("b200_gemm_skinny_partial_floats", n), dtype=torch.float32, device=x.device)
+    row_scale = torch.empty(16, dtype=torch.float32, device=x.device) if finish else None
+    partials = torch.empty((native.query("b200_gemm_skinny_partial_floats", n) // 16, 16), dtype=torch.float32, device=x.device)
     native.call("b200_gemm_skinny_residual", x.data_ptr(), weight.data_ptr(), native.ptr(bias), resid.data_ptr(), m, n, k, n,
-                next_weight.data_ptr(), float(eps), weighted.data_ptr(), row_scale.data_ptr(), partials.data_ptr(),
-                native.stream_ptr(), launches=2)
-    return weighted, row_scale
+                next_weight.data_ptr(), float(eps), weighted.data_ptr(), native.ptr(row_scale), partials.data_ptr(),
+                native.stream_ptr(), launches=2 if finish else 1)
+    return weighted, (row_scale if finish else partials)

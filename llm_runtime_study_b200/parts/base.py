@@ -239,13 +239,16 @@ class WeightedRows:
     its hands, and a batch of a few decoded tokens runs without norm kernels."""
 
     values: torch.Tensor        # [rows, width], activation type
-    scale: torch.Tensor         # [16] float32; the first ``rows`` entries count
+    scale: torch.Tensor | None  # [16] float32; the first ``rows`` entries count
+    sums: torch.Tensor | None = None    # instead of it: [parts, 16] float32, shares of the rows' sums of squares, and the norm's eps
+    eps: float = 0.0
 
     def normalised(self) -> torch.Tensor:
         """The normalised rows themselves, for a consumer that cannot apply the factor (plain tensor operations)."""
 
-        rows = self.values.shape[0]
-        return (self.values.float() * self.scale[:rows, None]).to(self.values.dtype)
+        rows, width = self.values.shape
+        scale = self.scale if self.sums is None else torch.rsqrt(self.sums.sum(dim=0) / width + self.eps)
+        return (self.values.float() * scale[:rows, None]).to(self.values.dtype)
 
 
 @dataclass

@@ -70,7 +70,7 @@ class Projection:
         if not isinstance(x, WeightedRows):
             return x, {}
         if self._streams(x.values.shape[0]) and x.values.is_contiguous():
-            return x.values, {"row_scale": x.scale}
+            return x.values, ({"row_scale": x.scale} if x.sums is None else {"sums": x.sums, "eps": x.eps})
         return x.normalised(), {}
 
     def swiglu(self, x: "torch.Tensor | WeightedRows", act: str = "silu") -> torch.Tensor:
@@ -119,7 +119,9 @@ class Projection:
             fusable = next_norm.fusable() if (next_norm is not None and self.FUSE_NORMS) else None
             if (fusable is not None and add_to is not None and out_dtype == torch.float32 and self._streams(m)
                     and fusable[0].shape[0] == self.out_features):
-                return WeightedRows(*gemm_bf16.linear_skinny_residual(x, self.weight, self.bias, add_to, *fusable))
+                finish = m > gemm_bf16.SUMMED_ROWS or self.out_features > gemm_bf16.SUMMED_WIDTH
+                rows, factors = gemm_bf16.linear_skinny_residual(x, self.weight, self.bias, add_to, *fusable, finish=finish)
+                return WeightedRows(rows, factors) if finish else WeightedRows(rows, None, factors, fusable[1])
             if m <= gemm_bf16.SKINNY_M:
                 if self.GEMM_BACKEND == "tcgen05" and gemm_bf16.few_rows_kernel(m, self.out_features, self.in_features) == "splitk":
                     if add_to is not None and out_dtype == torch.float32 and self.FUSE_RESIDUAL:

@@ -1118,6 +1118,28 @@ def test_embedding_prepares_the_first_norm(dtype, n, hidden, vocab):
     torch.testing.assert_close(scale[:n].cpu().double(), torch.rsqrt((want * want).mean(dim=1) + 1e-5), rtol=1e-5, atol=0)
 
 
+# one share, a last one of eight columns, the most; one row and the most; with and without the gated unit
+@pytest.mark.parametrize("m,n", [(1, 16), (8, 264), (5, 2048), (8, 2048)])
+def test_row_factors_out_of_shares_equal_the_finished_ones(m, n):
+    from llm_runtime_study_b200.errors import KernelError
+
+    torch.manual_seed(6)
+    x, w, resid = torch.randn(m, 96).bfloat16(), (torch.randn(n, 96) * 0.1).bfloat16(), torch.randn(m, n)
+    norm_weight, w2 = dev(1 + 0.05 * torch.randn(n)), dev((torch.randn(48, n) * 0.05).bfloat16())
+    made = [_gemm().linear_skinny_residual(dev(x), dev(w), None, dev(resid), norm_weight, 1e-5, finish=finish) for finish in (True, False)]
+    (rows, factors), (same, sums) = made
+    assert torch.equal(rows, same) and sums.shape == (-(-n // 16), 16)
+    # both are float32 sums of n squares, in another order: some roundings of 6e-8
+    torch.testing.assert_close(torch.rsqrt(sums.sum(dim=0)[:m] / n + 1e-5), factors[:m], rtol=1e-5, atol=0)
+    for swiglu, out in ((False, torch.float32), (True, torch.float32)):
+        want = _gemm().linear_skinny(rows, w2, None, out, swiglu=swiglu, row_scale=factors)
+        got = _gemm().linear_skinny(rows, w2, None, out, swiglu=swiglu, sums=sums, eps=1e-5)
+        torch.testing.assert_close(got, want, rtol=3e-5, atol=1e-5 * float(want.abs().max()))
+    nine = torch.zeros(9, n, dtype=torch.bfloat16, device="cuda")
+    with pytest.raises(KernelError):
+        _gemm().linear_skinny(nine, w2, None, torch.float32, sums=sums, eps=1e-5)
+
+
 def test_weighted_rows_through_projections_equal_the_norm_kernel():
     """The two halves together against the norm kernel followed by the plain product, on one layer's worth of
     shapes: rows prepared by a projection into the residual, finished by the projection after it."""
