@@ -119,9 +119,8 @@ __global__ void __launch_bounds__(128) decode_attention_tma_kernel(const __grid_
   __shared__ int sm_last;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  static_assert(WARPS * DEPTH <= 128, "a thread a barrier");
-  if (threadIdx.x < WARPS * DEPTH) {
-    mbar_init(&bars[threadIdx.x], 1);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < WARPS * DEPTH; ++i) mbar_init(&bars[i], 1);
     fence_barrier_init();
   }
   const int split = blockIdx.x, b = blockIdx.z;

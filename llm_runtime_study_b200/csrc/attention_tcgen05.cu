@@ -121,23 +121,19 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   const int head0 = kvh * p.group + slice * p.gs;
   const int tokens_per_cta = BM / p.gs;
 
-  if (threadIdx.x < 32) {                // a lane a barrier of each kind: one thread would take 30 ns for every one
-    const int s = threadIdx.x;
-    static_assert(KSTAGES <= 32, "a lane a stage");
-    if (s == 0) {
-      mbar_init(q_full, 1);
-      mbar_init(o_done, 1);
-    }
-    if (s < KSTAGES) {
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 1);
+    for (int s = 0; s < KSTAGES; ++s) {
       mbar_init(k_full + s, 1);
       mbar_init(k_empty + s, 1);
       mbar_init(v_full + s, 1);
       mbar_init(v_empty + s, 1);
     }
-    if (s < 2) {
+    for (int s = 0; s < 2; ++s) {
       mbar_init(s_full + s, 1);
       mbar_init(p_full + s, BM);
     }
+    mbar_init(o_done, 1);
     fence_barrier_init();
   }
   if (warp == 5) tmem_alloc(tmem_slot, TMEM_COLS);
@@ -462,24 +458,22 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
     return;
   }
 
-  if (threadIdx.x < 32) {
-    const int s = threadIdx.x;
-    static_assert(KSTAGES_P <= 32 && VSTAGES_P <= 32, "a lane a stage");
-    if (s == 0) mbar_init(q_full, 1);
-    if (s < KSTAGES_P) {
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 1);
+    for (int s = 0; s < KSTAGES_P; ++s) {
       mbar_init(k_full + s, 1);
       mbar_init(k_empty + s, 1);
     }
-    if (s < VSTAGES_P) {
+    for (int s = 0; s < VSTAGES_P; ++s) {
       mbar_init(v_full + s, 1);
       mbar_init(v_empty + s, 1);
     }
-    if (s < 2) {
-      mbar_init(s_full + s, 1);
-      mbar_init(p_full + 2 * s, 4);             // one arrival per softmax warp
-      mbar_init(p_full + 2 * s + 1, 4);
-      mbar_init(o_done + s, 1);
-      mbar_init(o_half + s, 1);
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(s_full + t, 1);
+      mbar_init(p_full + 2 * t, 4);             // one arrival per softmax warp
+      mbar_init(p_full + 2 * t + 1, 4);
+      mbar_init(o_done + t, 1);
+      mbar_init(o_half + t, 1);
     }
     fence_barrier_init();
   }
