@@ -75,6 +75,8 @@ def test_decode_parts_are_bounded_and_use_the_gpu():
         parts = attention_bf16.decode_splits(requests, kv_heads, 1, longest, slots)
         assert 1 <= parts <= 64
         assert parts == 1 or longest // parts >= 64            # a part is never shorter than a few key blocks
+    # parts that do not fit a cluster have to gain more than their meeting in memory costs
+    assert attention_bf16.decode_splits(1, 8, 1, 2001, 296, together=8) == 8 and attention_bf16.decode_splits(1, 8, 1, 32768, 296, together=8) >= 16
     # one long sequence is cut into many parts, a full batch into none
     assert attention_bf16.decode_splits(1, 8, 1, 32768, 296) >= 16
     assert attention_bf16.decode_splits(64, 8, 1, 2048, 592) == 1

@@ -528,6 +528,12 @@ def test_decode_attention_tma_uses_as_many_parts_as_the_batch_needs():
     mma.check_decode_tma_error(d)
 
 
+# as many parts as a cluster holds, one less, one more, and two clusters' worth with a group's heads in two slices
+@pytest.mark.parametrize("nq,nkv,d,page,splits", [(8, 2, 128, 16, 7), (8, 2, 128, 16, 8), (8, 2, 128, 16, 9), (24, 2, 64, 32, 8), (2, 1, 256, 64, 8)])
+def test_decode_attention_tma_in_parts_around_a_cluster(nq, nkv, d, page, splits):
+    test_decode_attention_tma(nq, nkv, d, page, splits)
+
+
 @pytest.mark.parametrize("nq,nkv,d,page", [(8, 2, 128, 16), (32, 8, 128, 16), (5, 1, 64, 16), (24, 2, 64, 32), (3, 3, 192, 16),
                                            (2, 1, 256, 64)])
 @pytest.mark.parametrize("splits,norm,rot", [(1, True, True), (4, True, True), (16, False, True), (3, True, False), (2, False, False)])
