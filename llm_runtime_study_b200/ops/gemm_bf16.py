@@ -166,6 +166,15 @@ def few_rows_kernel(m: int, n: int, k: int) -> str:
     return "splitk" if k >= 16384 and n * k >= SKINNY_LARGE else "skinny"
 
 
+def gated_in_one(n: int, k: int) -> bool:
+    """Whether a gated unit's projection of 17 to 127 rows goes to the split-K kernel, whose epilogue applies the gate, and not to the library and
+    a kernel for the gate behind it: where the weights are about 100 MB and more, and streaming them is all that counts (24,576 x 4,096 with 17, 64
+    and 96 rows 38.0, 39.5, 40.0 us, 38.7, 41.7, 43.2 with the library; a decode step of nine such layers 1,263 -> 1,232 with 24
+    requests, 1,553 -> 1,515 with 64).  Smaller ones are the library's (16,384 x 2,048 with 64 rows 18.6, 15.4; steps with them 1 % longer)."""
+
+    return n * k >= 60_000_000
+
+
 def gated_unit(swiglu: "bool | str") -> int:
     """The kernels' number of a gated unit: 0 for none, else its gate (``True``: SiLU)."""
 

@@ -90,7 +90,7 @@ class Projection:
                 return gemm_bf16.linear_skinny(x, self.weight, self.bias, torch.bfloat16, swiglu=act)
             if self.GEMM_BACKEND == "tcgen05" and m >= self.TCGEN05_MIN_ROWS:
                 return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act)
-            if self.GEMM_BACKEND == "tcgen05" and self.MID_ROWS == "splitk":
+            if self.GEMM_BACKEND == "tcgen05" and (self.MID_ROWS == "splitk" or gemm_bf16.gated_in_one(self.out_features, self.in_features)):
                 return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act, kernel="splitk")
         return F.silu_mul_interleaved(self(x), act)
 

@@ -70,6 +70,10 @@ def test_which_projections_go_by_features():
     assert not takes(405, 6144, 4096, False) and takes(640, 6144, 4096, False) and not takes(1024, 6144, 4096, False)
 
 
+def test_gated_projections_of_some_rows_in_one_launch_where_the_weights_are_large():
+    assert gemm_bf16.gated_in_one(24576, 4096) and gemm_bf16.gated_in_one(34816, 5120) and not gemm_bf16.gated_in_one(16384, 2048)
+
+
 def test_decode_parts_are_bounded_and_use_the_gpu():
     for requests, kv_heads, longest, slots in itertools.product((1, 3, 8, 64, 500), (1, 8), (1, 100, 2048, 32768, 1 << 20), (296, 592)):
         parts = attention_bf16.decode_splits(requests, kv_heads, 1, longest, slots)
