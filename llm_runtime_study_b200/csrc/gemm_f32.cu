@@ -24,25 +24,35 @@ inline int block_length(int K) {
 // ------------------------------------------------------------------------------------------ tiles
 // A cluster per BM x BN tile, one CTA for each block of K, (BM / TM) x (BN / TN) threads with TM x TN outputs each (rows
 // ty * 4 + g BM / (TM / 4), columns likewise: every fragment is one 16-byte read that neighbouring threads share or lay
-// side by side).  Two buffers of BK columns in shared memory and two more in registers: rows are asked for two steps ahead (with one, a step of
-// 0.8 us was the latency of its loads).  The
-// sums of finished segments wait in shared memory, one private 16-byte column per thread, so that registers hold one
+// side by side).  Two buffers of BK columns in shared memory and AHEAD more in registers.  AHEAD is two for tiles of 64 x 64, of which
+// an SM often holds only one or two CTAs (one step ahead: 509 x 1024 x 3072 80 us against 78), and one for tiles of 128 x 64, whose
+// registers are better spent on a third CTA an SM (509 x 6144 x 1024: 147 us with two steps and 170 registers, 140 with one and 168).
+// A wide read of shared memory takes two passes instead of four if lanes i and i ^ 1, or i and i ^ 2, read the same address: the
+// lowest bit of a lane is tx's, the next one ty's.  Transposed stores of four columns fall on four times the same bank; rows are
+// therefore kept at row ^ 2 k for the four-column group that starts at k.  The two took 509 x 1024 x 3072 from 89.6 to 77.7 us, 509 x 1024
+// x 2048 from 63.2 to 54.8, 509 x 4096 x 1024 from 108 to 97.
+// The sums of finished segments wait in shared memory, one private 16-byte column per thread, so that registers hold one
 // accumulator an output and two or three CTAs fit an SM; at the end the CTAs of a cluster share out the outputs and add the
-// blocks' sums up through distributed shared memory.  Bound by the FMA pipe and the reads of shared memory beside it:
-// 509 x 6144 x 1024 161 us (40 TFLOP/s of the 74 that the pipe could do; 292 us with one 64 x 64 tile kernel and 4-byte
-// accesses), 509 x 1024 x 3072 89 us (189).
+// blocks' sums up through distributed shared memory.  Bound by the FMA pipe, the reads of shared memory beside it and the last
+// wave: 509 x 6144 x 1024 140 us (46 TFLOP/s of the 74 that the pipe could do; 53 in the SMs that get three tiles of the 2.6 on
+// average).
 // VEC: rows of A and W start on 16-byte boundaries and K is a multiple of 4; otherwise elements are loaded one by one.
 constexpr int kBK = 16;
+constexpr size_t kMostSmem = 227 * 1024;
+// A cluster's CTAs lie in one GPC, whose last SMs may not hold another cluster.
+inline int usable_sms(int blocks) { return 148 - 4 * (blocks - 1); }
 constexpr size_t tile_smem(int bm, int bn) { return sizeof(float) * (static_cast<size_t>(bm) * bn + 2 * kBK * (bm + 4 + bn + 4)); }
 
 template <int BM, int BN, int TM, int TN, bool VEC>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), BM == 128 ? 3 : 4)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                      float* __restrict__ C, int M, int N, int K, int lda, int ldc, int block) {
   constexpr int THREADS = (BM / TM) * (BN / TN), BK = kBK, PA = BM + 4, PW = BN + 4;
   constexpr int RPP = THREADS / 4;                                  // rows a pass of 16-byte loads covers
   constexpr int LA = BM / RPP, LW = BN / RPP;
   constexpr int SM_ = BM / (TM / 4), SN_ = BN / (TN / 4);           // distance of a thread's groups of four rows, columns
+  constexpr int TX = BN / TN, AHEAD = BM == 128 ? 1 : 2;
+  static_assert((TX == 8 || TX == 16) && THREADS == 128 && SM_ % 32 == 0 && SN_ % 32 == 0, "lanes of a warp");
   static_assert(TM % 4 == 0 && TN % 4 == 0 && kSegment % BK == 0 && BM % RPP == 0 && BN % RPP == 0, "tile shape");
   extern __shared__ __align__(16) float smem[];
   float* As = smem;                                                 // [2][BK][PA]
@@ -55,7 +65,9 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x / blocks * BN;
   const int k_begin = rank * block, k_end = min(K, k_begin + block);
-  const int tx = tid % (BN / TN), ty = tid / (BN / TN);
+  // lane bits 0 .. 4: tx, ty, tx, tx, ty with eight columns of threads; tx, ty, tx, tx, tx with sixteen
+  const int tx = TX == 8 ? (tid & 1) | (tid >> 1 & 6) : (tid & 1) | (tid >> 1 & 2) | (tid >> 1 & 12);
+  const int ty = TX == 8 ? (tid >> 1 & 1) | (tid >> 3 & 2) | (tid >> 5) * 4 : (tid >> 1 & 1) | (tid >> 5) * 2;
   const int lrow = tid >> 2, lk = (tid & 3) * 4;
   struct Rows { float4 a[LA], w[LW]; };
 
@@ -72,8 +84,8 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
     for (int i = 0; i < LW; ++i) r.w[i] = load4(W, n0 + lrow + RPP * i, N, K, k0 + lk);
   };
   auto stash = [&](const Rows& r, int buf) {
-    float* as = As + (buf * BK + lk) * PA + lrow;
-    float* ws = Ws + (buf * BK + lk) * PW + lrow;
+    float* as = As + (buf * BK + lk) * PA + (lrow ^ 2 * lk);
+    float* ws = Ws + (buf * BK + lk) * PW + (lrow ^ 2 * lk);
 #pragma unroll
     for (int i = 0; i < LA; ++i) {
       as[RPP * i] = r.a[i].x; as[PA + RPP * i] = r.a[i].y; as[2 * PA + RPP * i] = r.a[i].z; as[3 * PA + RPP * i] = r.a[i].w;
@@ -94,24 +106,24 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
       for (int j = 0; j < TN / 2; ++j) acc[i][j] = make_float2(0.f, 0.f);
   };
   clear();
-  // `spent` goes on its way to hold the rows behind the next ones; `next` was asked for a step ago
+  // `spent` goes on its way to hold the rows AHEAD steps on; with two, `next` was asked for a step ago
   auto step = [&](int k0, int buf, Rows& spent, const Rows& next) {
     const bool more = k0 + BK < k_end;
-    fetch(spent, k0 + 2 * BK);
-    const float* as = As + buf * BK * PA + ty * 4;
-    const float* ws = Ws + buf * BK * PW + tx * 4;
+    fetch(spent, k0 + AHEAD * BK);
+    const float* as = As + buf * BK * PA;
+    const float* ws = Ws + buf * BK * PW;
 #pragma unroll
     for (int k = 0; k < BK; ++k) {
       float a[TM];
       float2 w[TN / 2];
 #pragma unroll
       for (int i = 0; i < TM; i += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(as + k * PA + i / 4 * SM_);
+        const float4 v = *reinterpret_cast<const float4*>(as + (ty * 4 ^ k / 4 * 8) + k * PA + i / 4 * SM_);
         a[i] = v.x; a[i + 1] = v.y; a[i + 2] = v.z; a[i + 3] = v.w;
       }
 #pragma unroll
       for (int j = 0; j < TN; j += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(ws + k * PW + j / 4 * SN_);
+        const float4 v = *reinterpret_cast<const float4*>(ws + (tx * 4 ^ k / 4 * 8) + k * PW + j / 4 * SN_);
         w[j / 2] = make_float2(v.x, v.y);
         w[j / 2 + 1] = make_float2(v.z, v.w);
       }
@@ -132,17 +144,17 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
         }
       clear();
     }
-    if (more) stash(next, buf ^ 1);
+    if (more) stash(AHEAD == 2 ? next : spent, buf ^ 1);
     __syncthreads();
   };
   Rows even, odd;
   fetch(even, k_begin);
-  fetch(odd, k_begin + BK);
+  if (AHEAD == 2) fetch(odd, k_begin + BK);
   stash(even, 0);
   __syncthreads();
   for (int k0 = k_begin; k0 < k_end; k0 += 2 * BK) {
     step(k0, 0, even, odd);
-    if (k0 + BK < k_end) step(k0 + BK, 1, odd, even);
+    if (k0 + BK < k_end) step(k0 + BK, 1, AHEAD == 2 ? odd : even, even);
   }
   if (blocks > 1) cluster.sync();                                   // every block's sums are in its CTA's shared memory
   const bool wide = VEC && ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
@@ -293,13 +305,17 @@ gemm_f32_short_kernel(const float* __restrict__ A, const float* __restrict__ W, 
 template <int BM, int BN, int TM, int TN, bool VEC>
 int launch_tiles(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, cudaStream_t stream) {
   static DeviceOnce once;
-  const int status = configure_once(once, gemm_f32_tile_kernel<BM, BN, TM, TN, VEC>, tile_smem(BM, BN));
+  const int status = configure_once(once, gemm_f32_tile_kernel<BM, BN, TM, TN, VEC>, kMostSmem);
   if (status) return status;
   const int block = block_length(K), blocks = (K + block - 1) / block;
+  // Launched while the kernel before still holds some SMs, the CTAs would crowd on the others, three where two suffice (509 x 4096 x
+  // 1024 in a prompt's layers: 144 us against 97 with two an SM): each takes the shared memory that leaves room for no more than an even share.
+  const long long share = (static_cast<long long>((N + BN - 1) / BN) * blocks * ((M + BM - 1) / BM) + usable_sms(blocks) - 1) / usable_sms(blocks);
+  const size_t even = share <= (BM == 128 ? 2 : 3) ? (kMostSmem + 1024) / share - 1024 : 0;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3((N + BN - 1) / BN * blocks, (M + BM - 1) / BM);
   config.blockDim = dim3((BM / TM) * (BN / TN));
-  config.dynamicSmemBytes = tile_smem(BM, BN);
+  config.dynamicSmemBytes = even > tile_smem(BM, BN) ? even / 128 * 128 : tile_smem(BM, BN);
   config.stream = stream;
   cudaLaunchAttribute attributes[2];
   attributes[0].id = cudaLaunchAttributeClusterDimension;
@@ -341,8 +357,11 @@ extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float
     // Up to 8 rows the weights cross once and that is the time (1 x 1024 x 3072: 7.9 us against 37.6 with tiles; 8 x 151,936 x
     // 1024: 285 against 495).  Every further eight rows read them again, from the L2 while the product is small: 24 x 6144
     // x 1024 37.5 against 39.0, 24 x 1024 x 3072 25.6 against 37.8, 64 x 6144 x 1024 83 against 40.
-    // Tiles of 128 rows do a third more arithmetic per byte of shared memory read; where they would be fewer than about
-    // 1.7 an SM, tiles of 64 fill the SMs better (509 x 4096 x 1024: 109 us against 116; 509 x 1024 x 3072: 109 against 89).
+    // Tiles of 128 rows do a third more arithmetic per byte of shared memory read, tiles of 64 leave less of the last wave empty.  A
+    // product takes 9 us and 22.9 for each 64 x 64 x 1024 that the busiest SM gets, or 11 and 43.2 for each 128 x 64 x 1024 (509 x
+    // 6144 x 1024: 140 us with 128 rows, 146 with 64; 700 x 4096 x 1024: 140, 123; 130 x 6144 x 1024: 96, 54; 2048 x 4096 x 1024:
+    // 313, 329).  One CTA of 128 rows an SM has nobody to work under its loads (509 x 1024 x 2048, the weights in HBM: 68 us, 57 with
+    // 64 rows).  Clusters cannot use every SM to the last slot (700 x 1024 x 3072, 96 clusters of three: 140, 100).
     // Few rows: up to about seven CTAs an SM at once (ten up to four rows), 8 us a round of them from K of 128 on (K beyond 512: as the weights
     // stream), where tiles take 3 us and 0.034 a column.  So beyond one round a short K goes to tiles (9 x 6400 x 256: 15.6 us against
     // 12.2, 24 x 9400 x 1024: 48 against 38), and so does K up to 160 beyond four rows (8 x 6400 x 64: 6.1 against 5.6, 20 x 2880 x 64: 9.0 against 5.4)
@@ -354,7 +373,12 @@ extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float
                      (K > 160 && (M <= 8 || (M <= 24 && small < 148)) && few_us <= tiles_us);
     if (vec && few) kernel = 1;
     else if (K <= (vec ? 32 : 112) && small <= 512) kernel = 4;
-    else kernel = large >= 250 && M > 64 ? 3 : 2;
+    else {
+      const int block = block_length(K), sms = usable_sms(blocks);
+      const float depth = (K < block ? K : block) / 1024.f;
+      const float small_us = 9.f + 22.9f * depth * ((small + sms - 1) / sms), large_us = 11.f + 43.2f * depth * ((large + sms - 1) / sms);
+      kernel = large > sms && large_us < small_us ? 3 : 2;
+    }
   }
   if ((M + 63) / 64 > 65535) return B200_ERR_TOO_LARGE;
   if (kernel == 1) {
