@@ -142,15 +142,23 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_poo
   }
 }
 
-// Prompt portions in float32: a CTA holds 32 rows (32 / group consecutive tokens of one request times the query heads
-// that share a key head) and walks the keys in the tiles of 32 that the kernel above takes them in; keys and values pass
+// Prompt portions in float32: 128 threads hold 32 rows (32 / group consecutive tokens of one request times the query heads
+// that share a key head) and walk the keys in the tiles of 32 that the kernel above takes them in; keys and values pass
 // through shared memory once for all rows, the next tile's on their way while this one is worked on.  A thread owns four
 // rows and, of a tile, the keys c and c + 16: the sum of its two weights and four shuffles are then the sum that 32 lanes
 // form by xor shuffles, and every other sum is one chain, so the results are the same bits.  A weight of zero reads no
 // value here either (a later token's value may be anything): only a warp that has one takes the loop that asks.
-// One warp per token and head reads every key for every row from the L2: 509 tokens, 16 heads of 128 over 8: 574 us; so: 133
-// (64 rows a CTA 161: fewer CTAs, one an SM).  Bound by the reads of shared memory beside the FMA pipe.
-constexpr int kTileRows = 32, kTileKeys = 32, kTileThreads = kTileRows * 4, kPPitch = kTileKeys + 4;
+// One warp per token and head reads every key for every row from the L2: 509 tokens, 16 heads of 128 over 8: 574 us; so: 77
+// (64 rows of keys and values at once 161; two rows a thread and twice the threads 87, 2,000 tokens in a window of 300 244 against 198).
+// A tile of keys takes 32 rows about 5 us, mostly latency: of the softmax (its steps are taken for all rows at once: 10 us less of 88)
+// and of reads of shared memory (lanes i and i ^ 1 read the same key: half the passes, 4 % at 1,021 keys).  So the time is that of the
+// SM with most tiles of keys.  More row tiles than SMs go in pairs, a CTA with two sets of threads that share nothing: the tile with most
+// keys beside that with fewest, the next beside the next; the CTAs take the shared memory that leaves room for no more than an even
+// share an SM.  Within a prompt's layers, where CTAs start while the kernel before still holds some SMs: 133 us one by one, 90 in pairs, 78 with
+// the softmax's steps taken together.
+constexpr int kTileRows = 32, kTileKeys = 32, kRowsOf = 4, kTileThreads = kTileRows / kRowsOf * 16, kPPitch = kTileKeys + 4;
+constexpr int kSms = 148;
+constexpr size_t kMostTileSmem = 227 * 1024;
 constexpr size_t attention_tile_smem(int dmax) {
   return sizeof(float) * (static_cast<size_t>(kTileRows + 2 * kTileKeys) * (dmax + 4) + kTileRows * kPPitch);
 }
@@ -158,23 +166,27 @@ constexpr size_t attention_tile_smem(int dmax) {
 struct TileParams {
   const float* q; const float* k_pool; const float* v_pool; float* out;
   const int* positions; const int* q_start; const int* block_table;
-  int entries, table_stride, page_size, nq, nkv, d, dv, per_tile, window, chunk, sink;
+  int entries, table_stride, page_size, nq, nkv, d, dv, per_tile, tiles, window, chunk, sink;
   float scale, softcap;
   const float* slopes; const float* log_r1; const float* log_r2; const float* sinks;
 };
 
 template <int DMAX>
-__global__ void __launch_bounds__(kTileThreads) paged_attention_tile_kernel(const TileParams p) {
+__global__ void __launch_bounds__(2 * kTileThreads) paged_attention_tile_kernel(const TileParams p) {
   constexpr int PITCH = DMAX + 4, CG = DMAX > 64 ? 2 : 1;   // CG: groups of four value columns a thread owns
+  constexpr size_t SET = attention_tile_smem(DMAX) / sizeof(float);
   extern __shared__ __align__(16) float smem[];
-  float* qs = smem;                                     // [32][PITCH]
+  float* qs = smem + threadIdx.x / kTileThreads * SET;   // [32][PITCH]
   float* ks = qs + kTileRows * PITCH;                   // [32][PITCH]
   float* vs = ks + kTileKeys * PITCH;                   // [32][PITCH]
   float* ps = vs + kTileKeys * PITCH;                   // [32][kPPitch]
   pdl_trigger();
   pdl_wait();
-  // the tile's request: every request has its own tiles, the last one (with most keys) first
-  int entry = 0, tile = blockIdx.x, first = 0, tokens = 0;
+  // the tile's request: every request has its own tiles, the last one (with most keys) first, for all key heads
+  const int half = threadIdx.x / kTileThreads, order = half ? p.tiles - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
+  if (half && 2 * static_cast<int>(blockIdx.x) + 1 == p.tiles) return;   // of an odd number the one in the middle has no partner
+  auto meet = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + half), "n"(kTileThreads) : "memory"); };
+  int entry = 0, tile = order / p.nkv, first = 0, tokens = 0;
   for (;; ++entry) {
     if (entry == p.entries) return;
     first = p.q_start[entry];
@@ -188,8 +200,8 @@ __global__ void __launch_bounds__(kTileThreads) paged_attention_tile_kernel(cons
   }
   first += tile * p.per_tile;
   tokens = min(p.per_tile, tokens - tile * p.per_tile);
-  const int tid = threadIdx.x, c = tid % 16, rg = tid / 16;
-  const int group = p.nq / p.nkv, kvh = blockIdx.y;
+  const int tid = threadIdx.x % kTileThreads, c = tid % 32 / 2, rg = tid / 32 * 2 + tid % 2;
+  const int group = p.nq / p.nkv, kvh = order % p.nkv;
   const int* table = p.block_table + static_cast<size_t>(entry) * p.table_stride;
   const int d = p.d, dv = p.dv, quads = d / 4, vquads = dv / 4;
 
@@ -200,13 +212,13 @@ __global__ void __launch_bounds__(kTileThreads) paged_attention_tile_kernel(cons
     *reinterpret_cast<float4*>(qs + row * PITCH + i) = v;
   }
   const float inv_cap = p.softcap > 0.f ? 1.f / p.softcap : 0.f;
-  float slope[4], r1[4], r2[4];
-  int pos[4], w0[4];
-  float m[4], l[4];
-  float2 acc[4][2 * CG];
+  float slope[kRowsOf], r1[kRowsOf], r2[kRowsOf];
+  int pos[kRowsOf], w0[kRowsOf];
+  float m[kRowsOf], l[kRowsOf];
+  float2 acc[kRowsOf][2 * CG];
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int row = rg * 4 + r, t = row / group, head = kvh * group + row % group;
+  for (int r = 0; r < kRowsOf; ++r) {
+    const int row = rg * kRowsOf + r, t = row / group, head = kvh * group + row % group;
     pos[r] = t < tokens ? p.positions[first + t] : -1;   // -1: no such row; it sees no key
     w0[r] = p.window > 0 ? max(0, pos[r] - p.window + 1) : 0;
     if (p.chunk > 0) w0[r] = max(w0[r], pos[r] / p.chunk * p.chunk);
@@ -241,25 +253,25 @@ __global__ void __launch_bounds__(kTileThreads) paged_attention_tile_kernel(cons
   ask(p.v_pool, vs, page, t0 + crow, dv, vquads);
   for (; t0 <= p_last; t0 += kTileKeys) {
     asm volatile("cp.async.wait_group 1;\n" ::: "memory");            // the keys; the values may still be on their way
-    __syncthreads();
+    meet();
     const int ahead_page = page_of(t0 + 2 * kTileKeys + crow);
     int key_page[2];
 #pragma unroll
     for (int n = 0; n < 2; ++n) key_page[n] = page_of(t0 + c + 16 * n);
-    float s[4][2];
+    float s[kRowsOf][2];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) s[r][0] = s[r][1] = 0.f;
-    const float* qrow = qs + rg * 4 * PITCH;
+    for (int r = 0; r < kRowsOf; ++r) s[r][0] = s[r][1] = 0.f;
+    const float* qrow = qs + rg * kRowsOf * PITCH;
     const float* krow = ks + c * PITCH;
 #pragma unroll 4
     for (int i = 0; i < d; i += 4) {
-      float4 qv[4], kv[2];
+      float4 qv[kRowsOf], kv[2];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) qv[r] = *reinterpret_cast<const float4*>(qrow + r * PITCH + i);
+      for (int r = 0; r < kRowsOf; ++r) qv[r] = *reinterpret_cast<const float4*>(qrow + r * PITCH + i);
 #pragma unroll
       for (int n = 0; n < 2; ++n) kv[n] = *reinterpret_cast<const float4*>(krow + n * 16 * PITCH + i);
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
+      for (int r = 0; r < kRowsOf; ++r)
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
           s[r][n] = fmaf(qv[r].x, kv[n].x, s[r][n]);
@@ -268,46 +280,55 @@ __global__ void __launch_bounds__(kTileThreads) paged_attention_tile_kernel(cons
           s[r][n] = fmaf(qv[r].w, kv[n].w, s[r][n]);
         }
     }
-    bool full = true;                                                 // no weight of this thread's is zero
+    // every step for all rows before the next one: their shuffles and exponentials then run side by side
+    bool valid[kRowsOf][2];
+    float top[kRowsOf], sum[kRowsOf], corr[kRowsOf];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 0; r < kRowsOf; ++r) {
       const ScoreRules rules{p.scale, p.softcap, inv_cap, slope[r], r1[r], r2[r], p.log_r1 != nullptr};
-      bool valid[2];
-      float top = -INFINITY;
+      top[r] = -INFINITY;
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
         const int t = t0 + c + 16 * n;
-        valid[n] = key_page[n] >= 0 && t <= pos[r] && t >= w0[r];
-        s[r][n] = valid[n] ? rules(s[r][n], pos[r] - t) : -INFINITY;
-        top = fmaxf(top, s[r][n]);
-      }
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-      float w[2] = {0.f, 0.f}, corr = 1.f;
-      const bool any = top != -INFINITY;
-      const float m_new = any ? fmaxf(m[r], top) : m[r];
-      if (any) {
-        corr = expf(m[r] - m_new);
-#pragma unroll
-        for (int n = 0; n < 2; ++n) w[n] = valid[n] ? expf(s[r][n] - m_new) : 0.f;
-      }
-      float sum = __fadd_rn(w[0], w[1]);
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (any) {
-        l[r] = __fmaf_rn(l[r], corr, sum);
-        m[r] = m_new;
-#pragma unroll
-        for (int j = 0; j < 2 * CG; ++j) { acc[r][j].x *= corr; acc[r][j].y *= corr; }
-      }
-#pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        ps[(rg * 4 + r) * kPPitch + c + 16 * n] = w[n];
-        full = full && w[n] != 0.f;
+        valid[r][n] = key_page[n] >= 0 && t <= pos[r] && t >= w0[r];
+        s[r][n] = valid[r][n] ? rules(s[r][n], pos[r] - t) : -INFINITY;
+        top[r] = fmaxf(top[r], s[r][n]);
       }
     }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+      for (int r = 0; r < kRowsOf; ++r) top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 2 * o));
+    bool full = true;                                                 // no weight of this thread's is zero
+#pragma unroll
+    for (int r = 0; r < kRowsOf; ++r) {
+      const bool any = top[r] != -INFINITY;                           // otherwise the row keeps what it has: a factor of one, weights of zero
+      const float m_new = any ? fmaxf(m[r], top[r]) : 0.f;
+      const float scaled = expf(m[r] - m_new);
+      corr[r] = any ? scaled : 1.f;
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const float w = expf(s[r][n] - m_new);
+        s[r][n] = any && valid[r][n] ? w : 0.f;
+        full = full && s[r][n] != 0.f;
+      }
+      sum[r] = __fadd_rn(s[r][0], s[r][1]);
+      m[r] = any ? m_new : m[r];
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+      for (int r = 0; r < kRowsOf; ++r) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2 * o);
+#pragma unroll
+    for (int r = 0; r < kRowsOf; ++r) {
+      l[r] = __fmaf_rn(l[r], corr[r], sum[r]);
+#pragma unroll
+      for (int j = 0; j < 2 * CG; ++j) { acc[r][j].x *= corr[r]; acc[r][j].y *= corr[r]; }
+#pragma unroll
+      for (int n = 0; n < 2; ++n) ps[(rg * kRowsOf + r) * kPPitch + c + 16 * n] = s[r][n];
+    }
     full = __all_sync(0xffffffffu, full);                             // then all 32 keys exist, for all rows of the warp
-    __syncthreads();                                                  // the keys have been read, all weights are written
+    meet();                                                  // the keys have been read, all weights are written
     const bool more = t0 + kTileKeys <= p_last;
     if (more) {
       ask(p.k_pool, ks, next_page, t0 + kTileKeys + crow, d, quads);
@@ -315,19 +336,19 @@ __global__ void __launch_bounds__(kTileThreads) paged_attention_tile_kernel(cons
     } else {
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
-    __syncthreads();
+    meet();
     auto add_values = [&](auto ask_first, int count) {
       for (int j = 0; j < count; j += 4) {
-        float4 pw[4];
+        float4 pw[kRowsOf];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) pw[r] = *reinterpret_cast<const float4*>(ps + (rg * 4 + r) * kPPitch + j);
+        for (int r = 0; r < kRowsOf; ++r) pw[r] = *reinterpret_cast<const float4*>(ps + (rg * kRowsOf + r) * kPPitch + j);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           float4 vv[CG];
 #pragma unroll
           for (int g = 0; g < CG; ++g) vv[g] = *reinterpret_cast<const float4*>(vs + (j + e) * PITCH + (g * 64 + c * 4) % DMAX);
 #pragma unroll
-          for (int r = 0; r < 4; ++r) {
+          for (int r = 0; r < kRowsOf; ++r) {
             const float w = e == 0 ? pw[r].x : e == 1 ? pw[r].y : e == 2 ? pw[r].z : pw[r].w;
             if (decltype(ask_first)::value && w == 0.f) continue;
 #pragma unroll
@@ -341,13 +362,13 @@ __global__ void __launch_bounds__(kTileThreads) paged_attention_tile_kernel(cons
     };
     if (full) add_values(std::false_type(), kTileKeys);
     else add_values(std::true_type(), min(kTileKeys, p_last - t0 + 1));
-    __syncthreads();                                                  // the values and the weights have been read
+    meet();                                                  // the values and the weights have been read
     if (more) ask(p.v_pool, vs, next_page, t0 + kTileKeys + crow, dv, vquads);
     next_page = ahead_page;
   }
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int row = rg * 4 + r, t = row / group;
+  for (int r = 0; r < kRowsOf; ++r) {
+    const int row = rg * kRowsOf + r, t = row / group;
     if (t >= tokens) continue;
     const float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
     float* orow = p.out + (static_cast<size_t>(first + t) * p.nq + kvh * group + row % group) * dv;
@@ -361,13 +382,17 @@ __global__ void __launch_bounds__(kTileThreads) paged_attention_tile_kernel(cons
 }
 
 template <int DMAX>
-int launch_attention_tiles(const TileParams& p, int n, cudaStream_t stream) {
+int launch_attention_tiles(const TileParams& p, cudaStream_t stream) {
   static DeviceOnce once;
-  const int status = configure_once(once, paged_attention_tile_kernel<DMAX>, attention_tile_smem(DMAX));
+  const int status = configure_once(once, paged_attention_tile_kernel<DMAX>, kMostTileSmem);
   if (status) return status;
-  const dim3 grid(n / p.per_tile + p.entries, p.nkv);                  // at least as many as there are tiles; the others return
-  if (grid.y > 65535) return B200_ERR_TOO_LARGE;
-  launch(paged_attention_tile_kernel<DMAX>, grid, dim3(kTileThreads), attention_tile_smem(DMAX), stream, p);
+  if (p.tiles <= kSms) {                                               // an SM for each: no pairs
+    launch(paged_attention_tile_kernel<DMAX>, dim3(p.tiles), dim3(kTileThreads), attention_tile_smem(DMAX), stream, p);
+    return launch_status();
+  }
+  const long long ctas = (p.tiles + 1LL) / 2, share = (ctas + kSms - 1) / kSms;
+  const size_t even = share <= 4 ? ((kMostTileSmem + 1024) / share - 1024) / 128 * 128 : 0, needed = 2 * attention_tile_smem(DMAX);
+  launch(paged_attention_tile_kernel<DMAX>, dim3(static_cast<unsigned>(ctas)), dim3(2 * kTileThreads), even > needed ? even : needed, stream, p);
   return launch_status();
 }
 
@@ -454,10 +479,13 @@ extern "C" int b200_paged_attention_tiles(
       (log_r1 == nullptr) != (log_r2 == nullptr))
     return B200_ERR_BAD_SIZE;
   if (d > 128 || dv > 128 || nq / nkv > kTileRows) return B200_ERR_TOO_LARGE;
+  const int per_tile = kTileRows / (nq / nkv);
+  const long long tiles = (static_cast<long long>(n) / per_tile + entries) * nkv;      // at least as many as there are; the others return
+  if (tiles > 0x7fffffff) return B200_ERR_TOO_LARGE;
   const TileParams p{q, k_pool, v_pool, out, positions, q_start, block_table, entries, table_stride, page_size, nq, nkv, d, dv,
-                     kTileRows / (nq / nkv), window, chunk, sink, scale, softcap, slopes, log_r1, log_r2, sinks};
+                     per_tile, static_cast<int>(tiles), window, chunk, sink, scale, softcap, slopes, log_r1, log_r2, sinks};
   const int widest = d > dv ? d : dv;
-  if (widest <= 32) return launch_attention_tiles<32>(p, n, stream);
-  if (widest <= 64) return launch_attention_tiles<64>(p, n, stream);
-  return launch_attention_tiles<128>(p, n, stream);
+  if (widest <= 32) return launch_attention_tiles<32>(p, stream);
+  if (widest <= 64) return launch_attention_tiles<64>(p, stream);
+  return launch_attention_tiles<128>(p, stream);
 }

@@ -332,6 +332,20 @@ def test_attention_tiles_give_the_bits_of_single_tokens(nq, nkv, d, dv, page, ru
     assert torch.equal(alone, tiled)
 
 
+# tiles (32 rows of each of nkv heads, and one more a head) go in pairs from 149 on, the first with the last: an odd number of them, the
+# fewest, and the most that go alone
+@pytest.mark.parametrize("nkv,tokens", [(15, 330), (149, 31), (37, 127)])
+def test_attention_tiles_in_pairs_give_the_bits_of_single_tokens(nkv, tokens):
+    d, page, past = 16, 8, 5
+    g = torch.Generator().manual_seed(nkv)
+    pages = -(-(past + tokens) // page)
+    q, k_pool, v_pool = dev(torch.randn(tokens, nkv, d, generator=g)), *(dev(torch.randn(pages, nkv, page, d, generator=g)) for _ in range(2))
+    positions, q_start = torch.arange(past, past + tokens, dtype=torch.int32), torch.tensor([0, tokens], dtype=torch.int32)
+    args = dict(positions=dev(positions), token_entry=dev(torch.zeros(tokens, dtype=torch.int32)), scale=d ** -0.5,
+                block_table=dev(torch.arange(pages, dtype=torch.int32).flip(0).view(1, -1).contiguous()))
+    assert torch.equal(F().paged_attention_simt(q, k_pool, v_pool, **args), F().paged_attention_simt(q, k_pool, v_pool, q_start=dev(q_start), **args))
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("window", [1, 7, 32, 33])
 def test_paged_attention_simt_window(dtype, window):
