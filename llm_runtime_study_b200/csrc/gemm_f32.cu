@@ -36,6 +36,9 @@ inline int block_length(int K) {
 // blocks' sums up through distributed shared memory.  Bound by the FMA pipe, the reads of shared memory beside it and the last
 // wave: 509 x 6144 x 1024 140 us (46 TFLOP/s of the 74 that the pipe could do; 53 in the SMs that get three tiles of the 2.6 on
 // average).
+// GATED: the columns are two factors in blocks of eight and act(g) * u leaves instead; a kernel less per feed-forward part (a step of few rows
+// through a small model is bound by its launches) and its pass over memory: 509 x 6144 x 1024 146 and 4.3 us in two kernels, 148 in
+// one (154 while only the half of the threads that own gate columns worked).
 // VEC: rows of A and W start on 16-byte boundaries and K is a multiple of 4; otherwise elements are loaded one by one.
 constexpr int kBK = 16;
 constexpr size_t kMostSmem = 227 * 1024;
@@ -43,10 +46,10 @@ constexpr size_t kMostSmem = 227 * 1024;
 inline int usable_sms(int blocks) { return 148 - 4 * (blocks - 1); }
 constexpr size_t tile_smem(int bm, int bn) { return sizeof(float) * (static_cast<size_t>(bm) * bn + 2 * kBK * (bm + 4 + bn + 4)); }
 
-template <int BM, int BN, int TM, int TN, bool VEC>
+template <int BM, int BN, int TM, int TN, bool VEC, bool GATED>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), BM == 128 ? 3 : 4)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                     float* __restrict__ C, int M, int N, int K, int lda, int ldc, int block) {
+                     float* __restrict__ C, int M, int N, int K, int lda, int ldc, int block, int act) {
   constexpr int THREADS = (BM / TM) * (BN / TN), BK = kBK, PA = BM + 4, PW = BN + 4;
   constexpr int RPP = THREADS / 4;                                  // rows a pass of 16-byte loads covers
   constexpr int LA = BM / RPP, LW = BN / RPP;
@@ -158,14 +161,37 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
   }
   if (blocks > 1) cluster.sync();                                   // every block's sums are in its CTA's shared memory
   const bool wide = VEC && ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
-  for (int q = rank; q < TM * TN / 4; q += blocks) {
-    const int i = q / (TN / 4), j = q % (TN / 4);
-    const int m = m0 + ty * 4 + i / 4 * SM_ + i % 4, n = n0 + tx * 4 + j * SN_;
+  auto total = [&](int q, int thread) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int b = 0; b < blocks; ++b) {
-      const float4 t = (blocks > 1 ? cluster.map_shared_rank(sums, b) : sums)[q * THREADS + tid];
+      const float4 t = (blocks > 1 ? cluster.map_shared_rank(sums, b) : sums)[q * THREADS + thread];
       v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
     }
+    return v;
+  };
+  if (GATED) {
+    // A thread's columns and those of the thread four behind it (tx + 2: eight columns on) are each other's factors: the two take turns.
+    const int upper = tid >> 2 & 1, gate = tid & ~4, n0_ = n0 + (tx & ~2) * 4;
+    for (int q = rank + blocks * upper; q < TM * TN / 4; q += 2 * blocks) {
+      const int i = q / (TN / 4), j = q % (TN / 4);
+      const int m = m0 + ty * 4 + i / 4 * SM_ + i % 4, n = n0_ + j * SN_;
+      if (m >= M || n >= N) continue;
+      const float4 v = total(q, gate), u = total(q, gate + 4);
+      float out[4] = {v.x, v.y, v.z, v.w};
+      const float other[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        out[e] = gate_act(bias ? out[e] + bias[n + e] : out[e], act) * (bias ? other[e] + bias[n + 8 + e] : other[e]);
+      float* c = C + static_cast<size_t>(m) * ldc + n / 16 * 8 + n % 8;
+      if (wide) *reinterpret_cast<float4*>(c) = make_float4(out[0], out[1], out[2], out[3]);
+      else
+#pragma unroll
+        for (int e = 0; e < 4; ++e) c[e] = out[e];
+    }
+  } else for (int q = rank; q < TM * TN / 4; q += blocks) {
+    const int i = q / (TN / 4), j = q % (TN / 4);
+    const int m = m0 + ty * 4 + i / 4 * SM_ + i % 4, n = n0 + tx * 4 + j * SN_;
+    const float4 v = total(q, tid);
     if (m >= M || n >= N) continue;
     float* c = C + static_cast<size_t>(m) * ldc + n;
     const float out[4] = {v.x, v.y, v.z, v.w};
@@ -192,7 +218,7 @@ constexpr size_t few_smem(int pitch) { return sizeof(float) * kRowsW * pitch; }
 template <int MB>
 __global__ void __launch_bounds__(kRowsW * kSegments)
 gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                    float* __restrict__ C, int M, int N, int K, int lda, int ldc, int pitch, int block) {
+                    float* __restrict__ C, int M, int N, int K, int lda, int ldc, int pitch, int block, int act) {
   extern __shared__ __align__(16) float ws[];                    // [kRowsW][pitch]
   __shared__ float sums[kSegments][MB][kRowsW];
   pdl_trigger();
@@ -200,14 +226,16 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, co
   const int tid = threadIdx.x;
   const int n0 = blockIdx.x * kRowsW, m0 = blockIdx.y * MB;
   const int n = tid % kRowsW, seg = tid / kRowsW;
+  // a gated product takes four rows of one factor and the four of the other eight rows on
+  auto row_of = [&](int r) { return act ? static_cast<int>(blockIdx.x) / 2 * 16 + blockIdx.x % 2 * 4 + r / 4 * 8 + r % 4 : n0 + r; };
   const int rows = min(MB, M - m0);
   const float* a0 = A + static_cast<size_t>(m0) * lda;
   float total = 0.f, part = 0.f;                                 // of output (tid / kRowsW, tid % kRowsW), for tid < MB * kRowsW
   for (int k0 = 0; k0 < K; k0 += kPass) {
     const int span = min(kPass, K - k0), quads = span / 4;       // K is a multiple of 4 here
     for (int r = tid / 32; r < kRowsW; r += kRowsW * kSegments / 32) {
-      if (n0 + r >= N) continue;                                 // never read: that row's outputs are not stored
-      const float* src = W + static_cast<size_t>(n0 + r) * K + k0;
+      if (row_of(r) >= N) continue;                              // never read: that row's outputs are not stored
+      const float* src = W + static_cast<size_t>(row_of(r)) * K + k0;
       const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(ws + r * pitch));
       for (int q = tid % 32; q < quads; q += 32)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + q * 16), "l"(src + q * 4) : "memory");
@@ -218,7 +246,7 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, co
 #pragma unroll
     for (int m = 0; m < MB; ++m) acc[m] = 0.f;
     const int first = seg * kSegment, last = min(first + kSegment, span);
-    if (n0 + n < N) {
+    if (row_of(n) < N) {
       const float* wrow = ws + n * pitch;
 #pragma unroll 4
       for (int k = first; k < last; k += 4) {
@@ -248,9 +276,14 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, co
     }
     __syncthreads();                                             // the sums and the rows have been read
   }
-  if (tid < MB * kRowsW) {
-    const int m = m0 + tid / kRowsW, nn = n0 + tid % kRowsW;
-    if (m < M && nn < N) C[static_cast<size_t>(m) * ldc + nn] = (K % block ? total + part : total) + (bias ? bias[nn] : 0.f);
+  const int m = m0 + tid / kRowsW, nn = row_of(n);
+  const bool stored = tid < MB * kRowsW && m < M && nn < N;
+  const float out = (K % block ? total + part : total) + (stored && bias ? bias[nn] : 0.f);
+  if (act) {
+    const float other = __shfl_down_sync(0xffffffffu, out, 4);
+    if (stored && n < 4) C[static_cast<size_t>(m) * ldc + blockIdx.x * 4 + n] = gate_act(out, act) * other;
+  } else if (stored) {
+    C[static_cast<size_t>(m) * ldc + nn] = out;
   }
 }
 
@@ -302,10 +335,10 @@ gemm_f32_short_kernel(const float* __restrict__ A, const float* __restrict__ W, 
   }
 }
 
-template <int BM, int BN, int TM, int TN, bool VEC>
-int launch_tiles(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, cudaStream_t stream) {
+template <int BM, int BN, int TM, int TN, bool VEC, bool GATED>
+int launch_tiles(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, int act, cudaStream_t stream) {
   static DeviceOnce once;
-  const int status = configure_once(once, gemm_f32_tile_kernel<BM, BN, TM, TN, VEC>, kMostSmem);
+  const int status = configure_once(once, gemm_f32_tile_kernel<BM, BN, TM, TN, VEC, GATED>, kMostSmem);
   if (status) return status;
   const int block = block_length(K), blocks = (K + block - 1) / block;
   // Launched while the kernel before still holds some SMs, the CTAs would crowd on the others, three where two suffice (509 x 4096 x
@@ -325,30 +358,33 @@ int launch_tiles(const float* A, const float* W, const float* bias, float* C, in
   attributes[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attributes;
   config.numAttrs = pdl_enabled() ? 2 : 1;
-  cudaLaunchKernelEx(&config, gemm_f32_tile_kernel<BM, BN, TM, TN, VEC>, A, W, bias, C, M, N, K, lda, ldc, block);
+  cudaLaunchKernelEx(&config, gemm_f32_tile_kernel<BM, BN, TM, TN, VEC, GATED>, A, W, bias, C, M, N, K, lda, ldc, block, act);
   return launch_status();
 }
 
 template <int MB>
-int launch_few(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, cudaStream_t stream) {
+int launch_few(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, int act, cudaStream_t stream) {
   static DeviceOnce once;
   const int status = configure_once(once, gemm_f32_few_kernel<MB>, few_smem(kPass + 4));
   if (status) return status;
   const dim3 grid((N + kRowsW - 1) / kRowsW, (M + MB - 1) / MB);
   const int pitch = (K < kPass ? K : kPass) + 4;      // a short K takes less shared memory: more CTAs an SM
   launch(gemm_f32_few_kernel<MB>, grid, dim3(kRowsW * kSegments), few_smem(pitch), stream, A, W, bias, C, M, N, K, lda, ldc, pitch,
-         block_length(K));
+         block_length(K), act);
   return launch_status();
 }
 
 }  // namespace b200
 
 // `kernel`: 0 chooses by size; 1: few rows, 2: tiles of 64 x 64, 3: tiles of 128 x 64, 4: short rows (for tests and measurements).
-extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,
-                                     int ldc, int kernel, cudaStream_t stream) {
+// `act` (ACT_SILU, ACT_GELU_TANH): the rows of W are two factors in blocks of eight, [g0..g7 | u0..u7 | ...], and C [M, N / 2] is act(g) * u,
+// each product rounded as it would be stored; otherwise 0.
+extern "C" int b200_gemm_f32_gated(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,
+                                   int ldc, int kernel, int act, cudaStream_t stream) {
   using namespace b200;
   if (M <= 0 || N <= 0) return 0;
-  if (K <= 0 || lda < K || ldc < N) return B200_ERR_BAD_SIZE;
+  if (K <= 0 || lda < K || ldc < (act ? N / 2 : N)) return B200_ERR_BAD_SIZE;
+  if (act && (N % 16 || M > 65535 || (act != ACT_SILU && act != ACT_GELU_TANH))) return B200_ERR_BAD_SIZE;
   const bool vec = K % 4 == 0 && lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(W) % 16 == 0;
   const int blocks = (K + block_length(K) - 1) / block_length(K);
   const long long small = static_cast<long long>((M + 63) / 64) * ((N + 63) / 64) * blocks;
@@ -372,7 +408,7 @@ extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float
     const bool few = M <= 2 || (M <= 24 && K <= 64 && ctas <= 400) || (M <= 4 && (K > 160 || ctas <= 10 * 148)) || (M <= 8 && K >= 512) ||
                      (K > 160 && (M <= 8 || (M <= 24 && small < 148)) && few_us <= tiles_us);
     if (vec && few) kernel = 1;
-    else if (K <= (vec ? 32 : 112) && small <= 512) kernel = 4;
+    else if (K <= (vec ? 32 : 112) && small <= 512 && !act) kernel = 4;
     else {
       const int block = block_length(K), sms = usable_sms(blocks);
       const float depth = (K < block ? K : block) / 1024.f;
@@ -383,21 +419,27 @@ extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float
   if ((M + 63) / 64 > 65535) return B200_ERR_TOO_LARGE;
   if (kernel == 1) {
     if (!vec) return B200_ERR_BAD_SIZE;
-    if (M == 1) return launch_few<1>(A, W, bias, C, M, N, K, lda, ldc, stream);
-    if (M == 2) return launch_few<2>(A, W, bias, C, M, N, K, lda, ldc, stream);
-    if (M <= 4) return launch_few<4>(A, W, bias, C, M, N, K, lda, ldc, stream);
-    return launch_few<8>(A, W, bias, C, M, N, K, lda, ldc, stream);
+    if (M == 1) return launch_few<1>(A, W, bias, C, M, N, K, lda, ldc, act, stream);
+    if (M == 2) return launch_few<2>(A, W, bias, C, M, N, K, lda, ldc, act, stream);
+    if (M <= 4) return launch_few<4>(A, W, bias, C, M, N, K, lda, ldc, act, stream);
+    return launch_few<8>(A, W, bias, C, M, N, K, lda, ldc, act, stream);
   }
   if (kernel == 4) {
-    if (K > kSegment) return B200_ERR_BAD_SIZE;
+    if (K > kSegment || act) return B200_ERR_BAD_SIZE;
     launch(gemm_f32_short_kernel, dim3((N + 63) / 64, (M + 63) / 64), dim3(256), 0, stream, A, W, bias, C, M, N, K, lda, ldc);
     return launch_status();
   }
-  if (kernel == 3)
-    return vec ? launch_tiles<128, 64, 8, 8, true>(A, W, bias, C, M, N, K, lda, ldc, stream)
-               : launch_tiles<128, 64, 8, 8, false>(A, W, bias, C, M, N, K, lda, ldc, stream);
-  return vec ? launch_tiles<64, 64, 8, 4, true>(A, W, bias, C, M, N, K, lda, ldc, stream)
-             : launch_tiles<64, 64, 8, 4, false>(A, W, bias, C, M, N, K, lda, ldc, stream);
+#define B200_F32_TILES(BM, TN, VEC)                                                                                 \
+  (act ? launch_tiles<BM, 64, 8, TN, VEC, true>(A, W, bias, C, M, N, K, lda, ldc, act, stream)                       \
+       : launch_tiles<BM, 64, 8, TN, VEC, false>(A, W, bias, C, M, N, K, lda, ldc, act, stream))
+  if (kernel == 3) return vec ? B200_F32_TILES(128, 8, true) : B200_F32_TILES(128, 8, false);
+  return vec ? B200_F32_TILES(64, 4, true) : B200_F32_TILES(64, 4, false);
+#undef B200_F32_TILES
+}
+
+extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,
+                                     int ldc, int kernel, cudaStream_t stream) {
+  return b200_gemm_f32_gated(A, W, bias, C, M, N, K, lda, ldc, kernel, 0, stream);
 }
 
 extern "C" int b200_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M,

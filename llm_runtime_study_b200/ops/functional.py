@@ -85,6 +85,24 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None 
 GATE_ACTS = {"silu": 1, "gelu_tanh": 2}     # as numbered in csrc/common.cuh
 
 
+def linear_f32_gated(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None, act: str = "silu") -> torch.Tensor:
+    """``silu_mul_interleaved(linear_f32(x, weight, bias), act)`` in one kernel, the same bits."""
+
+    require(x, "x", dtype=torch.float32, dims=2)
+    require(weight, "weight", dtype=torch.float32, dims=2)
+    m, k = x.shape
+    n = weight.shape[0]
+    if weight.shape[1] != k:
+        raise KernelError(f"linear: x has width {k}, weight expects {weight.shape[1]}")
+    if n % 16:
+        raise KernelError("a gated projection's rows must be a multiple of 16")
+    if bias is not None:
+        require(bias, "bias", dtype=torch.float32, shape=(n,))
+    out = torch.empty((m, n // 2), dtype=torch.float32, device=x.device)
+    call("b200_gemm_f32_gated", ptr(x), ptr(weight), ptr(bias), ptr(out), m, n, k, k, n // 2, 0, GATE_ACTS[act], stream_ptr())
+    return out
+
+
 def silu_mul(gate_up: torch.Tensor, act: str = "silu") -> torch.Tensor:
     """``silu(gate) * up`` for rows laid out as ``[gate | up]``."""
 

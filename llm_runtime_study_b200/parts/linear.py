@@ -92,6 +92,8 @@ class Projection:
                 return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act)
             if self.GEMM_BACKEND == "tcgen05" and (self.MID_ROWS == "splitk" or gemm_bf16.gated_in_one(self.out_features, self.in_features)):
                 return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act, kernel="splitk")
+        if self.runtime.dtype == torch.float32 and x.shape[-1] == self.in_features:
+            return F.linear_f32_gated(x, self.weight, self.bias, act)
         return F.silu_mul_interleaved(self(x), act)
 
     def __call__(self, x: "torch.Tensor | WeightedRows", out_dtype: torch.dtype | None = None, *,

@@ -136,6 +136,27 @@ def test_gemm_f32_of_short_rows_gives_the_bits_of_the_tiles(m, n, k):
     assert all(torch.equal(out, results[0]) for out in results[1:])
 
 
+# every kernel (few rows 1, tiles of 64 rows 2 and of 128 3, the choice 0) over parts of a tile of rows, of columns, one pair of eights, several
+# blocks of K (a cluster), rows that are no 16-byte vectors
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+@pytest.mark.parametrize("m,n,k", [(1, 16, 4), (3, 48, 260), (8, 544, 1028), (13, 544, 96), (70, 80, 2052), (129, 208, 35), (5, 32, 20)])
+def test_gemm_f32_gated_gives_the_bits_of_two_kernels(m, n, k, act):
+    from llm_runtime_study_b200.ops import native
+
+    torch.manual_seed(6)
+    x, w, b = dev(torch.randn(m, k)), dev(torch.randn(n, k)), dev(torch.randn(n))
+    for bias in (None, b):
+        want = F().silu_mul_interleaved(F().linear_f32(x, w, bias), act)
+        assert torch.equal(F().linear_f32_gated(x, w, bias, act), want)
+        for kernel in (1, 2, 3):
+            if kernel == 1 and k % 4:
+                continue                # 16-byte rows only
+            out = torch.full((m, n // 2), float("nan"), device=x.device)
+            native.call("b200_gemm_f32_gated", x.data_ptr(), w.data_ptr(), native.ptr(bias), out.data_ptr(), m, n, k, k, n // 2, kernel,
+                        F().GATE_ACTS[act], native.stream_ptr())
+            assert torch.equal(out, want), kernel
+
+
 def _scatter_to_pages(k, v, page_size, nkv, d, dtype, seed=0, extra_pages=3):
     """Put contiguous k, v [T, nkv, d] into shuffled pages; return pools + table row."""
 
