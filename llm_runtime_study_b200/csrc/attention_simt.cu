@@ -481,7 +481,7 @@ extern "C" int b200_paged_attention_tiles(
   if (d > 128 || dv > 128 || nq / nkv > kTileRows) return B200_ERR_TOO_LARGE;
   const int per_tile = kTileRows / (nq / nkv);
   const long long tiles = (static_cast<long long>(n) / per_tile + entries) * nkv;      // at least as many as there are; the others return
-  if (tiles > 0x7fffffff) return B200_ERR_TOO_LARGE;
+  if (nkv > 65535 || tiles > 0x7fffffff) return B200_ERR_TOO_LARGE;
   const TileParams p{q, k_pool, v_pool, out, positions, q_start, block_table, entries, table_stride, page_size, nq, nkv, d, dv,
                      per_tile, static_cast<int>(tiles), window, chunk, sink, scale, softcap, slopes, log_r1, log_r2, sinks};
   const int widest = d > dv ? d : dv;
