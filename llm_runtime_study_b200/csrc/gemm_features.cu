@@ -176,6 +176,7 @@ gemm_features_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         if (++s == stages) { s = 0; phase ^= 1; }
       }
     }
+    if (ok && !stages_returned(empty, stages, s, phase)) atomicExch(&g_features_error, 1);
   } else if (warp == 1) {
     // ---------------------------------------------------------------- tensor-core issue (leader)
     if (leader) {
@@ -244,7 +245,7 @@ gemm_features_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       }
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_addr(acc_empty + buf), leader_rank));
+      if (lane == 0 && accumulator_reused(item, clusters, buffers, items)) mbar_arrive_cluster(map_to_cta(smem_addr(acc_empty + buf), leader_rank));
     }
   } else {
     // ------------------------------------ epilogue of a shared tile: every pair hands the others their shares of its partial sums,
@@ -313,7 +314,7 @@ gemm_features_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   __syncwarp();
   tcgen05_fence_before();
   __syncthreads();
-  cluster_sync_relaxed();                 // nobody leaves while another CTA may still reach its shared memory or its barriers
+  cluster_sync_relaxed();                 // nobody leaves while the tensor cores of its pair still read its shared memory
   if (warp == 1) {
     __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");

@@ -336,7 +336,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_rows, con
 // per stage: both CTAs' TMA copies complete on the leader's `full` barrier (armed by the leader
 // for the bytes of both); the leader's commit arrives on `empty` in both CTAs.  Per tile: the
 // leader's commit arrives on `acc_full` in both CTAs; the eight epilogue warps of the pair arrive
-// on the leader's `acc_empty`.
+// on the leader's `acc_empty` if the buffer is filled again.  Every arrival is waited for by the CTA that it reaches, so the
+// barrier at the end has nothing to order.
 template <int BN, int STAGES, bool SWIGLU, typename OutT>
 __global__ void __launch_bounds__(kThreads)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, GemmParams p) {
@@ -394,6 +395,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __g
         if (++s == STAGES) { s = 0; phase ^= 1; }
       }
     }
+    if (ok && !stages_returned(empty, STAGES, s, phase)) atomicExch(&g_gemm_error, 1);
   } else if (warp == 1 && leader) {
     // ---------------------------------------------------------------- tensor-core issue (leader)
     constexpr uint32_t idesc = umma_idesc_pair(BN);
@@ -455,7 +457,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __g
       }
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_addr(acc_empty + buf), 0));
+      if (lane == 0 && accumulator_reused(tile, pairs, 2, tiles)) mbar_arrive_cluster(map_to_cta(smem_addr(acc_empty + buf), 0));
       if (!ok) break;
     }
   }
@@ -1103,6 +1105,11 @@ static int launch_pair(const CUtensorMap& rows, const CUtensorMap& cols, const G
 }  // namespace b200
 
 using namespace b200;
+
+// (the pair kernels' rule, callable without a GPU)
+extern "C" int b200_gemm_tcgen05_accumulator_reused(int item, int stride, int buffers, int items) {
+  return b200::accumulator_reused(item, stride, buffers, items) ? 1 : 0;
+}
 
 // Read and clear the error flag set by a bounded wait that ran out (0: none; 1: producer,
 // 2: tensor-core issue, 3: epilogue).  Synchronises the device.

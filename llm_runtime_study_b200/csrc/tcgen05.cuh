@@ -128,10 +128,23 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 // The barrier alone, for CTAs that only stay until the others are done with their shared memory: with release and acquire it also
-// waits for every store to global memory before it (0.65 us behind an epilogue, 0.2 without).
+// waits for every store to global memory before it (0.65 us behind an epilogue, 0.2 without).  It orders no memory access: whatever
+// this CTA did to another one's shared memory must be known to be over, values read from there used, arrivals there waited for.
 __device__ __forceinline__ void cluster_sync_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
   asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
+}
+// Whether the accumulator of item `item` is filled again: `buffers` take turns over the items item, item + stride, ... below `items`.  Only
+// then is its being free announced to the pair's leader: an arrival that nobody waits for could reach a CTA that has left.
+__host__ __device__ constexpr bool accumulator_reused(int item, int stride, int buffers, int items) { return item + stride * buffers < items; }
+// The end of a pair's producer: waits until the tensor cores have given back all stages (those never filled are free).  Their arrivals
+// come from the leader, so none is on its way to this CTA when it leaves.
+__device__ __forceinline__ bool stages_returned(uint64_t* empty, int stages, int s, uint32_t phase) {
+  for (int i = 0; i < stages; ++i) {
+    if (!mbar_wait_warp(empty + s, phase ^ 1)) return false;
+    if (++s == stages) { s = 0; phase ^= 1; }
+  }
+  return true;
 }
 // TMA copy into this CTA's shared memory whose bytes are counted on a barrier of the pair's leader
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t leader_bar, int x, int y) {

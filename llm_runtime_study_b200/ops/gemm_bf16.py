@@ -20,6 +20,7 @@ native.register_library(
                                       c_void_p],
         "b200_gemm_tcgen05_error": [],
         "b200_gemm_tcgen05_pair_width": [c_int, c_int, c_int, c_int],
+        "b200_gemm_tcgen05_accumulator_reused": [c_int, c_int, c_int, c_int],
         "b200_gemm_tcgen05_splitk_shape": [c_int, c_int, c_int, c_int, c_void_p, c_void_p],
         "b200_gemm_tcgen05_streamk_partial_floats": [],
         "b200_gemm_tcgen05_streamk_flags": [],

@@ -63,6 +63,21 @@ def test_tiles_of_the_projections_by_features():
     assert gemm_bf16.features_shape(160, 1024, 2048, 148)[2] == 4
 
 
+def test_accumulators_of_pairs_are_announced_only_to_a_wait():
+    """Every arrival on a pair's accumulator barrier belongs to a later item that waits for it: the first use of a buffer waits for none."""
+
+    from llm_runtime_study_b200.ops import native
+
+    for items, stride, buffers in itertools.product((1, 2, 3, 4, 5, 73, 74, 75, 148, 149, 400), (1, 2, 18, 37, 74), (1, 2)):
+        for cluster in range(min(items, stride)):
+            mine = range(cluster, items, stride)
+            arrivals, waits = [0] * buffers, [0] * buffers
+            for local, item in enumerate(mine):
+                waits[local % buffers] += local >= buffers
+                arrivals[local % buffers] += native.query("b200_gemm_tcgen05_accumulator_reused", item, stride, buffers, items)
+            assert arrivals == waits
+
+
 def test_which_projections_go_by_features():
     takes = gemm_bf16.by_features
     assert takes(405, 4096, 12288, True) and takes(129, 1024, 1024, True) and takes(1024, 4096, 4096, True) and takes(405, 4096, 4096, False)

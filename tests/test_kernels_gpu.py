@@ -823,6 +823,22 @@ def test_tcgen05_projection_by_features(m, n, k, tokens, splits, form):
     torch.testing.assert_close(got.cpu().double(), want + (resid.double() if form == "add" else 0), atol=(1e-2 if form == "bf16" else 2e-5) * scale, rtol=0)
 
 
+# one to five tiles for each pair of SMs, the numbers of tiles of two pairs not the same, K ranges shorter and longer than the ring
+@pytest.mark.parametrize("tiles", [1, 73, 74, 75, 149, 223, 297])
+@pytest.mark.parametrize("k", [64, 520])
+def test_pairs_that_leave_behind_any_number_of_tiles(tiles, k):
+    x, w, b, want = _gemm_case(256, 256 * tiles, k, True)
+    scale = float(want.abs().max())
+    for run in (lambda: _gemm().linear(dev(x), dev(w), dev(b), torch.float32, kernel="pair", pair_width=256),
+                lambda: _gemm().linear_features(dev(x), dev(w), dev(b), torch.float32, tokens=(256, 0), splits=1),
+                lambda: _gemm().linear_features(dev(x), dev(w), dev(b), torch.float32, tokens=(256, 64), splits=1)):
+        got = run()
+        assert torch.equal(got, run())
+        assert _gemm().native.query("b200_gemm_features_error") == 0
+        _gemm().check_error()
+        torch.testing.assert_close(got.cpu().double(), want, atol=2e-5 * scale, rtol=0)
+
+
 # by features (few columns, a short K range) and split-K; the fewest and the most rows that come here
 @pytest.mark.parametrize("m", [17, 64, 127])
 @pytest.mark.parametrize("n,k", [(300, 520), (2056, 2056), (2064, 96)])
