@@ -3,7 +3,7 @@
 // tile while it is in shared memory.  A pair of CTAs (cta_group::2) computes 256 features x (n1 + n2) tokens as one or two products
 // of up to 256 columns each; a tile's K range can be shared by 2 or 4 pairs (one cluster), which hand each other their shares of
 // the partial sums through distributed shared memory.
-//   warp 0   producer: TMA loads of 64-wide K blocks, the weights' first ring ahead of the wait for the kernel before;
+//   warp 0   producer: TMA loads of 64-wide K blocks, the first ring of weights that are at rest ahead of the wait for the kernel before;
 //   warp 1   tensor-core issue (in the pair's leader);
 //   warps 2-17  epilogue: a lane has a feature, a warp's stores are 32 neighbouring features of a row of C (64 or 128 bytes),
 //            where the kernels of gemm_tcgen05.cu write 16 bytes of 32 rows at a time.
@@ -43,6 +43,7 @@ struct FeatureParams {
   int share;           // splits > 1: columns of the tile that a pair finishes, a multiple of 16
   int wide;            // splits == 1: tiles that are computed whole; of those behind them the two products are items of their own
   int stages, accumulate;
+  int weight_ahead;    // no kernel that may still be running writes the weight
 };
 
 // What a cluster computes at a time: `count` tokens from `token` on of the 256 features from `feature` on, as the product with the first
@@ -130,8 +131,8 @@ gemm_features_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");   // every CTA's barriers exist before anything arrives on them
   const uint32_t pair_full = map_to_cta(smem_addr(full), leader_rank);
   int ahead = 0;
-  if (warp == 0 && cluster < items) {
-    // the weights do not depend on the kernel before this one: the first ring of them is asked for ahead of the wait
+  if (warp == 0 && cluster < items && p.weight_ahead) {
+    // weights that do not depend on the kernel before this one: the first ring of them is asked for ahead of the wait
     const FeatureItem it = feature_item(p, m_tiles, cluster);
     const uint32_t bytes = 2 * (W_BYTES + (it.first ? a1_bytes : 0) + (it.second ? a2_bytes : 0));
     const int y = it.feature + static_cast<int>(rank) * kFeatBM;
@@ -436,9 +437,10 @@ extern "C" int b200_gemm_features_shape(int M, int N, int K, int sm_count, int* 
 
 // C[M,N] (ldc) = A[M,K] * W[N,K]^T + bias, or (accumulate, float output) C += that.
 // n1, n2: tokens of a tile in its first and second product; splits: pairs of CTAs that share a tile's K range (1, 2, 4); all 0:
-// chosen by size.  M up to 16,384.
+// chosen by size.  M up to 16,384.  weight_ahead: no kernel that may still be running on the stream writes W, which is then read ahead of
+// the wait for it.
 extern "C" int b200_gemm_features(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, int ldc, int out_f32,
-                                  int accumulate, int n1, int n2, int splits, cudaStream_t stream) {
+                                  int accumulate, int n1, int n2, int splits, int weight_ahead, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || K % 8 != 0 || ldc < N) return B200_ERR_BAD_SIZE;
   if (accumulate && !out_f32) return B200_ERR_BAD_SIZE;
@@ -452,7 +454,7 @@ extern "C" int b200_gemm_features(const void* A, const void* W, const float* bia
   if (n1 < 32 || n1 > 256 || n1 % 32 || n2 < 0 || n2 > 256 || n2 % 32 || (splits != 1 && splits != 2 && splits != 4) || splits > (K + kFeatBK - 1) / kFeatBK)
     return B200_ERR_BAD_SIZE;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) return B200_ERR_BAD_SIZE;
-  FeatureParams p{C, bias, M, N, K, ldc, n1, n2, splits, 0, 0, 0, accumulate};
+  FeatureParams p{C, bias, M, N, K, ldc, n1, n2, splits, 0, 0, 0, accumulate, weight_ahead};
   CUtensorMap w, a1, a2;
   if (int e = features_map(&w, W, N, K, kFeatBM)) return e;
   if (int e = features_map(&a1, A, M, K, n1 / 2)) return e;

@@ -106,6 +106,7 @@ struct GemmParams {
   int group_rows;
   int act;            // 1: the square of relu on the way out (not with SWIGLU)
   int gate_act;       // SWIGLU: ACT_SILU or ACT_GELU_TANH
+  int weight_ahead;   // split-K: the weight is no work of a kernel that may still be running: it is read ahead of the wait
 };
 
 // What C holds in 32 columns of a row of it from column nb on, asked for a chunk ahead of its use (from L2 or HBM it takes
@@ -778,9 +779,9 @@ gemm_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_rows, const _
   bool ok = true;
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
-    // The weights do not depend on the kernel before this one: the first ring of weight tiles is asked
+    // Weights that do not depend on the kernel before this one: the first ring of their tiles is asked
     // for while that kernel is still finishing, the activations only after the wait.
-    const int ahead = min(stages, kb1 - kb0);
+    const int ahead = p.weight_ahead ? min(stages, kb1 - kb0) : 0;
     if (elect_one()) {
       for (int i = 0; i < ahead; ++i) {
         mbar_expect_tx(full + i, stage_bytes);
@@ -1134,6 +1135,7 @@ extern "C" int b200_gemm_tcgen05_error() {
 //   tile_n      128 or 256 columns per tile (kind 0; kind 2 takes 256): narrower tiles put a product
 //               with few rows on more SMs; kind 1: 128, 192, 224 or 256, 0: chosen from M, N and K so that the
 //               rounds of tiles are full (b200_gemm_tcgen05_pair_width)
+//   weight_ahead  split-K only: no kernel that may still be running on the stream writes W (the other kinds wait for it anyway)
 //   partials, flags  stream-K only: b200_gemm_tcgen05_streamk_partial_floats() floats and
 //               b200_gemm_tcgen05_streamk_flags() 32-bit words that are zero before the first launch
 //               (the kernel leaves them zero); launches that share them must not overlap
@@ -1175,7 +1177,7 @@ static int launch_variant(const CUtensorMap& rows, const CUtensorMap& cols, cons
 
 extern "C" int b200_gemm_tcgen05(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, int ldc,
                                  int out_f32, int swiglu, int accumulate, int kind, int tile_n, int splits, int stages,
-                                 float* partials, unsigned* flags, cudaStream_t stream) {
+                                 float* partials, unsigned* flags, int weight_ahead, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || K % 8 != 0 || ldc < (swiglu ? N / 2 : N) || (swiglu && N % 16 != 0) || swiglu < 0 || swiglu > ACT_GELU_TANH || kind < 0 || kind > 3) return B200_ERR_BAD_SIZE;
   if (kind == 1 ? (tile_n != 0 && tile_n != 128 && tile_n != 192 && tile_n != 224 && tile_n != 256)
@@ -1186,6 +1188,7 @@ extern "C" int b200_gemm_tcgen05(const void* A, const void* W, const float* bias
   if (kind == 2 && (!partials || !flags || (reinterpret_cast<uintptr_t>(partials) & 15))) return 10004;
   GemmParams p{C, bias, M, N, K, ldc, (ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) ? 1 : 0, accumulate, partials, flags, splits, BM, tile_n, 0};
   p.gate_act = swiglu;
+  p.weight_ahead = weight_ahead;
   if (kind == 1 && tile_n == 0) {
     int device = 0, sm_count = 0;
     cudaGetDevice(&device);

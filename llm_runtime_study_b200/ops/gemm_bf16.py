@@ -15,7 +15,7 @@ native.register_library(
     "b200_gemm_tcgen05", ("gemm_tcgen05.cu",),
     {
         "b200_gemm_tcgen05": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                              c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
+                              c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p],
         "b200_gemm_tcgen05_grouped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
                                       c_void_p],
         "b200_gemm_tcgen05_error": [],
@@ -45,7 +45,7 @@ native.register_library(
     "b200_gemm_features", ("gemm_features.cu",),
     {
         "b200_gemm_features": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                               c_void_p],
+                               c_int, c_void_p],
         "b200_gemm_features_error": [],
         "b200_gemm_features_shape": [c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
     },
@@ -184,7 +184,8 @@ def gated_unit(swiglu: "bool | str") -> int:
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None,
            out_dtype: torch.dtype = torch.bfloat16, *, swiglu: "bool | str" = False, add_to: torch.Tensor | None = None,
-           kernel: str | None = None, tile_n: int | None = None, splits: int = 0, stages: int = 0, pair_width: int = 0) -> torch.Tensor:
+           kernel: str | None = None, tile_n: int | None = None, splits: int = 0, stages: int = 0, pair_width: int = 0,
+           weight_at_rest: bool = False) -> torch.Tensor:
     """``x @ weight.T (+ bias)`` on the tcgen05 tensor cores; float32 accumulation; bfloat16 or
     float32 output.
 
@@ -196,7 +197,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     tiles: up to three SMs share a tile's K range) or "splitk" (few rows: a cluster of ``splits``
     <= 8 CTAs shares the K range of every 128 x ``tile_n`` tile, ``tile_n`` a multiple of 32; 0 for either
     lets the kernel choose so that the SMs are filled once; ``stages``: depth of its operand ring, 0 = as
-    deep as shared memory allows); chosen by shape when not given, the kernel of ``linear_features`` among them."""
+    deep as shared memory allows); chosen by shape when not given, the kernel of ``linear_features`` among them.
+    ``weight_at_rest``: no kernel that may still be running on the stream writes ``weight``, as with a model's weights; some kernels then
+    read it ahead of the wait for the kernel before."""
 
     native.require(x, "x", dtype=torch.bfloat16, dims=2)
     native.require(weight, "weight", dtype=torch.bfloat16, dims=2)
@@ -218,7 +221,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
             raise KernelError(f"unsupported output type {out_dtype}")
         out = torch.empty((m, n // 2 if swiglu else n), dtype=out_dtype, device=x.device)
     if not (kernel or tile_n or splits or stages or pair_width or swiglu) and by_features(m, n, k, out_dtype == torch.float32):
-        _by_features(x, weight, bias, out, add_to is not None, (0, 0), 0)
+        _by_features(x, weight, bias, out, add_to is not None, (0, 0), 0, weight_at_rest)
         return out
     picked_kernel, picked_width = pick_kernel(m, n, k)
     kernel = kernel or picked_kernel
@@ -239,19 +242,21 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     partials, flags = _streamk_workspace(x.device) if kernel == "streamk" else (None, None)
     native.call("b200_gemm_tcgen05", x.data_ptr(), weight.data_ptr(), native.ptr(bias), out.data_ptr(), m, n, k,
                 out.shape[1], 1 if out_dtype == torch.float32 else 0, gated_unit(swiglu), 0 if add_to is None else 1,
-                KERNELS[kernel], tile_n, splits, stages, native.ptr(partials), native.ptr(flags), native.stream_ptr())
+                KERNELS[kernel], tile_n, splits, stages, native.ptr(partials), native.ptr(flags), 1 if weight_at_rest else 0, native.stream_ptr())
     return out
 
 
 def _by_features(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, out: torch.Tensor, add: bool, tokens: tuple[int, int],
-                 splits: int) -> None:
+                 splits: int, weight_at_rest: bool) -> None:
     (m, k), n = x.shape, weight.shape[0]
     native.call("b200_gemm_features", x.data_ptr(), weight.data_ptr(), native.ptr(bias), out.data_ptr(), m, n, k, n,
-                1 if out.dtype == torch.float32 else 0, 1 if add else 0, tokens[0], tokens[1], splits, native.stream_ptr())
+                1 if out.dtype == torch.float32 else 0, 1 if add else 0, tokens[0], tokens[1], splits, 1 if weight_at_rest else 0,
+                native.stream_ptr())
 
 
 def linear_features(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None, out_dtype: torch.dtype = torch.bfloat16, *,
-                    add_to: torch.Tensor | None = None, tokens: tuple[int, int] = (0, 0), splits: int = 0) -> torch.Tensor:
+                    add_to: torch.Tensor | None = None, tokens: tuple[int, int] = (0, 0), splits: int = 0,
+                    weight_at_rest: bool = False) -> torch.Tensor:
     """As ``linear``, with the weight as the tensor cores' row operand: pairs of SMs on tiles of 256 features and ``tokens`` rows of
     ``x`` (the two numbers' sum, each a multiple of 32 up to 256, the second may be 0), ``splits`` (1, 2 or 4) pairs to a tile's K range;
     chosen by shape when not given."""
@@ -273,11 +278,11 @@ def linear_features(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | 
         if out_dtype not in (torch.bfloat16, torch.float32):
             raise KernelError(f"unsupported output type {out_dtype}")
         out = torch.empty((m, n), dtype=out_dtype, device=x.device)
-    _by_features(x, weight, bias, out, add_to is not None, tokens, splits)
+    _by_features(x, weight, bias, out, add_to is not None, tokens, splits, weight_at_rest)
     return out
 
 
-def linear_with_bias(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
+def linear_with_bias(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, *, weight_at_rest: bool = False) -> torch.Tensor:
     """``x @ weight.T + bias`` in bfloat16 for 17 to 127 rows.  Without a bias such products are the library's; behind one of those
     the sum is two launches more (the bias in bfloat16, the addition) and rounds twice.  With a K range or a number of columns up to 2,048 by
     features, else split-K, microseconds with 17, 64 and 127 rows against the library and the sum: 16,384 x 2,048 16.2, 17.1, 17.8
@@ -286,8 +291,8 @@ def linear_with_bias(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor) 
     added in place: as fast as these, so it stays.)"""
 
     if PAIR_ENABLED and (x.shape[1] <= 2048 or weight.shape[0] <= 2048):
-        return linear_features(x, weight, bias, torch.bfloat16)
-    return linear(x, weight, bias, torch.bfloat16, kernel="splitk")
+        return linear_features(x, weight, bias, torch.bfloat16, weight_at_rest=weight_at_rest)
+    return linear(x, weight, bias, torch.bfloat16, kernel="splitk", weight_at_rest=weight_at_rest)
 
 
 def features_shape(m: int, n: int, k: int, sm_count: int = 0) -> tuple[int, int, int]:
@@ -324,7 +329,7 @@ def linear_skinny(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | No
     ``swiglu``: see ``linear``.  ``row_scale`` (float32 ``[16]``): the rows of ``x`` still lack these factors
     (an RMS norm left half done, see ``linear_skinny_residual``); they are applied to the product, before the bias.
     ``sums`` (float32 ``[parts, 16]``, with the norm's ``eps``) instead of it: the shares of the rows' sums of squares that make the factors, for at
-    most eight rows."""
+    most eight rows.  ``weight`` is read ahead of the wait for the kernel before: that kernel must not write it."""
 
     native.require(x, "x", dtype=torch.bfloat16, dims=2)
     native.require(weight, "weight", dtype=torch.bfloat16, dims=2)

@@ -86,12 +86,12 @@ class Projection:
             m = x.shape[0]
             if m <= gemm_bf16.SKINNY_M:
                 if self.GEMM_BACKEND == "tcgen05" and gemm_bf16.few_rows_kernel(m, self.out_features, self.in_features) == "splitk":
-                    return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act, kernel="splitk")
+                    return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act, kernel="splitk", weight_at_rest=True)
                 return gemm_bf16.linear_skinny(x, self.weight, self.bias, torch.bfloat16, swiglu=act)
             if self.GEMM_BACKEND == "tcgen05" and m >= self.TCGEN05_MIN_ROWS:
-                return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act)
+                return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act, weight_at_rest=True)
             if self.GEMM_BACKEND == "tcgen05" and (self.MID_ROWS == "splitk" or gemm_bf16.gated_in_one(self.out_features, self.in_features)):
-                return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act, kernel="splitk")
+                return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act, kernel="splitk", weight_at_rest=True)
         if self.runtime.dtype == torch.float32 and x.shape[-1] == self.in_features:
             return F.linear_f32_gated(x, self.weight, self.bias, act)
         return F.silu_mul_interleaved(self(x), act)
@@ -127,22 +127,22 @@ class Projection:
             if m <= gemm_bf16.SKINNY_M:
                 if self.GEMM_BACKEND == "tcgen05" and gemm_bf16.few_rows_kernel(m, self.out_features, self.in_features) == "splitk":
                     if add_to is not None and out_dtype == torch.float32 and self.FUSE_RESIDUAL:
-                        gemm_bf16.linear(x, self.weight, self.bias, torch.float32, add_to=add_to, kernel="splitk")
+                        gemm_bf16.linear(x, self.weight, self.bias, torch.float32, add_to=add_to, kernel="splitk", weight_at_rest=True)
                         return None
-                    return gemm_bf16.linear(x, self.weight, self.bias, out_dtype, kernel="splitk")
+                    return gemm_bf16.linear(x, self.weight, self.bias, out_dtype, kernel="splitk", weight_at_rest=True)
                 return gemm_bf16.linear_skinny(x, self.weight, self.bias, out_dtype)
             if self.GEMM_BACKEND == "tcgen05" and m >= self.TCGEN05_MIN_ROWS:
                 if add_to is not None and out_dtype == torch.float32 and self.FUSE_RESIDUAL:
-                    gemm_bf16.linear(x, self.weight, self.bias, torch.float32, add_to=add_to)
+                    gemm_bf16.linear(x, self.weight, self.bias, torch.float32, add_to=add_to, weight_at_rest=True)
                     return None
-                return gemm_bf16.linear(x, self.weight, self.bias, out_dtype)
+                return gemm_bf16.linear(x, self.weight, self.bias, out_dtype, weight_at_rest=True)
             if self.GEMM_BACKEND == "tcgen05" and self.MID_ROWS == "splitk":
                 if add_to is not None and out_dtype == torch.float32 and self.FUSE_RESIDUAL:
-                    gemm_bf16.linear(x, self.weight, self.bias, torch.float32, add_to=add_to, kernel="splitk")
+                    gemm_bf16.linear(x, self.weight, self.bias, torch.float32, add_to=add_to, kernel="splitk", weight_at_rest=True)
                     return None
-                return gemm_bf16.linear(x, self.weight, self.bias, out_dtype, kernel="splitk")
+                return gemm_bf16.linear(x, self.weight, self.bias, out_dtype, kernel="splitk", weight_at_rest=True)
             if self.GEMM_BACKEND == "tcgen05" and self.bias is not None and out_dtype == torch.bfloat16:
-                return gemm_bf16.linear_with_bias(x, self.weight, self.bias)
+                return gemm_bf16.linear_with_bias(x, self.weight, self.bias, weight_at_rest=True)
         if out_dtype == torch.bfloat16:
             y = torch.mm(x, self.weight.t())
         else:

@@ -78,6 +78,32 @@ def test_accumulators_of_pairs_are_announced_only_to_a_wait():
             assert arrivals == waits
 
 
+def test_only_weights_at_rest_are_read_ahead(monkeypatch):
+    """The operations wait for the kernel before; a model's projections, whose weights no kernel writes, need not."""
+
+    import torch
+
+    from llm_runtime_study_b200.ops import native
+    from llm_runtime_study_b200.parts import Runtime
+    from llm_runtime_study_b200.parts.linear import Projection
+
+    asked = []
+    monkeypatch.setattr(native, "require", lambda *a, **k: None)
+    monkeypatch.setattr(native, "sm_count", lambda: 148)
+    monkeypatch.setattr(native, "stream_ptr", lambda: None)
+    monkeypatch.setattr(native, "call", lambda name, *args, **k: asked.append((name, args[-2])))
+    w, b, rows = torch.zeros(4096, 2048).bfloat16(), torch.zeros(4096), lambda m: torch.zeros(m, 2048).bfloat16()
+    gemm_bf16.linear(rows(405), w, None, torch.float32)
+    gemm_bf16.linear_features(rows(64), w)
+    gemm_bf16.linear_with_bias(rows(64), w, b)
+    gemm_bf16.linear(rows(64), w, kernel="splitk")
+    at_rest = len(asked)
+    plain, biased = (Projection([w], biases, Runtime(torch.device("cpu"), torch.bfloat16)) for biases in (None, [b]))
+    plain(rows(405), torch.float32), biased(rows(64)), plain(rows(200)), plain(rows(405), torch.float32, add_to=torch.zeros(405, 4096))
+    assert [flag for _, flag in asked] == [0] * at_rest + [1] * (len(asked) - at_rest) and len(asked) == at_rest + 4
+    assert {name for name, _ in asked} == {"b200_gemm_features", "b200_gemm_tcgen05"}
+
+
 def test_which_projections_go_by_features():
     takes = gemm_bf16.by_features
     assert takes(405, 4096, 12288, True) and takes(129, 1024, 1024, True) and takes(1024, 4096, 4096, True) and takes(405, 4096, 4096, False)

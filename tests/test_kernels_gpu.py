@@ -839,6 +839,25 @@ def test_pairs_that_leave_behind_any_number_of_tiles(tiles, k):
         torch.testing.assert_close(got.cpu().double(), want, atol=2e-5 * scale, rtol=0)
 
 
+# by features, split-K and what the shape picks; several rings of K blocks
+@pytest.mark.parametrize("m,kernel", [(405, "features"), (405, None), (64, "splitk"), (130, None)])
+def test_a_weight_that_the_kernel_before_writes(m, kernel):
+    """Nothing of the weight is read before that kernel's writes are there: every round's weight is another one in the same memory."""
+
+    n, k = 4096, 2048
+    x, gate_up = dev(torch.randn(m, k).bfloat16()), torch.empty(n, 2 * k, dtype=torch.bfloat16, device="cuda")
+    torch.manual_seed(2)
+    for _ in range(12):
+        gate_up.normal_()
+        weight = F().silu_mul(gate_up)
+        got = (_gemm().linear_features(x, weight, None, torch.float32) if kernel == "features"
+               else _gemm().linear(x, weight, None, torch.float32, kernel=kernel))
+        want = x.float() @ weight.float().T
+        torch.testing.assert_close(got, want, atol=2e-5 * float(want.abs().max()) * (k / 64) ** 0.5, rtol=0)
+        del weight
+    _gemm().check_error()
+
+
 # by features (few columns, a short K range) and split-K; the fewest and the most rows that come here
 @pytest.mark.parametrize("m", [17, 64, 127])
 @pytest.mark.parametrize("n,k", [(300, 520), (2056, 2056), (2064, 96)])
