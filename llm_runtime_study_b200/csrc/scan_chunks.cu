@@ -12,9 +12,9 @@
 //               B_ts = k_t . (D_t ... D_(s+1) k_s)            (the forward substitution of u_t, its steps gathered in T)
 //
 // Only products of decays between two tokens of a chunk are formed, never a quotient of two, so nothing overflows that
-// the recurrence does not, and every sum is over float32 products of float32 factors.  What does not depend on the
-// state is made for all chunks at once by a first kernel: per chunk and head a record of G_t q_t, E_s k_s, (G_t k_t,) A, (T)
-// and G_C, in float32.  The second walks the chunks.
+// the recurrence does not.  What does not depend on the state is made for all chunks at once by a first kernel, in float32: per chunk and
+// head a record of G_t q_t, E_s k_s, (G_t k_t,) A, (T), each number as three bfloat16 that hold its 24 bits, and G_C.  The second walks the
+// chunks on the tensor cores, its sums in float32.
 #include "common.cuh"
 #include "mma.cuh"
 #include "tcgen05.cuh"
@@ -58,14 +58,21 @@ constexpr int kSmallPitch = kChunkTokens + 8;
 __host__ __device__ constexpr int record_bytes(int dp, bool delta) {
   return (delta ? 9 : 6) * kChunkTokens * record_pitch(dp) * 2 + (delta ? 6 : 3) * kChunkTokens * kSmallPitch * 2 + dp * 4;
 }
-// x as the sum of three bfloat16, `plane` numbers apart
+// x as the sum of three bfloat16, `plane` numbers apart.  The first is at most the largest bfloat16, so that every finite number has such parts; an
+// infinity or NaN is the second one (number_of_parts).
 __device__ __forceinline__ void store_parts(__nv_bfloat16* to, int plane, float x) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const __nv_bfloat16 part = __float2bfloat16_rn(x);
-    to[i * plane] = part;
-    x -= __bfloat162float(part);
-  }
+  uint16_t bits;
+  asm("cvt.rn.satfinite.bf16.f32 %0, %1;\n" : "=h"(bits) : "f"(x));
+  __nv_bfloat16 part = __ushort_as_bfloat16(bits);
+  to[0] = part;
+  x -= __bfloat162float(part);
+  part = __float2bfloat16_rn(x);
+  to[plane] = part;
+  to[2 * plane] = __float2bfloat16_rn(x - __bfloat162float(part));
+}
+__device__ __forceinline__ float number_of_parts(const __nv_bfloat16* at, int plane) {
+  const float second = __bfloat162float(at[plane]);
+  return isfinite(second) ? (__bfloat162float(at[2 * plane]) + second) + __bfloat162float(at[0]) : second;
 }
 
 // (as in sequence_state.cu: SiLU of a value that was stored in 16 bits with the hardware's exponential and reciprocal)
@@ -291,8 +298,9 @@ __global__ void __launch_bounds__(128) scan_chunk_records_kernel(const ChunkPara
 // 16 rows x 32 columns each and exchanged every sum), delta rule with decays per channel 352 (460); 16 heads 232 and 300 (299, 424); three portions of
 // 578 tokens, 32 heads: decays per channel 159 (217), row gates 172 (250); one of 1,733 with row gates 213 (354).
 // ROW: the normaliser is one more column, behind the last value column, whose value is 1 for every token.
-// A value that is not finite must not reach the tokens before its own, whose weight for it is 0: where a warp meets one, the sums over
-// a chunk's tokens are formed one by one (up_to_now).
+// A number that is not finite has no three parts whose products add up to its own, nor has one beyond the largest bfloat16, and beside weights of
+// 0 such a value would reach the tokens before its own.  Any of them leaves a read-out or a cell of the state that is not finite; these are
+// looked at, and the CTA then takes its portion once more from its first token in float32 (scan_plainly).
 struct Triple { uint32_t part[3]; };        // two neighbouring values: three bfloat16 pairs that add up to them, largest first
 __device__ __forceinline__ Triple split_pair(float x, float y) {
   Triple s;
@@ -321,12 +329,102 @@ __device__ __forceinline__ void mma_free(float (&d)[4], const uint32_t (&a)[4], 
 // which parts of the two factors make the six products, smallest first; with one part only of the first factor, three
 __device__ constexpr int kPartA[6] = {2, 0, 1, 1, 0, 0}, kPartB[6] = {0, 2, 1, 0, 1, 0};
 
+// One CTA's portion with every sum over float32 products: a warp has a quarter of the rows, a lane a column.  For portions with numbers that the
+// tensor cores cannot take, so written for few registers beside the kernel that calls it, not for speed.  `shared`: 6 * 16 * 32 floats.
+template <typename TV, bool DELTA, bool ROW, bool VSPLIT, int DP>
+__device__ __noinline__ void scan_plainly(const ChunkParams& p, int entry, int h, int col0, int slot0, float* shared) {
+  constexpr int C = kChunkTokens, NC = kChunkCols, RECORD = record_bytes(DP, DELTA), PITCH = record_pitch(DP), ROWS = DP / 4;
+  float* us = shared;                                   // [C][NC]
+  float* vs = us + C * NC;                              // [C][NC]
+  float* red = vs + C * NC;                             // [4][C][NC]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, col = col0 + lane, row0 = warp * ROWS;
+  const Portion portion = portion_of(p, entry);
+  const size_t head = static_cast<size_t>(p.slots[entry]) * p.H + h;
+  const bool norm = ROW && col == p.dv, live = col < p.dv || norm;
+  auto cell = [&](int r) { return norm ? p.norm_state + head * p.d + r : p.state + (head * p.d + r) * p.dv + col; };
+  float S[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) S[r] = live && row0 + r < p.d ? *cell(row0 + r) : 0.f;
+  auto times_state = [&](const __nv_bfloat16* rows) {   // into `red`: this warp's rows' share of all tokens' sums
+#pragma unroll 1
+    for (int s = 0; s < C; ++s) {
+      float x = 0.f;
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) x = fmaf(S[r], number_of_parts(rows + s * PITCH + row0 + r, C * PITCH), x);
+      red[(warp * C + s) * NC + lane] = x;
+    }
+  };
+  auto whole_sum = [&](int s) { return (red[s * NC + lane] + red[(C + s) * NC + lane]) + (red[(2 * C + s) * NC + lane] + red[(3 * C + s) * NC + lane]); };
+  auto up_to_now = [&](const __nv_bfloat16* m, const float* x, int s, float sum) {
+#pragma unroll 1
+    for (int e = 0; e <= s; ++e) sum = fmaf(number_of_parts(m + s * kSmallPitch + e, C * kSmallPitch), x[e * NC + lane], sum);
+    return sum;
+  };
+#pragma unroll 1
+  for (int first = 0; first < portion.count; first += C) {
+    const int tokens = min(C, portion.count - first);
+    const unsigned char* record = static_cast<const unsigned char*>(p.records) + (static_cast<size_t>(slot0 + first / C) * p.H + h) * RECORD;
+    const __nv_bfloat16* rows = reinterpret_cast<const __nv_bfloat16*>(record);
+    const __nv_bfloat16* small = rows + (DELTA ? 9 : 6) * C * PITCH;
+    const float* whole = reinterpret_cast<const float*>(record + RECORD) - DP;
+    __syncthreads();
+#pragma unroll 1
+    for (int s = warp; s < C; s += 4) {
+      float x = norm && s < tokens ? 1.f : 0.f;
+      if (col < p.dv && s < tokens) {
+        x = to_float(static_cast<const TV*>(p.v)[static_cast<size_t>(portion.first + first + s) * p.ldv + static_cast<size_t>(h) * p.dv + col]);
+        if (VSPLIT && p.act) x = chunk_silu<TV>(x);
+      }
+      (DELTA ? vs : us)[s * NC + lane] = x;
+    }
+    if constexpr (DELTA) {
+      times_state(rows + 6 * C * PITCH);
+      __syncthreads();
+#pragma unroll 1
+      for (int s = warp; s < C; s += 4) vs[s * NC + lane] -= whole_sum(s);
+      __syncthreads();
+#pragma unroll 1
+      for (int s = warp; s < C; s += 4) us[s * NC + lane] = up_to_now(small + 3 * C * kSmallPitch, vs, s, 0.f);
+    }
+    times_state(rows);
+    __syncthreads();
+#pragma unroll 1
+    for (int s = warp; s < tokens; s += 4) {
+      const float o = up_to_now(small, us, s, whole_sum(s));
+      const size_t at = static_cast<size_t>(portion.first + first + s) * p.H + h;
+      if (norm) p.norm_out[at] = o;
+      else if (live) p.out[at * p.dv + col] = o;
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) S[r] *= whole[row0 + r];
+#pragma unroll 1
+    for (int s = 0; s < tokens; ++s) {
+      const float u = us[s * NC + lane];
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r)
+        if (row0 + r < p.d) S[r] = fmaf(number_of_parts(rows + 3 * C * PITCH + s * PITCH + row0 + r, C * PITCH), u, S[r]);     // (rows that are not there stay 0)
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+    if (live && row0 + r < p.d) *cell(row0 + r) = S[r];
+}
+
 constexpr int kChunkTiles = kChunkCols / 16, kChunkThreads = kChunkTiles * 64;
 // records in shared memory: as many as leave room for two CTAs an SM
 __host__ __device__ constexpr int record_ring(bool delta) { return delta ? 2 : 3; }
 __device__ int g_scan_error = 0;
+// Registers a thread.  Under another bound the compiler puts a chunk's instructions in another order, and its time follows: 2,048 tokens of 32 heads of
+// 128, one decay a head 205 to 217 us between 154 and 200 registers, delta rule 346 to 427 between 152 and 200; the best of them each.  Left to
+// itself it makes room for a third CTA an SM that the records do not leave (row gates 128 registers: 367 us, 239).  Small states need no bound but one (8 heads of 32, 509 tokens, a decay
+// a head: 30.3 us without, 26.0 with 96).
+constexpr int chunk_registers(int dt, bool delta, bool row) {
+  if (dt < 8) return dt == 2 && !delta && !row ? 96 : 255;
+  return delta ? 176 : (row ? 172 : 156);
+}
 template <typename TV, bool DELTA, bool ROW, bool VSPLIT, int DT>
-__global__ void __launch_bounds__(kChunkThreads) scan_chunk_kernel(const ChunkParams p) {
+__global__ void __launch_bounds__(kChunkThreads) __maxnreg__(chunk_registers(DT, DELTA, ROW))
+scan_chunk_kernel(const __grid_constant__ ChunkParams p) {
   constexpr int C = kChunkTokens, DP = DT * 16, RECORD = record_bytes(DP, DELTA), RING = record_ring(DELTA), PITCH = record_pitch(DP) * 2, HT = DT / 2;
   constexpr int PLANE = C * PITCH, SMALL = C * kSmallPitch * 2, UPARTS = VSPLIT || DELTA ? 3 : 1;
   extern __shared__ __align__(16) unsigned char ring[];   // [RING][RECORD]
@@ -442,59 +540,27 @@ __global__ void __launch_bounds__(kChunkThreads) scan_chunk_kernel(const ChunkPa
         out[nt][e] = (rest[0][nt][e] + rest[1][nt][e]) + lead[0][nt][e];
       }
   };
-  auto finite = [&](const float (&x)[2][4]) {           // of all lanes
-    bool bad = false;
+  // out[t] += sum over s <= t of M[t][s] x[s] for eight tokens from `first` on, M in three planes; x as row operands in `parts` planes
+  auto up_to_now = [&](uint32_t m, int first, const uint32_t (&a)[3][4], int parts, float (&out)[4]) {
+    uint32_t b[3][2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) bad |= !isfinite(x[i >> 2][i & 3]);
-    return !__any_sync(0xffffffffu, bad);
-  };
-  // out[t] += sum over s <= t of M[t][s] x[s] for eight tokens from `first` on, M in three planes; x also as row operands in `parts` planes
-  auto up_to_now = [&](uint32_t m, int first, const float (&x)[2][4], bool all_finite, const uint32_t (&a)[3][4], int parts, float (&out)[4]) {
-    if (all_finite) {
-      uint32_t b[3][2];
+    for (int i = 0; i < 3; ++i)
+      asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n"
+                   : "=r"(b[i][0]), "=r"(b[i][1])
+                   : "r"(m + i * SMALL + (first + (lane & 7)) * (kSmallPitch * 2) + half_n));
+    float lead[4] = {}, rest[2][4] = {};
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n"
-                     : "=r"(b[i][0]), "=r"(b[i][1])
-                     : "r"(m + i * SMALL + (first + (lane & 7)) * (kSmallPitch * 2) + half_n));
-      float lead[4] = {}, rest[2][4] = {};
-#pragma unroll
-      for (int i = 0; i < 6; ++i) {
-        if (kPartA[i] >= parts) continue;
-        mma_free(i == 5 ? lead : rest[i & 1], a[kPartA[i]], b[kPartB[i]][0], b[kPartB[i]][1]);
-      }
-#pragma unroll
-      for (int e = 0; e < 4; ++e) out[e] += (rest[0][e] + rest[1][e]) + lead[e];
-      return;
+    for (int i = 0; i < 6; ++i) {
+      if (kPartA[i] >= parts) continue;
+      mma_free(i == 5 ? lead : rest[i & 1], a[kPartA[i]], b[kPartB[i]][0], b[kPartB[i]][1]);
     }
-#pragma unroll 1
-    for (int s = 0; s < C; ++s) {
-      const int from = (lane & ~3) | ((s & 7) >> 1);
-      float x0 = 0.f, x1 = 0.f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {                     // (tile, parity) of token s
-        const float y0 = __shfl_sync(0xffffffffu, x[i >> 1][i & 1], from), y1 = __shfl_sync(0xffffffffu, x[i >> 1][2 + (i & 1)], from);
-        if ((s >> 3) * 2 + (s & 1) == i) { x0 = y0; x1 = y1; }
-      }
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int tok = first + 2 * t + i;
-        if (s > tok) continue;
-        float f = 0.f;
-#pragma unroll
-        for (int part = 2; part >= 0; --part) {
-          uint16_t bits;
-          asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(bits) : "r"(m + part * SMALL + (tok * kSmallPitch + s) * 2));
-          f += __uint_as_float(static_cast<uint32_t>(bits) << 16);
-        }
-        out[i] = fmaf(f, x0, out[i]);
-        out[2 + i] = fmaf(f, x1, out[2 + i]);
-      }
-    }
+    for (int e = 0; e < 4; ++e) out[e] += (rest[0][e] + rest[1][e]) + lead[e];
   };
 
   int slot = 0;
   uint32_t phase = 0;
+  float doubt = 0.f;                                    // NaN once something has not been finite
   for (int t0 = t_begin; t0 < t_end; t0 += C) {
     const bool ok = mbar_wait(full + slot, phase);
     if (!__syncthreads_and(ok)) {                       // (the record is there; the one before has been read)
@@ -537,11 +603,9 @@ __global__ void __launch_bounds__(kChunkThreads) scan_chunk_kernel(const ChunkPa
         u[i >> 2][i & 3] = 0.f;
       }
       split_tiles(w[0], w[1], a);
-      const bool plain = finite(w);
-      up_to_now(small + 3 * SMALL, 0, w, plain, a, 3, u[0]);
-      up_to_now(small + 3 * SMALL, 8, w, plain, a, 3, u[1]);
+      up_to_now(small + 3 * SMALL, 0, a, 3, u[0]);
+      up_to_now(small + 3 * SMALL, 8, a, 3, u[1]);
     }
-    const bool plain = finite(u);
     if constexpr (UPARTS == 3) {
       split_tiles(u[0], u[1], a);
     } else {                                            // the values are bfloat16
@@ -589,14 +653,23 @@ __global__ void __launch_bounds__(kChunkThreads) scan_chunk_kernel(const ChunkPa
     const float4 other = handed[0][tile][half ^ 1][lane];
     float mine[4] = {other.x + (half ? o[1][0] : o[0][0]), other.y + (half ? o[1][1] : o[0][1]), other.z + (half ? o[1][2] : o[0][2]),
                      other.w + (half ? o[1][3] : o[0][3])};
-    up_to_now(small, half * 8, u, plain, a, UPARTS, mine);
+    up_to_now(small, half * 8, a, UPARTS, mine);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
+      doubt = fmaf(mine[i], 0.f, doubt);
       const int tok = t0 + half * 8 + 2 * t + (i & 1), c = col0 + g + (i >> 1) * 8;
       if (tok >= t_end) continue;
       if (c < dv) p.out[(static_cast<size_t>(tok) * p.H + h) * dv + c] = mine[i];
       else if (ROW && c == dv) p.norm_out[static_cast<size_t>(tok) * p.H + h] = mine[i];
     }
+  }
+#pragma unroll
+  for (int j = 0; j < 2 * HT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) doubt = fmaf(S[j][e], 0.f, doubt);
+  if (__syncthreads_or(doubt != 0.f)) {                 // (nothing of the state has been written)
+    scan_plainly<TV, DELTA, ROW, VSPLIT, DP>(p, entry, h, blockIdx.x % col_blocks * kChunkCols, slot0, reinterpret_cast<float*>(ring));
+    return;
   }
   if (!working) return;
 #pragma unroll

@@ -250,3 +250,77 @@ def test_a_bad_value_in_a_chunk_reaches_its_own_column_and_later_tokens_only(for
     want = torch.ones(n, heads, dv, dtype=torch.bool)
     want[bad:, 1, 5] = False
     assert torch.equal(fine.cpu(), want)
+
+
+def _positive_case(form, heads, d, dv, n):
+    """Positive numbers throughout, so that an infinity adds up to an infinity and never to NaN: (rows q, k, v, state, norm_state, options, decay [n,
+    heads, d], gain or beta [n, heads])."""
+
+    g = torch.Generator().manual_seed(7)
+    rand = lambda *shape: 0.1 + 0.8 * torch.rand(*shape, generator=g)
+    delta = form.startswith("delta")
+    narrow = torch.float32 if delta or form == "head_float_qk" else torch.bfloat16
+    q, k = (rand(n, heads * d) for _ in range(2))
+    if delta:                                # rows of length one: the recurrence does not grow
+        q, k = (torch.nn.functional.normalize(x.view(n, heads, d), dim=-1).reshape(n, -1) for x in (q, k))
+    q, k, v = q.to(narrow), k.to(narrow), rand(n, heads * dv).to(torch.float32 if delta else torch.bfloat16)
+    head, channel, token, other = rand(heads), rand(n, heads, d), rand(n, heads), rand(n, heads)
+    options, wide = {"head": ({"decay": head}, head[None, :, None].expand(n, heads, d)), "channel": ({"gate": channel.reshape(n, -1)}, channel),
+                     "token": ({"row_decay": token}, token[..., None].expand(n, heads, d)), "row": ({"decay": token, "gain": other}, token[..., None].expand(n, heads, d)),
+                     }[form.split("_")[1] if delta else form.split("_")[0]]
+    if delta:
+        options["beta"] = other
+    return q, k, v, rand(1, heads, d, dv), rand(1, heads, d), options, wide, other
+
+
+# an infinity, and a number beyond bfloat16's largest (which rounds to an infinity), where a chunk meets them: in a value, a key, a query, the state
+# it starts from; the bad token in the first chunk and in a later one, tokens of its chunk before and behind it
+@pytest.mark.parametrize("where", ["v", "k", "q", "state", "large state", "large v", "large k"])
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("d,dv,n,bad", [(48, 40, 40, 5), (128, 33, 52, 37), (24, 32, 16, 9)])
+def test_infinities_and_the_largest_numbers_keep_their_value(form, where, d, dv, n, bad, monkeypatch):
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    heads, huge, delta = 2, 3.395e38, form.startswith("delta")
+    q, k, v, state, norm_state, options, wide, other = _positive_case(form, heads, d, dv, n)
+    if delta and where in ("k", "q", "state", "large k"):
+        pytest.skip("the delta rule subtracts: no sign of its infinities is the same in every order of its sums")
+    if where in ("large v", "large k") and {"large v": v, "large k": k}[where].dtype != torch.float32:
+        pytest.skip("16-bit rows hold no such number")
+    if delta and where == "v":
+        bad = n - 1                          # (the tokens behind it would subtract infinities)
+    if where in ("v", "k", "q"):
+        {"v": v, "k": k, "q": q}[where][bad, 3] = float("inf")
+    elif where == "state":
+        state[0, 0, 7, 3] = float("inf")
+    elif where == "large state":
+        state[0, 0, 7, 3] = huge
+        q *= 0.25                            # (the read-outs stay finite)
+    else:
+        {"large v": v, "large k": k}[where][bad, 3] = huge
+        q, k, v = q * 0.125, (k if where == "large k" else k * 0.25), (v if where == "large v" else v * 0.25)
+    monkeypatch.setattr(S, "portion_in_chunks", lambda *sizes: 1)
+    monkeypatch.setattr(S, "CHUNK_MIN_TOKENS", 1)
+    dev = lambda x: x.to(DEV)
+    s, ns = dev(state), dev(norm_state)
+    common = dict(heads=heads, dim=d, vdim=dv, state=s, q_start=torch.tensor([0, n], dtype=torch.int32, device=DEV), lens=[n],
+                  slots=torch.zeros(1, dtype=torch.int32, device=DEV), **{key: dev(x) for key, x in options.items()})
+    if form == "row":
+        out, den = S.linear_scan_row_gates(dev(q), dev(k), dev(v), norm_state=ns, **common)
+    else:
+        out = S.linear_scan(dev(q), dev(k), dev(v), qk_heads=heads, **common)
+    rows = [x.double().view(n, heads, -1) for x in (q, k, v)]
+    more = dict(decay=wide.double(), gain=other.double() if form == "row" else None, beta=other.double() if delta else None)
+    want, end = _reference(*rows, [n], state.double(), [0], **more)
+    pairs = [(out.view(n, heads, dv), want), (s, end)]
+    if form == "row":
+        nwant, nend = _reference(rows[0], rows[1], torch.ones(n, heads, 1, dtype=torch.float64), [n], norm_state.double()[..., None], [0], **more)
+        pairs += [(den, nwant[..., 0]), (ns, nend[..., 0])]
+    for got, ref in pairs:
+        got, ref = got.double().cpu(), ref.double()
+        assert not bool(ref.isnan().any()) and torch.equal(got.isinf() * got.sign(), ref.isinf() * ref.sign())
+        fine = ref.isfinite()
+        assert bool(fine.any())
+        # sums of up to 16 + 128 terms of one sign (the delta rule's: their largest counts), a float32 rounding each
+        scale = ref[fine].abs() if not delta else ref[fine].abs() + float(ref[fine].abs().max())
+        assert bool(((got[fine] - ref[fine]).abs() <= 1e-5 * scale).all())
