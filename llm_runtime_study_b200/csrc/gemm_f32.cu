@@ -211,11 +211,12 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
 // segment of one weight row against every row of A (1 x 151,936 x 1024: 93 us = 6.7 TB/s, where tiles took 708); kSegments segments of all the CTA's weight rows are in shared memory
 // at a time, copied there 16 bytes at a time without passing through registers, two or three CTAs an SM so that one's copies
 // run under the other's arithmetic.  Rows are padded by 16 bytes: the eight threads of a 128-byte phase then read from
-// different banks.
+// different banks.  GATED is a kernel of its own: chosen at run time, its rows cost every product 3 to 25 % (8 x 1024 x 3072 21.5 us, 18.0; 24 x 512
+// x 512 9.3, 7.7).
 constexpr int kRowsW = 8, kSegments = 16, kPass = kSegments * kSegment;
 constexpr size_t few_smem(int pitch) { return sizeof(float) * kRowsW * pitch; }
 
-template <int MB>
+template <int MB, bool GATED>
 __global__ void __launch_bounds__(kRowsW * kSegments)
 gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                     float* __restrict__ C, int M, int N, int K, int lda, int ldc, int pitch, int block, int act) {
@@ -227,7 +228,10 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, co
   const int n0 = blockIdx.x * kRowsW, m0 = blockIdx.y * MB;
   const int n = tid % kRowsW, seg = tid / kRowsW;
   // a gated product takes four rows of one factor and the four of the other eight rows on
-  auto row_of = [&](int r) { return act ? static_cast<int>(blockIdx.x) / 2 * 16 + blockIdx.x % 2 * 4 + r / 4 * 8 + r % 4 : n0 + r; };
+  auto row_of = [&](int r) {
+    if constexpr (GATED) return static_cast<int>(blockIdx.x) / 2 * 16 + blockIdx.x % 2 * 4 + r / 4 * 8 + r % 4;
+    else return n0 + r;
+  };
   const int rows = min(MB, M - m0);
   const float* a0 = A + static_cast<size_t>(m0) * lda;
   float total = 0.f, part = 0.f;                                 // of output (tid / kRowsW, tid % kRowsW), for tid < MB * kRowsW
@@ -246,7 +250,7 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, co
 #pragma unroll
     for (int m = 0; m < MB; ++m) acc[m] = 0.f;
     const int first = seg * kSegment, last = min(first + kSegment, span);
-    if (row_of(n) < N) {
+    if (n0 + n < N) {                                            // (as many of a gated product's rows are there: all)
       const float* wrow = ws + n * pitch;
 #pragma unroll 4
       for (int k = first; k < last; k += 4) {
@@ -276,14 +280,15 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, co
     }
     __syncthreads();                                             // the sums and the rows have been read
   }
-  const int m = m0 + tid / kRowsW, nn = row_of(n);
-  const bool stored = tid < MB * kRowsW && m < M && nn < N;
-  const float out = (K % block ? total + part : total) + (stored && bias ? bias[nn] : 0.f);
-  if (act) {
+  if constexpr (GATED) {
+    const int m = m0 + tid / kRowsW, nn = row_of(n);
+    const bool stored = tid < MB * kRowsW && m < M && nn < N;
+    const float out = (K % block ? total + part : total) + (stored && bias ? bias[nn] : 0.f);
     const float other = __shfl_down_sync(0xffffffffu, out, 4);
     if (stored && n < 4) C[static_cast<size_t>(m) * ldc + blockIdx.x * 4 + n] = gate_act(out, act) * other;
-  } else if (stored) {
-    C[static_cast<size_t>(m) * ldc + nn] = out;
+  } else if (tid < MB * kRowsW) {
+    const int m = m0 + tid / kRowsW, nn = n0 + tid % kRowsW;
+    if (m < M && nn < N) C[static_cast<size_t>(m) * ldc + nn] = (K % block ? total + part : total) + (bias ? bias[nn] : 0.f);
   }
 }
 
@@ -362,14 +367,14 @@ int launch_tiles(const float* A, const float* W, const float* bias, float* C, in
   return launch_status();
 }
 
-template <int MB>
+template <int MB, bool GATED>
 int launch_few(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, int act, cudaStream_t stream) {
   static DeviceOnce once;
-  const int status = configure_once(once, gemm_f32_few_kernel<MB>, few_smem(kPass + 4));
+  const int status = configure_once(once, gemm_f32_few_kernel<MB, GATED>, few_smem(kPass + 4));
   if (status) return status;
   const dim3 grid((N + kRowsW - 1) / kRowsW, (M + MB - 1) / MB);
   const int pitch = (K < kPass ? K : kPass) + 4;      // a short K takes less shared memory: more CTAs an SM
-  launch(gemm_f32_few_kernel<MB>, grid, dim3(kRowsW * kSegments), few_smem(pitch), stream, A, W, bias, C, M, N, K, lda, ldc, pitch,
+  launch(gemm_f32_few_kernel<MB, GATED>, grid, dim3(kRowsW * kSegments), few_smem(pitch), stream, A, W, bias, C, M, N, K, lda, ldc, pitch,
          block_length(K), act);
   return launch_status();
 }
@@ -419,10 +424,13 @@ extern "C" int b200_gemm_f32_gated(const float* A, const float* W, const float* 
   if ((M + 63) / 64 > 65535) return B200_ERR_TOO_LARGE;
   if (kernel == 1) {
     if (!vec) return B200_ERR_BAD_SIZE;
-    if (M == 1) return launch_few<1>(A, W, bias, C, M, N, K, lda, ldc, act, stream);
-    if (M == 2) return launch_few<2>(A, W, bias, C, M, N, K, lda, ldc, act, stream);
-    if (M <= 4) return launch_few<4>(A, W, bias, C, M, N, K, lda, ldc, act, stream);
-    return launch_few<8>(A, W, bias, C, M, N, K, lda, ldc, act, stream);
+#define B200_F32_FEW(MB)                                                                   \
+  (act ? launch_few<MB, true>(A, W, bias, C, M, N, K, lda, ldc, act, stream)                \
+       : launch_few<MB, false>(A, W, bias, C, M, N, K, lda, ldc, act, stream))
+    if (M == 1) return B200_F32_FEW(1);
+    if (M == 2) return B200_F32_FEW(2);
+    return M <= 4 ? B200_F32_FEW(4) : B200_F32_FEW(8);
+#undef B200_F32_FEW
   }
   if (kernel == 4) {
     if (K > kSegment || act) return B200_ERR_BAD_SIZE;
