@@ -347,13 +347,15 @@ int launch_tiles(const float* A, const float* W, const float* bias, float* C, in
   if (status) return status;
   const int block = block_length(K), blocks = (K + block - 1) / block;
   // Launched while the kernel before still holds some SMs, the CTAs would crowd on the others, three where two suffice (509 x 4096 x
-  // 1024 in a prompt's layers: 144 us against 97 with two an SM): each takes the shared memory that leaves room for no more than an even share.
+  // 1024 in a prompt's layers: 144 us against 97 with two an SM): each takes as much shared memory as leaves no room for one more than an even
+  // share, and no more than that: what is left caches the loads (64 x 1024 x 3072, one CTA an SM: 45.5 us with all of it, 40.0; 509 x 1024 x
+  // 3072, two: 80.6, 79.3).
   const long long share = (static_cast<long long>((N + BN - 1) / BN) * blocks * ((M + BM - 1) / BM) + usable_sms(blocks) - 1) / usable_sms(blocks);
-  const size_t even = share <= (BM == 128 ? 2 : 3) ? (kMostSmem + 1024) / share - 1024 : 0;
+  const size_t even = share <= (BM == 128 ? 2 : 3) ? ((kMostSmem + 1024) / (share + 1) / 128 + 1) * 128 - 1024 : 0;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3((N + BN - 1) / BN * blocks, (M + BM - 1) / BM);
   config.blockDim = dim3((BM / TM) * (BN / TN));
-  config.dynamicSmemBytes = even > tile_smem(BM, BN) ? even / 128 * 128 : tile_smem(BM, BN);
+  config.dynamicSmemBytes = even > tile_smem(BM, BN) ? even : tile_smem(BM, BN);
   config.stream = stream;
   cudaLaunchAttribute attributes[2];
   attributes[0].id = cudaLaunchAttributeClusterDimension;
