@@ -157,7 +157,6 @@ paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_poo
 // share an SM.  Within a prompt's layers, where CTAs start while the kernel before still holds some SMs: 133 us one by one, 90 in pairs, 78 with
 // the softmax's steps taken together.
 constexpr int kTileRows = 32, kTileKeys = 32, kRowsOf = 4, kTileThreads = kTileRows / kRowsOf * 16, kPPitch = kTileKeys + 4;
-constexpr int kSms = 148;
 constexpr size_t kMostTileSmem = 227 * 1024;
 constexpr size_t attention_tile_smem(int dmax) {
   return sizeof(float) * (static_cast<size_t>(kTileRows + 2 * kTileKeys) * (dmax + 4) + kTileRows * kPPitch);
@@ -384,13 +383,14 @@ __global__ void __launch_bounds__(2 * kTileThreads) paged_attention_tile_kernel(
 template <int DMAX>
 int launch_attention_tiles(const TileParams& p, cudaStream_t stream) {
   static DeviceOnce once;
-  const int status = configure_once(once, paged_attention_tile_kernel<DMAX>, kMostTileSmem);
+  int sms = 0;
+  const int status = configure_once(once, paged_attention_tile_kernel<DMAX>, kMostTileSmem, &sms);
   if (status) return status;
-  if (p.tiles <= kSms) {                                               // an SM for each: no pairs
+  if (p.tiles <= sms) {                                                // an SM for each: no pairs
     launch(paged_attention_tile_kernel<DMAX>, dim3(p.tiles), dim3(kTileThreads), attention_tile_smem(DMAX), stream, p);
     return launch_status();
   }
-  const long long ctas = (p.tiles + 1LL) / 2, share = (ctas + kSms - 1) / kSms;
+  const long long ctas = (p.tiles + 1LL) / 2, share = (ctas + sms - 1) / sms;
   const size_t even = share <= 4 ? ((kMostTileSmem + 1024) / share - 1024) / 128 * 128 : 0, needed = 2 * attention_tile_smem(DMAX);
   launch(paged_attention_tile_kernel<DMAX>, dim3(static_cast<unsigned>(ctas)), dim3(2 * kTileThreads), even > needed ? even : needed, stream, p);
   return launch_status();

@@ -43,7 +43,7 @@ inline int block_length(int K) {
 constexpr int kBK = 16;
 constexpr size_t kMostSmem = 227 * 1024;
 // A cluster's CTAs lie in one GPC, whose last SMs may not hold another cluster.
-inline int usable_sms(int blocks) { return 148 - 4 * (blocks - 1); }
+inline int usable_sms(int blocks, int sms) { return sms > 8 * (blocks - 1) ? sms - 4 * (blocks - 1) : (sms + 1) / 2; }
 constexpr size_t tile_smem(int bm, int bn) { return sizeof(float) * (static_cast<size_t>(bm) * bn + 2 * kBK * (bm + 4 + bn + 4)); }
 
 template <int BM, int BN, int TM, int TN, bool VEC, bool GATED>
@@ -340,17 +340,49 @@ gemm_f32_short_kernel(const float* __restrict__ A, const float* __restrict__ W, 
   }
 }
 
+// The kernel for a product by its size (vec: rows are 16-byte vectors) and the GPU's number of SMs.
+inline int choose_kernel(int M, int N, int K, bool vec, bool gated, int sms) {
+  const int blocks = (K + block_length(K) - 1) / block_length(K);
+  const long long small = static_cast<long long>((M + 63) / 64) * ((N + 63) / 64) * blocks;
+  const long long large = static_cast<long long>((M + 127) / 128) * ((N + 63) / 64) * blocks;
+  // Up to 8 rows the weights cross once and that is the time (1 x 1024 x 3072: 7.9 us against 37.6 with tiles; 8 x 151,936 x
+  // 1024: 285 against 495).  Every further eight rows read them again, from the L2 while the product is small: 24 x 6144
+  // x 1024 37.5 against 39.0, 24 x 1024 x 3072 25.6 against 37.8, 64 x 6144 x 1024 83 against 40.
+  // Tiles of 128 rows do a third more arithmetic per byte of shared memory read, tiles of 64 leave less of the last wave empty.  A
+  // product takes 9 us and 22.9 for each 64 x 64 x 1024 that the busiest SM gets, or 11 and 43.2 for each 128 x 64 x 1024 (509 x
+  // 6144 x 1024: 140 us with 128 rows, 146 with 64; 700 x 4096 x 1024: 140, 123; 130 x 6144 x 1024: 96, 54; 2048 x 4096 x 1024:
+  // 313, 329).  One CTA of 128 rows an SM has nobody to work under its loads (509 x 1024 x 2048, the weights in HBM: 68 us, 57 with
+  // 64 rows).  Clusters cannot use every SM to the last slot (700 x 1024 x 3072, 96 clusters of three: 140, 100).
+  // Few rows: up to about seven CTAs an SM at once (ten up to four rows), 8 us a round of them from K of 128 on (K beyond 512: as the weights
+  // stream), where tiles take 3 us and 0.034 a column.  So beyond one round a short K goes to tiles (9 x 6400 x 256: 15.6 us against
+  // 12.2, 24 x 9400 x 1024: 48 against 38), and so does K up to 160 beyond four rows (8 x 6400 x 64: 6.1 against 5.6, 20 x 2880 x 64: 9.0 against 5.4)
+  // except K up to 64 in a third of a round (8 x 64 x 64: 4.9 against 5.4, 24 x 512 x 64: 5.4 both).
+  // Short rows: up to 112 columns that are not whole 16-byte vectors and up to 32 that are, while the tiles are few.
+  const long long ctas = static_cast<long long>((N + kRowsW - 1) / kRowsW) * ((M + 7) / 8), rounds = (ctas + 7 * sms - 1) / (7 * sms);
+  const float few_us = rounds * (8.f + (K > 512 ? (K - 512) / 128.f : 0.f)), tiles_us = 3.f + 0.034f * (K < 1024 ? K : 1024);
+  const bool few = M <= 2 || (M <= 24 && K <= 64 && ctas <= 400) || (M <= 4 && (K > 160 || ctas <= 10 * sms)) || (M <= 8 && K >= 512) ||
+                   (K > 160 && (M <= 8 || (M <= 24 && small < sms)) && few_us <= tiles_us);
+  if (vec && few) return 1;
+  if (K <= (vec ? 32 : 112) && small <= 512 && !gated) return 4;
+  const int block = block_length(K), usable = usable_sms(blocks, sms);
+  const float depth = (K < block ? K : block) / 1024.f;
+  const float small_us = 9.f + 22.9f * depth * ((small + usable - 1) / usable), large_us = 11.f + 43.2f * depth * ((large + usable - 1) / usable);
+  return large > usable && large_us < small_us ? 3 : 2;
+}
+
 template <int BM, int BN, int TM, int TN, bool VEC, bool GATED>
 int launch_tiles(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, int act, cudaStream_t stream) {
   static DeviceOnce once;
-  const int status = configure_once(once, gemm_f32_tile_kernel<BM, BN, TM, TN, VEC, GATED>, kMostSmem);
+  int sms = 0;
+  const int status = configure_once(once, gemm_f32_tile_kernel<BM, BN, TM, TN, VEC, GATED>, kMostSmem, &sms);
   if (status) return status;
   const int block = block_length(K), blocks = (K + block - 1) / block;
   // Launched while the kernel before still holds some SMs, the CTAs would crowd on the others, three where two suffice (509 x 4096 x
   // 1024 in a prompt's layers: 144 us against 97 with two an SM): each takes as much shared memory as leaves no room for one more than an even
   // share, and no more than that: what is left caches the loads (64 x 1024 x 3072, one CTA an SM: 45.5 us with all of it, 40.0; 509 x 1024 x
   // 3072, two: 80.6, 79.3).
-  const long long share = (static_cast<long long>((N + BN - 1) / BN) * blocks * ((M + BM - 1) / BM) + usable_sms(blocks) - 1) / usable_sms(blocks);
+  const int usable = usable_sms(blocks, sms);
+  const long long share = (static_cast<long long>((N + BN - 1) / BN) * blocks * ((M + BM - 1) / BM) + usable - 1) / usable;
   const size_t even = share <= (BM == 128 ? 2 : 3) ? ((kMostSmem + 1024) / (share + 1) / 128 + 1) * 128 - 1024 : 0;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3((N + BN - 1) / BN * blocks, (M + BM - 1) / BM);
@@ -393,35 +425,11 @@ extern "C" int b200_gemm_f32_gated(const float* A, const float* W, const float* 
   if (K <= 0 || lda < K || ldc < (act ? N / 2 : N)) return B200_ERR_BAD_SIZE;
   if (act && (N % 16 || M > 65535 || (act != ACT_SILU && act != ACT_GELU_TANH))) return B200_ERR_BAD_SIZE;
   const bool vec = K % 4 == 0 && lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(W) % 16 == 0;
-  const int blocks = (K + block_length(K) - 1) / block_length(K);
-  const long long small = static_cast<long long>((M + 63) / 64) * ((N + 63) / 64) * blocks;
-  const long long large = static_cast<long long>((M + 127) / 128) * ((N + 63) / 64) * blocks;
   if (kernel == 0) {
-    // Up to 8 rows the weights cross once and that is the time (1 x 1024 x 3072: 7.9 us against 37.6 with tiles; 8 x 151,936 x
-    // 1024: 285 against 495).  Every further eight rows read them again, from the L2 while the product is small: 24 x 6144
-    // x 1024 37.5 against 39.0, 24 x 1024 x 3072 25.6 against 37.8, 64 x 6144 x 1024 83 against 40.
-    // Tiles of 128 rows do a third more arithmetic per byte of shared memory read, tiles of 64 leave less of the last wave empty.  A
-    // product takes 9 us and 22.9 for each 64 x 64 x 1024 that the busiest SM gets, or 11 and 43.2 for each 128 x 64 x 1024 (509 x
-    // 6144 x 1024: 140 us with 128 rows, 146 with 64; 700 x 4096 x 1024: 140, 123; 130 x 6144 x 1024: 96, 54; 2048 x 4096 x 1024:
-    // 313, 329).  One CTA of 128 rows an SM has nobody to work under its loads (509 x 1024 x 2048, the weights in HBM: 68 us, 57 with
-    // 64 rows).  Clusters cannot use every SM to the last slot (700 x 1024 x 3072, 96 clusters of three: 140, 100).
-    // Few rows: up to about seven CTAs an SM at once (ten up to four rows), 8 us a round of them from K of 128 on (K beyond 512: as the weights
-    // stream), where tiles take 3 us and 0.034 a column.  So beyond one round a short K goes to tiles (9 x 6400 x 256: 15.6 us against
-    // 12.2, 24 x 9400 x 1024: 48 against 38), and so does K up to 160 beyond four rows (8 x 6400 x 64: 6.1 against 5.6, 20 x 2880 x 64: 9.0 against 5.4)
-    // except K up to 64 in a third of a round (8 x 64 x 64: 4.9 against 5.4, 24 x 512 x 64: 5.4 both).
-    // Short rows: up to 112 columns that are not whole 16-byte vectors and up to 32 that are, while the tiles are few.
-    const long long ctas = static_cast<long long>((N + kRowsW - 1) / kRowsW) * ((M + 7) / 8), rounds = (ctas + 7 * 148 - 1) / (7 * 148);
-    const float few_us = rounds * (8.f + (K > 512 ? (K - 512) / 128.f : 0.f)), tiles_us = 3.f + 0.034f * (K < 1024 ? K : 1024);
-    const bool few = M <= 2 || (M <= 24 && K <= 64 && ctas <= 400) || (M <= 4 && (K > 160 || ctas <= 10 * 148)) || (M <= 8 && K >= 512) ||
-                     (K > 160 && (M <= 8 || (M <= 24 && small < 148)) && few_us <= tiles_us);
-    if (vec && few) kernel = 1;
-    else if (K <= (vec ? 32 : 112) && small <= 512 && !act) kernel = 4;
-    else {
-      const int block = block_length(K), sms = usable_sms(blocks);
-      const float depth = (K < block ? K : block) / 1024.f;
-      const float small_us = 9.f + 22.9f * depth * ((small + sms - 1) / sms), large_us = 11.f + 43.2f * depth * ((large + sms - 1) / sms);
-      kernel = large > sms && large_us < small_us ? 3 : 2;
-    }
+    static DeviceOnce once;
+    int sms = 0;
+    if (const int status = configure_once(once, gemm_f32_short_kernel, 0, &sms)) return status;
+    kernel = choose_kernel(M, N, K, vec, act != 0, sms);
   }
   if ((M + 63) / 64 > 65535) return B200_ERR_TOO_LARGE;
   if (kernel == 1) {
@@ -445,6 +453,11 @@ extern "C" int b200_gemm_f32_gated(const float* A, const float* W, const float* 
   if (kernel == 3) return vec ? B200_F32_TILES(128, 8, true) : B200_F32_TILES(128, 8, false);
   return vec ? B200_F32_TILES(64, 4, true) : B200_F32_TILES(64, 4, false);
 #undef B200_F32_TILES
+}
+
+// The kernel that is chosen for rows of 16-byte vectors on a GPU with `sm_count` SMs (callable without a GPU).
+extern "C" int b200_gemm_f32_choice(int M, int N, int K, int gated, int sm_count) {
+  return M > 0 && N > 0 && K > 0 && sm_count > 0 ? b200::choose_kernel(M, N, K, K % 4 == 0, gated != 0, sm_count) : 0;
 }
 
 extern "C" int b200_gemm_f32_variant(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,

@@ -72,6 +72,7 @@ _LIBRARIES = {
         ("gemm_f32.cu",),
         {"b200_gemm_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
          "b200_gemm_f32_variant": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+         "b200_gemm_f32_choice": [c_int, c_int, c_int, c_int, c_int],
          "b200_gemm_f32_gated": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]},
     ),
     "b200_attention_simt": (

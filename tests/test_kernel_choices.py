@@ -159,6 +159,18 @@ def test_split_k_shape_fills_the_sms_and_keeps_tiles_wide():
         assert shape(128, n, k) == (width, splits)     # the choice does not depend on the rows that came along
 
 
+def test_float32_tiles_go_by_the_gpus_own_number_of_multiprocessors():
+    """1: few rows, 2 and 3: tiles of 64 and 128 rows, 4: short rows; by a B200's 148 and by fewer."""
+
+    from llm_runtime_study_b200.ops import native
+
+    choice = lambda m, n, k, sms=148, gated=0: native.query("b200_gemm_f32_choice", m, n, k, gated, sms)
+    assert choice(8, 1024, 3072) == choice(24, 64, 64) == choice(1, 16, 4, gated=1) == 1 and choice(100, 16, 32) == 4
+    assert choice(509, 6144, 1024) == 3 and choice(700, 4096, 1024) == choice(130, 6144, 1024) == choice(509, 1024, 3072) == 2
+    assert choice(700, 4096, 1024, 100) == choice(509, 1024, 3072, 60) == 3 and choice(509, 6144, 1024, 60) == choice(9, 6400, 1024, 60) == 2 != choice(9, 6400, 1024)
+    assert all(choice(m, 4096, 9000, sms) in (2, 3) for m in (33, 200, 3000) for sms in (1, 8, 30, 57, 148, 160))
+
+
 def test_which_scans_go_in_chunks():
     from llm_runtime_study_b200.ops import sequence_state as S
 
