@@ -121,22 +121,28 @@ def pick_kernel(m: int, n: int, k: int) -> tuple[str, int]:
 def by_features(m: int, n: int, k: int, out_float32: bool) -> bool:
     """Whether a product of this shape goes to the kernel that has the weight as its row operand (``linear_features``) and not to the one that
     ``pick_kernel`` names.  Timed both ways at 18 numbers of rows (17 to 2,048), 11 of columns (256 to 12,288) and 8 of K (512 to
-    12,288), float32 sums and bfloat16 results.  Float32 rows are what it writes best: it is ahead from 129 rows on (0.40 to 0.97 of the time, 0.75
-    in the mean) but where other kernels fill the GPU better: around 2,048 columns up to 256 rows (1.05 to 1.14), 8,192
-    and more columns beyond 1,024 rows (0.97 to 1.05), short K with many rows (1.06 to 1.17).  Of the bfloat16 results those with few tiles
+    12,288), float32 sums and bfloat16 results, and at 22 numbers of rows (129 to 2,048) for 20 larger products, up to 151,936 columns and K of 28,672.
+    Float32 rows are what it writes best: it is ahead from 129 rows on (0.40 to 0.97 of the time, 0.75
+    in the mean; of the larger products 0.47 to 1.10, 0.87) but where other kernels fill the GPU better: around 2,048 columns up to 256 rows (1.05 to
+    1.26), 8,192 and more columns beyond 1,024 rows (0.97 to 1.12; with a long K or as an output head from 897 on: 1.03 to 1.11), short K with many rows
+    (1.06 to 1.17), 225 to 256 rows of 12,288 to 28,672 columns, which are one full round of pairs (0.93 to 1.15).  Of the bfloat16 results those with few tiles
     and a long K range (257 to 512 rows up to 4,096 columns 0.48 to 1.07, mean 0.73; to 1,024 rows up to 2,048 columns 0.51 to 0.99), 129
-    to 256 rows whose 128-row tiles are half empty (3,072 to 6,144 columns: 0.65 to 1.03), and 513 to 896 rows of wide products, whose
-    256-row tiles are (0.73 to 1.05, mean 0.92)."""
+    to 256 rows whose 128-row tiles are half empty (3,072 to 6,144 columns: 0.65 to 1.04; with 4,096 columns and K beyond 16,384 1.08 to 1.11), and 513 to
+    896 rows of wide products, whose 256-row tiles are (0.71 to 1.05, mean 0.90), but not 641 to 768 and more than 832 rows of some 16,000 to 20,000 columns
+    (1.02 to 1.09) and 641 to 768 of some 5,000 with a long K (1.05 to 1.07)."""
 
     if not (PAIR_ENABLED and 128 < m <= 2048):
         return False
     if out_float32:
-        return not ((176 < m <= 256 and 1536 < n <= 2560) or (m > 1024 and (n >= 8192 or k < 1024)))
+        return not ((176 < m <= 256 and 1536 < n <= 2560) or (224 < m <= 256 and 12288 <= n <= 28672 and k >= 4096)
+                    or (m > 896 and k >= 4096 and n * k >= 200_000_000 and (n >= 65536 or k > 16384)) or (m > 1024 and (n >= 8192 or k < 1024)))
     if m <= 256:
-        return 3072 <= n <= 4096 or (m <= 208 and 4096 < n <= 6144)
+        return (3072 <= n <= 4096 and k <= 16384) or (m <= 208 and 4096 < n <= 6144)
     if m <= 512:
         return n <= 4096 and k >= 3072
-    return (m <= 1024 and n <= 2048 and k >= 3072) or (m <= 896 and n >= 5120)
+    if n >= 5120 and m <= 896:
+        return not (14336 < n <= 20480 and (640 < m <= 768 or m > 832)) and not (n < 6144 and k > 12288 and 640 < m <= 768)
+    return m <= 1024 and n <= 2048 and k >= 3072
 
 
 # weight elements from which 9 to 16 rows go to the tcgen05 split-K kernel

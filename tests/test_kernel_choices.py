@@ -111,6 +111,18 @@ def test_which_projections_go_by_features():
     assert not takes(405, 6144, 4096, False) and takes(640, 6144, 4096, False) and not takes(1024, 6144, 4096, False)
 
 
+def test_which_larger_projections_go_by_features():
+    """Output heads and long K ranges: where the other kernels are ahead (timed both ways) they keep the product."""
+
+    takes = gemm_bf16.by_features
+    assert takes(512, 151936, 4096, True) and not takes(1024, 151936, 4096, True) and takes(1024, 151936, 1024, True)
+    assert takes(640, 8192, 28672, True) and not takes(960, 8192, 28672, True) and takes(1024, 5120, 25600, True)
+    assert not takes(256, 24576, 4096, True) and not takes(230, 12288, 16384, True) and takes(224, 24576, 4096, True) and takes(256, 32000, 4096, True)
+    assert takes(200, 4096, 14336, False) and not takes(200, 4096, 20480, False) and takes(200, 5120, 25600, False)
+    assert takes(640, 16384, 4096, False) and not takes(768, 16384, 4096, False) and takes(832, 16384, 4096, False) and not takes(896, 20480, 5120, False)
+    assert takes(640, 5120, 25600, False) and not takes(704, 5120, 25600, False) and takes(832, 5120, 25600, False) and takes(704, 5120, 4096, False)
+
+
 def test_gated_projections_of_some_rows_in_one_launch_where_the_weights_are_large():
     assert gemm_bf16.gated_in_one(24576, 4096) and gemm_bf16.gated_in_one(34816, 5120) and not gemm_bf16.gated_in_one(16384, 2048)
 
