@@ -175,11 +175,15 @@ def few_rows_kernel(m: int, n: int, k: int) -> str:
 
 def gated_in_one(n: int, k: int) -> bool:
     """Whether a gated unit's projection of 17 to 127 rows goes to the split-K kernel, whose epilogue applies the gate, and not to the library and
-    a kernel for the gate behind it: where the weights are about 100 MB and more, and streaming them is all that counts (24,576 x 4,096 with 17, 64
+    a kernel for the gate behind it: where the weights are 160 MB and more with 20,000 rows of 3,072 columns or more, and streaming them is all that
+    counts (24,576 x 4,096 with 17, 64
     and 96 rows 38.0, 39.5, 40.0 us, 38.7, 41.7, 43.2 with the library; a decode step of nine such layers 1,263 -> 1,232 with 24
-    requests, 1,553 -> 1,515 with 64).  Smaller ones are the library's (16,384 x 2,048 with 64 rows 18.6, 15.4; steps with them 1 % longer)."""
+    requests, 1,553 -> 1,515 with 64).  Smaller ones are the library's (16,384 x 2,048 with 64 rows 18.6, 15.4; steps with them 1 % longer), and
+    so are short columns, whose products are over before the next tile's begin (98,304 x 640 1.03 to 1.32 of the library's time, 49,152 x 2,048
+    0.95 to 1.05), and fewer rows, which are too few tiles (8,192 x 8,192 and 8,192 x 12,288 1.37 to 1.71, 14,336 x 5,120 1.06 to 1.14, 16,384 x 4,096
+    1.02 to 1.07; 24,576 x 4,096 0.85 to 0.99, 28,672 x 8,192 0.87 to 1.01)."""
 
-    return n * k >= 60_000_000
+    return n >= 20_000 and k >= 3072 and n * k >= 80_000_000
 
 
 def gated_unit(swiglu: "bool | str") -> int:

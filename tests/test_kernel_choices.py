@@ -127,6 +127,14 @@ def test_gated_projections_of_some_rows_in_one_launch_where_the_weights_are_larg
     assert gemm_bf16.gated_in_one(24576, 4096) and gemm_bf16.gated_in_one(34816, 5120) and not gemm_bf16.gated_in_one(16384, 2048)
 
 
+def test_gated_projections_of_few_or_short_rows_stay_with_the_library():
+    """Products of as many weights that the split-K kernel takes longer for."""
+
+    assert gemm_bf16.gated_in_one(51200, 5120) and gemm_bf16.gated_in_one(57344, 8192)
+    for n, k in ((8192, 8192), (8192, 12288), (2048, 32768), (14336, 5120), (16384, 4096), (98304, 640), (65536, 1024), (49152, 2048)):
+        assert not gemm_bf16.gated_in_one(n, k)
+
+
 def test_decode_parts_are_bounded_and_use_the_gpu():
     for requests, kv_heads, longest, slots in itertools.product((1, 3, 8, 64, 500), (1, 8), (1, 100, 2048, 32768, 1 << 20), (296, 592)):
         parts = attention_bf16.decode_splits(requests, kv_heads, 1, longest, slots)
