@@ -24,8 +24,10 @@ native.register_error_probe("b200_scan_chunks", "b200_scan_chunks_error", "linea
 
 CHUNK_TOKENS, CHUNK_MAX_DIM = 16, 128     # tokens a chunk, largest key size of the chunked kernel
 CHUNK_MIN_TOKENS = 48                     # tokens beyond one per request from which a batch may be scanned in chunks
-CHUNK_MAX_BYTES = 1 << 30                 # records of a batch at most (2,048 tokens of 32 heads of 128: 0.11 GB)
-CHUNK_SLICE_BYTES = 1 << 27               # of which at most so much is there at once
+CHUNK_MAX_NUMBERS = 1 << 28               # numbers in the records of a batch at most: a limit on work (2,048 tokens of 32 heads of 128: 1 << 24.7)
+# Bytes of records that are there at once, in one launch.  2,048 tokens of 32 heads of 128 with the delta rule are 181 MB (a number is three bfloat16);
+# cut in two the scan takes 20 to 30 us more, 32 portions of 34 tokens of 64 heads 1.4 times as long.
+CHUNK_SLICE_BYTES = 1 << 28
 MOST_RUNS = 4                             # launches a batch of long and short portions is cut into at most
 
 
@@ -39,22 +41,21 @@ def _lengths(lens: "Sequence[int] | None", n: int, entries: int) -> "Sequence[in
     return lens
 
 
-def _record_bytes(n: int, entries: int, heads: int, dim: int) -> int:
-    """What the numbers of a batch's records take in float32 (the larger form, the delta rule's; the records themselves, whose
-    numbers are three bfloat16 each, half as much again: they are held in slices)."""
+def _record_numbers(n: int, entries: int, heads: int, dim: int) -> int:
+    """How many numbers the records of a batch hold (the larger form, the delta rule's)."""
 
     dim = 32 if dim <= 32 else (64 if dim <= 64 else 128)
-    return (n // CHUNK_TOKENS + entries) * heads * 4 * (3 * CHUNK_TOKENS * dim + 2 * CHUNK_TOKENS * CHUNK_TOKENS + dim)
+    return (n // CHUNK_TOKENS + entries) * heads * (3 * CHUNK_TOKENS * dim + 2 * CHUNK_TOKENS * CHUNK_TOKENS + dim)
 
 
 def scans_in_chunks(n: int, entries: int, heads: int, dim: int, fixed_order: bool) -> bool:
     """Whether a batch of ``n`` tokens of ``entries`` requests can hold portions that are scanned sixteen tokens at a time
     (``csrc/scan_chunks.cu``; ``portion_in_chunks`` says which): batches with portions of prompts beside 16-bit activations.  With
-    ``fixed_order`` a token's sums must not depend on where a step's chunks begin.  Batches whose records would take more than a
-    gigabyte of memory are scanned token by token."""
+    ``fixed_order`` a token's sums must not depend on where a step's chunks begin.  Batches of more than ``CHUNK_MAX_NUMBERS`` are scanned
+    token by token (the memory that records take is bounded by ``CHUNK_SLICE_BYTES`` whatever the batch)."""
 
     return (not fixed_order and dim <= CHUNK_MAX_DIM and n - entries >= CHUNK_MIN_TOKENS
-            and _record_bytes(n, entries, heads, dim) <= CHUNK_MAX_BYTES)
+            and _record_numbers(n, entries, heads, dim) <= CHUNK_MAX_NUMBERS)
 
 
 def portion_in_chunks(lens: "Sequence[int]", heads: int, dim: int, columns: int, delta: bool) -> int:

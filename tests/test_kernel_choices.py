@@ -220,6 +220,20 @@ def test_records_of_long_portions_come_in_slices():
                 assert sum(held for _, _, held in slices) == whole
 
 
+def test_records_of_one_prompt_are_there_at_once():
+    """With the size that the records have: prompts and batches up to some 2,400 tokens of 32 heads of 128 are one launch."""
+
+    from llm_runtime_study_b200.ops import native
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    size = lambda dim, delta: native.query("b200_scan_chunks_record_floats", dim, delta) * 4
+    assert size(128, 1) == 44_288 and size(128, 0) == 28_928
+    for heads, dim, delta, lens in ((32, 128, 1, [2048]), (32, 128, 1, [800, 800, 800]), (32, 128, 0, [3700]), (64, 128, 0, [34] * 32), (64, 64, 1, [2300]), (64, 32, 0, [6300])):
+        chunks = sum(-(-m // 16) for m in lens)
+        assert len(S.chunk_slices(lens, sum(lens), len(lens), chunks, heads * size(dim, delta))) == 1
+    assert len(S.chunk_slices([9000], 9000, 1, 563, 32 * size(128, 1))) > 1
+
+
 def test_which_portions_go_in_chunks(monkeypatch):
     """By a portion's own length: many short ones beside each other, or single tokens beside a long one, are no reason."""
 
