@@ -58,23 +58,31 @@ def scans_in_chunks(n: int, entries: int, heads: int, dim: int, fixed_order: boo
             and _record_numbers(n, entries, heads, dim) <= CHUNK_MAX_NUMBERS)
 
 
-def portion_in_chunks(lens: "Sequence[int]", heads: int, dim: int, columns: int, delta: bool) -> int:
+def portion_in_chunks(lens: "Sequence[int]", heads: int, dim: int, columns: int, delta: bool, row_gates: bool = False) -> int:
     """The number of tokens from which a portion of a batch is scanned in chunks (0: none is); ``columns``: of a head's state.
 
-    A chunk costs 1.4 to 1.8 us (2.2 when the sums below were taken: with a kernel of its time) behind some 8 us for the records; a token of a chain 0.2 us as long as the chains' CTAs of 8 columns
-    all run at once, two an SM, and 0.3 to 0.5 us beyond that.  A chunk takes the same 0.06 us a head (0.13 with the
+    ``row_gates``: the state has the normaliser as one more column.
+
+    A chunk costs 1.6 us, 2.6 with the delta rule, behind some 8 us for the records; a token of a chain 0.2 us as long as the chains' CTAs of 8 columns
+    all run at once, two an SM, and 0.3 to 0.5 us beyond that.  A chunk takes the same 0.04 us a head (0.06 with the
     delta rule) whether it holds sixteen tokens or one.  So what counts is the portion's own length, not the batch's.  Microseconds in
-    chunks and as a chain, 128 x 128: 4 heads, one portion of 64 tokens 21.6, 22.8 (delta rule, a decay per channel 28.3, 24.6), of 96
-    26.4, 31.3 (34.4, 32.8); 16 heads, 64 tokens 23.5, 24.8 (29.6, 28.7), 96 tokens 27.6, 34.8 (35.8, 39.6); 32 heads, eight of 24 48, 55 (83, 74), two of
-    48 25.8, 42.3 (39.9, 57.3), eight of 48 60.4, 98.3 (112, 129), 64 of 2 206, 90 (404, 107).  With key sizes up to 64 and enough chains to
-    fill the GPU with CTAs of 32 columns a chain is as fast or faster at any length (8 heads of 64, 64 portions of 64: 62.4, 53.3;
-    96.2, 65.5).  Few chains beside requests of another kernel pay for that launch too (4 heads, 64 tokens beside one token: 26, 23)."""
+    chunks and as a chain, 128 x 128, one decay a head (delta rule, a decay per channel): 4 heads, one portion of 64 tokens 11.9, 13.8 (18.2, 19.5), of 96
+    14.0, 19.3 (21.5, 27.8); 16 heads, 64 tokens 12.0, 15.8 (18.4, 24.3), 96 tokens 14.1, 22.2 (21.5, 34.9); 32 heads, eight of 24 28.7, 41.8 (41.5, 66.6), two of
+    48 14.1, 29.5 (22.1, 50.3), eight of 48 37.0, 75.0 (61.7, 121.9), 64 of 2 167, 82 (224, 100).  With key sizes up to 64 and enough chains to
+    fill the GPU with CTAs of 32 columns a chain is as fast or faster for short values (8 heads of 64, 64 portions of 64: 49.4, 38.1;
+    82.7, 58.4).  Few chains beside requests of another kernel pay for that launch too (4 heads, 64 tokens beside one token: 15.3, 13.8).
+    With row gates a head of 128 columns is five blocks of 32, and short portions pay only from 28 tokens on (16 heads, eight of 24 to 28 tokens 1.01 to
+    0.91 of the chain's time) and where their CTAs are not just more than fit at once, two an SM (four of 32: 23.6, 21.8, six 0.76); with 96 rows of state, which
+    are worked on as 128, not at all (four to 32 of 32 tokens: 0.90 to 1.40).  These lines hold with what runs today but lie on the chain's side: several short portions with the
+    delta rule and single ones of 64 tokens would be faster in chunks."""
 
     sms = native.sm_count()
     if not delta and dim > 64:                 # many portions, each as long as two chunks or nearly
-        short = sum(m >= 24 for m in lens)
-        if short >= 4 and short * heads * -(-columns // 8) > 4 * sms:
-            return 24
+        least = 28 if row_gates else 24
+        short = sum(m >= least for m in lens)
+        ctas = short * heads * -(-columns // 32)
+        if short >= 4 and short * heads * -(-columns // 8) > 4 * sms and not (row_gates and (dim <= 96 or 2 * sms < ctas <= 3 * sms)):
+            return least
     long = sum(m >= 48 for m in lens)
     if not long or (dim <= 64 and long * heads * -(-columns // 32) >= 2 * sms):
         return 0
@@ -117,7 +125,7 @@ def _scan_plan(lens, n: int, entries: int, heads: int, dim: int, vdim: int, colu
 
     least = 0
     if scans_in_chunks(n, entries, heads, dim, fixed_order):
-        least = portion_in_chunks(lens if lens else [n // entries] * entries, heads, dim, columns, delta)
+        least = portion_in_chunks(lens if lens else [n // entries] * entries, heads, dim, columns, delta, columns > vdim)
     if not lens:
         return [("chunks" if least and n >= least * entries else "chain", 0, entries)]
     singles = scans_single(1, 1, dim, vdim, fixed_order)

@@ -258,6 +258,21 @@ def test_which_portions_go_in_chunks(monkeypatch):
     assert plan(None, 405, 25) == [("chain", 0, 25)] and plan(None, 1200, 25) == [("chunks", 0, 25)] and plan(None, 8, 8) == [("chain", 0, 8)]
 
 
+def test_short_portions_with_row_gates_go_in_chunks_where_they_fill_them(monkeypatch):
+    """The normaliser is a 129th column, a block of its own: nearly two full chunks a portion, and no second round of CTAs that is nearly empty."""
+
+    from llm_runtime_study_b200.ops import sequence_state as S
+
+    monkeypatch.setattr(S.native, "sm_count", lambda: 148)
+    least = lambda lens, heads, dim=128, columns=129: S.portion_in_chunks(lens, heads, dim, columns, False, True)
+    assert least([24] * 8, 16) == least([27] * 32, 64) == 0 and least([28] * 8, 16) == least([34] * 6, 16) == 28
+    assert least([32] * 4, 16) == least([32] * 16, 4) == least([32] * 8, 8) == 0 and least([48] * 4, 16) == 48      # 320 CTAs, two an SM
+    assert least([40] * 32, 16, 96) == 0 and least([48] * 32, 16, 96) == 48
+    assert S.portion_in_chunks([24] * 8, 16, 128, 128, False) == 24
+    assert S._scan_plan([24] * 8, 192, 8, 16, 128, 128, 129, False, False) == [("chain", 0, 8)]
+    assert S._scan_plan([24] * 8, 192, 8, 16, 128, 128, 128, False, False) == [("chunks", 0, 8)]
+
+
 def test_parts_of_a_single_tokens_keys_over_shared_rows(monkeypatch):
     """Rows too wide for two CTAs a multiprocessor are cut into at most one round of CTAs, narrow ones into two."""
 
