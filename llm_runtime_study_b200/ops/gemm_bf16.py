@@ -321,15 +321,17 @@ native.register_error_probe("b200_gemm_features", "b200_gemm_features_error", "t
 
 
 def check_error() -> None:
-    """Synchronise and raise if a bounded wait inside the kernel ran out."""
+    """Synchronise and raise if a bounded wait inside one of the tcgen05 kernels of this module ran out."""
 
-    code = native.query("b200_gemm_tcgen05_error")
-    if code:
-        where = {1: "producer", 2: "tensor-core issue", 3: "epilogue", 4: "accumulator buffer", 5: "flag of a shared tile",
-                 -1: "device error"}.get(code, str(code))
+    where = {1: "producer", 2: "tensor-core issue", 3: "epilogue", 4: "accumulator buffer", 5: "flag or exchange of a shared tile", -1: "device error"}
+    codes = [(what, native.query(probe)) for what, probe in (("tcgen05 projection", "b200_gemm_tcgen05_error"),
+                                                             ("tcgen05 projection by features", "b200_gemm_features_error"))]
+    if codes[0][1]:
         for _, flags in _STREAMK_WORKSPACE.values():     # a wait that ran out may have left flags behind
             flags.zero_()
-        raise KernelError(f"tcgen05 projection: a bounded wait ran out ({where})")
+    for what, code in codes:
+        if code:
+            raise KernelError(f"{what}: a bounded wait ran out ({where.get(code, str(code))})")
 
 
 def linear_skinny(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None,

@@ -111,6 +111,23 @@ def test_which_projections_go_by_features():
     assert not takes(405, 6144, 4096, False) and takes(640, 6144, 4096, False) and not takes(1024, 6144, 4096, False)
 
 
+def test_a_wait_that_ran_out_is_reported_whichever_kernel_it_was_in(monkeypatch):
+    import pytest
+
+    from llm_runtime_study_b200.errors import KernelError
+    from llm_runtime_study_b200.ops import native
+
+    codes = {"b200_gemm_tcgen05_error": 0, "b200_gemm_features_error": 0}
+    monkeypatch.setattr(native, "query", lambda name: codes[name])
+    gemm_bf16.check_error()
+    codes["b200_gemm_features_error"] = 5
+    with pytest.raises(KernelError, match="by features.*shared tile"):
+        gemm_bf16.check_error()
+    codes.update(b200_gemm_tcgen05_error=2, b200_gemm_features_error=0)
+    with pytest.raises(KernelError, match="projection: .*issue"):
+        gemm_bf16.check_error()
+
+
 def test_which_larger_projections_go_by_features():
     """Output heads and long K ranges: where the other kernels are ahead (timed both ways) they keep the product."""
 
