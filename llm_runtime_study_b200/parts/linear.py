@@ -29,7 +29,7 @@ class Projection:
         ``LLM_RUNTIME_STUDY_B200_GEMM_MID=splitk`` sends these row counts to our cluster
         split-K kernel instead.
     K must be a multiple of 8 for our bfloat16 kernels (16-byte rows); other
-    widths go to the library product.
+    widths go to the library product, and so do 17 to 127 rows that start off a 16-byte boundary.
 
     The weight-streaming kernel also carries the RMS norms of a decode step: given
     ``add_to`` and ``next_norm`` it adds its product into the residual rows and returns
@@ -90,7 +90,8 @@ class Projection:
                 return gemm_bf16.linear_skinny(x, self.weight, self.bias, torch.bfloat16, swiglu=act)
             if self.GEMM_BACKEND == "tcgen05" and m >= self.TCGEN05_MIN_ROWS:
                 return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act, weight_at_rest=True)
-            if self.GEMM_BACKEND == "tcgen05" and (self.MID_ROWS == "splitk" or gemm_bf16.gated_in_one(self.out_features, self.in_features)):
+            if self.GEMM_BACKEND == "tcgen05" and (self.MID_ROWS == "splitk" or (gemm_bf16.gated_in_one(self.out_features, self.in_features)
+                                                                                 and x.data_ptr() % 16 == 0)):
                 return gemm_bf16.linear(x, self.weight, self.bias, torch.bfloat16, swiglu=act, kernel="splitk", weight_at_rest=True)
         if self.runtime.dtype == torch.float32 and x.shape[-1] == self.in_features:
             return F.linear_f32_gated(x, self.weight, self.bias, act)
@@ -141,7 +142,7 @@ class Projection:
                     gemm_bf16.linear(x, self.weight, self.bias, torch.float32, add_to=add_to, kernel="splitk", weight_at_rest=True)
                     return None
                 return gemm_bf16.linear(x, self.weight, self.bias, out_dtype, kernel="splitk", weight_at_rest=True)
-            if self.GEMM_BACKEND == "tcgen05" and self.bias is not None and out_dtype == torch.bfloat16:
+            if self.GEMM_BACKEND == "tcgen05" and self.bias is not None and out_dtype == torch.bfloat16 and x.data_ptr() % 16 == 0:
                 return gemm_bf16.linear_with_bias(x, self.weight, self.bias, weight_at_rest=True)
         if out_dtype == torch.bfloat16:
             y = torch.mm(x, self.weight.t())

@@ -132,6 +132,30 @@ def test_attention_part_whole_and_in_portions(dtype, bias, qk_norm, heads):
         torch.testing.assert_close(torch.cat(outs).double().cpu(), want, **TOL[dtype])
 
 
+@pytest.mark.parametrize("rows", [17, 64, 127])
+@pytest.mark.parametrize("offset", [0, 1, 4])
+def test_rows_of_any_alignment_between_the_streaming_and_the_tiled_kernels(rows, offset):
+    """A view that starts off a 16-byte boundary, which TMA cannot read: with a bias, and through a gated unit large enough for one launch."""
+
+    from llm_runtime_study_b200.parts.linear import Projection
+
+    torch.manual_seed(4)
+    for n, k, gated in ((300, 520, False), (2064, 2056, False), (20016, 4104, True)):
+        w = (0.05 * torch.randn(n, k)).bfloat16()
+        bias = None if gated else torch.randn(n)
+        part = Projection([w], None if gated else [bias], runtime(torch.bfloat16))
+        x = torch.randn(rows * k + offset).bfloat16().cuda()[offset:].view(rows, k)
+        want = x.double() @ w.double().cuda().T
+        if gated:
+            blocks = want.view(rows, n // 16, 2, 8)
+            want = (torch.nn.functional.silu(blocks[:, :, 0]) * blocks[:, :, 1]).reshape(rows, n // 2)
+        else:
+            want = want + bias.double().cuda()
+        got = part.swiglu(x) if gated else part(x)
+        # bfloat16 results, and roundings of the library's product and of the bias before the sum (the gate's factors) in between: 2^-8 each
+        torch.testing.assert_close(got.double(), want, atol=1e-2 * float(want.abs().max()), rtol=2e-2)
+
+
 def test_unknown_kind_and_bad_sizes():
     from llm_runtime_study_b200.errors import RegistryError
     from llm_runtime_study_b200.parts import FEED_FORWARDS, MIXERS
