@@ -492,9 +492,9 @@ __device__ ArgMax block_argmax(ArgMax v, ArgMax* scratch) {
 // One cluster of CTAs per row (gridDim.x = rows * cluster size): each CTA scans its slice of the row and
 // the CTAs combine their results through distributed shared memory.  STAGED: the slice is read from memory and divided by
 // the temperature once and kept in shared memory for the passes over it (`staged`: room for it).  32 rows of 151,936 entries, 19 of
-// them filtered: 58 us, half of it the passes' arithmetic and half the meetings of the clusters (118 us when each threshold took eight passes of
+// them filtered: 59 us, half of it the passes' arithmetic and half the meetings of the clusters (117 us when each threshold took eight passes of
 // find_threshold, which weighs elements against fifteen candidates, and rows without filters two launches of their own); one row with
-// top-k 25 us (40), with top-p 46 (60).
+// top-k 24 us (41), with top-p 40 (52).
 template <bool STAGED, int STEPS>
 __global__ void __launch_bounds__(1024)
 sample_kernel(const float* __restrict__ logits, int ld, int vocab, RowParams params,

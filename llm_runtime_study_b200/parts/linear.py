@@ -17,13 +17,17 @@ class Projection:
     """One weight matrix (possibly several checkpoint tensors stacked along the
     output axis, so that q/k/v or gate/up are one product) and an optional bias.
 
-    float32 runtime: our FFMA kernel.  bfloat16 runtime, float32 accumulation,
+    float32 runtime: our FFMA kernels, gated units with the gate in their epilogue
+    (``functional.linear_f32_gated``).  bfloat16 runtime, float32 accumulation,
     bfloat16 or float32 output:
       * up to 16 rows (decoding): our weight-streaming mma.sync kernel, or, for 9 to 16 rows
         and weights of more than about 100 MB, our tcgen05 split-K kernel
         (``gemm_bf16.few_rows_kernel``);
-      * 128 rows and more (prompts): our tcgen05/TMEM/TMA kernels;
-      * in between, and everywhere when ``LLM_RUNTIME_STUDY_B200_GEMM=library``: a
+      * 128 rows and more (prompts): our tcgen05/TMEM/TMA kernels, the one with the weight as
+        its row operand among them (``gemm_bf16.by_features``);
+      * 17 to 127 rows: our kernels for bfloat16 results with a bias (``gemm_bf16.linear_with_bias``)
+        and for large gated units (``gemm_bf16.gated_in_one``), else, and everywhere when
+        ``LLM_RUNTIME_STUDY_B200_GEMM=library``, a
         library product (the reference's projections are ``nn.Linear``, i.e. library
         products: mini_llm/nn/attention.py:102-111), which is the faster one there;
         ``LLM_RUNTIME_STUDY_B200_GEMM_MID=splitk`` sends these row counts to our cluster
@@ -75,9 +79,9 @@ class Projection:
 
     def swiglu(self, x: "torch.Tensor | WeightedRows", act: str = "silu") -> torch.Tensor:
         """For a projection whose rows are gate and up features interleaved in blocks of
-        eight: ``silu(gate(x)) * up(x)`` (``act``: or another gate) in the activation type.  Our bfloat16 kernels apply
-        the activation in their epilogue, so the ``[tokens, 2 I]`` intermediate is never
-        written; the other paths run the projection and then the interleaved SiLU kernel."""
+        eight: ``silu(gate(x)) * up(x)`` (``act``: or another gate) in the activation type.  Our kernels, bfloat16 and
+        float32, apply the activation in their epilogue, so the ``[tokens, 2 I]`` intermediate is never
+        written; library products (17 to 127 rows of smaller units, odd widths) are followed by the interleaved SiLU kernel."""
 
         x, norm = self._unweighted(x)
         if norm:
